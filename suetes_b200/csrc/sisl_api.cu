@@ -3,6 +3,7 @@
 // orchestration of SISLStepper3D.step (steppers.py:720-1073).
 #include "../../include/sisl_b200.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -313,7 +314,7 @@ GWork<T> carve_gmres(Carver& cv, const Dims& d, int R, bool refine) {
   g.npad = o;
   g.gs = (GState*)cv.take(sizeof(GState));
   g.dview = (GHostView*)cv.take(sizeof(GHostView));
-  g.partial = (double*)cv.take(sizeof(double) * GM_MAXBLOCKS * (GM_MAXR + 2));
+  g.partial = (double*)cv.take(sizeof(double) * gm_partial_doubles(R));
   g.vec = (T*)cv.take(sizeof(T) * g.npad * (size_t)(R + 4));
   g.tmp = (T*)cv.take(sizeof(T) * field_size(d, LOC_M));
   g.scal = (double*)cv.take(sizeof(double));
@@ -371,6 +372,33 @@ double precond_bytes(const Dims& d, size_t es) {
   return es * (vec + 2 * fw + fm + fm + 6 * fw);
 }
 
+// Columns per orthogonalisation block of the Krylov cycles.  The monomial
+// basis M A V, (M A)^2 V, .. of a block is well conditioned when the operator
+// M A = I + E is dominated by E, the horizontal acoustic coupling, whose
+// spectrum is close to imaginary with radius alpha dt times the grid's largest
+// acoustic frequency.  From radius 3 a block of 6 loses nothing against
+// one-step orthogonalisation (flat mountain wave, float32 vectors, residual
+// after 3 cycles 3.7823e-10 against 3.7836e-10 at radius 3.8, and the same
+// digits at 7, 15 and 61); at 1.9, where one cycle already converges to
+// the vectors' rounding, the first cycle ends at 1.6e-6 against 5.8e-7, so
+// such small steps keep one column at a time.
+//
+// The forward solves of a float32 step recorded for its VJP keep one column
+// too: the objective of a gradient run is compared between runs (finite
+// differences, Taylor tests) as a float32 number, where the last bit of the
+// state shows in full, and one column per block forms the states to the bit
+// as the one-step Arnoldi process does.  128x128x64 float32, two steps and
+// their sweep: 243 ms with one column everywhere, 187 ms with blocks in the
+// transposed solves only (this rule), 152 ms with blocks in both.
+int block_columns(const SislCore* c, bool taped) {
+  if (taped && c->grid.dtype == SISL_F32) return 1;
+  const Scalars& s = c->s;
+  const double sound = std::sqrt(s.cp / s.cvd * s.Rd * 300.0);
+  const double radius =
+      2.0 * s.alpha * s.dt * sound * std::sqrt(1.0 / (c->d.dx * c->d.dx) + 1.0 / (c->d.dy * c->d.dy));
+  return radius >= 3.0 ? GM_S : 1;
+}
+
 // Restarted GMRES on the packed vectors g.bg (rhs) and g.xg (initial guess).
 // transpose = 1 runs the same iteration on A^T with the preconditioner M^T
 // (the bwd_solve of steppers.py:473-481).
@@ -384,13 +412,14 @@ double precond_bytes(const Dims& d, size_t es) {
 // host synchronisation: the whole solve replays inside one graph launch.
 template <typename T>
 int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, SislSolveInfo* info,
-              int transpose = 0, GDevInfo* dev_info = nullptr) {
+              int transpose = 0, GDevInfo* dev_info = nullptr, bool taped = false) {
   const Dims& d = c->d;
   const int R = g.R;
   const size_t n = g.npad;
   const int method = (transpose && c->adj_method >= 0) ? c->adj_method : c->prm.solve_method;
   const double eps = (sizeof(T) == 8) ? 2.220446049250313e-16 : 1.1920928955078125e-07;
   GState* gs = g.gs;
+  const int S = block_columns(c, taped);
   CVec5<T> none{};
   const double es = sizeof(T), vb = es * (double)n;
   const double mvb = matvec_bytes(d, sizeof(T)), pcb = precond_bytes(d, sizeof(T));
@@ -410,7 +439,7 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
   {
     KScope k(c, SISL_K_OTHER, st);
     const double tol = (transpose && c->adj_tol > 0.0) ? c->adj_tol : c->prm.solver_tol;
-    gm_setup(gs, eps, tol, c->prm.solver_atol, R, method, st);
+    gm_setup(gs, eps, tol, c->prm.solver_atol, R, method, S, st);
   }
   {
     KScope k(c, SISL_K_DOTS, st);
@@ -475,28 +504,42 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
       gm_dots<T>(g.V(0), n, 0, g.V(0), n, g.partial, gs, 3 /*RNORM*/, 0, s);
     }
   };
-  // one restart cycle: R Arnoldi steps, the small least-squares solve, x update
+  // one restart cycle: R Arnoldi steps in blocks, the small least-squares solve, x update
+  int cols[GM_MAXR];
+  const int nblocks = gm_block_plan(R, S, method, cols);
   auto cycle = [&](cudaStream_t s) {
     {
       KScope k(c, SISL_K_OTHER, s);
       gm_begin_cycle(gs, s);
     }
-    for (int j = 0; j < R; ++j) {
-      {
-        KScope k(c, SISL_K_MATVEC, s, na, mvb);
-        apply_A(g.V(j), &gs->s[j], none, g.V(j + 1), &gs->active, s);
+    for (int b = 0, j0 = 0; b < nblocks; j0 += cols[b++]) {
+      const int sc = cols[b];
+      for (int j = j0; j < j0 + sc; ++j) {
+        {
+          KScope k(c, SISL_K_MATVEC, s, na, mvb);
+          apply_A(g.V(j), &gs->s[j], none, g.V(j + 1), &gs->active, s);
+        }
+        {
+          KScope k(c, SISL_K_PRECOND, s, nm, pcb);
+          apply_M_after_A(g.V(j + 1), &gs->active, s);
+        }
+      }
+      if (S == 1) {
+        {
+          KScope k(c, SISL_K_DOTS, s, 1, vb * (j0 + 2));  // reads V_0..V_j and w
+          gm_dots<T>(g.V(0), n, j0 + 1, g.V(j0 + 1), n, g.partial, gs, 0 /*PROJ*/, 1, s);
+        }
+        KScope k(c, SISL_K_UPDATE, s, 1, vb * (j0 + 3));  // reads V_0..V_j, reads and writes w
+        gm_update<T>(g.V(0), n, j0 + 1, g.V(j0 + 1), n, -1.0, g.partial, gs, 1 /*ARNOLDI*/, 1, 0, s);
+        continue;
       }
       {
-        KScope k(c, SISL_K_PRECOND, s, nm, pcb);
-        apply_M_after_A(g.V(j + 1), &gs->active, s);
+        KScope k(c, SISL_K_DOTS, s, 1, vb * (j0 + 1 + sc));  // reads V_0 .. V_j0 and the new vectors
+        gm_block_dots<T>(g.V(0), n, j0, sc, n, g.partial, gs, s);
       }
       {
-        KScope k(c, SISL_K_DOTS, s, 1, vb * (j + 2));  // reads V_0..V_j and w
-        gm_dots<T>(g.V(0), n, j + 1, g.V(j + 1), n, g.partial, gs, 0 /*PROJ*/, 1, s);
-      }
-      {
-        KScope k(c, SISL_K_UPDATE, s, 1, vb * (j + 3));  // reads V_0..V_j, reads and writes w
-        gm_update<T>(g.V(0), n, j + 1, g.V(j + 1), n, -1.0, g.partial, gs, 1 /*ARNOLDI*/, 1, 0, s);
+        KScope k(c, SISL_K_UPDATE, s, 1, vb * (j0 + 1 + 2 * sc));  // the same, and writes the new ones
+        gm_block_update<T>(g.V(0), n, j0, sc, n, g.partial, gs, s);
       }
     }
     {
@@ -656,7 +699,7 @@ int solve_t_prep(SislCore* c, const Coef<T>& cf, GWork<T>& g, CVec5<T> xbar, con
   if (c->adj_normalize) {
     const int nb = 2 * 148;
     KScope k(c, SISL_K_OTHER, st, 4);
-    gm_setup(g.gs, 0.0, c->prm.solver_tol, c->prm.solver_atol, g.R, c->prm.solve_method, st);
+    gm_setup(g.gs, 0.0, c->prm.solver_tol, c->prm.solver_atol, g.R, c->prm.solve_method, 1, st);
     gm_dots<T>(g.V(0), g.npad, 0, g.bg(), g.npad, g.partial, g.gs, 1 /*BNORM*/, 0, st);
     keep_norm_kernel<<<1, 1, 0, st>>>(g.gs, g.scal);
     scale_packed_kernel<T><<<nb, 256, 0, st>>>(g.bg(), g.npad, g.scal, 0);
@@ -970,7 +1013,7 @@ int step_impl(SislCore* c, const SislState* in, const SislState* out, const Sisl
   for (int it = 0; it < 2; ++it) {
     step_pre_solve<T>(r, it);
     SislSolveInfo si{};
-    rc = gmres_run<T>(c, r.cf, r.w.g, st, &si, 0, dev_info ? dev_info + it : nullptr);
+    rc = gmres_run<T>(c, r.cf, r.w.g, st, &si, 0, dev_info ? dev_info + it : nullptr, tape != nullptr);
     rc = step_post_solve<T>(r, it, rc, si);
     if (rc) return rc;
   }
@@ -2422,6 +2465,8 @@ int capture_members(int n, SislCore* const* cores, F&& record, SislStepGraph** o
 template <typename T>
 int gmres_group_run(const GroupLaunch<T>& gl, cudaStream_t st, cudaStream_t side, int slot, int transpose) {
   const int R = gl.R;
+  int cols[GM_MAXR];
+  const int nblocks = gm_block_plan(R, gl.S, gl.method, cols);
   grp_setup<T>(gl, transpose, st);
   if (gl.refine) grp_convert<T>(gl, 0, st);
   grp_dots<T>(gl, 0, GV_B, 1 /*BNORM*/, 0, st);
@@ -2457,16 +2502,23 @@ int gmres_group_run(const GroupLaunch<T>& gl, cudaStream_t st, cudaStream_t side
   };
   auto cycle = [&](cudaStream_t s) {
     grp_begin_cycle<T>(gl, s);
-    for (int j = 0; j < R; ++j) {
-      if (transpose) {
-        grp_matvec_t<T>(gl, 0, j, s);
-        grp_precond_t<T>(gl, 0, j + 1, 1, s);
-      } else {
-        grp_matvec<T>(gl, 0, j, s);
-        grp_precond<T>(gl, 0, j + 1, 1, s);
+    for (int b = 0, j0 = 0; b < nblocks; j0 += cols[b++]) {
+      for (int j = j0; j < j0 + cols[b]; ++j) {
+        if (transpose) {
+          grp_matvec_t<T>(gl, 0, j, s);
+          grp_precond_t<T>(gl, 0, j + 1, 1, s);
+        } else {
+          grp_matvec<T>(gl, 0, j, s);
+          grp_precond<T>(gl, 0, j + 1, 1, s);
+        }
       }
-      grp_dots<T>(gl, j + 1, GV_V0 + j + 1, 0 /*PROJ*/, 1, s);
-      grp_update_arnoldi<T>(gl, j + 1, s);
+      if (gl.S == 1) {
+        grp_dots<T>(gl, j0 + 1, GV_V0 + j0 + 1, 0 /*PROJ*/, 1, s);
+        grp_update_arnoldi<T>(gl, j0 + 1, s);
+      } else {
+        grp_block_dots<T>(gl, j0, cols[b], s);
+        grp_block_update<T>(gl, j0, cols[b], s);
+      }
     }
     grp_small_solve<T>(gl, s);
     grp_update_x<T>(gl, s);
@@ -2517,7 +2569,7 @@ int gmres_group_run(const GroupLaunch<T>& gl, cudaStream_t st, cudaStream_t side
 // grouped GMRES over all members (gmres_group_run).  transpose: the solves
 // are the reverse sweep's transposed ones, the step's second solve first.
 template <typename T, typename Open, typename Work, typename Phase>
-int capture_grouped(int n, SislCore* const* cores, int transpose, Open&& open, Work&& gwork, Phase&& phase,
+int capture_grouped(int n, SislCore* const* cores, int transpose, bool taped, Open&& open, Work&& gwork, Phase&& phase,
                     SislStepGraph** out) {
   SislStepGraph* g = new (std::nothrow) SislStepGraph();
   if (!g) return SISL_ERR_ARG;
@@ -2588,6 +2640,8 @@ int capture_grouped(int n, SislCore* const* cores, int transpose, Open&& open, W
   gl.R = R;
   gl.method = method;
   gl.refine = refine;
+  gl.S = GM_S;
+  for (int m = 0; m < n; ++m) gl.S = std::min(gl.S, block_columns(cores[m], taped));
   gl.first_h.assign((size_t)NT * (n + 1), 0);
   gl.nz_h.resize(n);
   for (int m = 0; m < n; ++m) {
@@ -2628,6 +2682,8 @@ int capture_grouped(int n, SislCore* const* cores, int transpose, Open&& open, W
     cnt[GT_ATM] = group_at_blocks(c->d, 1);
     cnt[GT_PTM] = group_pt_blocks(c->d, 0);
     cnt[GT_PTU] = group_pt_blocks(c->d, 1);
+    cnt[GT_BDOT] = gm_block_dots_blocks<T>(np);
+    cnt[GT_BUPD] = gm_block_update_blocks<T>(np);
     for (int q = 0; q <= R; ++q) cnt[GT_DOTS0 + q] = gm_dots_blocks<T>(q, np);
     for (int t = 0; t < NT; ++t) {
       int* row = gl.first_h.data() + (size_t)t * (n + 1);
@@ -2684,7 +2740,7 @@ int capture_grouped_step(int n, SislCore* const* cores, const SislState* ins, co
   std::vector<StepRun<T>> runs(n);
   const SislSolveInfo none{};
   return capture_grouped<T>(
-      n, cores, 0,
+      n, cores, 0, solves != nullptr,
       [&](int m, cudaStream_t s) {
         return step_open<T>(runs[m], cores[m], &ins[m], &outs[m], relax ? relax[m] : nullptr, ws[m], ws_bytes[m],
                             s, nullptr, solves ? solves + 10 * m : nullptr, nullptr);
@@ -2718,7 +2774,7 @@ int capture_grouped_vjp(int n, SislCore* const* cores, const SislState* ins, voi
   std::vector<VjpRun<T>> runs(n);
   const SislSolveInfo none{};
   return capture_grouped<T>(
-      n, cores, 1,
+      n, cores, 1, false,
       [&](int m, cudaStream_t s) {
         return vjp_open<T>(runs[m], cores[m], &ins[m], solves + 10 * m, relax ? relax[m] : nullptr, &out_bars[m],
                            &in_bars[m], ws[m], ws_bytes[m], s, nullptr);

@@ -7,14 +7,38 @@
 // equations + Cholesky for the Hessenberg least-squares problem) or the
 // 'incremental' cycle (Givens rotations, early exit on the rotated residual).
 //
-// A basis vector V_i is stored unnormalised next to its inverse norm s_i, so
+// A classical basis vector V_i is stored unnormalised next to its inverse norm s_i, so
 // normalisation never costs a pass over memory: the matvec scales its input
 // on load, projections use h_i = s_i <V_i, w>, updates use h_i s_i V_i.
-// Every reduction accumulates in float64; the last block of a reduction
-// kernel (ticket counter) finishes the sum and runs the scalar logic.
+// The classical projection reads the whole basis twice per Arnoldi step (once
+// for the inner products, once for the update), which was two thirds of a
+// solve.  Here up to GM_S steps share those two reads: the operator is
+// applied to its own output s times, Z_1 = M A V_j, Z_i = M A Z_{i-1}, and
+// the s new vectors are orthogonalised together (s-step Arnoldi with a
+// monomial basis; Hoemmen, Communication-avoiding Krylov subspace methods,
+// Berkeley 2010).  block_dots forms all products of the basis with Z and of Z
+// with itself in one pass over memory, block_update the new vectors in a
+// second one, and the Hessenberg columns follow from the small matrices
+// (block_finish), so a cycle spans the same Krylov space and minimises over
+// it as the one-step form does.  256x256x80 float32, restart 30: vector passes
+// per cycle 1020 -> 220.
+//
+// One column per block is the classical form: the dots and update kernels with
+// their one-step bookkeeping.  It stays for the cores and calls whose rule
+// says so (block_columns in sisl_api.cu).
+//
+// The block form's stored vectors V carry a small triangular factor per block (GState::B)
+// instead of being normalised in memory: the Gram matrix of the vectors as
+// stored is summed while they are written and its Cholesky factor is carried
+// in the small algebra, so rounding of the stored vectors never enters the
+// Arnoldi relation.  Every reduction accumulates in float64; the last block
+// of a reduction kernel (ticket counter) finishes the sum and runs the small
+// algebra.
 #include "sisl_group.cuh"
 
 #include <math.h>
+
+#include <type_traits>
 
 namespace sisl {
 namespace {
@@ -29,6 +53,15 @@ template <typename T>
 __device__ __forceinline__ void load16(const T* p, T* r) {
   using VT = typename V16<T>::type;
   VT v = __ldg(reinterpret_cast<const VT*>(p));
+  const T* q = reinterpret_cast<const T*>(&v);
+#pragma unroll
+  for (int e = 0; e < V16<T>::n; ++e) r[e] = q[e];
+}
+// the same through the coherent path: memory this kernel also writes
+template <typename T>
+__device__ __forceinline__ void load16_rw(const T* p, T* r) {
+  using VT = typename V16<T>::type;
+  VT v = *reinterpret_cast<const VT*>(p);
   const T* q = reinterpret_cast<const T*>(&v);
 #pragma unroll
   for (int e = 0; e < V16<T>::n; ++e) r[e] = q[e];
@@ -180,8 +213,16 @@ __device__ __forceinline__ void dots_body(const T* __restrict__ Vb, size_t strid
       const bool use = nrm > gs->eps;
       gs->s[0] = use ? 1.0 / nrm : 0.0;
       gs->rnorm = use ? nrm : 0.0;
+      gs->B[0][0] = gs->s[0];  // block form: V_0 is a block of its own
+      gs->bstart[0] = 0;
+      gs->clast[0] = gs->rnorm;
+      gs->cstart = 0;
+      gs->clen = 1;
     }
   }
+  // block form: a cycle's vectors enter the operator unscaled until their block is finished
+  if (mode == DM_RNORM && gs->columns > 1)
+    for (int q = 1 + tid; q < GM_MAXR + 2; q += nt) gs->s[q] = 1.0;
 }
 
 template <typename T>
@@ -192,6 +233,510 @@ __global__ void dots_kernel(const T* __restrict__ Vb, size_t stride, int m, cons
 }
 
 enum UpdMode { UM_NONE = 0, UM_ARNOLDI = 1 };
+
+// ---------------------------------------------------------------------------
+// block Arnoldi: inner products
+// ---------------------------------------------------------------------------
+// d += a b on the float64 tensor path (the fifth-generation tensor cores have
+// no float64 kind).  Lane l holds A[row l / 4][k l % 4], B[k l % 4][col l / 4]
+// and D[row l / 4][cols 2 (l % 4), + 1]; every product and sum is a float64
+// fused multiply-add.
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
+// One warp per summed matrix row and thread 0 for the s x s factor: the
+// coefficients of the block's update from the summed products w[r][i] =
+// <row r, Z_i>, rows V_0 .. V_j0 then Z_1 .. Z_s.  r1s: scratch, rows x 8.
+//
+// Projections in the orthonormal basis: r1 = B^T w.  The part of Z outside
+// the basis has the Gram matrix G - r1^T r1 = r2^T r2; a column whose pivot
+// there is lost in rounding (Z_i depends on the earlier ones to the
+// precision of the stored vectors) ends the block before it, never before its
+// first column, which needs no pivot: its norm is taken from the stored
+// result.
+__device__ __forceinline__ void block_coefs(GState* gs, const double* w, double* r1s, int j0, int s) {
+  __shared__ double g[GM_S][GM_S], r2[GM_S][GM_S], u[GM_S][GM_S];
+  const int m = j0 + 1, tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+  for (int q = tid; q < m * 8; q += GT) {
+    const int l = q >> 3, i = q & 7;
+    double v = 0.0;
+    if (i < s) {
+      const int st = gs->bstart[l];
+      for (int p = st; p <= l; ++p) v += gs->B[l][p - st] * w[p * 8 + i];
+      gs->r1[l][i] = v;
+    }
+    r1s[q] = v;
+  }
+  __syncthreads();
+  int pair = 0;
+  for (int i = 0; i < s; ++i)
+    for (int k = i; k < s; ++k, ++pair) {
+      if ((pair & 7) != wp) continue;
+      double v = 0.0;
+      for (int l = lane; l < m; l += 32) v += r1s[l * 8 + i] * r1s[l * 8 + k];
+      v = warp_sum(v);
+      if (lane == 0) g[i][k] = w[(m + i) * 8 + k] - v;
+    }
+  __syncthreads();
+  if (tid == 0) {
+    int keep = s;
+    const double lost = 32.0 * gs->eps;
+    for (int i = 0; i < GM_S; ++i)
+      for (int k = 0; k < GM_S; ++k) { r2[i][k] = 0.0; u[i][k] = 0.0; }
+    for (int i = 0; i < keep; ++i) {
+      double piv = g[i][i];
+      for (int q = 0; q < i; ++q) {
+        double v = g[q][i];
+        for (int p = 0; p < q; ++p) v -= r2[p][q] * r2[p][i];
+        v /= r2[q][q];
+        r2[q][i] = v;
+        piv -= v * v;
+      }
+      const double own = w[(m + i) * 8 + i];  // ||Z_i||^2
+      if (piv > lost * own) {
+        r2[i][i] = sqrt(piv);
+      } else if (i == 0) {  // scaled by its own length; alone in its block
+        r2[0][0] = own > 0.0 ? sqrt(own) : 1.0;
+        keep = 1;
+      } else {
+        for (int q = 0; q < i; ++q) r2[q][i] = 0.0;
+        keep = i;
+      }
+    }
+    for (int i = 0; i < keep; ++i) {  // u = r2^-1
+      u[i][i] = 1.0 / r2[i][i];
+      for (int q = i - 1; q >= 0; --q) {
+        double v = 0.0;
+        for (int p = q + 1; p <= i; ++p) v -= r2[q][p] * u[p][i];
+        u[q][i] = v / r2[q][q];
+      }
+    }
+    gs->bs = keep;
+    for (int i = 0; i < GM_S; ++i)
+      for (int k = 0; k < GM_S; ++k) { gs->r2[i][k] = r2[i][k]; gs->u[i][k] = u[i][k]; }
+  }
+  __syncthreads();
+  // r1 u, then back to the stored vectors: cv = B (r1 u)
+  double t[GM_S];
+  for (int l = tid; l < m; l += GT) {
+    for (int i = 0; i < s; ++i) {
+      t[i] = 0.0;
+      for (int k = 0; k <= i; ++k) t[i] += r1s[l * 8 + k] * u[k][i];
+    }
+    for (int i = 0; i < s; ++i) r1s[l * 8 + i] = t[i];
+  }
+  __syncthreads();
+  for (int q = tid; q < m * 8; q += GT) {
+    const int k = q >> 3, i = q & 7;
+    if (i >= s) continue;
+    const int st = gs->bstart[k];
+    double v = 0.0;
+    for (int l = k; l < m && gs->bstart[l] == st; ++l) v += gs->B[l][k - st] * r1s[l * 8 + i];
+    gs->cv[k][i] = v;
+  }
+}
+
+// Products of the m + s stored vectors V_0 .. V_j0, Z_1 .. Z_s (contiguous
+// slots, m = j0 + 1) with Z_1 .. Z_s: an (m + s) x s x n contraction, float64
+// tensor tiles of 8 rows x 8 columns x 4 elements.  The operands of both
+// sides have the same lane layout (row l / 4, element l % 4), so a lane loads
+// 16-byte pieces of its row straight from memory and the order of the
+// elements within a piece does not matter; NT row tiles stay in registers
+// for the whole pass and need no shuffles.  Rows and columns past the end
+// repeat the last one and are ignored.
+//
+// Bound by reading the m + s vectors: the tensor work of a pass (8 of 8
+// columns for 6 vectors) stays below the loads' time.  256x256x80 float32,
+// the inner products of a cycle of 30: 9.1 ms in one-step form, 2.71 ms here
+// (3.7 TB/s of the rows read once; the float64 tensor pipe 60 % busy).
+//
+// The partial tiles are summed in two levels (groups of GM_GROUP blocks, then
+// the groups), in a fixed order: the same bits on every run.
+template <typename T, int NT>
+__device__ __forceinline__ void block_dots_body(const T* __restrict__ Vb, size_t stride, int j0, int s, size_t n,
+                                                double* partial, GState* gs, int bid, int nblk) {
+  constexpr int VN = V16<T>::n;
+  constexpr int KW = 8 * VN;  // elements of every row a warp takes per pass: two 16-byte pieces per lane
+  constexpr int GRP = NT < 4 ? NT : 4;
+  __shared__ double red[8][GRP * 64];
+  __shared__ double w[NT * 64], r1s[NT * 64];
+  const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+  const int m = j0 + 1, rows = m + s;
+  const int r = lane >> 2;
+  const size_t kq = (size_t)(lane & 3) * VN;
+  const T* zp = Vb + (size_t)(m + min(r, s - 1)) * stride + kq;
+  const T* v0 = Vb + kq;
+  double acc[NT][2];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = 0.0;
+  for (size_t k = ((size_t)bid * 8 + wp) * KW; k < n; k += (size_t)nblk * 8 * KW) {
+    T z[2 * VN];
+    load16(zp + k, z);
+    load16(zp + k + 4 * VN, z + VN);
+#pragma unroll
+    for (int t0 = 0; t0 < NT; t0 += GRP) {
+      T a[GRP][2 * VN];
+#pragma unroll
+      for (int t = 0; t < GRP; ++t) {
+        if (t0 + t >= NT) continue;
+        const T* v = v0 + (size_t)min(8 * (t0 + t) + r, rows - 1) * stride + k;
+        load16(v, a[t]);
+        load16(v + 4 * VN, a[t] + VN);
+      }
+#pragma unroll
+      for (int e = 0; e < 2 * VN; ++e) {
+        const double zd = (double)z[e];
+#pragma unroll
+        for (int t = 0; t < GRP; ++t)
+          if (t0 + t < NT) dmma(acc[t0 + t], (double)a[t][e], zd);
+      }
+    }
+  }
+  double* mine = partial + (size_t)bid * (NT * 64);
+#pragma unroll
+  for (int t0 = 0; t0 < NT; t0 += GRP) {
+#pragma unroll
+    for (int t = 0; t < GRP; ++t)
+      if (t0 + t < NT) {
+        red[wp][t * 64 + r * 8 + 2 * (lane & 3)] = acc[t0 + t][0];
+        red[wp][t * 64 + r * 8 + 2 * (lane & 3) + 1] = acc[t0 + t][1];
+      }
+    __syncthreads();
+    const int cnt = min(GRP, NT - t0) * 64;
+    for (int q = tid; q < cnt; q += GT) {
+      double v = 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v += red[k][q];
+      mine[t0 * 64 + q] = v;
+    }
+    __syncthreads();
+  }
+  const int grp = bid / GM_GROUP, ng = (nblk + GM_GROUP - 1) / GM_GROUP;
+  const int gsz = min(GM_GROUP, nblk - grp * GM_GROUP);
+  if (!last_block(&gs->group_counter[grp], (unsigned)gsz)) return;
+  double* gpart = partial + (size_t)nblk * (NT * 64);
+  const double* first = partial + (size_t)grp * GM_GROUP * (NT * 64);
+  for (int q = tid; q < NT * 64; q += GT) {
+    double v = 0.0;
+    for (int b = 0; b < gsz; ++b) v += __ldcg(first + (size_t)b * (NT * 64) + q);
+    gpart[(size_t)grp * (NT * 64) + q] = v;
+  }
+  if (tid == 0) gs->group_counter[grp] = 0;
+  __syncthreads();  // every thread has read last_block's verdict before the next one is written
+  if (!last_block(&gs->counter, (unsigned)ng)) return;
+  for (int q = tid; q < NT * 64; q += GT) {
+    double v = 0.0;
+    for (int b = 0; b < ng; ++b) v += __ldcg(gpart + (size_t)b * (NT * 64) + q);
+    w[q] = v;
+  }
+  if (tid == 0) gs->counter = 0;
+  __syncthreads();
+  block_coefs(gs, w, r1s, j0, s);
+}
+
+template <typename T, int NT>
+__global__ void __launch_bounds__(GT, 2) block_dots_kernel(const T* __restrict__ Vb, size_t stride, int j0, int s,
+                                                           size_t n, double* partial, GState* gs) {
+  if (gs->active == 0) return;
+  block_dots_body<T, NT>(Vb, stride, j0, s, n, partial, gs, blockIdx.x, gridDim.x);
+}
+
+// ---------------------------------------------------------------------------
+// block Arnoldi: update
+// ---------------------------------------------------------------------------
+// The Hessenberg columns of the block's steps from gram[i][k] = <V_{m+i},
+// V_{m+k}> of the new vectors as stored, then the cycle's bookkeeping.
+//
+// With rc^T rc = gram the new orthonormal vectors are Q_{m+i} = sum_q V_{m+q}
+// (rc^-1)[q][i], and in the basis Q the operator's inputs and outputs are
+// known columns C: C_0 the scaled V_j0, C_{i+1} = [r1_i; (rc r2)_i] the
+// vector Z_{i+1} = M A (input i).  H C_t = C_{t+1} gives the new columns of
+// H one after the other (a row per thread: a row of column t needs only the
+// same row of earlier columns).  For one column this is the classical
+// Arnoldi step.
+__device__ __forceinline__ void block_finish(GState* gs, const double (&gram)[GM_S][GM_S], int j0, int s) {
+  constexpr int P = GM_MAXR + 2;
+  __shared__ double C[GM_S + 1][P], hn[GM_S][P], gv[GM_MAXR][2];
+  __shared__ double rc[GM_S][GM_S], ri[GM_S][GM_S], t2[GM_S][GM_S], len2[GM_S];
+  __shared__ int keep_s, done_s;
+  const int m = j0 + 1, R = gs->restart, tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+  const bool rotate = gs->method != 0;
+  if (tid == 0) {
+    int keep = gs->bs;
+    for (int i = 0; i < GM_S; ++i)
+      for (int k = 0; k < GM_S; ++k) { rc[i][k] = 0.0; ri[i][k] = 0.0; t2[i][k] = 0.0; }
+    for (int i = 0; i < keep; ++i) {
+      double piv = gram[i][i];
+      for (int q = 0; q < i; ++q) {
+        double v = gram[q][i];
+        for (int p = 0; p < q; ++p) v -= rc[p][q] * rc[p][i];
+        v /= rc[q][q];
+        rc[q][i] = v;
+        piv -= v * v;
+      }
+      if (i > 0 && !(piv > 1e-4 * gram[i][i])) {  // not independent of the earlier columns as stored
+        for (int q = 0; q < i; ++q) rc[q][i] = 0.0;
+        keep = i;
+        break;
+      }
+      rc[i][i] = piv > 0.0 ? sqrt(piv) : 0.0;
+      if (!(rc[i][i] > 0.0)) keep = i + 1;  // i = 0: nothing left of Z_1
+    }
+    for (int i = 0; i < keep; ++i) {
+      ri[i][i] = rc[i][i] > 0.0 ? 1.0 / rc[i][i] : 0.0;
+      for (int q = i - 1; q >= 0; --q) {
+        double v = 0.0;
+        for (int p = q + 1; p <= i; ++p) v -= rc[q][p] * ri[p][i];
+        ri[q][i] = v * ri[q][q];
+      }
+      for (int q = 0; q <= i; ++q) {
+        double v = 0.0;
+        for (int p = q; p <= i; ++p) v += rc[q][p] * gs->r2[p][i];
+        t2[q][i] = v;
+      }
+    }
+    keep_s = keep;
+  }
+  for (int q = tid; q < 2 * j0; q += GT) (&gv[0][0])[q] = (&gs->givens[0][0])[q];
+  __syncthreads();
+  const int keep = keep_s;
+  const double start = gs->s[j0];
+  const int cst = gs->cstart, cln = gs->clen;
+  for (int p = tid; p < m + keep; p += GT) {
+    C[0][p] = (p >= cst && p < cst + cln) ? start * gs->clast[p - cst] : 0.0;
+    for (int i = 0; i < keep; ++i) C[i + 1][p] = p < m ? gs->r1[p][i] : (p - m <= i ? t2[p - m][i] : 0.0);
+  }
+  __syncthreads();
+  for (int p = tid; p < m + keep; p += GT) {
+    double a[GM_S], h[GM_S];
+    for (int t = 0; t < GM_S; ++t) a[t] = 0.0;
+    for (int c = p > 0 ? p - 1 : 0; c < j0; ++c) {  // known columns (Hessenberg: row p starts at column p - 1)
+      const double hv = gs->hraw[c][p];
+#pragma unroll
+      for (int t = 0; t < GM_S; ++t) a[t] += hv * (t < keep ? C[t][c] : 0.0);
+    }
+#pragma unroll
+    for (int t = 0; t < GM_S; ++t) {
+      h[t] = 0.0;
+      if (t < keep) {
+        double v = C[t + 1][p] - a[t];
+#pragma unroll
+        for (int k = 0; k < GM_S; ++k)
+          if (k < t) v -= h[k] * C[t][j0 + k];
+        h[t] = p <= j0 + t + 1 ? v / C[t][j0 + t] : 0.0;
+        hn[t][p] = h[t];
+      }
+    }
+  }
+  __syncthreads();
+  if (wp < keep) {  // ||M A Q_j||^2
+    double v = 0.0;
+    for (int p = lane; p < m + keep; p += 32) v += hn[wp][p] * hn[wp][p];
+    v = warp_sum(v);
+    if (lane == 0) len2[wp] = v;
+  }
+  __syncthreads();
+  // breakdown (jax _kth_arnoldi_iteration): nothing new left of a column
+  if (tid < keep && !(hn[tid][m + tid] > gs->eps * sqrt(len2[tid]))) {
+    hn[tid][m + tid] = 0.0;
+    len2[tid] = -1.0;
+  }
+  __syncthreads();
+  for (int q = tid; q < keep * (R + 1); q += GT) {
+    const int t = q / (R + 1), p = q - t * (R + 1);
+    gs->hraw[j0 + t][p] = p < m + keep ? hn[t][p] : 0.0;
+  }
+  __syncthreads();
+  if (rotate && tid < keep)  // the cycle's earlier rotations, a column per thread
+    for (int i = 0; i < j0; ++i) {
+      const double c = gv[i][0], sn = gv[i][1], x1 = hn[tid][i], y1 = hn[tid][i + 1];
+      hn[tid][i] = c * x1 - sn * y1;
+      hn[tid][i + 1] = sn * x1 + c * y1;
+    }
+  __syncthreads();
+  if (tid == 0) {
+    int done = 0, active = 1;
+    for (int t = 0; t < keep && active; ++t) {
+      const int j = j0 + t;
+      done = t + 1;
+      if (!rotate) {
+        if (len2[t] < 0.0) { gs->breakdown = 1; active = 0; }
+        continue;
+      }
+      double* row = hn[t];
+      for (int i = j0; i < j; ++i) {
+        const double c = gv[i][0], sn = gv[i][1], x1 = row[i], y1 = row[i + 1];
+        row[i] = c * x1 - sn * y1;
+        row[i + 1] = sn * x1 + c * y1;
+      }
+      // _givens_rotation(a, b)
+      const double a = row[j], b = row[j + 1];
+      double cs, sn;
+      if (b == 0.0) {
+        cs = 1.0; sn = 0.0;
+      } else if (fabs(a) < fabs(b)) {
+        const double q = -a / b, r = 1.0 / sqrt(1.0 + q * q);
+        cs = r * q; sn = r;
+      } else {
+        const double q = -b / a, r = 1.0 / sqrt(1.0 + q * q);
+        cs = r; sn = r * q;
+      }
+      gv[j][0] = gs->givens[j][0] = cs;
+      gv[j][1] = gs->givens[j][1] = sn;
+      row[j] = cs * a - sn * b;
+      row[j + 1] = sn * a + cs * b;
+      const double b0 = gs->beta[j], b1 = gs->beta[j + 1];
+      gs->beta[j] = cs * b0 - sn * b1;
+      gs->beta[j + 1] = sn * b0 + cs * b1;
+      gs->err = fabs(gs->beta[j + 1]);
+      if (!(gs->err > gs->ptol)) active = 0;
+    }
+    if (keep < s) active = 0;  // a shortened block ends its cycle
+    gs->kdone = j0 + done;
+    gs->active = active;
+    done_s = done;
+    // the block's last vector feeds the next one
+    const int last = keep - 1;
+    gs->s[m + last] = ri[last][last];
+    gs->cstart = m;
+    gs->clen = keep;
+    for (int q = 0; q <= last; ++q) gs->clast[q] = rc[q][last];
+  }
+  for (int q = tid; q < keep * GM_S; q += GT) {
+    const int i = q / GM_S, p = q - i * GM_S;
+    gs->B[m + i][p] = p <= i ? ri[p][i] : 0.0;
+    if (p == 0) gs->bstart[m + i] = m;
+  }
+  __syncthreads();
+  for (int q = tid; q < done_s * (R + 1); q += GT) {
+    const int t = q / (R + 1), p = q - t * (R + 1);
+    gs->H[j0 + t][p] = p <= m + t ? hn[t][p] : 0.0;
+  }
+}
+
+// V_{m+i} <- sum_k u[k][i] Z_k - sum_l cv[l][i] V_l for the S new vectors
+// (m = j0 + 1) and the Gram matrix of the results as stored.  One 16-byte
+// chunk of all S vectors per thread, four basis vectors' loads in flight.
+// Bound by reading m + S and writing S vectors.  Tiles are taken from the end
+// of the vectors: block_dots has just walked them from the front, so the
+// last tens of MB of every row are still in the 126 MB L2.  256x256x80
+// float32, the updates of a cycle of 30: 8.2 ms in one-step form, 2.43 ms
+// here (5.4 TB/s).
+template <typename T, int S>
+__device__ __forceinline__ void block_update_body(T* Vb, size_t stride, int j0, size_t n, double* partial,
+                                                  GState* gs, int bid, int nblk) {
+  constexpr int VN = V16<T>::n;
+  constexpr int NP = S * (S + 1) / 2;
+  constexpr int LD = 8;  // coefficients per row, padded for vector loads
+  __shared__ __align__(16) T cf[(GM_MAXR + 1) * LD];
+  __shared__ double red[NP][GT / 32];
+  __shared__ double gram[GM_S][GM_S];
+  const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+  const int m = j0 + 1;
+  for (int q = tid; q < (m + S) * LD; q += GT) {
+    const int l = q / LD, i = q - l * LD;
+    cf[q] = i >= S ? T(0) : (T)(l < m ? -gs->cv[l][i] : gs->u[l - m][i]);
+  }
+  __syncthreads();
+  const T* cu = cf + m * LD;
+  T* zb = Vb + (size_t)m * stride;
+  double g[NP];
+#pragma unroll
+  for (int q = 0; q < NP; ++q) g[q] = 0.0;
+  const size_t tile = (size_t)GT * VN;
+  for (long long t = (long long)((n + tile - 1) / tile) - 1 - bid; t >= 0; t -= nblk) {
+    const size_t off = (size_t)t * tile + (size_t)tid * VN;
+    if (off >= n) continue;
+    T acc[S][VN];
+    {
+      T z[S][VN];
+#pragma unroll
+      for (int k = 0; k < S; ++k) load16_rw(zb + (size_t)k * stride + off, z[k]);
+#pragma unroll
+      for (int i = 0; i < S; ++i)
+#pragma unroll
+        for (int e = 0; e < VN; ++e) {
+          T v = cu[i] * z[0][e];
+#pragma unroll
+          for (int k = 1; k <= i; ++k) v += cu[k * LD + i] * z[k][e];
+          acc[i][e] = v;
+        }
+    }
+    const T* v = Vb + off;
+    int l = 0;
+    for (; l + 4 <= m; l += 4, v += 4 * stride) {
+      T x[4][VN];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) load16_rw(v + (size_t)q * stride, x[q]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int i = 0; i < S; ++i) {
+          const T c = cf[(l + q) * LD + i];
+#pragma unroll
+          for (int e = 0; e < VN; ++e) acc[i][e] += c * x[q][e];
+        }
+    }
+    for (; l < m; ++l, v += stride) {
+      T x[VN];
+      load16_rw(v, x);
+#pragma unroll
+      for (int i = 0; i < S; ++i) {
+        const T c = cf[l * LD + i];
+#pragma unroll
+        for (int e = 0; e < VN; ++e) acc[i][e] += c * x[e];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < S; ++i) store16(zb + (size_t)i * stride + off, acc[i]);
+#pragma unroll
+    for (int e = 0; e < VN; ++e) {
+      double d[S];
+#pragma unroll
+      for (int i = 0; i < S; ++i) d[i] = (double)acc[i][e];
+      int q = 0;
+#pragma unroll
+      for (int i = 0; i < S; ++i)
+#pragma unroll
+        for (int k = i; k < S; ++k) g[q++] += d[i] * d[k];
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < NP; ++q) {
+    const double v = warp_sum(g[q]);
+    if (lane == 0) red[q][wp] = v;
+  }
+  __syncthreads();
+  if (tid < NP) {
+    double v = 0.0;
+    for (int k = 0; k < GT / 32; ++k) v += red[tid][k];
+    partial[(size_t)bid * NP + tid] = v;
+  }
+  if (!last_block(&gs->counter, (unsigned)nblk)) return;
+  for (int q = wp; q < NP; q += GT / 32) {
+    double v = 0.0;
+    for (int b = lane; b < nblk; b += 32) v += __ldcg(partial + (size_t)b * NP + q);
+    v = warp_sum(v);
+    if (lane == 0) {
+      int i = 0, r = q;
+      while (r >= S - i) { r -= S - i; ++i; }
+      gram[i][i + r] = v;
+    }
+  }
+  if (tid == 0) gs->counter = 0;
+  __syncthreads();
+  block_finish(gs, gram, j0, S);
+}
+
+template <typename T, int S>
+__global__ void __launch_bounds__(GT, 2) block_update_kernel(T* Vb, size_t stride, int j0, size_t n, double* partial,
+                                                             GState* gs) {
+  if (gs->active == 0) return;
+  block_update_body<T, S>(Vb, stride, j0, n, partial, gs, blockIdx.x, gridDim.x);
+}
 
 // x64 += sum_{i < min(m, kdone)} coef_i V_i with a float64 solution (the
 // end-of-cycle update of GMRES with iterative refinement)
@@ -371,13 +916,15 @@ __global__ void __launch_bounds__(GT) update_kernel(const T* __restrict__ Vb, si
   update_body<T>(Vb, stride, m, w, n, sign, partial, gs, mode, limit_kdone, blockIdx.x, gridDim.x);
 }
 
-__device__ void setup_state(GState* gs, double eps, double tol, double atol_in, int restart, int method) {
+__device__ void setup_state(GState* gs, double eps, double tol, double atol_in, int restart, int method, int columns) {
   gs->eps = eps;
   gs->tol = tol;
   gs->atol_in = atol_in;
   gs->restart = restart;
   gs->method = method;
+  gs->columns = columns;
   gs->counter = 0;
+  for (int q = 0; q < GM_BLOCKS / GM_GROUP + 1; ++q) gs->group_counter[q] = 0;
   gs->active = 1;
   gs->kdone = 0;
   gs->breakdown = 0;
@@ -385,8 +932,9 @@ __device__ void setup_state(GState* gs, double eps, double tol, double atol_in, 
   gs->steps = 0;
   for (int q = 0; q < GM_MAXR + 2; ++q) gs->s[q] = 0.0;
 }
-__global__ void setup_kernel(GState* gs, double eps, double tol, double atol_in, int restart, int method) {
-  setup_state(gs, eps, tol, atol_in, restart, method);
+__global__ void setup_kernel(GState* gs, double eps, double tol, double atol_in, int restart, int method,
+                             int columns) {
+  setup_state(gs, eps, tol, atol_in, restart, method, columns);
 }
 
 // Graph mode: after a residual, count the finished cycle and set the WHILE
@@ -437,10 +985,12 @@ __device__ void begin_cycle_state(GState* gs) {
 }
 __global__ void begin_cycle_kernel(GState* gs) { begin_cycle_state(gs); }
 
-// y from the cycle's small problem; coef_i = y_i s_i.
+// y from the cycle's small problem; coef_i = y_i s_i, or B y in the block
+// form, whose triangular solves run on one warp (a row's inner product over
+// the lanes).
 __device__ void small_solve_state(GState* gs) {
   extern __shared__ double a2[];  // R * R
-  const int R = gs->restart;
+  const int R = gs->restart, kd = gs->kdone, lane = threadIdx.x & 31;
   __shared__ double b2[GM_MAXR];
   __shared__ double y[GM_MAXR];
   if (gs->method == 0) {
@@ -470,7 +1020,24 @@ __device__ void small_solve_state(GState* gs) {
       }
       __syncthreads();
     }
-    if (threadIdx.x == 0) {
+    if (gs->columns > 1) {
+      if (threadIdx.x < 32) {
+        for (int i = 0; i < R; ++i) {  // L z = b2
+          double s = 0.0;
+          for (int k = lane; k < i; k += 32) s += a2[i * R + k] * y[k];
+          s = warp_sum(s);
+          if (lane == 0) y[i] = (b2[i] - s) / a2[i * R + i];
+          __syncwarp();
+        }
+        for (int i = R - 1; i >= 0; --i) {  // L^T y = z
+          double s = 0.0;
+          for (int k = i + 1 + lane; k < R; k += 32) s += a2[k * R + i] * y[k];
+          s = warp_sum(s);
+          if (lane == 0) y[i] = (y[i] - s) / a2[i * R + i];
+          __syncwarp();
+        }
+      }
+    } else if (threadIdx.x == 0) {
       for (int i = 0; i < R; ++i) {  // L z = b2
         double s = b2[i];
         for (int k = 0; k < i; ++k) s -= a2[i * R + k] * y[k];
@@ -484,9 +1051,17 @@ __device__ void small_solve_state(GState* gs) {
       for (int i = 0; i < R; ++i) gs->coef[i] = y[i] * gs->s[i];
     }
   } else {
-    if (threadIdx.x == 0) {
-      // back substitution with the rotated rows: sum_j R[j][i] y_j = beta_i
-      const int kd = gs->kdone;
+    // back substitution with the rotated rows: sum_j R[j][i] y_j = beta_i
+    if (gs->columns > 1) {
+      if (threadIdx.x < 32)
+        for (int i = kd - 1; i >= 0; --i) {
+          double s = 0.0;
+          for (int jj = i + 1 + lane; jj < kd; jj += 32) s += gs->H[jj][i] * y[jj];
+          s = warp_sum(s);
+          if (lane == 0) y[i] = (gs->beta[i] - s) / gs->H[i][i];
+          __syncwarp();
+        }
+    } else if (threadIdx.x == 0) {
       for (int i = kd - 1; i >= 0; --i) {
         double s = gs->beta[i];
         for (int jj = i + 1; jj < kd; ++jj) s -= gs->H[jj][i] * y[jj];
@@ -494,6 +1069,16 @@ __device__ void small_solve_state(GState* gs) {
       }
       for (int i = 0; i < R; ++i) gs->coef[i] = (i < kd) ? y[i] * gs->s[i] : 0.0;
     }
+  }
+  if (gs->columns == 1) return;
+  __syncthreads();
+  for (int k = threadIdx.x; k < R; k += blockDim.x) {
+    double v = 0.0;
+    if (k < kd) {
+      const int st = gs->bstart[k];
+      for (int l = k; l < kd && gs->bstart[l] == st; ++l) v += gs->B[l][k - st] * y[l];
+    }
+    gs->coef[k] = v;
   }
 }
 __global__ void small_solve_kernel(GState* gs) { small_solve_state(gs); }
@@ -525,6 +1110,26 @@ __global__ void group_dots_kernel(GroupMember<T>* mem, const int* __restrict__ f
   dots_body<T>(gvec(g, GV_V0), g.npad, m, gvec(g, wv), g.npad, g.partial, g.gs, mode, b - f0, first[mi + 1] - f0);
 }
 
+template <typename T, int NT>
+__global__ void __launch_bounds__(GT, 2) group_block_dots_kernel(GroupMember<T>* mem, const int* __restrict__ first,
+                                                                 int M, int j0, int s) {
+  const int b = blockIdx.x;
+  const int mi = group_find(first, M, b);
+  const GroupMember<T>& g = mem[mi];
+  if (!g.running || g.gs->active == 0) return;
+  const int f0 = first[mi];
+  block_dots_body<T, NT>(gvec(g, GV_V0), g.npad, j0, s, g.npad, g.partial, g.gs, b - f0, first[mi + 1] - f0);
+}
+template <typename T, int S>
+__global__ void __launch_bounds__(GT, 2) group_block_update_kernel(GroupMember<T>* mem, const int* __restrict__ first,
+                                                                   int M, int j0) {
+  const int b = blockIdx.x;
+  const int mi = group_find(first, M, b);
+  const GroupMember<T>& g = mem[mi];
+  if (!g.running || g.gs->active == 0) return;
+  const int f0 = first[mi];
+  block_update_body<T, S>(gvec(g, GV_V0), g.npad, j0, g.npad, g.partial, g.gs, b - f0, first[mi + 1] - f0);
+}
 // final_x = 0: Arnoldi projection of V_m out of V_0 .. V_{m-1} (gated);
 // final_x = 1: x += sum coef_i V_i over the cycle's basis
 template <typename T>
@@ -591,11 +1196,11 @@ __global__ void __launch_bounds__(256) group_convert_kernel(GroupMember<T>* mem,
 
 // one thread per member
 template <typename T>
-__global__ void group_setup_kernel(GroupMember<T>* mem, int M, int R, int method, int transpose) {
+__global__ void group_setup_kernel(GroupMember<T>* mem, int M, int R, int method, int transpose, int columns) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= M) return;
   GroupMember<T>& g = mem[m];
-  setup_state(g.gs, g.eps, transpose ? g.tol_t : g.tol, g.atol_in, R, method);
+  setup_state(g.gs, g.eps, transpose ? g.tol_t : g.tol, g.atol_in, R, method, columns);
   g.running = 1;
 }
 template <typename T>
@@ -680,6 +1285,63 @@ int gm_x64_blocks_t(size_t n) {
 // ---------------------------------------------------------------------------
 // host wrappers
 // ---------------------------------------------------------------------------
+// calls f with the row tile count (a compile-time constant) for `rows` rows
+template <typename F>
+void with_row_tiles(int rows, F&& f) {
+  switch (gm_row_tiles(rows)) {
+    case 1: f(std::integral_constant<int, 1>{}); break;
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 3: f(std::integral_constant<int, 3>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    case 5: f(std::integral_constant<int, 5>{}); break;
+    case 6: f(std::integral_constant<int, 6>{}); break;
+    case 8: f(std::integral_constant<int, 8>{}); break;
+    case 10: f(std::integral_constant<int, 10>{}); break;
+    case 13: f(std::integral_constant<int, 13>{}); break;
+    default: f(std::integral_constant<int, 17>{}); break;
+  }
+}
+// the same for the columns of a block
+template <typename F>
+void with_columns(int s, F&& f) {
+  switch (s) {
+    case 1: f(std::integral_constant<int, 1>{}); break;
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 3: f(std::integral_constant<int, 3>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    case 5: f(std::integral_constant<int, 5>{}); break;
+    default: f(std::integral_constant<int, 6>{}); break;
+  }
+}
+
+int capped(size_t want) { return want < 1 ? 1 : want > (size_t)GM_BLOCKS ? GM_BLOCKS : (int)want; }
+// two passes of a block's 8 warps; one chunk per thread
+template <typename T>
+int gm_block_dots_blocks(size_t n) {
+  return capped((n + 128 * V16<T>::n - 1) / (128 * V16<T>::n));
+}
+template <typename T>
+int gm_block_update_blocks(size_t n) {
+  return capped((n + GT * V16<T>::n - 1) / (GT * V16<T>::n));
+}
+
+template <typename T>
+void gm_block_dots(const T* Vb, size_t stride, int j0, int s, size_t n, double* partial, GState* gs,
+                   cudaStream_t st) {
+  const int g = gm_block_dots_blocks<T>(n);
+  with_row_tiles(j0 + 1 + s, [&](auto nt) {
+    block_dots_kernel<T, decltype(nt)::value><<<g, GT, 0, st>>>(Vb, stride, j0, s, n, partial, gs);
+  });
+}
+
+template <typename T>
+void gm_block_update(T* Vb, size_t stride, int j0, int s, size_t n, double* partial, GState* gs, cudaStream_t st) {
+  const int g = gm_block_update_blocks<T>(n);
+  with_columns(s, [&](auto sc) {
+    block_update_kernel<T, decltype(sc)::value><<<g, GT, 0, st>>>(Vb, stride, j0, n, partial, gs);
+  });
+}
+
 // shared memory of the dots kernel: (m + 1) per-warp slots of 8 warps
 constexpr size_t DOTS_SMEM_MAX = (size_t)(GM_MAXR + 1) * 8 * sizeof(double);
 constexpr int DOTS_THREADS = 256;
@@ -709,8 +1371,9 @@ void gm_update_x64(const T* Vb, size_t stride, int m, double* x, size_t n, const
   update_x64_kernel<T><<<gm_x64_blocks_t<T>(n), 256, 0, st>>>(Vb, stride, m, x, n, gs);
 }
 
-void gm_setup(GState* gs, double eps, double tol, double atol_in, int restart, int method, cudaStream_t st) {
-  setup_kernel<<<1, 1, 0, st>>>(gs, eps, tol, atol_in, restart, method);
+void gm_setup(GState* gs, double eps, double tol, double atol_in, int restart, int method, int columns,
+              cudaStream_t st) {
+  setup_kernel<<<1, 1, 0, st>>>(gs, eps, tol, atol_in, restart, method, columns);
 }
 void gm_init_tol(GState* gs, cudaStream_t st) { init_tol_kernel<<<1, 1, 0, st>>>(gs); }
 void gm_gate(GState* gs, cudaGraphConditionalHandle h, int maxiter, int after_cycle, cudaStream_t st) {
@@ -752,7 +1415,7 @@ int group_convert_blocks(size_t n) { return flat_grid(n, 256 * 8) < 296 ? flat_g
 
 template <typename T>
 void grp_setup(const GroupLaunch<T>& g, int transpose, cudaStream_t st) {
-  group_setup_kernel<T><<<(g.M + 127) / 128, 128, 0, st>>>(g.mem, g.M, g.R, g.method, transpose);
+  group_setup_kernel<T><<<(g.M + 127) / 128, 128, 0, st>>>(g.mem, g.M, g.R, g.method, transpose, g.S);
 }
 template <typename T>
 void grp_dots(const GroupLaunch<T>& g, int m, int w, int mode, int gated, cudaStream_t st) {
@@ -761,6 +1424,20 @@ void grp_dots(const GroupLaunch<T>& g, int m, int w, int mode, int gated, cudaSt
   const int nt = gm_dots_threads<T>(m);
   const size_t smem = (size_t)(m + 1) * (nt / 32) * sizeof(double);
   group_dots_kernel<T><<<g.blocks(GT_DOTS0 + m), nt, smem, st>>>(g.mem, g.row(GT_DOTS0 + m), g.M, m, w, mode, gated);
+}
+template <typename T>
+void grp_block_dots(const GroupLaunch<T>& g, int j0, int s, cudaStream_t st) {
+  with_row_tiles(j0 + 1 + s, [&](auto nt) {
+    group_block_dots_kernel<T, decltype(nt)::value>
+        <<<g.blocks(GT_BDOT), GT, 0, st>>>(g.mem, g.row(GT_BDOT), g.M, j0, s);
+  });
+}
+template <typename T>
+void grp_block_update(const GroupLaunch<T>& g, int j0, int s, cudaStream_t st) {
+  with_columns(s, [&](auto sc) {
+    group_block_update_kernel<T, decltype(sc)::value>
+        <<<g.blocks(GT_BUPD), GT, 0, st>>>(g.mem, g.row(GT_BUPD), g.M, j0);
+  });
 }
 template <typename T>
 void grp_update_arnoldi(const GroupLaunch<T>& g, int m, cudaStream_t st) {
@@ -799,6 +1476,10 @@ void grp_info(const GroupLaunch<T>& g, int solve, cudaStream_t st) {
 }
 
 #define SISL_GROUP_INST(T)                                                                           \
+  template int gm_block_dots_blocks<T>(size_t);                                                      \
+  template int gm_block_update_blocks<T>(size_t);                                                    \
+  template void grp_block_dots<T>(const GroupLaunch<T>&, int, int, cudaStream_t);                    \
+  template void grp_block_update<T>(const GroupLaunch<T>&, int, int, cudaStream_t);                  \
   template int gm_dots_threads<T>(int);                                                              \
   template int gm_dots_blocks<T>(int, size_t);                                                       \
   template int gm_update_blocks<T>(size_t);                                                          \
@@ -816,6 +1497,10 @@ SISL_GROUP_INST(float)
 SISL_GROUP_INST(double)
 #undef SISL_GROUP_INST
 
+template void gm_block_dots<float>(const float*, size_t, int, int, size_t, double*, GState*, cudaStream_t);
+template void gm_block_dots<double>(const double*, size_t, int, int, size_t, double*, GState*, cudaStream_t);
+template void gm_block_update<float>(float*, size_t, int, int, size_t, double*, GState*, cudaStream_t);
+template void gm_block_update<double>(double*, size_t, int, int, size_t, double*, GState*, cudaStream_t);
 template void gm_dots<float>(const float*, size_t, int, const float*, size_t, double*, GState*, int, int,
                              cudaStream_t);
 template void gm_dots<double>(const double*, size_t, int, const double*, size_t, double*, GState*, int, int,

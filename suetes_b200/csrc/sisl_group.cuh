@@ -42,6 +42,8 @@ enum GroupTable {
   GT_MV = 0,  // column-march matvec
   GT_PC,      // pipelined column preconditioner
   GT_UPD,     // multi-axpy (+ norm)
+  GT_BDOT,    // block dots
+  GT_BUPD,    // block update
   GT_X64,     // float64 solution update
   GT_CVT,     // packed conversions and copies
   GT_ATG,     // transposed matvec, stage 1 (mass points)
@@ -59,6 +61,7 @@ struct GroupLaunch {
   std::vector<int> first_h;  // host copy
   std::vector<int> nz_h;     // members' level counts (preconditioner shared memory)
   int M = 0, R = 0, method = 0;
+  int S = 1;                 // columns per orthogonalisation block, the same for every member
   bool refine = false;
   const int* row(int t) const { return first + (size_t)t * (M + 1); }
   int blocks(int t) const { return first_h[(size_t)t * (M + 1) + M]; }
@@ -81,6 +84,8 @@ enum GroupVec { GV_X = 0, GV_B = 1, GV_Z = 2, GV_V0 = 3 };  // GV_V0 + i: basis 
 // per-member block counts of the standalone launches
 template <typename T> int gm_dots_threads(int m);
 template <typename T> int gm_dots_blocks(int m, size_t n);
+template <typename T> int gm_block_dots_blocks(size_t n);
+template <typename T> int gm_block_update_blocks(size_t n);
 template <typename T> int gm_update_blocks(size_t n);
 int gm_x64_blocks(size_t n);
 int group_matvec_blocks(const Dims& d);
@@ -97,6 +102,11 @@ void grp_setup(const GroupLaunch<T>& g, int transpose, cudaStream_t st);
 // result over basis vectors V_0 .. V_{m-1} and vector `w` (GroupVec), mode as gm_dots
 template <typename T>
 void grp_dots(const GroupLaunch<T>& g, int m, int w, int mode, int gated, cudaStream_t st);
+// block Arnoldi step: as gm_block_dots, gm_block_update (gated)
+template <typename T>
+void grp_block_dots(const GroupLaunch<T>& g, int j0, int s, cudaStream_t st);
+template <typename T>
+void grp_block_update(const GroupLaunch<T>& g, int j0, int s, cudaStream_t st);
 // Arnoldi: V_{m} -= sum_{i<m} h_i s_i V_i and finish step m - 1 (gated);
 // final: x += sum_{i<min(R, kdone)} coef_i V_i (float64 x with refinement)
 template <typename T>
