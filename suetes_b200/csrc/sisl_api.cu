@@ -372,6 +372,40 @@ double precond_bytes(const Dims& d, size_t es) {
   return es * (vec + 2 * fw + fm + fm + 6 * fw);
 }
 
+// Launch shapes of a core that has not been tuned; every shape gives the same
+// bits, so only time decides.  Lines drawn from whole solves (us per Arnoldi
+// step, cold coefficients) at grids from 48x41x33 to 384x384x96.
+//
+// Matvec.  The column march (6) holds one thread per column: it needs
+// four blocks on every SM to hide memory, and then beats the
+// several-levels-per-thread shapes (4: two, 5: four), which hide latency with
+// threads instead (256x256x80 float32 449 against 473; 192x192x64, at 0.6 of a
+// wave, 255 against 237; 64x64x48 104 against 70).  Past one wave of blocks,
+// four z chunks (8) even out the second one (384x384x96 1202 against 1257).
+// In float64 the march has half the threads resident and never wins by more
+// than 1 %; shape 5 from about 20,000 columns (150x131x60 222.5 against 224.2,
+// 96x96x48 114 against 110).
+int default_matvec(const Dims& d, size_t es) {
+  if (es == 8) return d.nx * d.ny < 20000 ? 4 : 5;
+  const int blocks = ((d.nx + 1 + 31) / 32) * ((d.ny + 1 + 3) / 4), wave = 4 * 148;
+  return blocks > wave ? 8 : 10 * blocks >= 8 * wave ? 6 : 4;
+}
+// Preconditioner.  The 32-column tile with batched loads (4) works on a
+// column with eight threads outside the tridiagonal sweep, the pipelined
+// march (6) with one: the tile wins while the columns alone do not fill the
+// chip (64x64x48 float32 46 against 70, 192x192x64 227 against 237, float64
+// 150x131x60 216 against 224) and loses after (256x256x80 487 against 473.5,
+// float64 192x192x64 385 against 380).  Of the transposed ones the batched
+// tile is never slower (256x256x80 float32 613 against 643, float64 948
+// against 1118).
+void default_shapes(Dims& d, size_t es) {
+  d.tune_mv = default_matvec(d, es);
+  const bool fits = d.nz >= 2 && (size_t)(5 * d.nz + 1) * 32 * es <= 200 * 1024;
+  d.tune_pc = fits && d.nx * d.ny < (es == 4 ? 50000 : 30000) ? 4 : 6;
+  d.tune_mvt = 0;
+  d.tune_pct = d.nz >= 2 ? 4 : 0;
+}
+
 // Columns per orthogonalisation block of the Krylov cycles.  The monomial
 // basis M A V, (M A)^2 V, .. of a block is well conditioned when the operator
 // M A = I + E is dominated by E, the horizontal acoustic coupling, whose
@@ -488,7 +522,9 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
         launch_matvec_t<double>(d, cf64, x5, nullptr, b5, r5, g.tmp64, nullptr, s);
         convert_packed_kernel<double, T><<<nconv, 256, 0, s>>>(g.r64, g.z(), g.z(), n, n);
       } else {
-        launch_matvec<double>(d, cf64, x5, nullptr, b5, r5, nullptr, s);
+        Dims d64 = d;  // the float64 operator's own shape: the march waits on b at every level
+        d64.tune_mv = default_matvec(d, sizeof(double));
+        launch_matvec<double>(d64, cf64, x5, nullptr, b5, r5, nullptr, s);
         convert_packed_kernel<double, T><<<nconv, 256, 0, s>>>(g.r64, g.V(0), g.z(), g.off[2], n);
       }
     } else {
@@ -1744,6 +1780,7 @@ int sisl_core_create(const SislGrid* grid, const SislParams* prm, const SislBack
   c->s = Scalars{prm->dt, prm->alpha, prm->g, prm->cp, prm->Rd, prm->cvd, prm->p0, prm->pi_scale, prm->nu_div,
                  prm->nu_h};
   const size_t es = esize(grid->dtype);
+  default_shapes(c->d, es);
   size_t total = 0, offs[C_COUNT];
   for (int q = 0; q < C_COUNT; ++q) {
     offs[q] = total;

@@ -52,10 +52,9 @@ struct Dims {
   int nx, ny, nz;
   int px, py;          // periodic flags for x and y
   double dx, dy, dz;
-  // launch shapes chosen by the autotuner (sisl_autotune): the Helmholtz
-  // matvec (default 6: the column march), its transpose (stencil block), the
-  // column preconditioner (default 6: the pipelined column march) and its
-  // transpose (column tile)
+  // launch shapes, set by default_shapes or chosen by the autotuner
+  // (sisl_autotune): the Helmholtz matvec, its transpose (stencil block), the
+  // column preconditioner and its transpose (column tile)
   int tune_mv = 6, tune_pc = 6, tune_mvt = 0, tune_pct = 0;
 };
 
