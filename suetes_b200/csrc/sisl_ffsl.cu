@@ -3,10 +3,11 @@
 // FluxFormAdvector.advect_3d_split (steppers.py:596-647) with advect_1d
 // (steppers.py:552-594): cell masses rho dx dy / m^2 dz_m, one sweep per
 // axis (x, y, z) remapping the cumulative mass to the departure interfaces
-// with linear interpolation.  One thread per grid line; the cumulative mass
-// of each line is accumulated in float64 in a line-interleaved scratch array
-// (position-major, line-fastest, so neighbouring threads touch neighbouring
-// words).  Periodic axes use the three-copy extension of steppers.py:569-582
+// with linear interpolation.  A block per 32 grid lines with the cumulative
+// mass of its lines, float64, in shared memory; lines too long for that, the
+// VJPs and advect_1d take one thread per line with a line-interleaved scratch
+// array (position-major, line-fastest, so neighbouring threads touch
+// neighbouring words).  Periodic axes use the three-copy extension of steppers.py:569-582
 // evaluated in closed form: M_ext(p) = floor(p / N) S + M(p mod N).
 #include "sisl_core.cuh"
 
@@ -98,6 +99,172 @@ __global__ void ffsl_sweep_kernel(Dims d, Coef<T> c, int axis, const T* __restri
     out[p] = (T)val;
     prev = nxt;
   }
+}
+
+// One sweep with a block per 32 lines: the lines' cells go to shared memory
+// as float64 (from density when from_density: mass = rho dx dy / m^2 dz_m,
+// rounded to T as ffsl_mass_kernel stores it), eight warps each sum one
+// segment of every line and shift it by the segments before it, and the
+// departure sums read the shared cumulative mass.  Global memory sees every
+// cell, every face velocity and every result once, in rows: along x the lanes
+// walk a line, along y and z they sit on neighbouring lines.
+//
+// ffsl_sweep_kernel walks a line with one thread, which leaves a chain of N
+// dependent memory round trips and (along x) a row of N cells per lane:
+// 201x160x64 float64 173 us a sweep.  Here: 45 us along x (its density to mass
+// product included), 22 along y, 27 along z, bound by the float64 arithmetic of
+// the departure sums.  The line length
+// is bounded by shared memory ((N + 1) x 33 float64); longer lines take the
+// one-thread form.
+constexpr int FL = 32;      // lines per block
+constexpr int FW = 8;       // warps: segments per line
+constexpr int FLD = FL + 1;  // row of the shared cumulative mass: no bank conflicts along either index
+
+inline size_t ffsl_tile_bytes(int N) { return sizeof(double) * ((size_t)(N + 1) * FLD + FW * FL); }
+
+template <typename T, int AXIS>
+__global__ void __launch_bounds__(FL* FW) ffsl_tile_kernel(Dims d, Coef<T> c, const T* __restrict__ in,
+                                                           const T* __restrict__ vel, T* __restrict__ out,
+                                                           int periodic, double scale, int from_density,
+                                                           int to_density) {
+  extern __shared__ double M[];  // [N + 1][FLD] cumulative mass, then the segment sums
+  const int N = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;
+  const int nlines = AXIS == 0 ? d.ny * d.nz : AXIS == 1 ? d.nx * d.nz : d.nx * d.ny;
+  const int na = AXIS == 0 ? d.ny : d.nx;
+  double* seg = M + (size_t)(N + 1) * FLD;  // [FW][FL]
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int line0 = blockIdx.x * FL;
+  auto point = [&](int line, int q, int& i, int& j, int& k) {
+    const int a = line % na, b = line / na;
+    i = AXIS == 0 ? q : a;
+    j = AXIS == 0 ? a : AXIS == 1 ? q : b;
+    k = AXIS == 2 ? q : b;
+  };
+  auto mass = [&](int line, int q) -> double {
+    int i, j, k;
+    point(line, q, i, j, k);
+    T v = ld(in, im(d, i, j, k));
+    if (from_density) v = v * cell_volume(d, c, i, j, k);
+    return (double)v;
+  };
+  if constexpr (AXIS == 0) {
+    for (int l = wp; l < FL && line0 + l < nlines; l += FW)
+#pragma unroll 8
+      for (int q = lane; q < N; q += 32) M[(size_t)(q + 1) * FLD + l] = mass(line0 + l, q);
+  } else if (line0 + lane < nlines) {
+#pragma unroll 8
+    for (int q = wp; q < N; q += FW) M[(size_t)(q + 1) * FLD + lane] = mass(line0 + lane, q);
+  }
+  if (wp == 0) M[lane] = 0.0;
+  __syncthreads();
+  // cumulative mass: segment sums, then every segment shifted by those before it
+  const int len = (N + FW - 1) / FW;
+  const int q0 = min(wp * len, N), q1 = min(q0 + len, N);
+  double s = 0.0;
+  if (line0 + lane < nlines)
+    for (int q = q0; q < q1; ++q) {
+      s += M[(size_t)(q + 1) * FLD + lane];
+      M[(size_t)(q + 1) * FLD + lane] = s;
+    }
+  seg[wp * FL + lane] = s;
+  __syncthreads();
+  if (wp > 0 && line0 + lane < nlines) {
+    double off = seg[lane];
+    for (int v = 1; v < wp; ++v) off += seg[v * FL + lane];
+    for (int q = q0; q < q1; ++q) M[(size_t)(q + 1) * FLD + lane] += off;
+  }
+  __syncthreads();
+  auto courant = [&](int l, int q) -> double {  // at interface q (steppers.py:614-616)
+    int i, j, k;
+    point(line0 + l, q, i, j, k);
+    if (AXIS == 0) return (double)ld(vel, iu(d, i, j, k)) * (double)ld(c.mu, h_u(d, i, j)) * scale;
+    if (AXIS == 1) return (double)ld(vel, iv(d, i, j, k)) * (double)ld(c.mv, h_v(d, i, j)) * scale;
+    return (double)ld(vel, iw(d, i, j, k)) * scale;
+  };
+  // mass left of interface q's departure point
+  auto departed = [&](int l, int q, double c0) -> double {
+    if (periodic) {
+      const double S = M[(size_t)N * FLD + l];
+      const double dep = (double)(q + N) - c0;
+      const double lo = floor(dep), w = dep - lo;
+      const long long L = 3LL * N + 1;
+      long long i0 = (long long)lo, i1 = i0 + 1;
+      i0 = i0 < 0 ? 0 : (i0 > L - 1 ? L - 1 : i0);
+      i1 = i1 < 0 ? 0 : (i1 > L - 1 ? L - 1 : i1);
+      const int p0 = (int)i0, p1 = (int)i1, b0 = p0 / N, b1 = p1 / N;
+      return (1.0 - w) * ((double)b0 * S + M[(size_t)(p0 - b0 * N) * FLD + l]) +
+             w * ((double)b1 * S + M[(size_t)(p1 - b1 * N) * FLD + l]);
+    }
+    const double dep = fmin(fmax((double)q - c0, 0.0), (double)N);
+    const double lo = floor(dep), w = dep - lo;
+    const int i0 = min(max((int)lo, 0), N), i1 = min(i0 + 1, N);
+    return (1.0 - w) * M[(size_t)i0 * FLD + l] + w * M[(size_t)i1 * FLD + l];
+  };
+  auto store = [&](int l, int q, double val) {
+    int i, j, k;
+    point(line0 + l, q, i, j, k);
+    if (to_density) val /= (double)cell_volume(d, c, i, j, k);
+    out[im(d, i, j, k)] = (T)val;
+  };
+  constexpr int U = 4;  // interfaces whose velocities are in flight together
+  if constexpr (AXIS == 0) {
+    // 31 cells a step: lane 31 only supplies the last one's right interface
+    for (int l = wp; l < FL && line0 + l < nlines; l += FW)
+      for (int qb = 0; qb < N; qb += 31 * U) {  // uniform over the warp
+        double c0[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) c0[u] = courant(l, min(qb + 31 * u + lane, N));
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int q = qb + 31 * u + lane;
+          const double lo = departed(l, min(q, N), c0[u]);
+          const double hi = __shfl_down_sync(0xffffffffu, lo, 1);
+          if (lane < 31 && q < N) store(l, q, hi - lo);
+        }
+      }
+  } else if (line0 + lane < nlines && q0 < q1) {
+    double prev = departed(lane, q0, courant(lane, q0));
+    for (int q = q0; q < q1; q += U) {
+      double c0[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) c0[u] = courant(lane, min(q + u + 1, q1));
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (q + u >= q1) break;
+        const double next = departed(lane, q + u + 1, c0[u]);
+        store(lane, q + u, next - prev);
+        prev = next;
+      }
+    }
+  }
+}
+
+// One sweep along `axis` in the form that fits; returns whether the tile form
+// (the only one that takes densities) was launched.
+template <typename T, int AXIS>
+bool launch_ffsl_tile(const Dims& d, const Coef<T>& c, const T* in, const T* vel, T* out, int periodic, double dt,
+                      int from_density, int to_density, cudaStream_t st) {
+  const int N = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;
+  const int nlines = AXIS == 0 ? d.ny * d.nz : AXIS == 1 ? d.nx * d.nz : d.nx * d.ny;
+  const size_t smem = ffsl_tile_bytes(N);
+  if (smem > 224 * 1024) return false;
+  static SmemLimit attr_bytes;  // per instantiation
+  ensure_smem_limit((const void*)ffsl_tile_kernel<T, AXIS>, attr_bytes, smem);
+  const double scale = AXIS == 0 ? dt / d.dx : AXIS == 1 ? dt / d.dy : dt;  // of the interface Courant number
+  ffsl_tile_kernel<T, AXIS><<<(nlines + FL - 1) / FL, FL * FW, smem, st>>>(d, c, in, vel, out, periodic, scale,
+                                                                         from_density, to_density);
+  return true;
+}
+template <typename T>
+void launch_ffsl_sweep(const Dims& d, const Coef<T>& c, int axis, const T* in, const T* vel, T* out, double* M,
+                       int periodic, double dt, int to_density, cudaStream_t st) {
+  const bool done = axis == 0   ? launch_ffsl_tile<T, 0>(d, c, in, vel, out, periodic, dt, 0, to_density, st)
+                    : axis == 1 ? launch_ffsl_tile<T, 1>(d, c, in, vel, out, periodic, dt, 0, to_density, st)
+                                : launch_ffsl_tile<T, 2>(d, c, in, vel, out, periodic, dt, 0, to_density, st);
+  if (done) return;
+  const int nlines = axis == 0 ? d.ny * d.nz : axis == 1 ? d.nx * d.nz : d.nx * d.ny;
+  const int tb = 128;
+  ffsl_sweep_kernel<T><<<(nlines + tb - 1) / tb, tb, 0, st>>>(d, c, axis, in, vel, out, M, periodic, dt, to_density);
 }
 
 // advect_1d (steppers.py:552-594) on nlines independent lines: scalar is
@@ -304,14 +471,17 @@ size_t ffsl_scratch_doubles(const Dims& d) {
 template <typename T>
 int launch_ffsl(const Dims& d, const Coef<T>& c, const T* field, const T* u, const T* v, const T* eta, T* out, T* tmp0,
                 T* tmp1, double* M, cudaStream_t st) {
-  dim3 blk(32, 4, 2);
-  ffsl_mass_kernel<T><<<box3(d, blk), blk, 0, st>>>(d, c, field, tmp0);
-  const int tb = 128;
   const double dt = c.s.dt;
-  ffsl_sweep_kernel<T><<<(d.ny * d.nz + tb - 1) / tb, tb, 0, st>>>(d, c, 0, tmp0, u, tmp1, M, d.px, dt, 0);
-  ffsl_sweep_kernel<T><<<(d.nx * d.nz + tb - 1) / tb, tb, 0, st>>>(d, c, 1, tmp1, v, tmp0, M, d.py, dt, 0);
-  ffsl_sweep_kernel<T><<<(d.nx * d.ny + tb - 1) / tb, tb, 0, st>>>(d, c, 2, tmp0, eta, out, M, 0, dt, 1);
-  return 4;  // kernels launched
+  int kernels = 3;
+  if (!launch_ffsl_tile<T, 0>(d, c, field, u, tmp1, d.px, dt, 1, 0, st)) {
+    const dim3 blk(32, 4, 2);
+    ffsl_mass_kernel<T><<<box3(d, blk), blk, 0, st>>>(d, c, field, tmp0);
+    launch_ffsl_sweep<T>(d, c, 0, tmp0, u, tmp1, M, d.px, dt, 0, st);
+    ++kernels;
+  }
+  launch_ffsl_sweep<T>(d, c, 1, tmp1, v, tmp0, M, d.py, dt, 0, st);
+  launch_ffsl_sweep<T>(d, c, 2, tmp0, eta, out, M, 0, dt, 1, st);
+  return kernels;
 }
 
 // field_bar (and u_bar, v_bar, eta_bar where non-null) of out = FFSL(field)
@@ -327,8 +497,8 @@ int launch_ffsl_vjp(const Dims& d, const Coef<T>& c, const T* field, const T* u,
   T *mass = tmp[0], *mx = tmp[1], *my = tmp[2], *b1 = tmp[3], *b2 = tmp[4];
   // recompute the sweeps' inputs
   ffsl_mass_kernel<T><<<box3(d, blk), blk, 0, st>>>(d, c, field, mass);
-  ffsl_sweep_kernel<T><<<(d.ny * d.nz + tb - 1) / tb, tb, 0, st>>>(d, c, 0, mass, u, mx, M, d.px, dt, 0);
-  ffsl_sweep_kernel<T><<<(d.nx * d.nz + tb - 1) / tb, tb, 0, st>>>(d, c, 1, mx, v, my, M, d.py, dt, 0);
+  launch_ffsl_sweep<T>(d, c, 0, mass, u, mx, M, d.px, dt, 0, st);
+  launch_ffsl_sweep<T>(d, c, 1, mx, v, my, M, d.py, dt, 0, st);
   // reverse z, y, x
   ffsl_sweep_vjp_kernel<T><<<(d.nx * d.ny + tb - 1) / tb, tb, 0, st>>>(d, c, 2, my, eta, out_bar, b1, eta_bar, M,
                                                                      Mb, 0, dt, 1, 0);
