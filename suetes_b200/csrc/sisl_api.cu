@@ -1675,13 +1675,10 @@ int split_vjp_impl(SislCore* c, const SislState* in, const SislState* ob, const 
     a.dtau = (T)dts[stage]; a.alpha = (T)alpha; a.nu_div = (T)c->s.nu_div;
     int A = 0;  // b.upp[A]: cotangent of u'' after the current sub-step
     for (int n = nst[stage] - 1; n >= 0; --n) {
-      if (!zero(b.upp[1 - A], LOC_U) || !zero(b.vpp[1 - A], LOC_V) || !zero(b.uh, LOC_U) || !zero(b.vh, LOC_V) ||
-          !zero(b.gx0, LOC_U) || !zero(b.gy0, LOC_V))
-        return SISL_ERR_CUDA;
       a.upp2 = b.upp[A]; a.vpp2 = b.vpp[A];
       a.upp = b.upp[1 - A]; a.vpp = b.vpp[1 - A];
-      KScope k(c, SISL_K_OTHER, st, 9);
-      launch_split_substep_vjp<T>(d, cf, a, b.det, st);
+      KScope k(c, SISL_K_OTHER, st, 4);
+      launch_split_substep_vjp<T>(d, cf, a, st);
       A = 1 - A;
     }
     {
@@ -1691,7 +1688,7 @@ int split_vjp_impl(SislCore* c, const SislState* in, const SislState* ob, const 
         if (!zero(b.adv[q], LOC_M)) return SISL_ERR_CUDA;
       launch_split_slow_vjp<T>(d, (const T* const*)b.sf, b.tend, b.adv, b.det, st);
       launch_split_adv_vjp<T>(d, cf, cur[0], cur[1], cur[2], cur[3], cur[5], (T)eps_l, (const T* const*)b.adv, Cb[0],
-                              Cb[1], Cb[2], Cb[3], Cb[5], b.det, st);
+                              Cb[1], Cb[2], Cb[3], Cb[5], b.tmp4, st);
     }
     // explicit tendencies (mode 1) at the stage start; their hyperdiffusion input
     const bool hyp = hyp_s || hyp_t;

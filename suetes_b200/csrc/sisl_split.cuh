@@ -62,13 +62,14 @@ void launch_split_axpy(size_t n, const T* b, T* a, cudaStream_t st);
 // Reverse sweep (sisl_step_vjp.cu).  Every acoustic sub-step is linear in
 // the state (its matrices are background coefficients), so its transposes
 // need no recorded intermediates; the slow tendencies are re-formed at the
-// recomputed stage-start states.  Scatters go through a fixed-point sink
-// when det_scratch is given (det_scatter_scratch_bytes), so the cotangents
-// are the same bits on every run.
+// recomputed stage-start states.  The sub-steps and the advection gather;
+// the other scatters go through a fixed-point sink when det_scratch is given
+// (det_scatter_scratch_bytes), so the cotangents are the same bits on every
+// run.
 // ---------------------------------------------------------------------------
 template <typename T>
 struct SplitBar {
-  T *upp, *vpp;              // u'', v'' at the sub-step start (accumulated)
+  T *upp, *vpp;              // u'', v'' at the sub-step start
   const T *upp2, *vpp2;      // u'', v'' after the corrector
   T *wpp, *ppp;              // w'', pi'' (in place: after -> before)
   T *uh, *vh, *gx0, *gy0;    // midpoint winds and old pressure gradients
@@ -86,8 +87,7 @@ void launch_split_diag_vjp(const Dims& d, const Coef<T>& c, T* wb, T* eb, T* ub,
                            cudaStream_t st);
 // the reverse of one acoustic sub-step: corrector, column, predictor
 template <typename T>
-void launch_split_substep_vjp(const Dims& d, const Coef<T>& c, const SplitBar<T>& b, void* det_scratch,
-                              cudaStream_t st);
+void launch_split_substep_vjp(const Dims& d, const Coef<T>& c, const SplitBar<T>& b, cudaStream_t st);
 // split_end^T: out6 (u, v, w, eta, pi, th cotangents of the stage state) ->
 // stage-start c6 (accumulated; th into the step start's th0b), u'', v'', w'',
 // pi'' (written) and the th' slow forcing (written, times dtau nsteps)
@@ -102,10 +102,10 @@ void launch_split_init_vjp(const Dims& d, const T* upp, const T* vpp, const T* w
 template <typename T>
 void launch_split_slow_vjp(const Dims& d, const T* const* sf5, T* const* tend6, T* const* adv4, void* det_scratch,
                            cudaStream_t st);
-// split_adv^T at the stage-start state: adv4 -> u, v, w, eta_dot, th' (accumulated)
+// split_adv^T at the stage-start state: adv4 -> u, v, w, eta_dot, th' (accumulated); tmp4: mass-point scratch
 template <typename T>
 void launch_split_adv_vjp(const Dims& d, const Coef<T>& c, const T* u, const T* v, const T* w, const T* eta,
                           const T* th, T eps_l, const T* const* adv4, T* ub, T* vb, T* wb, T* eb, T* thb,
-                          void* det_scratch, cudaStream_t st);
+                          T* const* tmp4, cudaStream_t st);
 
 }  // namespace sisl

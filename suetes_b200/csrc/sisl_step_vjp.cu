@@ -7,13 +7,13 @@
 // m->u, m->v of a non-periodic axis and the levels 0 and nz of m->w carry no
 // cotangent).
 //
-// Stencils whose transposes fan out to a handful of points (explicit and
-// corrector kernels) scatter, one thread per output point, mirroring the
+// Stencils whose transposes fan out to a handful of points (explicit,
+// corrector and slow-forcing kernels) scatter, one thread per output point, mirroring the
 // forward kernels' point functions -- with a scratch buffer as fixed-point
 // sums (DetSink: the same bits on every run), without one as float atomic
-// adds; the two horizontal Laplacians of the hyperdiffusion are transposed
-// in gather form (two passes per Laplacian: face gradients, then mass
-// points).
+// adds; the two horizontal Laplacians of the hyperdiffusion (two passes per
+// Laplacian: face gradients, then mass points), the split-explicit core's
+// acoustic sub-steps and its upwind advection are transposed in gather form.
 #include "sisl_explicit_dev.cuh"
 #include "sisl_step_vjp.cuh"
 
@@ -848,44 +848,6 @@ __device__ __forceinline__ void kinematic_adj(const Dims& d, const Coef<T>& c, c
   WA.vw(i, j, k, m * ld(c.zew, p));
 }
 
-// horizontal divergence of (uc + up, vc + vp) at cell (i, j, k): cotangent x
-template <typename T>
-__device__ __forceinline__ void cell_div_adj(const Dims& d, const Coef<T>& c, T* ucb, T* upb, T* vcb, T* vpb, int i,
-                                             int j, int k, T x) {
-  const T mm = ld(c.mm, h_m(d, i, j));
-  const int u0 = iu(d, i, j, k), v0 = iv(d, i, j, k);
-  const T sx = x * mm / (T)d.dx, sy = x * mm / (T)d.dy;
-  radd(ucb, u0 + 1, sx);
-  radd(upb, u0 + 1, sx);
-  radd(ucb, u0, -sx);
-  radd(upb, u0, -sx);
-  radd(vcb, v0 + d.nx, sy);
-  radd(vpb, v0 + d.nx, sy);
-  radd(vcb, v0, -sy);
-  radd(vpb, v0, -sy);
-}
-// the divergence-damping gradient at u face i / v face j (never a padded face here)
-template <typename T>
-__device__ __forceinline__ void div_grad_x_adj(const Dims& d, const Coef<T>& c, T* ucb, T* upb, T* vcb, T* vpb, int i,
-                                               int j, int k, T x) {
-  if (x == T(0)) return;
-  int l, r;
-  face_pair(i, d.nx, d.px, l, r);
-  const T s = x / (T)d.dx * ld(c.mu, h_u(d, i, j));
-  cell_div_adj(d, c, ucb, upb, vcb, vpb, r, j, k, s);
-  cell_div_adj(d, c, ucb, upb, vcb, vpb, l, j, k, -s);
-}
-template <typename T>
-__device__ __forceinline__ void div_grad_y_adj(const Dims& d, const Coef<T>& c, T* ucb, T* upb, T* vcb, T* vpb, int i,
-                                               int j, int k, T x) {
-  if (x == T(0)) return;
-  int l, r;
-  face_pair(j, d.ny, d.py, l, r);
-  const T s = x / (T)d.dy * ld(c.mv, h_v(d, i, j));
-  cell_div_adj(d, c, ucb, upb, vcb, vpb, i, r, k, s);
-  cell_div_adj(d, c, ucb, upb, vcb, vpb, i, l, k, -s);
-}
-
 // split_diag_kernel^T (steppers.py:1272-1310): one thread per w point
 template <typename T>
 __global__ void __launch_bounds__(256) split_diag_vjp_kernel(Dims d, Coef<T> c, T* wb, T* eb, T* ub, T* vb,
@@ -910,165 +872,261 @@ __global__ void __launch_bounds__(256) split_diag_vjp_kernel(Dims d, Coef<T> c, 
   det_end<T>();
 }
 
-// split_correct_kernel^T (steppers.py:1607-1626): one thread per union point
-template <typename T>
-__global__ void __launch_bounds__(256) split_correct_vjp_kernel(Dims d, Coef<T> c, SplitBar<T> b, DetSink<T> sink) {
-  det_begin(sink);
+// ---------------------------------------------------------------------------
+// The reverse of one acoustic sub-step, in gather form: every output element
+// is summed by one thread (float64 sums, one rounding), so a launch needs
+// no atomics, no zeroed targets and no pass to find the contributions' range,
+// and repeats bitwise.  The scatter form ran each kernel twice with up to 40
+// 64-bit atomics per point.  109x90x50 float64, us per sub-step, scattered
+// and gathered: corrector 370 -> 74, column 182 -> 37 and 21 (its faces),
+// predictor 268 -> 82, and no longer 38 clears and three finishing passes.
+// What bounds the face kernels now is the issue of their loads (about 90 per
+// point, nearly all of them hits in L1 and L2).
+// ---------------------------------------------------------------------------
+
+// Cotangents at the faces of the predictor (PRED) and corrector updates of
+// u'' and v'': x the cotangent of the updated wind, h that of the pressure
+// gradient, with the periodic duplicate face's share on face 0 and nothing on
+// the open boundary faces (they copy the step-start winds).
+template <typename T, bool PRED>
+struct FaceBar {
+  const Dims& d;
+  const Coef<T>& c;
+  const SplitBar<T>& b;
+  T wt;  // the update's weight: dtau, or dtau / 2 in the predictor
+  __device__ __forceinline__ static T pick(const T* __restrict__ f, int p, int p0, int pn, bool edge, bool per) {
+    if (!edge) return ld(f, p);
+    return per ? ld(f, p0) + ld(f, pn) : T(0);
+  }
+  __device__ __forceinline__ T xu(int f, int j, int k) const {
+    return pick(PRED ? b.uh : b.upp2, iu(d, f, j, k), iu(d, 0, j, k), iu(d, d.nx, j, k), f == 0 || f == d.nx, d.px);
+  }
+  __device__ __forceinline__ T xv(int i, int f, int k) const {
+    return pick(PRED ? b.vh : b.vpp2, iv(d, i, f, k), iv(d, i, 0, k), iv(d, i, d.ny, k), f == 0 || f == d.ny, d.py);
+  }
+  __device__ __forceinline__ int fu(int f) const { return d.px && f == d.nx ? 0 : f; }
+  __device__ __forceinline__ int fv(int f) const { return d.py && f == d.ny ? 0 : f; }
+  __device__ __forceinline__ T hu(int f, int j, int k) const {
+    const T cp = (T)c.s.cp, th = ld(c.thu, iu(d, fu(f), j, k)), x = xu(f, j, k);
+    if (!PRED) return -wt * T(0.5) * cp * th * x;
+    return pick(b.gx0, iu(d, f, j, k), iu(d, 0, j, k), iu(d, d.nx, j, k), f == 0 || f == d.nx, d.px) -
+           wt * cp * th * x;
+  }
+  __device__ __forceinline__ T hv(int i, int f, int k) const {
+    const T cp = (T)c.s.cp, th = ld(c.thv, iv(d, i, fv(f), k)), x = xv(i, f, k);
+    if (!PRED) return -wt * T(0.5) * cp * th * x;
+    return pick(b.gy0, iv(d, i, f, k), iv(d, i, 0, k), iv(d, i, d.ny, k), f == 0 || f == d.ny, d.py) -
+           wt * cp * th * x;
+  }
+  // cotangent of the horizontal divergence of cell (i, j), through the damping gradient at its four faces
+  __device__ __forceinline__ double div(int i, int j, int k) const {
+    const T n = b.nu_div * wt, dx = (T)d.dx, dy = (T)d.dy;
+    return (double)(n * xu(i, j, k) / dx * ld(c.mu, h_u(d, i, j))) -
+           (double)(n * xu(i + 1, j, k) / dx * ld(c.mu, h_u(d, fu(i + 1), j))) +
+           (double)(n * xv(i, j, k) / dy * ld(c.mv, h_v(d, i, j))) -
+           (double)(n * xv(i, j + 1, k) / dy * ld(c.mv, h_v(d, i, fv(j + 1))));
+  }
+  // cotangent of the mass-level vertical gradient of column (i, j), through the terrain slope at its four faces
+  __device__ __forceinline__ double slope(int i, int j, int k) const {
+    return -0.5 * ((double)(ld(c.zxu, iu(d, i, j, k)) * hu(i, j, k)) +
+                   (double)(ld(c.zxu, iu(d, fu(i + 1), j, k)) * hu(i + 1, j, k)) +
+                   (double)(ld(c.zev, iv(d, i, j, k)) * hv(i, j, k)) +
+                   (double)(ld(c.zev, iv(d, i, fv(j + 1), k)) * hv(i, j + 1, k)));
+  }
+};
+
+// split_correct_kernel^T (steppers.py:1607-1626) and split_predict_kernel^T
+// (steppers.py:1561-1579): a thread per column of the union box and VJP_KC
+// levels, the columns' slope terms carried from level to level.
+constexpr int VJP_KC = 4;
+template <typename T, bool PRED>
+__global__ void __launch_bounds__(256) split_faces_vjp_kernel(Dims d, Coef<T> c, SplitBar<T> b) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z * blockDim.z + threadIdx.z;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  if (i <= nx && j <= ny && k <= nz) {
-    const T cp = (T)c.s.cp, dtau = b.dtau;
-    const GradAdj<T> GA{d, c, b.ppp};
-    if (j < ny && k < nz) {
-      const int p = iu(d, i, j, k);
-      const T x = b.upp2[p];
-      if (!d.px && (i == 0 || i == nx)) {
-        radd(b.u0, p, x);
-        radd(b.uc, p, -x);
-      } else if (x != T(0)) {
-        const int ie = (d.px && i == nx) ? 0 : i, pe = iu(d, ie, j, k);
-        radd(b.upp, pe, x);
-        radd(b.sfu, pe, dtau * x);
-        const T h = -dtau * T(0.5) * cp * ld(c.thu, pe) * x;
-        radd(b.gx0, pe, h);
-        GA.gx(ie, j, k, h);
-        div_grad_x_adj(d, c, b.uc, b.uh, b.vc, b.vh, ie, j, k, b.nu_div * dtau * x);
+  if (i > nx || j > ny) return;
+  const int k0 = blockIdx.z * VJP_KC, k1 = min(k0 + VJP_KC, nz + 1);
+  const T dtau = b.dtau, dx = (T)d.dx, dy = (T)d.dy;
+  const FaceBar<T, PRED> F{d, c, b, PRED ? T(0.5) * dtau : dtau};
+  const bool cell = i < nx && j < ny, damp = b.nu_div != T(0);
+  double ym = 0.0, y0 = 0.0;
+  if (cell) {
+    if (k0 > 0) ym = F.slope(i, j, k0 - 1);
+    if (k0 < nz) y0 = F.slope(i, j, k0);
+  }
+  for (int k = k0; k < k1; ++k) {
+    if (k < nz) {
+      double de = 0.0;  // own cell's divergence cotangent
+      if (damp && cell) de = F.div(i, j, k) * (double)ld(c.mm, h_m(d, i, j));
+      if (j < ny) {
+        const int p = iu(d, i, j, k);
+        const bool edge = i == 0 || i == nx;
+        double e = 0.0;
+        if (damp) {
+          if (i > 0) e += F.div(i - 1, j, k) * (double)ld(c.mm, h_m(d, i - 1, j));
+          e = (e - de) / (double)dx;
+        }
+        const T x = F.xu(i, j, k), own = d.px && i == nx ? T(0) : x;  // the duplicate face: on face 0
+        if (edge && !d.px) {  // u''(boundary) = u0 - uc
+          const T v = PRED ? b.uh[p] : b.upp2[p];
+          b.u0[p] += v;
+          b.uc[p] += (T)(e - (double)v);
+        } else {
+          b.uc[p] += (T)e;
+          b.sfu[p] += F.wt * own;
+        }
+        if (PRED) {
+          b.upp[p] += (T)((double)own + e);
+        } else {
+          b.upp[p] = own;
+          b.uh[p] = (T)e;
+          b.gx0[p] = d.px && i == nx ? T(0) : F.hu(i, j, k);
+        }
+      }
+      if (i < nx) {
+        const int p = iv(d, i, j, k);
+        const bool edge = j == 0 || j == ny;
+        double e = 0.0;
+        if (damp) {
+          if (j > 0) e += F.div(i, j - 1, k) * (double)ld(c.mm, h_m(d, i, j - 1));
+          e = (e - de) / (double)dy;
+        }
+        const T x = F.xv(i, j, k), own = d.py && j == ny ? T(0) : x;
+        if (edge && !d.py) {
+          const T v = PRED ? b.vh[p] : b.vpp2[p];
+          b.v0[p] += v;
+          b.vc[p] += (T)(e - (double)v);
+        } else {
+          b.vc[p] += (T)e;
+          b.sfv[p] += F.wt * own;
+        }
+        if (PRED) {
+          b.vpp[p] += (T)((double)own + e);
+        } else {
+          b.vpp[p] = own;
+          b.vh[p] = (T)e;
+          b.gy0[p] = d.py && j == ny ? T(0) : F.hv(i, j, k);
+        }
       }
     }
-    if (i < nx && k < nz) {
-      const int p = iv(d, i, j, k);
-      const T x = b.vpp2[p];
-      if (!d.py && (j == 0 || j == ny)) {
-        radd(b.v0, p, x);
-        radd(b.vc, p, -x);
-      } else if (x != T(0)) {
-        const int je = (d.py && j == ny) ? 0 : j, pe = iv(d, i, je, k);
-        radd(b.vpp, pe, x);
-        radd(b.sfv, pe, dtau * x);
-        const T h = -dtau * T(0.5) * cp * ld(c.thv, pe) * x;
-        radd(b.gy0, pe, h);
-        GA.gy(i, je, k, h);
-        div_grad_y_adj(d, c, b.uc, b.uh, b.vc, b.vh, i, je, k, b.nu_div * dtau * x);
-      }
-    }
-    if (i < nx && j < ny) {  // w'' = (wc + w'') / (1 + dtau tau) - wc at every w level
+    if (!cell) continue;
+    if (!PRED) {  // w'' = (wc + w'') / (1 + dtau tau) - wc at every w level
       const int p = iw(d, i, j, k);
       const T x = b.wpp[p];
       const T f = T(1) / (T(1) + dtau * ld(b.tau, p));
-      wr(b.wpp, p, x * f);
-      radd(b.wc, p, x * (f - T(1)));
+      b.wpp[p] = x * f;
+      b.wc[p] += x * (f - T(1));
+    }
+    if (k < nz) {  // pi'' of the pressure gradient; the edge levels of the vertical one are padded copies
+      const double y1 = k + 1 < nz ? F.slope(i, j, k + 1) : 0.0;
+      double a = ((double)(F.hu(i, j, k) * ld(c.mu, h_u(d, i, j))) -
+                  (double)(F.hu(i + 1, j, k) * ld(c.mu, h_u(d, F.fu(i + 1), j)))) * (1.0 / d.dx) +
+                 ((double)(F.hv(i, j, k) * ld(c.mv, h_v(d, i, j))) -
+                  (double)(F.hv(i, j + 1, k) * ld(c.mv, h_v(d, i, F.fv(j + 1))))) * (1.0 / d.dy);
+      if (k > 0) a += 0.5 * (ym + y0) * (double)ld(c.idzw, iw(d, i, j, k));
+      if (k + 1 < nz) a -= 0.5 * (y0 + y1) * (double)ld(c.idzw, iw(d, i, j, k + 1));
+      const int p = im(d, i, j, k);
+      b.ppp[p] += (T)a;
+      ym = y0;
+      y0 = y1;
     }
   }
-  det_end<T>();
+}
+
+// Cotangents of w level kw (0 < kw < nz) of a column from the solved r below
+// and above it: the eta_dot flux (per unit of w_av - kinematic)
+template <typename T>
+__device__ __forceinline__ T col_flux_bar(const Dims& d, const Coef<T>& c, T dtau, int pw, T r_lo, T r_hi) {
+  // div_z = (fz(k + 1) - fz(k)) / dz_m, rhs = -dtau C_pi (div_h + div_z)
+  const T lo = -dtau * ld(c.cpidz, pw - d.nx * d.ny) * r_lo, hi = -dtau * ld(c.cpidz, pw) * r_hi;
+  return (lo - hi) * ld(c.rhow, pw) * ld(c.thw, pw);
 }
 
 // split_column_kernel^T (steppers.py:1584-1605, 1635-1737): one thread per
 // column.  x (the pi'' increment) is the column solve of T x = rhs, so
-// rhs_bar = T^-T x_bar, swept with the transposed bands; the w'' and eta_dot
-// flux terms are re-formed per level on the way down.
+// rhs_bar = T^-T x_bar, swept with the transposed bands; r = rhs_bar goes to
+// s2 for the faces' kernel.
 template <typename T>
-__global__ void __launch_bounds__(128) split_column_vjp_kernel(Dims d, Coef<T> c, SplitBar<T> b, T a2cp, T adcp,
-                                                               DetSink<T> sink) {
-  det_begin(sink);
+__global__ void __launch_bounds__(128) split_column_vjp_kernel(Dims d, Coef<T> c, SplitBar<T> b, T a2cp, T adcp) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  if (i < nx && j < ny) {
-    const T al = b.alpha, dtau = b.dtau, cp = (T)c.s.cp;
-    const T mm = ld(c.mm, h_m(d, i, j));
-    const T dx = (T)d.dx, dy = (T)d.dy;
-    const GradAdj<T> GA{d, c, b.ppp};
-    const WindsAdj<T> WA{d, c, b.uh, b.vh};
-    auto gam = [&](int kw) -> T {  // acoustic coupling at w level kw (zero at the ground and lid)
-      if (kw <= 0 || kw >= nz) return T(0);
-      const int pw = iw(d, i, j, kw);
-      const T thw = ld(c.thw, pw);
-      return a2cp * thw * ld(c.rhow, pw) * thw / ld(c.dzw, pw);
-    };
-    auto wcoef = [&](int kw) -> T {  // d w''(kw) / d x(kw) = -adcp thw / dz_w (interior levels)
-      if (kw <= 0 || kw >= nz) return T(0);
-      const int pw = iw(d, i, j, kw);
-      return adcp * ld(c.thw, pw) * ld(c.idzw, pw);
-    };
-    // upward: x_bar(k) and the forward sweep of T^T r = x_bar
-    T cprev = T(0), dprev = T(0), g_lo = T(0), g_hi = gam(1);
-    for (int k = 0; k < nz; ++k) {
-      const int p = im(d, i, j, k);
-      T xb = b.ppp[p];
-      if (k >= 1) xb -= wcoef(k) * b.wpp[iw(d, i, j, k)];
-      if (k + 1 <= nz - 1) xb += wcoef(k + 1) * b.wpp[iw(d, i, j, k + 1)];
-      const T cpidz = ld(c.cpidz, p);
-      const T mainv = T(1) + cpidz * (g_lo + g_hi);  // 1 - lower - upper
-      const T sub = (k >= 1) ? -ld(c.cpidz, p - nx * ny) * g_lo : T(0);  // upper(k - 1)
-      const T g_next = gam(k + 2);
-      const T sup = (k + 1 < nz) ? -ld(c.cpidz, p + nx * ny) * g_hi : T(0);  // lower(k + 1)
-      const T inv = T(1) / (mainv - sub * cprev);
-      const T cpk = sup * inv, dpk = (xb - sub * dprev) * inv;
-      b.s1[p] = cpk;
-      b.s2[p] = dpk;
-      cprev = cpk;
-      dprev = dpk;
-      g_lo = g_hi;
-      g_hi = g_next;
-    }
-    // downward: r(k), then the cotangents of level k and of w level k + 1
-    T rh = T(0), dh_hi = T(0);  // r(k + 1) and the div_z weight of level k + 1
-    for (int k = nz - 1; k >= 0; --k) {
-      const int p = im(d, i, j, k);
-      const T r = (k == nz - 1) ? b.s2[p] : b.s2[p] - b.s1[p] * rh;
-      radd(b.sfp, p, dtau * r);
-      const T cpidz = ld(c.cpidz, p), dzm = ld(c.dzm, p);
-      const T dh = -dtau * cpidz * dzm * r;  // cotangent of div_h + div_z
-      // div_h = m (dFx/dx m / dz_m + dFy/dy m / dz_m), F = u_h rdu thu, v_h rdv thv
-      const T e = dh * mm * mm / dzm;
-      const int u0 = iu(d, i, j, k), v0 = iv(d, i, j, k);
-      radd(b.uh, u0 + 1, e / dx * ld(c.rdu, u0 + 1) * ld(c.thu, u0 + 1));
-      radd(b.uh, u0, -e / dx * ld(c.rdu, u0) * ld(c.thu, u0));
-      radd(b.vh, v0 + nx, e / dy * ld(c.rdv, v0 + nx) * ld(c.thv, v0 + nx));
-      radd(b.vh, v0, -e / dy * ld(c.rdv, v0) * ld(c.thv, v0));
-      const T fz_w = dh / dzm;  // div_z = (fz(k + 1) - fz(k)) / dz_m
-      if (k + 1 <= nz - 1) {    // w level k + 1: fz_bar = fz_w(k) - fz_w(k + 1)
-        const int kw = k + 1, pw = iw(d, i, j, kw);
-        const T thw = ld(c.thw, pw), rw = ld(c.rhow, pw);
-        const T q = (fz_w - dh_hi) * rw * thw;  // cotangent of w_av - kinematic
-        kinematic_adj(d, c, WA, i, j, kw, -q);
-        const T wex_b = al * q + b.wpp[pw];
-        const T wold_b = (T(1) - al) * q + wex_b;
-        radd(b.sfw, pw, dtau * wex_b);
-        GA.gzw(i, j, kw, -dtau * cp * thw * wex_b);
-        wr(b.wpp, pw, wold_b);
-      }
-      rh = r;
-      dh_hi = fz_w;
-    }
-    // the ground value is the kinematic one of padded winds and the lid is
-    // zero: w'' there carries no cotangent back
-    wr(b.wpp, iw(d, i, j, 0), T(0));
-    wr(b.wpp, iw(d, i, j, nz), T(0));
+  if (i >= nx || j >= ny) return;
+  const T al = b.alpha, dtau = b.dtau, cp = (T)c.s.cp;
+  auto gam = [&](int kw) -> T {  // acoustic coupling at w level kw (zero at the ground and lid)
+    if (kw <= 0 || kw >= nz) return T(0);
+    const int pw = iw(d, i, j, kw);
+    const T thw = ld(c.thw, pw);
+    return a2cp * thw * ld(c.rhow, pw) * thw / ld(c.dzw, pw);
+  };
+  auto wcoef = [&](int kw) -> T {  // d w''(kw) / d x(kw) = -adcp thw / dz_w (interior levels)
+    if (kw <= 0 || kw >= nz) return T(0);
+    const int pw = iw(d, i, j, kw);
+    return adcp * ld(c.thw, pw) * ld(c.idzw, pw);
+  };
+  // upward: x_bar(k) and the forward sweep of T^T r = x_bar
+  T cprev = T(0), dprev = T(0), g_lo = T(0), g_hi = gam(1);
+  for (int k = 0; k < nz; ++k) {
+    const int p = im(d, i, j, k);
+    T xb = b.ppp[p];
+    if (k >= 1) xb -= wcoef(k) * b.wpp[iw(d, i, j, k)];
+    if (k + 1 <= nz - 1) xb += wcoef(k + 1) * b.wpp[iw(d, i, j, k + 1)];
+    const T cpidz = ld(c.cpidz, p);
+    const T mainv = T(1) + cpidz * (g_lo + g_hi);  // 1 - lower - upper
+    const T sub = (k >= 1) ? -ld(c.cpidz, p - nx * ny) * g_lo : T(0);  // upper(k - 1)
+    const T g_next = gam(k + 2);
+    const T sup = (k + 1 < nz) ? -ld(c.cpidz, p + nx * ny) * g_hi : T(0);  // lower(k + 1)
+    const T inv = T(1) / (mainv - sub * cprev);
+    const T cpk = sup * inv, dpk = (xb - sub * dprev) * inv;
+    b.s1[p] = cpk;
+    b.s2[p] = dpk;
+    cprev = cpk;
+    dprev = dpk;
+    g_lo = g_hi;
+    g_hi = g_next;
   }
-  det_end<T>();
+  // downward: r(k), then the cotangents of level k and of w level k + 1
+  T rh = T(0), s_hi = T(0);  // r(k + 1) and the vertical gradient's share of w level k + 1
+  for (int k = nz - 1; k >= 0; --k) {
+    const int p = im(d, i, j, k);
+    const T r = (k == nz - 1) ? b.s2[p] : b.s2[p] - b.s1[p] * rh;
+    b.s2[p] = r;
+    b.sfp[p] += dtau * r;
+    T s_lo = T(0);  // of w level k
+    if (k > 0) {
+      const int pw = iw(d, i, j, k);
+      const T r_lo = b.s2[p - nx * ny] - b.s1[p - nx * ny] * r;
+      const T q = col_flux_bar(d, c, dtau, pw, r_lo, r);
+      const T wex_b = al * q + b.wpp[pw];
+      b.sfw[pw] += dtau * wex_b;
+      b.wpp[pw] = (T(1) - al) * q + wex_b;
+      s_lo = -dtau * cp * ld(c.thw, pw) * wex_b * ld(c.idzw, pw);
+    }
+    b.ppp[p] += s_lo - s_hi;
+    rh = r;
+    s_hi = s_lo;
+  }
+  // the ground value is the kinematic one of padded winds and the lid is
+  // zero: w'' there carries no cotangent back
+  b.wpp[iw(d, i, j, 0)] = T(0);
+  b.wpp[iw(d, i, j, nz)] = T(0);
 }
 
-// split_column_vjp_kernel on tiles of PC columns (one block per tile and row
-// j): A forms x_bar and the transposed bands at every (level, column) pair,
-// B one thread per column sweeps T^T r = x_bar in shared memory, C scatters
-// the cotangents of every (level, column) pair.  Arithmetic term for term
-// that of split_column_vjp_kernel, with the scatters spread over the block.
+// The same on tiles of PC columns (one block per tile and row j): A forms
+// x_bar and the transposed bands at every (level, column) pair, B one thread
+// per column sweeps T^T r = x_bar in shared memory, C1 the w levels and C2
+// the mass levels.
 template <typename T, int PT, int PC>
-__global__ void __launch_bounds__(PT) split_column_vjp_tile_kernel(Dims d, Coef<T> c, SplitBar<T> b, T a2cp, T adcp,
-                                                                   DetSink<T> sink) {
-  det_begin(sink);
+__global__ void __launch_bounds__(PT) split_column_vjp_tile_kernel(Dims d, Coef<T> c, SplitBar<T> b, T a2cp,
+                                                                   T adcp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  const int nx = d.nx, nz = d.nz;
   T* s_x = reinterpret_cast<T*>(smem_raw);  // [nz][PC] x_bar -> r
-  T* s_sub = s_x + nz * PC;                  // [nz][PC] upper(k - 1)
+  T* s_sub = s_x + nz * PC;                  // [nz][PC] upper(k - 1) -> the vertical gradient's share of w level k
   T* s_sup = s_sub + nz * PC;                // [nz][PC] lower(k + 1) -> c'
   T* s_mn = s_sup + nz * PC;                 // [nz][PC] main
   const int i0 = blockIdx.x * PC, j = blockIdx.y, tid = threadIdx.x;
   const T al = b.alpha, dtau = b.dtau, cp = (T)c.s.cp;
-  const T dx = (T)d.dx, dy = (T)d.dy;
   auto gam = [&](int i, int kw) -> T {
     if (kw <= 0 || kw >= nz) return T(0);
     const int pw = iw(d, i, j, kw);
@@ -1096,8 +1154,8 @@ __global__ void __launch_bounds__(PT) split_column_vjp_tile_kernel(Dims d, Coef<
     s_x[q] = xb;
     const T g_lo = gam(i, k), g_hi = gam(i, k + 1);
     s_mn[q] = T(1) + ld(c.cpidz, p) * (g_lo + g_hi);
-    s_sub[q] = (k >= 1) ? -ld(c.cpidz, p - nx * ny) * g_lo : T(0);
-    s_sup[q] = (k + 1 < nz) ? -ld(c.cpidz, p + nx * ny) * g_hi : T(0);
+    s_sub[q] = (k >= 1) ? -ld(c.cpidz, p - nx * d.ny) * g_lo : T(0);
+    s_sup[q] = (k + 1 < nz) ? -ld(c.cpidz, p + nx * d.ny) * g_hi : T(0);
   }
   __syncthreads();
   if (tid < PC) {  // B
@@ -1120,91 +1178,93 @@ __global__ void __launch_bounds__(PT) split_column_vjp_tile_kernel(Dims d, Coef<
     }
   }
   __syncthreads();
-  const GradAdj<T> GA{d, c, b.ppp};
-  const WindsAdj<T> WA{d, c, b.uh, b.vh};
-  for (int q = tid; q < (nz + 1) * PC; q += PT) {  // C: level k (< nz) and w level k + 1
+  for (int q = tid; q < (nz + 1) * PC; q += PT) {  // C1: w level k
     const int k = q / PC, i = i0 + q % PC;
     if (i >= nx) continue;
-    if (k == nz) {  // ground and lid: no cotangent back through w''
-      wr(b.wpp, iw(d, i, j, 0), T(0));
-      wr(b.wpp, iw(d, i, j, nz), T(0));
+    const int pw = iw(d, i, j, k);
+    if (k == 0 || k == nz) {  // ground and lid: no cotangent back through w''
+      b.wpp[pw] = T(0);
+      if (k == 0) s_sub[q] = T(0);
       continue;
     }
-    const int p = im(d, i, j, k);
-    const T r = s_x[q];
-    radd(b.sfp, p, dtau * r);
-    const T cpidz = ld(c.cpidz, p), dzm = ld(c.dzm, p);
-    const T dh = -dtau * cpidz * dzm * r;
-    const T mm = ld(c.mm, h_m(d, i, j));
-    const T e = dh * mm * mm / dzm;
-    const int u0 = iu(d, i, j, k), v0 = iv(d, i, j, k);
-    radd(b.uh, u0 + 1, e / dx * ld(c.rdu, u0 + 1) * ld(c.thu, u0 + 1));
-    radd(b.uh, u0, -e / dx * ld(c.rdu, u0) * ld(c.thu, u0));
-    radd(b.vh, v0 + nx, e / dy * ld(c.rdv, v0 + nx) * ld(c.thv, v0 + nx));
-    radd(b.vh, v0, -e / dy * ld(c.rdv, v0) * ld(c.thv, v0));
-    if (k + 1 <= nz - 1) {
-      const int kw = k + 1, pw = iw(d, i, j, kw);
-      const int p1 = p + nx * ny;
-      const T fz_lo = dh / dzm;
-      const T fz_hi = (-dtau * ld(c.cpidz, p1) * ld(c.dzm, p1) * s_x[q + PC]) / ld(c.dzm, p1);
-      const T thw = ld(c.thw, pw), rw = ld(c.rhow, pw);
-      const T qq = (fz_lo - fz_hi) * rw * thw;
-      kinematic_adj(d, c, WA, i, j, kw, -qq);
-      const T wex_b = al * qq + b.wpp[pw];
-      const T wold_b = (T(1) - al) * qq + wex_b;
-      radd(b.sfw, pw, dtau * wex_b);
-      GA.gzw(i, j, kw, -dtau * cp * thw * wex_b);
-      wr(b.wpp, pw, wold_b);
-    }
+    const T x = col_flux_bar(d, c, dtau, pw, s_x[q - PC], s_x[q]);
+    const T wex_b = al * x + b.wpp[pw];
+    b.sfw[pw] += dtau * wex_b;
+    b.wpp[pw] = (T(1) - al) * x + wex_b;
+    s_sub[q] = -dtau * cp * ld(c.thw, pw) * wex_b * ld(c.idzw, pw);
   }
-  det_end<T>();
+  __syncthreads();
+  for (int q = tid; q < nz * PC; q += PT) {  // C2: mass level k
+    const int k = q / PC, i = i0 + q % PC;
+    if (i >= nx) continue;
+    const int p = im(d, i, j, k);
+    b.s2[p] = s_x[q];
+    b.sfp[p] += dtau * s_x[q];
+    b.ppp[p] += s_sub[q] - (k + 1 < nz ? s_sub[q + PC] : T(0));
+  }
 }
 
-// split_predict_kernel^T (steppers.py:1561-1579): one thread per union point
+// The column solve's cotangents at the faces: uh, vh += the horizontal flux
+// of div_h and the kinematic winds at the w levels, from r = s2.  A thread
+// per column of the union box and VJP_KC levels.
 template <typename T>
-__global__ void __launch_bounds__(256) split_predict_vjp_kernel(Dims d, Coef<T> c, SplitBar<T> b, DetSink<T> sink) {
-  det_begin(sink);
+__global__ void __launch_bounds__(256) split_column_faces_vjp_kernel(Dims d, Coef<T> c, SplitBar<T> b) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z * blockDim.z + threadIdx.z;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  if (i <= nx && j <= ny && k < nz) {
-    const T cp = (T)c.s.cp, hdt = T(0.5) * b.dtau;
-    const GradAdj<T> GA{d, c, b.ppp};
+  if (i > nx || j > ny) return;
+  const int k0 = blockIdx.z * VJP_KC, k1 = min(k0 + VJP_KC, nz);
+  const T dtau = b.dtau;
+  // kinematic winds of w level kw of cell (a, bb): cotangents of the x and y slope terms
+  struct Kin {
+    double x, y;
+  };
+  auto kin = [&](int a, int bb, int kw) -> Kin {
+    if (kw <= 0 || kw >= nz) return Kin{0.0, 0.0};
+    const int pw = iw(d, a, bb, kw);
+    const T q = -col_flux_bar(d, c, dtau, pw, ld(b.s2, pw - nx * ny), ld(b.s2, pw)) * ld(c.mm, h_m(d, a, bb));
+    return Kin{(double)(q * ld(c.zxw, pw)), (double)(q * ld(c.zew, pw))};
+  };
+  // cotangent of div_h times m^2 / dz_m
+  auto ediv = [&](int a, int bb, int k) -> double {
+    const int p = im(d, a, bb, k);
+    const T m = ld(c.mm, h_m(d, a, bb));
+    return (double)(-dtau * ld(c.cpidz, p) * ld(b.s2, p) * m * m);
+  };
+  const bool own = i < nx && j < ny, west = i > 0 && j < ny, south = j > 0 && i < nx;
+  Kin o0{0.0, 0.0}, w0{0.0, 0.0}, s0{0.0, 0.0};
+  if (own) o0 = kin(i, j, k0);
+  if (west) w0 = kin(i - 1, j, k0);
+  if (south) s0 = kin(i, j - 1, k0);
+  for (int k = k0; k < k1; ++k) {
+    Kin o1{0.0, 0.0}, w1{0.0, 0.0}, s1{0.0, 0.0};
+    double eo = 0.0, ew = 0.0, es = 0.0;
+    if (own) {
+      o1 = kin(i, j, k + 1);
+      eo = ediv(i, j, k);
+    }
+    if (west) {
+      w1 = kin(i - 1, j, k + 1);
+      ew = ediv(i - 1, j, k);
+    }
+    if (south) {
+      s1 = kin(i, j - 1, k + 1);
+      es = ediv(i, j - 1, k);
+    }
     if (j < ny) {
       const int p = iu(d, i, j, k);
-      const int ie = (d.px && i == nx) ? 0 : i, pe = iu(d, ie, j, k);
-      const T x = b.uh[p];
-      T g0 = b.gx0[p];
-      if (!d.px && (i == 0 || i == nx)) {
-        radd(b.u0, p, x);
-        radd(b.uc, p, -x);
-      } else if (x != T(0)) {
-        radd(b.upp, pe, x);
-        radd(b.sfu, pe, hdt * x);
-        g0 -= hdt * cp * ld(c.thu, pe) * x;
-        div_grad_x_adj(d, c, b.uc, b.upp, b.vc, b.vpp, ie, j, k, b.nu_div * hdt * x);
-      }
-      if (g0 != T(0)) GA.gx(ie, j, k, g0);
+      b.uh[p] += (T)((ew - eo) / d.dx * (double)(ld(c.rdu, p) * ld(c.thu, p)) +
+                     0.25 * (o0.x + o1.x + w0.x + w1.x));
     }
     if (i < nx) {
       const int p = iv(d, i, j, k);
-      const int je = (d.py && j == ny) ? 0 : j, pe = iv(d, i, je, k);
-      const T x = b.vh[p];
-      T g0 = b.gy0[p];
-      if (!d.py && (j == 0 || j == ny)) {
-        radd(b.v0, p, x);
-        radd(b.vc, p, -x);
-      } else if (x != T(0)) {
-        radd(b.vpp, pe, x);
-        radd(b.sfv, pe, hdt * x);
-        g0 -= hdt * cp * ld(c.thv, pe) * x;
-        div_grad_y_adj(d, c, b.uc, b.upp, b.vc, b.vpp, i, je, k, b.nu_div * hdt * x);
-      }
-      if (g0 != T(0)) GA.gy(i, je, k, g0);
+      b.vh[p] += (T)((es - eo) / d.dy * (double)(ld(c.rdv, p) * ld(c.thv, p)) +
+                     0.25 * (o0.y + o1.y + s0.y + s1.y));
     }
+    o0 = o1;
+    w0 = w1;
+    s0 = s1;
   }
-  det_end<T>();
 }
 
 // split_end_kernel^T: pointwise
@@ -1316,130 +1376,204 @@ __global__ void __launch_bounds__(256) split_slow_vjp_kernel(Dims d, PtrTable<T>
   det_end<T>();
 }
 
-// cotangent g of F (q4 + sg qb), the 3rd-order upwind-biased face flux
+// split_adv_kernel^T (steppers.py:1312-1465) in gather form, two launches:
+// the cotangents of the four advected mass-point fields (each point collects
+// from the four faces per axis whose upwind stencils read it), then at the
+// faces and w levels those of the winds: the averages to mass points and
+// the advecting fluxes.  Sums in float64, one rounding.  Bound by float64
+// arithmetic and load issue; 109x90x50 float64, us: 1930 as two scattering
+// passes, 128 and 69 here.
 template <typename T>
-__device__ __forceinline__ void upwind_flux_adj(T qm2, T qm1, T q0, T qp1, T F, T eps_l, T g, T& bm2, T& bm1, T& b0,
-                                                T& bp1, T& bF) {
-  const T q4 = T(7.0 / 12.0) * (q0 + qm1) - T(1.0 / 12.0) * (qp1 + qm2);
-  const T qb = T(1.0 / 12.0) * ((qp1 - qm2) - T(3) * (q0 - qm1));
-  const T cf = (fabs(F) < eps_l) ? T(0) : F;
-  const T sg = (cf > T(0)) ? T(1) : ((cf < T(0)) ? T(-1) : T(0));
-  bF += g * (q4 + sg * qb);
-  const T t4 = g * F, tb = g * F * sg;
-  b0 += T(7.0 / 12.0) * t4 - T(3.0 / 12.0) * tb;
-  bm1 += T(7.0 / 12.0) * t4 + T(3.0 / 12.0) * tb;
-  bp1 += -T(1.0 / 12.0) * t4 + T(1.0 / 12.0) * tb;
-  bm2 += -T(1.0 / 12.0) * t4 - T(1.0 / 12.0) * tb;
-}
+struct AdvIn {
+  const T *u, *v, *w, *eta, *th;
+  const T* o[4];  // cotangents of the advection tendencies
+  T eps_l;
+};
+template <typename T>
+struct AdvBar {
+  const Dims& d;
+  const Coef<T>& c;
+  const T* __restrict__ u;
+  const T* __restrict__ v;
+  const T* __restrict__ w;
+  const T* __restrict__ eta;
+  const T* __restrict__ th;
+  const T* const* o;
+  T eps_l;
+  __device__ __forceinline__ T at(int f, int i, int j, int k) const {  // as AdvFields::at
+    switch (f) {
+      case 0: return ld(th, im(d, i, j, k));
+      case 1: return T(0.5) * (ld(u, iu(d, i, j, k)) + ld(u, iu(d, i + 1, j, k)));
+      case 2: return T(0.5) * (ld(v, iv(d, i, j, k)) + ld(v, iv(d, i, j + 1, k)));
+      default: return T(0.5) * (ld(w, iw(d, i, j, k)) + ld(w, iw(d, i, j, k + 1)));
+    }
+  }
+  __device__ __forceinline__ T U(int i, int j, int k) const {
+    return ld(u, iu(d, i, j, k)) / ld(c.mu, h_u(d, i, j));
+  }
+  __device__ __forceinline__ T V(int i, int j, int k) const {
+    return ld(v, iv(d, i, j, k)) / ld(c.mv, h_v(d, i, j));
+  }
+  __device__ __forceinline__ T W(int i, int j, int k) const {
+    return ld(eta, iw(d, i, j, k)) * ld(c.dzw, iw(d, i, j, k));
+  }
+  // sign the upwind bias takes from a flux
+  __device__ __forceinline__ T sign(T F) const {
+    return fabs(F) < eps_l ? T(0) : (F > T(0) ? T(1) : (F < T(0) ? T(-1) : T(0)));
+  }
+  // weight of the stencil's value q (0: two cells below the face .. 3: one above) in the face value
+  __device__ __forceinline__ static T weight(int q, T sg) {
+    switch (q) {
+      case 0: return -T(1.0 / 12.0) - T(1.0 / 12.0) * sg;
+      case 1: return T(7.0 / 12.0) + T(3.0 / 12.0) * sg;
+      case 2: return T(7.0 / 12.0) - T(3.0 / 12.0) * sg;
+      default: return -T(1.0 / 12.0) + T(1.0 / 12.0) * sg;
+    }
+  }
+  // cotangent of the flux difference of cell (i, j, k) per axis
+  __device__ __forceinline__ double gx(const T* __restrict__ of, int i, int j, int k) const {
+    const double m = (double)ld(c.mm, h_m(d, i, j));
+    return -m * m * m / d.dx * (double)ld(of, im(d, i, j, k));
+  }
+  __device__ __forceinline__ double gy(const T* __restrict__ of, int i, int j, int k) const {
+    const double m = (double)ld(c.mm, h_m(d, i, j));
+    return -m * m * m / d.dy * (double)ld(of, im(d, i, j, k));
+  }
+  __device__ __forceinline__ double gz(const T* __restrict__ of, int i, int j, int k) const {
+    const int p = im(d, i, j, k);
+    return -(double)ld(of, p) / (double)ld(c.dzm, p);
+  }
+};
 
-// split_adv_kernel^T (steppers.py:1312-1465): one thread per mass point
+// cotangent of the advected fields at mass points; field 0 is added to thb, 1 to 3 are written to qb
 template <typename T>
-__global__ void __launch_bounds__(256) split_adv_vjp_kernel(Dims d, Coef<T> c, const T* __restrict__ u,
-                                                            const T* __restrict__ v, const T* __restrict__ w,
-                                                            const T* __restrict__ eta, const T* __restrict__ th,
-                                                            T eps_l, PtrTable<T> ab, T* ub, T* vb, T* wb, T* eb,
-                                                            T* thb, DetSink<T> sink) {
-  det_begin(sink);
+__global__ void __launch_bounds__(256) split_adv_vjp_mass_kernel(Dims d, Coef<T> c, AdvIn<T> in, PtrTable<T> qb,
+                                                                 T* thb) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  if (i < nx && j < ny && k < nz) {
-    auto at = [&](int f, int a, int bq, int cz) -> T {  // the advected fields, as AdvFields::at
-      switch (f) {
-        case 0: return ld(th, im(d, a, bq, cz));
-        case 1: return T(0.5) * (ld(u, iu(d, a, bq, cz)) + ld(u, iu(d, a + 1, bq, cz)));
-        case 2: return T(0.5) * (ld(v, iv(d, a, bq, cz)) + ld(v, iv(d, a, bq + 1, cz)));
-        default: return T(0.5) * (ld(w, iw(d, a, bq, cz)) + ld(w, iw(d, a, bq, cz + 1)));
-      }
-    };
-    auto to = [&](int f, int a, int bq, int cz, T x) {  // cotangent x of at(f, a, bq, cz)
-      if (x == T(0)) return;
-      switch (f) {
-        case 0: radd(thb, im(d, a, bq, cz), x); break;
-        case 1:
-          radd(ub, iu(d, a, bq, cz), T(0.5) * x);
-          radd(ub, iu(d, a + 1, bq, cz), T(0.5) * x);
-          break;
-        case 2:
-          radd(vb, iv(d, a, bq, cz), T(0.5) * x);
-          radd(vb, iv(d, a, bq + 1, cz), T(0.5) * x);
-          break;
-        default:
-          radd(wb, iw(d, a, bq, cz), T(0.5) * x);
-          radd(wb, iw(d, a, bq, cz + 1), T(0.5) * x);
-          break;
-      }
-    };
-    const T mm = ld(c.mm, h_m(d, i, j));
-    const T dx = (T)d.dx, dy = (T)d.dy;
-    const T mu0 = ld(c.mu, h_u(d, i, j)), mu1 = ld(c.mu, h_u(d, i + 1, j));
-    const T mv0 = ld(c.mv, h_v(d, i, j)), mv1 = ld(c.mv, h_v(d, i, j + 1));
-    const T dz0 = ld(c.dzw, iw(d, i, j, k)), dz1 = ld(c.dzw, iw(d, i, j, k + 1));
-    const T U0 = ld(u, iu(d, i, j, k)) / mu0, U1 = ld(u, iu(d, i + 1, j, k)) / mu1;
-    const T V0 = ld(v, iv(d, i, j, k)) / mv0, V1 = ld(v, iv(d, i, j + 1, k)) / mv1;
-    const T W0 = ld(eta, iw(d, i, j, k)) * dz0, W1 = ld(eta, iw(d, i, j, k + 1)) * dz1;
-    const T dzm = ld(c.dzm, im(d, i, j, k));
-    const T zfac = (T)d.dz / dzm;
-    const T dU = (U1 - U0) / dx * mm, dV = (V1 - V0) / dy * mm;
-    const T dW = (W1 - W0) / (T)d.dz * zfac;
-    int xi[5], yj[5], zk[5];
+  if (i >= nx || j >= ny || k >= nz) return;
+  const AdvBar<T> A{d, c, in.u, in.v, in.w, in.eta, in.th, in.o, in.eps_l};
+  const double mm = (double)ld(c.mm, h_m(d, i, j));
+  // -(a - q d) differentiated by the q of its second part
+  const double dU = ((double)A.U(i + 1, j, k) - (double)A.U(i, j, k)) / d.dx * mm;
+  const double dV = ((double)A.V(i, j + 1, k) - (double)A.V(i, j, k)) / d.dy * mm;
+  const double dW = ((double)A.W(i, j, k + 1) - (double)A.W(i, j, k)) / (double)ld(c.dzm, im(d, i, j, k));
+  const double own = mm * mm * (dU + dV) + dW;
+  double acc[4];
 #pragma unroll
-    for (int o = 0; o < 5; ++o) {
-      xi[o] = wrap_or_clamp(i - 2 + o, nx, d.px);
-      yj[o] = wrap_or_clamp(j - 2 + o, ny, d.py);
-      zk[o] = min(max(k - 2 + o, 0), nz - 1);
+  for (int f = 0; f < 4; ++f) acc[f] = own * (double)ld(A.o[f], im(d, i, j, k));
+  // stencil positions v that read this point: itself and, at an edge, those clamped (or wrapped) onto it
+  auto first = [](int a, int n, int per) { return per ? a - n * ((a + 2) / n) : (a == 0 ? -2 : a); };
+  auto last = [](int a, int n, int per) { return per ? n + 1 : (a == n - 1 ? n + 1 : a); };
+  for (int v = first(i, nx, d.px), e = last(i, nx, d.px); v <= e; v += d.px ? nx : 1)
+    for (int f = max(v - 1, 0); f <= min(v + 2, nx); ++f) {
+      const T F = A.U(f, j, k);
+      const double wt = (double)F * (double)AdvBar<T>::weight(v - f + 2, A.sign(F));
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        acc[q] += wt * ((f > 0 ? A.gx(A.o[q], f - 1, j, k) : 0.0) - (f < nx ? A.gx(A.o[q], f, j, k) : 0.0));
     }
-    T U0b = T(0), U1b = T(0), V0b = T(0), V1b = T(0), W0b = T(0), W1b = T(0), dUb = T(0), dVb = T(0), dWb = T(0);
-    const int p = im(d, i, j, k);
-#pragma unroll 1
+  for (int v = first(j, ny, d.py), e = last(j, ny, d.py); v <= e; v += d.py ? ny : 1)
+    for (int f = max(v - 1, 0); f <= min(v + 2, ny); ++f) {
+      const T F = A.V(i, f, k);
+      const double wt = (double)F * (double)AdvBar<T>::weight(v - f + 2, A.sign(F));
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        acc[q] += wt * ((f > 0 ? A.gy(A.o[q], i, f - 1, k) : 0.0) - (f < ny ? A.gy(A.o[q], i, f, k) : 0.0));
+    }
+  for (int v = first(k, nz, 0), e = last(k, nz, 0); v <= e; ++v)
+    for (int f = max(v - 1, 0); f <= min(v + 2, nz); ++f) {
+      const T F = A.W(i, j, f);
+      const double wt = (double)F * (double)AdvBar<T>::weight(v - f + 2, A.sign(F));
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        acc[q] += wt * ((f > 0 ? A.gz(A.o[q], i, j, f - 1) : 0.0) - (f < nz ? A.gz(A.o[q], i, j, f) : 0.0));
+    }
+  const int p = im(d, i, j, k);
+  thb[p] += (T)acc[0];
+#pragma unroll
+  for (int q = 1; q < 4; ++q) qb.p[q][p] = (T)acc[q];
+}
+
+// u, v, w += the averages' share of qb; u, v, eta_dot += the advecting fluxes' cotangent.  Union box.
+template <typename T>
+__global__ void __launch_bounds__(256) split_adv_vjp_faces_kernel(Dims d, Coef<T> c, AdvIn<T> in, PtrTable<T> qb,
+                                                                  T* ub, T* vb, T* wb, T* eb) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int k = blockIdx.z * blockDim.z + threadIdx.z;
+  const int nx = d.nx, ny = d.ny, nz = d.nz;
+  if (i > nx || j > ny || k > nz) return;
+  const AdvBar<T> A{d, c, in.u, in.v, in.w, in.eta, in.th, in.o, in.eps_l};
+  // cotangent of a face's flux: its upwind value times the flux differences', and the cells' q dU, q dV, q dW
+  // (the difference's own factor is the flux difference's, with the opposite sign and q for the face value)
+  if (j < ny && k < nz) {
+    double Fb = 0.0;
+    const T sg = A.sign(A.U(i, j, k));
+#pragma unroll
     for (int f = 0; f < 4; ++f) {
-      const T o = ab.p[f][p];
-      if (o == T(0)) continue;
-      T qx[5], qy[5], qz[5];
+      const double gl = i > 0 ? A.gx(A.o[f], i - 1, j, k) : 0.0, gr = i < nx ? A.gx(A.o[f], i, j, k) : 0.0;
+      double val = 0.0;
 #pragma unroll
-      for (int q = 0; q < 5; ++q) {
-        qx[q] = at(f, xi[q], j, k);
-        qy[q] = at(f, i, yj[q], k);
-        qz[q] = at(f, i, j, zk[q]);
+      for (int q = 0; q < 4; ++q) {
+        const T x = A.at(f, wrap_or_clamp(i - 2 + q, nx, d.px), j, k);
+        val += (double)AdvBar<T>::weight(q, sg) * (double)x;
+        if (q == 1) Fb -= gl * (double)x;
+        if (q == 2) Fb += gr * (double)x;
       }
-      const T q = qx[2];
-      // out = -(m^2)(ax - q dU + ay - q dV) - (az - q dW)
-      const T axb = -(mm * mm) * o, azb = -o;
-      T bx[5] = {T(0), T(0), T(0), T(0), T(0)}, by[5] = {T(0), T(0), T(0), T(0), T(0)},
-        bz[5] = {T(0), T(0), T(0), T(0), T(0)};
-      bx[2] += (mm * mm) * (dU + dV) * o + dW * o;
-      dUb += (mm * mm) * q * o;
-      dVb += (mm * mm) * q * o;
-      dWb += q * o;
-      const T gx = axb / dx * mm, gy = axb / dy * mm, gz = azb / (T)d.dz * zfac;
-      upwind_flux_adj(qx[1], qx[2], qx[3], qx[4], U1, eps_l, gx, bx[1], bx[2], bx[3], bx[4], U1b);
-      upwind_flux_adj(qx[0], qx[1], qx[2], qx[3], U0, eps_l, -gx, bx[0], bx[1], bx[2], bx[3], U0b);
-      upwind_flux_adj(qy[1], qy[2], qy[3], qy[4], V1, eps_l, gy, by[1], by[2], by[3], by[4], V1b);
-      upwind_flux_adj(qy[0], qy[1], qy[2], qy[3], V0, eps_l, -gy, by[0], by[1], by[2], by[3], V0b);
-      upwind_flux_adj(qz[1], qz[2], qz[3], qz[4], W1, eps_l, gz, bz[1], bz[2], bz[3], bz[4], W1b);
-      upwind_flux_adj(qz[0], qz[1], qz[2], qz[3], W0, eps_l, -gz, bz[0], bz[1], bz[2], bz[3], W0b);
-#pragma unroll
-      for (int q2 = 0; q2 < 5; ++q2) {
-        to(f, xi[q2], j, k, bx[q2]);
-        to(f, i, yj[q2], k, by[q2]);
-        to(f, i, j, zk[q2], bz[q2]);
-      }
+      Fb += (gl - gr) * val;
     }
-    U1b += dUb / dx * mm;
-    U0b -= dUb / dx * mm;
-    V1b += dVb / dy * mm;
-    V0b -= dVb / dy * mm;
-    W1b += dWb / (T)d.dz * zfac;
-    W0b -= dWb / (T)d.dz * zfac;
-    if (U0b != T(0)) radd(ub, iu(d, i, j, k), U0b / mu0);
-    if (U1b != T(0)) radd(ub, iu(d, i + 1, j, k), U1b / mu1);
-    if (V0b != T(0)) radd(vb, iv(d, i, j, k), V0b / mv0);
-    if (V1b != T(0)) radd(vb, iv(d, i, j + 1, k), V1b / mv1);
-    if (W0b != T(0)) radd(eb, iw(d, i, j, k), W0b * dz0);
-    if (W1b != T(0)) radd(eb, iw(d, i, j, k + 1), W1b * dz1);
+    double a = Fb / (double)ld(c.mu, h_u(d, i, j));
+    if (i > 0) a += 0.5 * (double)ld(qb.p[1], im(d, i - 1, j, k));
+    if (i < nx) a += 0.5 * (double)ld(qb.p[1], im(d, i, j, k));
+    ub[iu(d, i, j, k)] += (T)a;
   }
-  det_end<T>();
+  if (i < nx && k < nz) {
+    double Fb = 0.0;
+    const T sg = A.sign(A.V(i, j, k));
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      const double gl = j > 0 ? A.gy(A.o[f], i, j - 1, k) : 0.0, gr = j < ny ? A.gy(A.o[f], i, j, k) : 0.0;
+      double val = 0.0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const T x = A.at(f, i, wrap_or_clamp(j - 2 + q, ny, d.py), k);
+        val += (double)AdvBar<T>::weight(q, sg) * (double)x;
+        if (q == 1) Fb -= gl * (double)x;
+        if (q == 2) Fb += gr * (double)x;
+      }
+      Fb += (gl - gr) * val;
+    }
+    double a = Fb / (double)ld(c.mv, h_v(d, i, j));
+    if (j > 0) a += 0.5 * (double)ld(qb.p[2], im(d, i, j - 1, k));
+    if (j < ny) a += 0.5 * (double)ld(qb.p[2], im(d, i, j, k));
+    vb[iv(d, i, j, k)] += (T)a;
+  }
+  if (i < nx && j < ny) {
+    double Fb = 0.0;
+    const T sg = A.sign(A.W(i, j, k));
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      const double gl = k > 0 ? A.gz(A.o[f], i, j, k - 1) : 0.0, gr = k < nz ? A.gz(A.o[f], i, j, k) : 0.0;
+      double val = 0.0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const T x = A.at(f, i, j, min(max(k - 2 + q, 0), nz - 1));
+        val += (double)AdvBar<T>::weight(q, sg) * (double)x;
+        if (q == 1) Fb -= gl * (double)x;
+        if (q == 2) Fb += gr * (double)x;
+      }
+      Fb += (gl - gr) * val;
+    }
+    const int p = iw(d, i, j, k);
+    eb[p] += (T)(Fb * (double)ld(c.dzw, p));
+    double a = 0.0;
+    if (k > 0) a += 0.5 * (double)ld(qb.p[3], im(d, i, j, k - 1));
+    if (k < nz) a += 0.5 * (double)ld(qb.p[3], im(d, i, j, k));
+    wb[p] += (T)a;
+  }
 }
 
 }  // namespace
@@ -1573,45 +1707,26 @@ void launch_split_diag_vjp(const Dims& d, const Coef<T>& c, T* wb, T* eb, T* ub,
 }
 
 template <typename T>
-void launch_split_substep_vjp(const Dims& d, const Coef<T>& c, const SplitBar<T>& b, void* det_scratch,
-                              cudaStream_t st) {
-  dim3 blk(32, 4, 2);
-  const unsigned fu = (unsigned)field_size(d, LOC_U), fv = (unsigned)field_size(d, LOC_V);
-  const unsigned fw = (unsigned)field_size(d, LOC_W), fm = (unsigned)field_size(d, LOC_M);
-  {  // corrector^T
-    T* dst[14] = {b.upp, b.vpp, b.sfu, b.sfv, b.gx0, b.gy0, b.ppp, b.uh, b.vh, b.uc, b.vc, b.wc, b.u0, b.v0};
-    const unsigned len[14] = {fu, fv, fu, fv, fu, fv, fm, fu, fv, fu, fv, fw, fu, fv};
-    det_run<T>(det_make<T>(det_scratch, dst, len, 14), [&](const DetSink<T>& s) {
-      split_correct_vjp_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, c, b, s);
-    }, st);
-  }
+void launch_split_substep_vjp(const Dims& d, const Coef<T>& c, const SplitBar<T>& b, cudaStream_t st) {
+  const dim3 blk(32, 8, 1);
+  const dim3 grd((d.nx + 32) / 32, (d.ny + 8) / 8, (d.nz + VJP_KC) / VJP_KC);
+  split_faces_vjp_kernel<T, false><<<grd, blk, 0, st>>>(d, c, b);  // corrector^T
   {  // column^T, with the forward's alpha dtau products
     const double ad = (double)b.alpha * (double)b.dtau;
     const T a2cp = (T)(ad * ad * c.s.cp), adcp = (T)(ad * c.s.cp);
-    T* dst[5] = {b.ppp, b.uh, b.vh, b.sfw, b.sfp};
-    const unsigned len[5] = {fm, fu, fv, fw, fm};
     constexpr int PT = 256, PC = 32;
     const size_t smem = (size_t)(4 * d.nz) * PC * sizeof(T);
     if (smem <= 200 * 1024) {  // tiles of 32 columns; the one-thread-per-column march beyond
       static SmemLimit attr_bytes;  // per instantiation
       ensure_smem_limit((const void*)split_column_vjp_tile_kernel<T, PT, PC>, attr_bytes, smem);
-      det_run<T>(det_make<T>(det_scratch, dst, len, 5), [&](const DetSink<T>& s) {
-        split_column_vjp_tile_kernel<T, PT, PC>
-            <<<dim3((d.nx + PC - 1) / PC, d.ny), PT, smem, st>>>(d, c, b, a2cp, adcp, s);
-      }, st);
+      split_column_vjp_tile_kernel<T, PT, PC>
+          <<<dim3((d.nx + PC - 1) / PC, d.ny), PT, smem, st>>>(d, c, b, a2cp, adcp);
     } else {
-      det_run<T>(det_make<T>(det_scratch, dst, len, 5), [&](const DetSink<T>& s) {
-        split_column_vjp_kernel<T><<<dim3((d.nx + 127) / 128, d.ny), 128, 0, st>>>(d, c, b, a2cp, adcp, s);
-      }, st);
+      split_column_vjp_kernel<T><<<dim3((d.nx + 127) / 128, d.ny), 128, 0, st>>>(d, c, b, a2cp, adcp);
     }
+    split_column_faces_vjp_kernel<T><<<grd, blk, 0, st>>>(d, c, b);
   }
-  {  // predictor^T
-    T* dst[9] = {b.upp, b.vpp, b.sfu, b.sfv, b.ppp, b.uc, b.vc, b.u0, b.v0};
-    const unsigned len[9] = {fu, fv, fu, fv, fm, fu, fv, fu, fv};
-    det_run<T>(det_make<T>(det_scratch, dst, len, 9), [&](const DetSink<T>& s) {
-      split_predict_vjp_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz, blk), blk, 0, st>>>(d, c, b, s);
-    }, st);
-  }
+  split_faces_vjp_kernel<T, true><<<grd, blk, 0, st>>>(d, c, b);  // predictor^T
 }
 
 template <typename T>
@@ -1658,23 +1773,19 @@ void launch_split_slow_vjp(const Dims& d, const T* const* sf5, T* const* tend6, 
 template <typename T>
 void launch_split_adv_vjp(const Dims& d, const Coef<T>& c, const T* u, const T* v, const T* w, const T* eta,
                           const T* th, T eps_l, const T* const* adv4, T* ub, T* vb, T* wb, T* eb, T* thb,
-                          void* det_scratch, cudaStream_t st) {
-  dim3 blk(32, 4, 2);
-  PtrTable<T> a{};
-  for (int q = 0; q < 4; ++q) a.p[q] = const_cast<T*>(adv4[q]);
-  const unsigned fw = (unsigned)field_size(d, LOC_W), fm = (unsigned)field_size(d, LOC_M);
-  T* dst[5] = {ub, vb, wb, eb, thb};
-  const unsigned len[5] = {(unsigned)field_size(d, LOC_U), (unsigned)field_size(d, LOC_V), fw, fw, fm};
-  det_run<T>(det_make<T>(det_scratch, dst, len, 5), [&](const DetSink<T>& s) {
-    split_adv_vjp_kernel<T><<<box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st>>>(d, c, u, v, w, eta, th, eps_l, a, ub,
-                                                                            vb, wb, eb, thb, s);
-  }, st);
+                          T* const* tmp4, cudaStream_t st) {
+  const dim3 blk(32, 4, 2);
+  AdvIn<T> in{u, v, w, eta, th, {adv4[0], adv4[1], adv4[2], adv4[3]}, eps_l};
+  PtrTable<T> qb{};
+  for (int q = 0; q < 4; ++q) qb.p[q] = tmp4[q];
+  split_adv_vjp_mass_kernel<T><<<box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st>>>(d, c, in, qb, thb);
+  split_adv_vjp_faces_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, c, in, qb, ub, vb, wb,
+                                                                                           eb);
 }
 
 #define SISL_INST_SPLIT_VJP(T)                                                                                 \
   template void launch_split_diag_vjp<T>(const Dims&, const Coef<T>&, T*, T*, T*, T*, void*, cudaStream_t);    \
-  template void launch_split_substep_vjp<T>(const Dims&, const Coef<T>&, const SplitBar<T>&, void*,            \
-                                            cudaStream_t);                                                     \
+  template void launch_split_substep_vjp<T>(const Dims&, const Coef<T>&, const SplitBar<T>&, cudaStream_t);    \
   template void launch_split_end_vjp<T>(const Dims&, const T* const*, T* const*, T*, T*, T*, T*, T*, T*, T,   \
                                         cudaStream_t);                                                         \
   template void launch_split_init_vjp<T>(const Dims&, const T*, const T*, const T*, const T*, T* const*,       \
@@ -1682,7 +1793,7 @@ void launch_split_adv_vjp(const Dims& d, const Coef<T>& c, const T* u, const T* 
   template void launch_split_slow_vjp<T>(const Dims&, const T* const*, T* const*, T* const*, void*,            \
                                          cudaStream_t);                                                        \
   template void launch_split_adv_vjp<T>(const Dims&, const Coef<T>&, const T*, const T*, const T*, const T*,   \
-                                        const T*, T, const T* const*, T*, T*, T*, T*, T*, void*, cudaStream_t);
+                                        const T*, T, const T* const*, T*, T*, T*, T*, T*, T* const*, cudaStream_t);
 SISL_INST_SPLIT_VJP(float)
 SISL_INST_SPLIT_VJP(double)
 #undef SISL_INST_SPLIT_VJP
