@@ -54,14 +54,16 @@ __global__ void split_diag_kernel(Dims d, Coef<T> c, const T* __restrict__ u, co
 }
 
 
-// flux * q_face of the 3rd-order upwind-biased face value (steppers.py:1312-1360)
+// 3rd-order upwind-biased face value (steppers.py:1312-1360), sg the sign of the flux through the face
 template <typename T>
-__device__ __forceinline__ T upwind_flux(T qm2, T qm1, T q0, T qp1, T F, T eps_l) {
+__device__ __forceinline__ T upwind_value(T qm2, T qm1, T q0, T qp1, T sg) {
   const T q4 = T(7.0 / 12.0) * (q0 + qm1) - T(1.0 / 12.0) * (qp1 + qm2);
   const T qb = T(1.0 / 12.0) * ((qp1 - qm2) - T(3) * (q0 - qm1));
-  const T cf = (fabs(F) < eps_l) ? T(0) : F;
-  const T sg = (cf > T(0)) ? T(1) : ((cf < T(0)) ? T(-1) : T(0));
-  return F * (q4 + sg * qb);
+  return q4 + sg * qb;
+}
+template <typename T>
+__device__ __forceinline__ T flux_sign(T F, T eps_l) {
+  return fabs(F) < eps_l ? T(0) : (F > T(0) ? T(1) : (F < T(0) ? T(-1) : T(0)));
 }
 
 // the four advected fields at mass point (i, j, k): th', u_m, v_m, w_m
@@ -82,73 +84,100 @@ struct AdvFields {
   }
 };
 
-// Blocks of AX x AY mass points of one level.  For each of the four fields
-// the block forms the field's values at the (AX + 4) x (AY + 4) cells of its
-// x and y stencils once into shared memory (indices wrapped or clamped as
-// the point form wraps them), instead of five times per point and axis; the
-// z stencil is read per point.
+// Blocks of AX x AY columns walk `chunk` levels.  Per level the block forms
+// the four fields' values at the (AX + 4) x (AY + 4) cells of its x and y
+// stencils once in shared memory (indices wrapped or clamped as the point
+// form wraps them; two buffers, one barrier a level); a thread keeps the
+// five levels of its z stencil in registers and the face value below its cell
+// from the level before.
+//
+// The flux-form difference less q times the velocity's divergence is taken as
+// F1 (q1 - q) - F0 (q0 - q) of the two faces: the fluxes' signs and factors are
+// formed once for the four fields, there is no division per field and axis,
+// and the two large terms of the direct form no longer cancel.  Bound by the
+// issue of arithmetic and shared loads: 256x256x64 float32 598 us a call with
+// a block per level, every face twice and three divisions per field.
 constexpr int AX = 32, AY = 8;
 
 template <typename T>
-__global__ void __launch_bounds__(AX * AY) split_adv_kernel(Dims d, Coef<T> c, const T* __restrict__ u,
-                                                            const T* __restrict__ v, const T* __restrict__ w,
-                                                            const T* __restrict__ eta, const T* __restrict__ th,
-                                                            T eps_l, PtrTable<T> out) {
-  __shared__ T Qt[AY + 4][AX + 4];
-  const int i0 = blockIdx.x * AX, j0 = blockIdx.y * AY, k = blockIdx.z;
+__global__ void __launch_bounds__(AX * AY, sizeof(T) == 4 ? 3 : 2) split_adv_kernel(
+    Dims d, Coef<T> c, const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ w,
+    const T* __restrict__ eta, const T* __restrict__ th, T eps_l, PtrTable<T> out, int chunk) {
+  __shared__ T Qt[2][4][AY + 4][AX + 4];
+  const int i0 = blockIdx.x * AX, j0 = blockIdx.y * AY;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  const int i = i0 + tx, j = j0 + ty;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  const bool live = i < nx && j < ny;
+  const bool live = i0 + tx < nx && j0 + ty < ny;
+  const int i = min(i0 + tx, nx - 1), j = min(j0 + ty, ny - 1);
+  const int k0 = blockIdx.z * chunk, k1 = min(k0 + chunk, nz);
   const AdvFields<T> F{d, u, v, w, th};
-  const T dx = (T)d.dx, dy = (T)d.dy;
-  T mm = T(0), U0 = T(0), U1 = T(0), V0 = T(0), V1 = T(0), W0 = T(0), W1 = T(0), zfac = T(0);
-  T dU = T(0), dV = T(0), dW = T(0);
-  int zk[5];
-  if (live) {
-    mm = ld(c.mm, h_m(d, i, j));
-    // U = u / m_u, V = v / m_v, W = eta dz_w at the cell's faces (steppers.py:1397-1399)
-    U0 = ld(u, iu(d, i, j, k)) / ld(c.mu, h_u(d, i, j));
-    U1 = ld(u, iu(d, i + 1, j, k)) / ld(c.mu, h_u(d, i + 1, j));
-    V0 = ld(v, iv(d, i, j, k)) / ld(c.mv, h_v(d, i, j));
-    V1 = ld(v, iv(d, i, j + 1, k)) / ld(c.mv, h_v(d, i, j + 1));
-    W0 = ld(eta, iw(d, i, j, k)) * ld(c.dzw, iw(d, i, j, k));
-    W1 = ld(eta, iw(d, i, j, k + 1)) * ld(c.dzw, iw(d, i, j, k + 1));
-    const T dzm = ld(c.dzm, im(d, i, j, k));
-    zfac = (T)d.dz / dzm;
-    dU = (U1 - U0) / dx * mm;
-    dV = (V1 - V0) / dy * mm;
-    dW = (W1 - W0) / (T)d.dz * zfac;
-  }
-#pragma unroll
-  for (int o = 0; o < 5; ++o) zk[o] = min(max(k - 2 + o, 0), nz - 1);
   const int t = tx + AX * ty;
-#pragma unroll 1
-  for (int f = 0; f < 4; ++f) {
-    for (int q = t; q < (AX + 4) * (AY + 4); q += AX * AY) {
-      const int x = q % (AX + 4), y = q / (AX + 4);
-      Qt[y][x] = F.at(f, wrap_or_clamp(i0 - 2 + x, nx, d.px), wrap_or_clamp(j0 - 2 + y, ny, d.py), k);
+  constexpr int CELLS = (AX + 4) * (AY + 4), FILL = (CELLS + AX * AY - 1) / (AX * AY);
+  int ci[FILL], cj[FILL];
+#pragma unroll
+  for (int n = 0; n < FILL; ++n) {
+    const int q = t + n * AX * AY;
+    ci[n] = wrap_or_clamp(i0 - 2 + q % (AX + 4), nx, d.px);
+    cj[n] = wrap_or_clamp(j0 - 2 + q / (AX + 4), ny, d.py);
+  }
+  const T mm = ld(c.mm, h_m(d, i, j)), m2 = mm * mm;
+  const T sx = mm / (T)d.dx, sy = mm / (T)d.dy;
+  const T mu0 = ld(c.mu, h_u(d, i, j)), mu1 = ld(c.mu, h_u(d, i + 1, j));
+  const T mv0 = ld(c.mv, h_v(d, i, j)), mv1 = ld(c.mv, h_v(d, i, j + 1));
+  auto zat = [&](int f, int k) { return F.at(f, i, j, min(max(k, 0), nz - 1)); };
+  T qz[4][5], gb[4];  // levels k - 2 .. k + 2; face value below the cell
+  T W0 = ld(eta, iw(d, i, j, k0)) * ld(c.dzw, iw(d, i, j, k0));
+  {
+    const T sg = flux_sign(W0, eps_l);
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+#pragma unroll
+      for (int o = 0; o < 4; ++o) qz[f][o + 1] = zat(f, k0 - 2 + o);
+      gb[f] = upwind_value(qz[f][1], qz[f][2], qz[f][3], qz[f][4], sg);
     }
-    __syncthreads();
-    if (live) {
-      T qx[5], qy[5], qz[5];
+  }
+#pragma unroll 1
+  for (int k = k0, s = 0; k < k1; ++k, s ^= 1) {
+#pragma unroll
+    for (int n = 0; n < FILL; ++n) {
+      const int q = t + n * AX * AY;
+      if (q < CELLS) {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) (&Qt[s][f][0][0])[q] = F.at(f, ci[n], cj[n], k);
+      }
+    }
+    const T U0 = ld(u, iu(d, i, j, k)) / mu0, U1 = ld(u, iu(d, i + 1, j, k)) / mu1;
+    const T V0 = ld(v, iv(d, i, j, k)) / mv0, V1 = ld(v, iv(d, i, j + 1, k)) / mv1;
+    const T W1 = ld(eta, iw(d, i, j, k + 1)) * ld(c.dzw, iw(d, i, j, k + 1));
+    const T sz = T(1) / ld(c.dzm, im(d, i, j, k));
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+#pragma unroll
+      for (int o = 0; o < 4; ++o) qz[f][o] = qz[f][o + 1];
+      qz[f][4] = zat(f, k + 2);
+    }
+    const T su0 = flux_sign(U0, eps_l), su1 = flux_sign(U1, eps_l), sv0 = flux_sign(V0, eps_l),
+            sv1 = flux_sign(V1, eps_l), sw1 = flux_sign(W1, eps_l);
+    __syncthreads();  // the other buffer was last read before the previous level's barrier
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      T qx[5], qy[5];
 #pragma unroll
       for (int o = 0; o < 5; ++o) {
-        qx[o] = Qt[ty + 2][tx + o];
-        qy[o] = Qt[ty + o][tx + 2];
-        qz[o] = (o == 2) ? Qt[ty + 2][tx + 2] : F.at(f, i, j, zk[o]);
+        qx[o] = Qt[s][f][ty + 2][tx + o];
+        qy[o] = Qt[s][f][ty + o][tx + 2];
       }
-      const T q = qx[2];
-      // faces i (q at i-2..i+1) and i+1 (q at i-1..i+2)
-      const T ax = (upwind_flux(qx[1], qx[2], qx[3], qx[4], U1, eps_l) -
-                    upwind_flux(qx[0], qx[1], qx[2], qx[3], U0, eps_l)) / dx * mm;
-      const T ay = (upwind_flux(qy[1], qy[2], qy[3], qy[4], V1, eps_l) -
-                    upwind_flux(qy[0], qy[1], qy[2], qy[3], V0, eps_l)) / dy * mm;
-      const T az = (upwind_flux(qz[1], qz[2], qz[3], qz[4], W1, eps_l) -
-                    upwind_flux(qz[0], qz[1], qz[2], qz[3], W0, eps_l)) / (T)d.dz * zfac;
-      out.p[f][im(d, i, j, k)] = -(mm * mm) * (ax - q * dU + ay - q * dV) - (az - q * dW);
+      const T q = qz[f][2];
+      const T ax = U1 * (upwind_value(qx[1], qx[2], qx[3], qx[4], su1) - q) -
+                   U0 * (upwind_value(qx[0], qx[1], qx[2], qx[3], su0) - q);
+      const T ay = V1 * (upwind_value(qy[1], qy[2], qy[3], qy[4], sv1) - q) -
+                   V0 * (upwind_value(qy[0], qy[1], qy[2], qy[3], sv0) - q);
+      const T gt = upwind_value(qz[f][1], qz[f][2], qz[f][3], qz[f][4], sw1);
+      const T az = W1 * (gt - q) - W0 * (gb[f] - q);
+      gb[f] = gt;
+      if (live) out.p[f][im(d, i, j, k)] = -m2 * (ax * sx + ay * sy) - az * sz;
     }
-    __syncthreads();  // the next field refills the tile
+    W0 = W1;
   }
 }
 
@@ -586,7 +615,11 @@ void launch_split_adv(const Dims& d, const Coef<T>& c, const T* u, const T* v, c
   const dim3 blk(AX, AY, 1);
   PtrTable<T> o{};
   for (int q = 0; q < 4; ++q) o.p[q] = adv4[q];
-  split_adv_kernel<T><<<box(d.nx, d.ny, d.nz, blk), blk, 0, st>>>(d, c, u, v, w, eta, th, eps_l, o);
+  // 16 levels a block where that leaves two blocks an SM, else 8: a chunk's start reads four levels more
+  const int tiles = ((d.nx + AX - 1) / AX) * ((d.ny + AY - 1) / AY);
+  const int chunk = tiles * ((d.nz + 15) / 16) >= 2 * 148 ? 16 : 8;
+  split_adv_kernel<T><<<dim3((d.nx + AX - 1) / AX, (d.ny + AY - 1) / AY, (d.nz + chunk - 1) / chunk), blk, 0, st>>>(
+      d, c, u, v, w, eta, th, eps_l, o, chunk);
 }
 
 template <typename T>
