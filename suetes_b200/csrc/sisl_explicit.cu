@@ -41,57 +41,116 @@ __global__ void hyper_src_kernel(Dims d, const T* __restrict__ u, const T* __res
   out.p[3][p] = ld(th, p);
 }
 
-// The Cartesian horizontal Laplacian (diffusion.py:93-129) in two passes:
-// the terrain-following gradients at every u face and v face once
-// (hyper_grad_kernel, HLap::Gx/Gy), then the divergence of the stored
-// gradients (hyper_div_kernel), instead of re-forming twelve face
-// gradients per point (the one-pass form this replaced computed the same
-// values in registers; the fields agree bitwise).
-template <typename T>
-__global__ void hyper_grad_kernel(Dims d, Coef<T> c, PtrTable<T> src, PtrTable<T> gxy) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int kz = blockIdx.z * blockDim.z + threadIdx.z;
-  const int f = kz / d.nz, k = kz % d.nz;
-  if (i > d.nx || j > d.ny || f >= 4) return;
-  HLap<T> L{d, c, src.p[f]};
-  if (j < d.ny) gxy.p[f][iu(d, i, j, k)] = L.Gx(i, j, k);
-  if (i < d.nx) gxy.p[4 + f][iv(d, i, j, k)] = L.Gy(i, j, k);
-}
-
-template <typename T>
-__global__ void hyper_div_kernel(Dims d, Coef<T> c, PtrTable<T> gxy, PtrTable<T> dst, T scale) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int kz = blockIdx.z * blockDim.z + threadIdx.z;
-  const int f = kz / d.nz, k = kz % d.nz;
-  if (i >= d.nx || j >= d.ny || f >= 4) return;
-  const int nz = d.nz;
-  const T* __restrict__ gx = gxy.p[f];
-  const T* __restrict__ gy = gxy.p[4 + f];
-  const int kl = max(k - 1, 0), kh = min(k + 1, nz - 1);
-  const int lv[3] = {kl, k, kh};
-  T gxm[3], gym[3], gx0 = T(0), gx1 = T(0), gy0 = T(0), gy1 = T(0);
+// The Cartesian horizontal Laplacian (diffusion.py:93-129) of NF fields:
+// blocks of LX x LY columns walk HL_KC levels.  Per level every cell of the
+// tile and its rim is read once, with the level above already in hand: its value and
+// mass-level vertical derivative (HLap::dzm) go to shared memory (two buffers,
+// one barrier a level), and a thread forms the terrain-following gradients
+// (HLap::Gx, Gy) at its four faces from there, one level ahead of the
+// divergence.  As two passes through stored face gradients (eight more
+// fields, read back at three levels) it was bound by L1 and L2 traffic:
+// 256x256x64 float32, the four fields: 452 us; a thread per column and field,
+// reading its four neighbours itself: 361 us.
+constexpr int LX = 32, LY = 8, HL_KC = 16;
+template <typename T, int NF>
+__global__ void __launch_bounds__(LX * LY, 2) hyper_lap_kernel(Dims d, Coef<T> c, PtrTable<T> src, PtrTable<T> dst,
+                                                               T scale) {
+  constexpr int TX = LX + 2, TY = LY + 2, CELLS = TX * TY, SLOTS = (CELLS + LX * LY - 1) / (LX * LY);
+  __shared__ T sF[2][NF][CELLS], sD[2][NF][CELLS];
+  const int nx = d.nx, ny = d.ny, nz = d.nz, pm = nx * ny;
+  const int i0 = blockIdx.x * LX, j0 = blockIdx.y * LY;
+  const int tx = threadIdx.x, ty = threadIdx.y, t = tx + LX * ty;
+  const bool live = i0 + tx < nx && j0 + ty < ny;
+  const int i = min(i0 + tx, nx - 1), j = min(j0 + ty, ny - 1);
+  const int f0 = (blockIdx.z % (4 / NF)) * NF, k0 = (blockIdx.z / (4 / NF)) * HL_KC, k1 = min(k0 + HL_KC, nz);
+  const int qs = max(k0 - 1, 0), qe = min(k1, nz - 1);
+  // this thread's cells of the tile: value at level l, difference to the level below, derivative at w level l
+  int col[SLOTS];
+  T Fc[SLOTS][NF], df[SLOTS][NF], zl[SLOTS][NF];
 #pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    const T a0 = ld(gx, iu(d, i, j, lv[q])), a1 = ld(gx, iu(d, i + 1, j, lv[q]));
-    const T b0 = ld(gy, iv(d, i, j, lv[q])), b1 = ld(gy, iv(d, i, j + 1, lv[q]));
-    gxm[q] = T(0.5) * (a0 + a1);
-    gym[q] = T(0.5) * (b0 + b1);
-    if (q == 1) { gx0 = a0; gx1 = a1; gy0 = b0; gy1 = b1; }
+  for (int n = 0; n < SLOTS; ++n) {
+    const int q = min(t + n * LX * LY, CELLS - 1);
+    col[n] = wrap_or_clamp(i0 - 1 + q % TX, nx, d.px) + nx * wrap_or_clamp(j0 - 1 + q / TX, ny, d.py);
+    const T iz = ld(c.idzw, col[n] + qs * pm);
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      const T* __restrict__ q_ = src.p[f0 + f];
+      Fc[n][f] = ld(q_, col[n] + qs * pm);
+      const T other = ld(q_, col[n] + (qs > 0 ? qs - 1 : 1) * pm);
+      df[n][f] = qs > 0 ? Fc[n][f] - other : other - Fc[n][f];  // the ground repeats the lowest pair
+      zl[n][f] = df[n][f] * iz;
+    }
   }
-  auto lvl = [&](int kk) { return kk == kl ? 0 : (kk == k ? 1 : 2); };
-  int al, ar, bl, br;
-  level_pair(k, nz, al, ar);
-  level_pair(k + 1, nz, bl, br);
-  const T iz0 = ld(c.idzw, iw(d, i, j, k)), iz1 = ld(c.idzw, iw(d, i, j, k + 1));
-  const T ex0 = (gxm[lvl(ar)] - gxm[lvl(al)]) * iz0, ex1 = (gxm[lvl(br)] - gxm[lvl(bl)]) * iz1;
-  const T ey0 = (gym[lvl(ar)] - gym[lvl(al)]) * iz0, ey1 = (gym[lvl(br)] - gym[lvl(bl)]) * iz1;
-  const T m = ld(c.mm, h_m(d, i, j));
-  const int p = im(d, i, j, k);
-  const T divx = m * (gx1 - gx0) * (T)(1.0 / d.dx) - ld(c.zxm, p) * T(0.5) * (ex0 + ex1);
-  const T divy = m * (gy1 - gy0) * (T)(1.0 / d.dy) - ld(c.zem, p) * T(0.5) * (ey0 + ey1);
-  dst.p[f][p] = scale * (divx + divy);
+  const T idx = (T)(1.0 / d.dx), idy = (T)(1.0 / d.dy);
+  const T mu0 = ld(c.mu, h_u(d, i, j)), mu1 = ld(c.mu, h_u(d, i + 1, j));
+  const T mv0 = ld(c.mv, h_v(d, i, j)), mv1 = ld(c.mv, h_v(d, i, j + 1)), m = ld(c.mm, h_m(d, i, j));
+  // tile positions of the two cells of each face; an open boundary face repeats its neighbour's pair (face_pair)
+  const int own = (ty + 1) * TX + tx + 1;
+  const int wl = i == 0 && !d.px ? own : own - 1, el = i == nx - 1 && !d.px ? own - 1 : own;
+  const int sl = j == 0 && !d.py ? own : own - TX, nl = j == ny - 1 && !d.py ? own - TX : own;
+  const int h = i + nx * j;
+  T gmx[NF], gmy[NF], dgx[NF], dgy[NF], ex[NF], ey[NF];  // of level l - 1; ex, ey: w level l - 1
+#pragma unroll
+  for (int f = 0; f < NF; ++f) gmx[f] = gmy[f] = dgx[f] = dgy[f] = ex[f] = ey[f] = T(0);
+#pragma unroll 1
+  for (int l = qs, s = 0; l <= qe; ++l, s ^= 1) {
+#pragma unroll
+    for (int n = 0; n < SLOTS; ++n) {
+      const int q = t + n * LX * LY;
+      if (q < CELLS) {
+        const T iz = ld(c.idzw, col[n] + (l + 1) * pm);
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+          const T Fn = ld(src.p[f0 + f], col[n] + min(l + 1, nz - 1) * pm);
+          if (l + 1 < nz) df[n][f] = Fn - Fc[n][f];  // the lid repeats the highest pair
+          const T zh = df[n][f] * iz;
+          sF[s][f][q] = Fc[n][f];
+          sD[s][f][q] = T(0.5) * (zl[n][f] + zh);
+          zl[n][f] = zh;
+          Fc[n][f] = Fn;
+        }
+      }
+    }
+    const int u0 = iu(d, i, j, l), v0 = iv(d, i, j, l);
+    const T zx0 = ld(c.zxu, u0), zx1 = ld(c.zxu, u0 + 1), ze0 = ld(c.zev, v0), ze1 = ld(c.zev, v0 + nx);
+    const T izl = ld(c.idzw, h + l * pm), izt = ld(c.idzw, h + (l + 1) * pm), izg = ld(c.idzw, h);
+    const int p = h + max(l - 1, 0) * pm;
+    const T zxm = ld(c.zxm, p), zem = ld(c.zem, p);
+    __syncthreads();  // the other buffer was last read before the previous level's barrier
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      const T* F = sF[s][f];
+      const T* D = sD[s][f];
+      auto face = [&](int a, int b, T id, T mf, T z) {
+        const T g = (F[b] - F[a]) * id * mf;
+        return g - z * T(0.5) * (D[a] + D[b]);
+      };
+      const T gx0 = face(wl, wl + 1, idx, mu0, zx0), gx1 = face(el, el + 1, idx, mu1, zx1);
+      const T gy0 = face(sl, sl + TX, idy, mv0, ze0), gy1 = face(nl, nl + TX, idy, mv1, ze1);
+      const T ax = T(0.5) * (gx0 + gx1), ay = T(0.5) * (gy0 + gy1);
+      const T lx = ax - gmx[f], ly = ay - gmy[f];
+      auto put = [&](int p_, T zx, T ze, T ex1, T ey1) {
+        const T divx = m * dgx[f] * idx - zx * T(0.5) * (ex[f] + ex1);
+        const T divy = m * dgy[f] * idy - ze * T(0.5) * (ey[f] + ey1);
+        if (live) dst.p[f0 + f][p_] = scale * (divx + divy);
+      };
+      if (l > qs) {  // w level l, and with it mass level l - 1
+        const T ex1 = lx * izl, ey1 = ly * izl;
+        if (l == 1) {  // the ground repeats the lowest pair
+          ex[f] = lx * izg;
+          ey[f] = ly * izg;
+        }
+        if (l > k0) put(p, zxm, zem, ex1, ey1);
+        ex[f] = ex1;
+        ey[f] = ey1;
+      }
+      gmx[f] = ax;
+      gmy[f] = ay;
+      dgx[f] = gx1 - gx0;
+      dgy[f] = gy1 - gy0;
+      if (l + 1 == nz) put(h + l * pm, ld(c.zxm, h + l * pm), ld(c.zem, h + l * pm), lx * izt, ly * izt);
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -345,14 +404,14 @@ __global__ void __launch_bounds__(256) finalize_kernel(Dims d, Coef<T> c, Finali
 
 template <typename T>
 void launch_hyper(const Dims& d, const Coef<T>& c, const T* u, const T* v, const T* w, const T* th,
-                  PtrTable<T> tmp4, PtrTable<T> out4, PtrTable<T> gxy8, cudaStream_t st) {
+                  PtrTable<T> tmp4, PtrTable<T> out4, cudaStream_t st) {
   dim3 blk(32, 4, 2);
   hyper_src_kernel<T><<<box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st>>>(d, u, v, w, th, out4);
-  const dim3 gg = box_grid(d.nx + 1, d.ny + 1, 4 * d.nz, blk), gd = box_grid(d.nx, d.ny, 4 * d.nz, blk);
-  hyper_grad_kernel<T><<<gg, blk, 0, st>>>(d, c, out4, gxy8);
-  hyper_div_kernel<T><<<gd, blk, 0, st>>>(d, c, gxy8, tmp4, T(1));
-  hyper_grad_kernel<T><<<gg, blk, 0, st>>>(d, c, tmp4, gxy8);
-  hyper_div_kernel<T><<<gd, blk, 0, st>>>(d, c, gxy8, out4, (T)(-c.s.nu_h));
+  // float64 takes two fields a block: the state of four would not fit the registers of two resident blocks
+  constexpr int NF = sizeof(T) == 4 ? 4 : 2;
+  const dim3 lb(LX, LY, 1), lg((d.nx + LX - 1) / LX, (d.ny + LY - 1) / LY, (4 / NF) * ((d.nz + HL_KC - 1) / HL_KC));
+  hyper_lap_kernel<T, NF><<<lg, lb, 0, st>>>(d, c, out4, tmp4, T(1));
+  hyper_lap_kernel<T, NF><<<lg, lb, 0, st>>>(d, c, tmp4, out4, (T)(-c.s.nu_h));
 }
 
 template <typename T>
@@ -424,7 +483,7 @@ void launch_finalize(const Dims& d, const Coef<T>& c, const FinalizeArgs<T>& fa,
 
 #define SISL_INST_EX(T)                                                                                        \
   template void launch_hyper<T>(const Dims&, const Coef<T>&, const T*, const T*, const T*, const T*,           \
-                                PtrTable<T>, PtrTable<T>, PtrTable<T>, cudaStream_t);                          \
+                                PtrTable<T>, PtrTable<T>, cudaStream_t);                          \
   template void launch_explicit<T>(const Dims&, const Coef<T>&, const ExplicitIn<T>&, const ExplicitOut<T>&,   \
                                    int, cudaStream_t);                                                         \
   template void launch_corrector_theta<T>(const Dims&, const Coef<T>&, const T*, const T*, const T*, const T*, \
