@@ -88,6 +88,7 @@ __device__ __forceinline__ void at_gzm_block(const Dims& d, const Coef<T>& c, co
 template <typename T>
 __global__ void at_gzm_kernel(Dims d, Coef<T> c, const T* __restrict__ yu, const T* __restrict__ yv, const double* yscale,
                               T* __restrict__ gzm, const int* active) {
+  grid_chain();
   if (active && *active == 0) return;
   at_gzm_block<T>(d, c, yu, yv, yscale, gzm, blockIdx.x, blockIdx.y, blockIdx.z);
 }
@@ -265,6 +266,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) at_main_kernel(Dims d, Coef<T> c, CVec5<T> y, const double* yscale,
                                                       const T* __restrict__ gzm, CVec5<T> b, Vec5<T> out,
                                                       const int* active) {
+  grid_chain();
   if (active && *active == 0) return;
   at_main_block<T>(d, c, y, yscale, gzm, b, out, blockIdx.x, blockIdx.y, blockIdx.z);
 }
@@ -295,6 +297,7 @@ __global__ void __launch_bounds__(256) at_main_kernel(Dims d, Coef<T> c, CVec5<T
 template <typename T, int TPT, int TPC>
 __global__ void __launch_bounds__(TPT) pt_column_kernel(Dims d, Coef<T> c, CVec5<T> y, Vec5<T> out,
                                                         const int* active) {
+  grid_chain();
   if (active && *active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
@@ -497,6 +500,7 @@ __device__ __forceinline__ void pt_column_batched_block(const Dims& d, const Coe
 template <typename T, int TPT, int TPC, int PU>
 __global__ void __launch_bounds__(TPT) pt_column_batched_kernel(Dims d, Coef<T> c, CVec5<T> y, Vec5<T> out,
                                                                 const int* active) {
+  grid_chain();
   if (active && *active == 0) return;
   pt_column_batched_block<T, TPT, TPC, PU>(d, c, y, out, blockIdx.x, blockIdx.y, blockIdx.z);
 }
@@ -544,6 +548,7 @@ __device__ __forceinline__ void pt_uv_block(const Dims& d, const Coef<T>& c, con
 }
 template <typename T>
 __global__ void __launch_bounds__(256) pt_uv_kernel(Dims d, Coef<T> c, CVec5<T> y, Vec5<T> out, const int* active) {
+  grid_chain();
   if (active && *active == 0) return;
   pt_uv_block<T>(d, c, y, out, blockIdx.x, blockIdx.y, blockIdx.z);
 }
@@ -774,6 +779,7 @@ __global__ void __launch_bounds__(256) tricubic_vjp_kernel(int sx, int sy, int s
                                                            const T* __restrict__ cy, const T* __restrict__ cz,
                                                            const T* __restrict__ cot, T* grad, int limiter,
                                                            T scale) {
+  grid_chain();
   tricubic_vjp_point(sx, sy, sz, dx, dy, dz, f, cx, cy, cz, cot, AtomicAcc<T>{grad}, limiter, scale);
 }
 
@@ -785,6 +791,7 @@ __global__ void __launch_bounds__(256) tricubic_vjp_count_kernel(int sx, int sy,
                                                                  const T* __restrict__ cx, const T* __restrict__ cy,
                                                                  const T* __restrict__ cz, const T* __restrict__ cot,
                                                                  T scale, int* cnt, DetHdr* hdr) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -819,6 +826,7 @@ __global__ void __launch_bounds__(256) tricubic_vjp_fixed_kernel(int sx, int sy,
                                                                  const T* __restrict__ cy, const T* __restrict__ cz,
                                                                  const T* __restrict__ cot, unsigned long long* acc,
                                                                  const DetHdr* hdr, int limiter, T scale) {
+  grid_chain();
   if (hdr->max_count == 0) return;  // no cotangent at all
   const FixedAcc<T> a = make_fixed_acc<T>(acc, (size_t)sx * sy * sz, hdr);
   tricubic_vjp_point<T, FixedAcc<T>, REL>(sx, sy, sz, dx, dy, dz, f, cx, cy, cz, cot, a, limiter, scale);
@@ -828,6 +836,7 @@ __global__ void __launch_bounds__(256) tricubic_vjp_fixed_kernel(int sx, int sy,
 template <typename T>
 __global__ void tricubic_vjp_finish_kernel(size_t n, const unsigned long long* __restrict__ acc,
                                            const DetHdr* hdr, T* __restrict__ grad) {
+  grid_chain();
   if (hdr->max_count == 0) return;
   const double inv = ldexp(1.0, -det_exponent(hdr));
   const double finv = sizeof(T) == 8 ? ldexp(1.0, -det_fraction_bits(hdr)) : 0.0;
@@ -845,7 +854,8 @@ template <typename T>
 void launch_tricubic_vjp(int sx, int sy, int sz, int dx, int dy, int dz, const T* field, const T* const* coords3,
                          const T* cot, T* grad, int use_limiter, T scale, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  tricubic_vjp_kernel<T><<<box_grid(dx, dy, dz, blk), blk, 0, st>>>(sx, sy, sz, dx, dy, dz, field, coords3[0],
+  launch_chained(tricubic_vjp_kernel<T>, box_grid(dx, dy, dz, blk), blk, 0, st, sx, sy, sz, dx, dy, dz, field,
+                 coords3[0],
                                                                     coords3[1], coords3[2], cot, grad,
                                                                     use_limiter, scale);
 }
@@ -866,20 +876,23 @@ void launch_tricubic_vjp_det(int sx, int sy, int sz, int dx, int dy, int dz, con
   cudaMemsetAsync(scratch, 0, 256 + sizeof(int) * n, st);  // header and the counts (in acc's memory)
   const dim3 grd = box_grid(dx, dy, dz, blk);
   if (relative)
-    tricubic_vjp_count_kernel<T, 1><<<grd, blk, 0, st>>>(sx, sy, sz, dx, dy, dz, coords3[0], coords3[1],
+    launch_chained(tricubic_vjp_count_kernel<T, 1>, grd, blk, 0, st, sx, sy, sz, dx, dy, dz, coords3[0], coords3[1],
                                                          coords3[2], cot, scale, (int*)acc, hdr);
   else
-    tricubic_vjp_count_kernel<T, 0><<<grd, blk, 0, st>>>(sx, sy, sz, dx, dy, dz, coords3[0], coords3[1],
+    launch_chained(tricubic_vjp_count_kernel<T, 0>, grd, blk, 0, st, sx, sy, sz, dx, dy, dz, coords3[0], coords3[1],
                                                          coords3[2], cot, scale, (int*)acc, hdr);
   cudaMemsetAsync(acc, 0, (sizeof(T) == 8 ? 2 : 1) * sizeof(unsigned long long) * n, st);
   if (relative)
-    tricubic_vjp_fixed_kernel<T, 1><<<grd, blk, 0, st>>>(sx, sy, sz, dx, dy, dz, field, coords3[0], coords3[1],
+    launch_chained(tricubic_vjp_fixed_kernel<T, 1>, grd, blk, 0, st, sx, sy, sz, dx, dy, dz, field, coords3[0],
+                   coords3[1],
                                                          coords3[2], cot, acc, hdr, use_limiter, scale);
   else
-    tricubic_vjp_fixed_kernel<T, 0><<<grd, blk, 0, st>>>(sx, sy, sz, dx, dy, dz, field, coords3[0], coords3[1],
+    launch_chained(tricubic_vjp_fixed_kernel<T, 0>, grd, blk, 0, st, sx, sy, sz, dx, dy, dz, field, coords3[0],
+                   coords3[1],
                                                          coords3[2], cot, acc, hdr, use_limiter, scale);
   const size_t nb = (n + 255) / 256;
-  tricubic_vjp_finish_kernel<T><<<(unsigned)(nb < 148 * 16 ? nb : 148 * 16), 256, 0, st>>>(n, acc, hdr, grad);
+  launch_chained(tricubic_vjp_finish_kernel<T>, (unsigned)(nb < 148 * 16 ? nb : 148 * 16), 256, 0, st, n, acc, hdr,
+                 grad);
 }
 template void launch_tricubic_vjp_det<float>(int, int, int, int, int, int, const float*, const float* const*,
                                              const float*, float*, int, float, void*, int, cudaStream_t);
@@ -955,6 +968,7 @@ __device__ __forceinline__ void pt_march_block(const Dims& d, const Coef<T>& c, 
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT) pt_march_kernel(Dims d, Coef<T> c, CVec5<T> y, Vec5<T> out,
                                                       const int* active) {
+  grid_chain();
   if (active && *active == 0) return;
   pt_march_block<T, NT>(d, c, y, out, blockIdx.x, blockIdx.y, blockIdx.z);
 }
@@ -982,6 +996,7 @@ __device__ __forceinline__ void group_box(int t, int ex, int ey, int& bx, int& b
 template <typename T, typename U>
 __global__ void __launch_bounds__(256) group_at_kernel(GroupMember<T>* mem, const int* __restrict__ first, int M,
                                                        int stage, int mode, int j) {
+  grid_chain();
   const int b = blockIdx.x;
   const int mi = group_find(first, M, b);
   const GroupMember<T>& g = mem[mi];
@@ -1024,6 +1039,7 @@ __global__ void __launch_bounds__(256) group_at_kernel(GroupMember<T>* mem, cons
 template <typename T>
 __global__ void __launch_bounds__(256) group_pt_kernel(GroupMember<T>* mem, const int* __restrict__ first, int M,
                                                        int stage, int mode, int tv, int gated) {
+  grid_chain();
   const int b = blockIdx.x;
   const int mi = group_find(first, M, b);
   const GroupMember<T>& g = mem[mi];
@@ -1065,9 +1081,11 @@ void grp_matvec_t(const GroupLaunch<T>& g, int mode, int j, cudaStream_t st) {
     const int tb = stage ? GT_ATM : GT_ATG;
     if (mode == 2) {
       if constexpr (sizeof(T) == 4)
-        group_at_kernel<T, double><<<g.blocks(tb), dim3(32, 4, 2), 0, st>>>(g.mem, g.row(tb), g.M, stage, 2, 0);
+        launch_chained(group_at_kernel<T, double>, g.blocks(tb), dim3(32, 4, 2), 0, st, g.mem, g.row(tb), g.M, stage,
+                       2, 0);
     } else {
-      group_at_kernel<T, T><<<g.blocks(tb), dim3(32, 4, 2), 0, st>>>(g.mem, g.row(tb), g.M, stage, mode, j);
+      launch_chained(group_at_kernel<T, T>, g.blocks(tb), dim3(32, 4, 2), 0, st, g.mem, g.row(tb), g.M, stage, mode,
+                     j);
     }
   }
 }
@@ -1079,8 +1097,9 @@ void grp_precond_t(const GroupLaunch<T>& g, int mode, int t, int gated, cudaStre
   const size_t smem = (size_t)(4 * nz_max) * 32 * sizeof(T);
   static SmemLimit attr_bytes;
   ensure_smem_limit((const void*)group_pt_kernel<T>, attr_bytes, smem);
-  group_pt_kernel<T><<<g.blocks(GT_PTM), 256, smem, st>>>(g.mem, g.row(GT_PTM), g.M, 0, mode, t, gated);
-  group_pt_kernel<T><<<g.blocks(GT_PTU), dim3(32, 4, 2), 0, st>>>(g.mem, g.row(GT_PTU), g.M, 1, mode, t, gated);
+  launch_chained(group_pt_kernel<T>, g.blocks(GT_PTM), 256, smem, st, g.mem, g.row(GT_PTM), g.M, 0, mode, t, gated);
+  launch_chained(group_pt_kernel<T>, g.blocks(GT_PTU), dim3(32, 4, 2), 0, st, g.mem, g.row(GT_PTU), g.M, 1, mode, t,
+                 gated);
 }
 
 template void grp_matvec_t<float>(const GroupLaunch<float>&, int, int, cudaStream_t);
@@ -1094,7 +1113,7 @@ void launch_pt_march(const Dims& d, const Coef<T>& c, CVec5<T> y, Vec5<T> out, c
   const size_t smem = (size_t)d.nz * NT * sizeof(T);
   static SmemLimit attr_bytes;  // per instantiation
   ensure_smem_limit((const void*)pt_march_kernel<T, NT>, attr_bytes, smem);
-  pt_march_kernel<T, NT><<<dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st>>>(d, c, y, out, active);
+  launch_chained(pt_march_kernel<T, NT>, dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st, d, c, y, out, active);
 }
 
 template <typename T, int TPT, int TPC>
@@ -1103,7 +1122,8 @@ void launch_pt_column(const Dims& d, const Coef<T>& c, CVec5<T> y, Vec5<T> out, 
   const size_t smem = (size_t)(4 * d.nz) * TPC * sizeof(T);
   static SmemLimit attr_bytes;  // per instantiation
   ensure_smem_limit((const void*)pt_column_kernel<T, TPT, TPC>, attr_bytes, smem);
-  pt_column_kernel<T, TPT, TPC><<<dim3((d.nx + TPC - 1) / TPC, d.ny), TPT, smem, st>>>(d, c, y, out, active);
+  launch_chained(pt_column_kernel<T, TPT, TPC>, dim3((d.nx + TPC - 1) / TPC, d.ny), TPT, smem, st, d, c, y, out,
+                 active);
 }
 
 template <typename T, int TPT, int TPC, int PU>
@@ -1112,8 +1132,8 @@ void launch_pt_column_batched(const Dims& d, const Coef<T>& c, CVec5<T> y, Vec5<
   const size_t smem = (size_t)(4 * d.nz) * TPC * sizeof(T);
   static SmemLimit attr_bytes;  // per instantiation
   ensure_smem_limit((const void*)pt_column_batched_kernel<T, TPT, TPC, PU>, attr_bytes, smem);
-  pt_column_batched_kernel<T, TPT, TPC, PU>
-      <<<dim3((d.nx + TPC - 1) / TPC, d.ny), TPT, smem, st>>>(d, c, y, out, active);
+  launch_chained(pt_column_batched_kernel<T, TPT, TPC, PU>, dim3((d.nx + TPC - 1) / TPC, d.ny), TPT, smem, st, d, c,
+                 y, out, active);
 }
 
 template <typename T>
@@ -1129,7 +1149,7 @@ void launch_precond_t(const Dims& d, const Coef<T>& c, CVec5<T> y, Vec5<T> out, 
     default: launch_pt_column<T, 256, 32>(d, c, y, out, active, st); break;
   }
   const dim3 blk = stencil_block(d.tune_mvt);
-  pt_uv_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz, blk), blk, 0, st>>>(d, c, y, out, active);
+  launch_chained(pt_uv_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz, blk), blk, 0, st, d, c, y, out, active);
 }
 
 template void launch_precond_t<float>(const Dims&, const Coef<float>&, CVec5<float>, Vec5<float>, const int*,
@@ -1143,8 +1163,10 @@ template <typename T>
 void launch_matvec_t(const Dims& d, const Coef<T>& c, CVec5<T> y, const double* yscale, CVec5<T> b, Vec5<T> out,
                      T* gzm_tmp, const int* active, cudaStream_t st) {
   const dim3 blk = stencil_block(d.tune_mvt);
-  at_gzm_kernel<T><<<box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st>>>(d, c, y.f[0], y.f[1], yscale, gzm_tmp, active);
-  at_main_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, c, y, yscale, gzm_tmp, b, out,
+  launch_chained(at_gzm_kernel<T>, box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st, d, c, y.f[0], y.f[1], yscale,
+                 gzm_tmp, active);
+  launch_chained(at_main_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, c, y, yscale,
+                 gzm_tmp, b, out,
                                                                               active);
 }
 

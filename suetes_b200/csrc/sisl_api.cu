@@ -145,6 +145,7 @@ int loc_of_field(int q) {  // solver vector field -> stagger
 template <typename T>
 __global__ void scale5_kernel(Dims d, CVec5<T> src, Vec5<T> dst, T pi_mul, int eta_mode, const T* __restrict__ dzw,
                               const T* __restrict__ idzw) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -166,6 +167,7 @@ __global__ void scale5_kernel(Dims d, CVec5<T> src, Vec5<T> dst, T pi_mul, int e
 template <typename T>
 __global__ void zero_gaps_kernel(T* base, size_t npad, int nvec, size_t o0, size_t o1, size_t o2, size_t o3,
                                  size_t o4, size_t s0, size_t s1, size_t s2, size_t s3, size_t s4) {
+  grid_chain();
   const size_t off[5] = {o0, o1, o2, o3, o4};
   const size_t sz[5] = {s0, s1, s2, s3, s4};
   const int v = blockIdx.x;
@@ -205,6 +207,7 @@ constexpr int CONVERT_BLOCKS = 8 * 148;
 template <typename S, typename D>
 __global__ void __launch_bounds__(256) convert_packed_kernel(const S* __restrict__ src, D* dst_lo, D* dst_hi,
                                                              size_t split, size_t n) {
+  grid_chain();
   const size_t n4 = n / 4;
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n4; q += (size_t)gridDim.x * blockDim.x) {
     const size_t e = 4 * q;
@@ -219,10 +222,11 @@ __global__ void __launch_bounds__(256) convert_packed_kernel(const S* __restrict
 
 // norm of a packed vector kept for the transposed solve; v *= 1/norm (mode 0)
 // or v *= norm (mode 1), a zero norm leaving v unchanged
-__global__ void keep_norm_kernel(const GState* gs, double* scal) { *scal = gs->bnorm; }
+__global__ void keep_norm_kernel(const GState* gs, double* scal) { grid_chain(); *scal = gs->bnorm; }
 
 template <typename T>
 __global__ void scale_packed_kernel(T* v, size_t n, const double* scal, int mode) {
+  grid_chain();
   const double nrm = *scal;
   if (!(nrm > 0.0)) return;
   const T f = (T)(mode == 0 ? 1.0 / nrm : nrm);
@@ -235,6 +239,7 @@ __global__ void scale_packed_kernel(T* v, size_t n, const double* scal, int mode
 template <typename T>
 __global__ void sl_fixup_kernel(Dims d, T* rhs_u, T* rhs_v, const T* __restrict__ u0, const T* __restrict__ v0,
                                 T* reta) {
+  grid_chain();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;  // generic 2-D index
   const int k = blockIdx.y;
   // u faces 0 and nx for every (j, k)
@@ -345,7 +350,8 @@ template <typename T>
 void scale5(SislCore* c, const Coef<T>& cf, CVec5<T> src, Vec5<T> dst, T pi_mul, int eta_mode, cudaStream_t st) {
   KScope k(c, SISL_K_OTHER, st);
   dim3 blk(32, 4, 2);
-  scale5_kernel<T><<<box(c->d.nx + 1, c->d.ny + 1, c->d.nz + 1, blk), blk, 0, st>>>(c->d, src, dst, pi_mul,
+  launch_chained(scale5_kernel<T>, box(c->d.nx + 1, c->d.ny + 1, c->d.nz + 1, blk), blk, 0, st, c->d, src, dst,
+                 pi_mul,
                                                                                    eta_mode, cf.dzw, cf.idzw);
 }
 
@@ -465,8 +471,8 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
   if (refine) {
     cf64 = coef64_of(c);
     KScope k(c, SISL_K_OTHER, st, 2);
-    convert_packed_kernel<T, double><<<nconv, 256, 0, st>>>(g.bg(), g.b64, g.b64, n, n);
-    convert_packed_kernel<T, double><<<nconv, 256, 0, st>>>(g.xg(), g.x64, g.x64, n, n);
+    launch_chained(convert_packed_kernel<T, double>, nconv, 256, 0, st, g.bg(), g.b64, g.b64, n, n);
+    launch_chained(convert_packed_kernel<T, double>, nconv, 256, 0, st, g.xg(), g.x64, g.x64, n, n);
     // the operator writes no padding gaps: they stay zero for the norms
     if (cudaMemsetAsync(g.r64, 0, sizeof(double) * n, st) != cudaSuccess) return SISL_ERR_CUDA;
   }
@@ -520,12 +526,12 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
       }
       if (transpose) {
         launch_matvec_t<double>(d, cf64, x5, nullptr, b5, r5, g.tmp64, nullptr, s);
-        convert_packed_kernel<double, T><<<nconv, 256, 0, s>>>(g.r64, g.z(), g.z(), n, n);
+        launch_chained(convert_packed_kernel<double, T>, nconv, 256, 0, s, g.r64, g.z(), g.z(), n, n);
       } else {
         Dims d64 = d;  // the float64 operator's own shape: the march waits on b at every level
         d64.tune_mv = default_matvec(d, sizeof(double));
         launch_matvec<double>(d64, cf64, x5, nullptr, b5, r5, nullptr, s);
-        convert_packed_kernel<double, T><<<nconv, 256, 0, s>>>(g.r64, g.V(0), g.z(), g.off[2], n);
+        launch_chained(convert_packed_kernel<double, T>, nconv, 256, 0, s, g.r64, g.V(0), g.z(), g.off[2], n);
       }
     } else {
       KScope k(c, SISL_K_MATVEC, s, na);
@@ -591,7 +597,7 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
   auto finish_x = [&]() {
     if (refine) {
       KScope k(c, SISL_K_OTHER, st);
-      convert_packed_kernel<double, T><<<nconv, 256, 0, st>>>(g.x64, g.xg(), g.xg(), n, n);
+      launch_chained(convert_packed_kernel<double, T>, nconv, 256, 0, st, g.x64, g.xg(), g.xg(), n, n);
     }
   };
   const int maxiter = c->prm.solver_maxiter;
@@ -691,7 +697,8 @@ template <typename T>
 void solve_prep(SislCore* c, const Coef<T>& cf, GWork<T>& g, CVec5<T> rhs, const CVec5<T>* x0, cudaStream_t st) {
   {
     KScope k(c, SISL_K_OTHER, st);
-    zero_gaps_kernel<T><<<g.R + 4, 256, 0, st>>>(g.vec, g.npad, g.R + 4, g.off[0], g.off[1], g.off[2], g.off[3],
+    launch_chained(zero_gaps_kernel<T>, g.R + 4, 256, 0, st, g.vec, g.npad, g.R + 4, g.off[0], g.off[1], g.off[2],
+                   g.off[3],
                                                 g.off[4], g.sz[0], g.sz[1], g.sz[2], g.sz[3], g.sz[4]);
   }
   const T ps = (T)c->s.ps;
@@ -721,7 +728,8 @@ template <typename T>
 int solve_t_prep(SislCore* c, const Coef<T>& cf, GWork<T>& g, CVec5<T> xbar, const CVec5<T>* x0, cudaStream_t st) {
   {
     KScope k(c, SISL_K_OTHER, st);
-    zero_gaps_kernel<T><<<g.R + 4, 256, 0, st>>>(g.vec, g.npad, g.R + 4, g.off[0], g.off[1], g.off[2], g.off[3],
+    launch_chained(zero_gaps_kernel<T>, g.R + 4, 256, 0, st, g.vec, g.npad, g.R + 4, g.off[0], g.off[1], g.off[2],
+                   g.off[3],
                                                 g.off[4], g.sz[0], g.sz[1], g.sz[2], g.sz[3], g.sz[4]);
   }
   scale5<T>(c, cf, xbar, g.view(g.bg()), (T)(1.0 / c->s.ps), 2, st);  // pi / ps, eta / dz_w
@@ -737,9 +745,9 @@ int solve_t_prep(SislCore* c, const Coef<T>& cf, GWork<T>& g, CVec5<T> xbar, con
     KScope k(c, SISL_K_OTHER, st, 4);
     gm_setup(g.gs, 0.0, c->prm.solver_tol, c->prm.solver_atol, g.R, c->prm.solve_method, 1, st);
     gm_dots<T>(g.V(0), g.npad, 0, g.bg(), g.npad, g.partial, g.gs, 1 /*BNORM*/, 0, st);
-    keep_norm_kernel<<<1, 1, 0, st>>>(g.gs, g.scal);
-    scale_packed_kernel<T><<<nb, 256, 0, st>>>(g.bg(), g.npad, g.scal, 0);
-    if (x0) scale_packed_kernel<T><<<nb, 256, 0, st>>>(g.xg(), g.npad, g.scal, 0);
+    launch_chained(keep_norm_kernel, 1, 1, 0, st, g.gs, g.scal);
+    launch_chained(scale_packed_kernel<T>, nb, 256, 0, st, g.bg(), g.npad, g.scal, 0);
+    if (x0) launch_chained(scale_packed_kernel<T>, nb, 256, 0, st, g.xg(), g.npad, g.scal, 0);
   }
   return SISL_OK;
 }
@@ -747,7 +755,7 @@ template <typename T>
 void solve_t_finish(SislCore* c, const Coef<T>& cf, GWork<T>& g, Vec5<T> bbar, cudaStream_t st) {
   if (c->adj_normalize) {
     KScope k(c, SISL_K_OTHER, st);
-    scale_packed_kernel<T><<<2 * 148, 256, 0, st>>>(g.xg(), g.npad, g.scal, 1);
+    launch_chained(scale_packed_kernel<T>, 2 * 148, 256, 0, st, g.xg(), g.npad, g.scal, 1);
   }
   scale5<T>(c, cf, g.cview(g.xg()), bbar, (T)c->s.ps, 0, st);  // pi * ps
 }
@@ -908,7 +916,7 @@ void step_explicit(StepRun<T>& r) {
   {
     KScope k(c, SISL_K_OTHER, st);
     const int na = (d.nx > d.ny ? d.nx : d.ny) + 1;
-    sl_fixup_kernel<T><<<dim3((na + 127) / 128, d.nz), 128, 0, st>>>(d, w.ru, w.rv, u, v, w.reta);
+    launch_chained(sl_fixup_kernel<T>, dim3((na + 127) / 128, d.nz), 128, 0, st, d, w.ru, w.rv, u, v, w.reta);
   }
 }
 
@@ -1234,7 +1242,7 @@ int vjp_forward(VjpRun<T>& r) {
     launch_sl_advect<T>(d, LOC_V, dt, w.vel + 6, iters, 1, fv, ov, one, lim, st);
     launch_sl_advect<T>(d, LOC_M, dt, w.vel + 0, iters, 1, fm, om, one, lim, st);
     const int na = (d.nx > d.ny ? d.nx : d.ny) + 1;
-    sl_fixup_kernel<T><<<dim3((na + 127) / 128, d.nz), 128, 0, st>>>(d, w.ru, w.rv, u, vv, w.reta);
+    launch_chained(sl_fixup_kernel<T>, dim3((na + 127) / 128, d.nz), 128, 0, st, d, w.ru, w.rv, u, vv, w.reta);
   }
   {
     KScope k(c, SISL_K_EXPLICIT, st, 2);

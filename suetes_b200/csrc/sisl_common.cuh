@@ -46,6 +46,34 @@ inline void ensure_smem_limit(const void* fn, SmemLimit& limit, size_t bytes) {
     current.store(bytes);
 }
 
+// Chained launches.  A step is hundreds of kernels that each read what the one
+// before wrote; on small grids, where they take a few microseconds, a fifth of
+// the time was the drain of one grid and the launch of the next.  A kernel
+// launched with launch_chained is set up while the previous kernel of its
+// stream still runs and starts when that one's last block has ended; its
+// first statement, grid_chain, waits until every earlier grid has completed
+// and its writes are visible.  A kernel that is launched this way touches no memory before
+// grid_chain.  No kernel releases its successor earlier (griddepcontrol.
+// launch_dependents): waiting blocks then fill the slots that come free first,
+// unevenly over the SMs (256x256x80 float32 step 79.2 ms against 69.3 without
+// chaining and 68.6 this way; 48x41x33 9.4 against 9.8 and 8.1; 61x47x40
+// float64 gradient 54.5 against 56.4 and 47.2).
+__device__ __forceinline__ void grid_chain() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 enum Loc { LOC_M = 0, LOC_U = 1, LOC_V = 2, LOC_W = 3 };
 
 struct Dims {

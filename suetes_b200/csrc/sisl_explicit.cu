@@ -30,6 +30,7 @@ dim3 box_grid(int ex, int ey, int ez, dim3 blk) {
 template <typename T>
 __global__ void hyper_src_kernel(Dims d, const T* __restrict__ u, const T* __restrict__ v,
                                  const T* __restrict__ w, const T* __restrict__ th, PtrTable<T> out) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -55,6 +56,7 @@ constexpr int LX = 32, LY = 8, HL_KC = 16;
 template <typename T, int NF>
 __global__ void __launch_bounds__(LX * LY, 2) hyper_lap_kernel(Dims d, Coef<T> c, PtrTable<T> src, PtrTable<T> dst,
                                                                T scale) {
+  grid_chain();
   constexpr int TX = LX + 2, TY = LY + 2, CELLS = TX * TY, SLOTS = (CELLS + LX * LY - 1) / (LX * LY);
   __shared__ T sF[2][NF][CELLS], sD[2][NF][CELLS];
   const int nx = d.nx, ny = d.ny, nz = d.nz, pm = nx * ny;
@@ -160,6 +162,7 @@ __global__ void __launch_bounds__(LX * LY, 2) hyper_lap_kernel(Dims d, Coef<T> c
 template <typename T>
 __global__ void __launch_bounds__(256) explicit_kernel(Dims d, Coef<T> c, ExplicitIn<T> in, ExplicitOut<T> out,
                                                        int mode) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -259,6 +262,7 @@ __global__ void __launch_bounds__(256) explicit_kernel(Dims d, Coef<T> c, Explic
 template <typename T>
 __global__ void corrector_theta_kernel(Dims d, Coef<T> c, const T* __restrict__ th_adv, const T* __restrict__ tth,
                                        const T* __restrict__ w_now, const T* __restrict__ w_next, T* th_next) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -272,6 +276,7 @@ __global__ void corrector_theta_kernel(Dims d, Coef<T> c, const T* __restrict__ 
 
 template <typename T>
 __global__ void __launch_bounds__(256) corrector_rhs_kernel(Dims d, Coef<T> c, CorrectorIn<T> in, Vec5<T> out) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -331,6 +336,7 @@ __global__ void __launch_bounds__(256) corrector_rhs_kernel(Dims d, Coef<T> c, C
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void hdiv_kernel(Dims d, Coef<T> c, const T* __restrict__ u, const T* __restrict__ v, T* div) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -350,6 +356,7 @@ __device__ __forceinline__ T blend(T val, const T* mask, int h, T ext) {
 
 template <typename T>
 __global__ void __launch_bounds__(256) finalize_kernel(Dims d, Coef<T> c, FinalizeArgs<T> fa) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -406,39 +413,40 @@ template <typename T>
 void launch_hyper(const Dims& d, const Coef<T>& c, const T* u, const T* v, const T* w, const T* th,
                   PtrTable<T> tmp4, PtrTable<T> out4, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  hyper_src_kernel<T><<<box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st>>>(d, u, v, w, th, out4);
+  launch_chained(hyper_src_kernel<T>, box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st, d, u, v, w, th, out4);
   // float64 takes two fields a block: the state of four would not fit the registers of two resident blocks
   constexpr int NF = sizeof(T) == 4 ? 4 : 2;
   const dim3 lb(LX, LY, 1), lg((d.nx + LX - 1) / LX, (d.ny + LY - 1) / LY, (4 / NF) * ((d.nz + HL_KC - 1) / HL_KC));
-  hyper_lap_kernel<T, NF><<<lg, lb, 0, st>>>(d, c, out4, tmp4, T(1));
-  hyper_lap_kernel<T, NF><<<lg, lb, 0, st>>>(d, c, tmp4, out4, (T)(-c.s.nu_h));
+  launch_chained(hyper_lap_kernel<T, NF>, lg, lb, 0, st, d, c, out4, tmp4, T(1));
+  launch_chained(hyper_lap_kernel<T, NF>, lg, lb, 0, st, d, c, tmp4, out4, (T)(-c.s.nu_h));
 }
 
 template <typename T>
 void launch_explicit(const Dims& d, const Coef<T>& c, const ExplicitIn<T>& in, const ExplicitOut<T>& out, int mode,
                      cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  explicit_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, c, in, out, mode);
+  launch_chained(explicit_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, c, in, out, mode);
 }
 
 template <typename T>
 void launch_corrector_theta(const Dims& d, const Coef<T>& c, const T* th_adv, const T* tth, const T* w_now,
                             const T* w_next, T* th_next, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  corrector_theta_kernel<T><<<box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st>>>(d, c, th_adv, tth, w_now, w_next,
+  launch_chained(corrector_theta_kernel<T>, box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st, d, c, th_adv, tth, w_now,
+                 w_next,
                                                                             th_next);
 }
 
 template <typename T>
 void launch_corrector_rhs(const Dims& d, const Coef<T>& c, const CorrectorIn<T>& in, Vec5<T> out, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  corrector_rhs_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, c, in, out);
+  launch_chained(corrector_rhs_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, c, in, out);
 }
 
 template <typename T>
 void launch_hdiv(const Dims& d, const Coef<T>& c, const T* u, const T* v, T* div, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  hdiv_kernel<T><<<box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st>>>(d, c, u, v, div);
+  launch_chained(hdiv_kernel<T>, box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st, d, c, u, v, div);
 }
 
 // Euler3D.metric_curvature_tendencies (euler.py:188-206): the map-curvature
@@ -449,6 +457,7 @@ void launch_hdiv(const Dims& d, const Coef<T>& c, const T* u, const T* v, T* div
 template <typename T>
 __global__ void curvature_kernel(Dims d, Coef<T> c, const T* __restrict__ u, const T* __restrict__ v,
                                  T* __restrict__ ou, T* __restrict__ ov) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -472,13 +481,13 @@ __global__ void curvature_kernel(Dims d, Coef<T> c, const T* __restrict__ u, con
 template <typename T>
 void launch_curvature(const Dims& d, const Coef<T>& c, const T* u, const T* v, T* ou, T* ov, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  curvature_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz, blk), blk, 0, st>>>(d, c, u, v, ou, ov);
+  launch_chained(curvature_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz, blk), blk, 0, st, d, c, u, v, ou, ov);
 }
 
 template <typename T>
 void launch_finalize(const Dims& d, const Coef<T>& c, const FinalizeArgs<T>& fa, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  finalize_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, c, fa);
+  launch_chained(finalize_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, c, fa);
 }
 
 #define SISL_INST_EX(T)                                                                                        \

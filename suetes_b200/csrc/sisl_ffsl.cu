@@ -26,6 +26,7 @@ __device__ __forceinline__ T cell_volume(const Dims& d, const Coef<T>& c, int i,
 
 template <typename T>
 __global__ void ffsl_mass_kernel(Dims d, Coef<T> c, const T* __restrict__ rho, T* mass) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -37,6 +38,7 @@ __global__ void ffsl_mass_kernel(Dims d, Coef<T> c, const T* __restrict__ rho, T
 template <typename T>
 __global__ void ffsl_sweep_kernel(Dims d, Coef<T> c, int axis, const T* __restrict__ in, const T* __restrict__ vel,
                                   T* out, double* __restrict__ M, int periodic, double dt, int to_density) {
+  grid_chain();
   const int line = blockIdx.x * blockDim.x + threadIdx.x;
   int N, nlines, a, b;
   if (axis == 0) { N = d.nx; nlines = d.ny * d.nz; a = line % d.ny; b = line / d.ny; }
@@ -127,6 +129,7 @@ __global__ void __launch_bounds__(FL* FW) ffsl_tile_kernel(Dims d, Coef<T> c, co
                                                            const T* __restrict__ vel, T* __restrict__ out,
                                                            int periodic, double scale, int from_density,
                                                            int to_density) {
+  grid_chain();
   extern __shared__ double M[];  // [N + 1][FLD] cumulative mass, then the segment sums
   const int N = AXIS == 0 ? d.nx : AXIS == 1 ? d.ny : d.nz;
   const int nlines = AXIS == 0 ? d.ny * d.nz : AXIS == 1 ? d.nx * d.nz : d.nx * d.ny;
@@ -251,7 +254,8 @@ bool launch_ffsl_tile(const Dims& d, const Coef<T>& c, const T* in, const T* vel
   static SmemLimit attr_bytes;  // per instantiation
   ensure_smem_limit((const void*)ffsl_tile_kernel<T, AXIS>, attr_bytes, smem);
   const double scale = AXIS == 0 ? dt / d.dx : AXIS == 1 ? dt / d.dy : dt;  // of the interface Courant number
-  ffsl_tile_kernel<T, AXIS><<<(nlines + FL - 1) / FL, FL * FW, smem, st>>>(d, c, in, vel, out, periodic, scale,
+  launch_chained(ffsl_tile_kernel<T, AXIS>, (nlines + FL - 1) / FL, FL * FW, smem, st, d, c, in, vel, out, periodic,
+                 scale,
                                                                          from_density, to_density);
   return true;
 }
@@ -264,7 +268,8 @@ void launch_ffsl_sweep(const Dims& d, const Coef<T>& c, int axis, const T* in, c
   if (done) return;
   const int nlines = axis == 0 ? d.ny * d.nz : axis == 1 ? d.nx * d.nz : d.nx * d.ny;
   const int tb = 128;
-  ffsl_sweep_kernel<T><<<(nlines + tb - 1) / tb, tb, 0, st>>>(d, c, axis, in, vel, out, M, periodic, dt, to_density);
+  launch_chained(ffsl_sweep_kernel<T>, (nlines + tb - 1) / tb, tb, 0, st, d, c, axis, in, vel, out, M, periodic, dt,
+                 to_density);
 }
 
 // advect_1d (steppers.py:552-594) on nlines independent lines: scalar is
@@ -272,6 +277,7 @@ void launch_ffsl_sweep(const Dims& d, const Coef<T>& c, int axis, const T* in, c
 template <typename T>
 __global__ void ffsl_line_kernel(int N, int nlines, const T* __restrict__ sc, const T* __restrict__ cf, T* out,
                                  double* __restrict__ M, int periodic) {
+  grid_chain();
   const int line = blockIdx.x * blockDim.x + threadIdx.x;
   if (line >= nlines) return;
   const T* s_ = sc + (size_t)line * N;
@@ -382,6 +388,7 @@ __global__ void ffsl_sweep_vjp_kernel(Dims d, Coef<T> c, int axis, const T* __re
                                       const T* __restrict__ vel, const T* __restrict__ ob, T* ib, T* velb,
                                       double* __restrict__ M, double* __restrict__ Mb, int periodic, double dt,
                                       int ob_density, int ib_density) {
+  grid_chain();
   const int line = blockIdx.x * blockDim.x + threadIdx.x;
   int N, nlines, a, b;
   if (axis == 0) { N = d.nx; nlines = d.ny * d.nz; a = line % d.ny; b = line / d.ny; }
@@ -430,6 +437,7 @@ template <typename T>
 __global__ void ffsl_line_vjp_kernel(int N, int nlines, const T* __restrict__ sc, const T* __restrict__ cf,
                                      const T* __restrict__ ob, T* sb, T* cb, double* __restrict__ M,
                                      double* __restrict__ Mb, int periodic) {
+  grid_chain();
   const int line = blockIdx.x * blockDim.x + threadIdx.x;
   if (line >= nlines) return;
   const size_t s0 = (size_t)line * N, c0 = (size_t)line * (N + 1);
@@ -445,6 +453,7 @@ __global__ void ffsl_line_vjp_kernel(int N, int nlines, const T* __restrict__ sc
 
 template <typename T>
 __global__ void eos_kernel(Dims d, Coef<T> c, const T* __restrict__ th, const T* __restrict__ pi, T* rho) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -475,7 +484,7 @@ int launch_ffsl(const Dims& d, const Coef<T>& c, const T* field, const T* u, con
   int kernels = 3;
   if (!launch_ffsl_tile<T, 0>(d, c, field, u, tmp1, d.px, dt, 1, 0, st)) {
     const dim3 blk(32, 4, 2);
-    ffsl_mass_kernel<T><<<box3(d, blk), blk, 0, st>>>(d, c, field, tmp0);
+    launch_chained(ffsl_mass_kernel<T>, box3(d, blk), blk, 0, st, d, c, field, tmp0);
     launch_ffsl_sweep<T>(d, c, 0, tmp0, u, tmp1, M, d.px, dt, 0, st);
     ++kernels;
   }
@@ -496,15 +505,18 @@ int launch_ffsl_vjp(const Dims& d, const Coef<T>& c, const T* field, const T* u,
   const double dt = c.s.dt;
   T *mass = tmp[0], *mx = tmp[1], *my = tmp[2], *b1 = tmp[3], *b2 = tmp[4];
   // recompute the sweeps' inputs
-  ffsl_mass_kernel<T><<<box3(d, blk), blk, 0, st>>>(d, c, field, mass);
+  launch_chained(ffsl_mass_kernel<T>, box3(d, blk), blk, 0, st, d, c, field, mass);
   launch_ffsl_sweep<T>(d, c, 0, mass, u, mx, M, d.px, dt, 0, st);
   launch_ffsl_sweep<T>(d, c, 1, mx, v, my, M, d.py, dt, 0, st);
   // reverse z, y, x
-  ffsl_sweep_vjp_kernel<T><<<(d.nx * d.ny + tb - 1) / tb, tb, 0, st>>>(d, c, 2, my, eta, out_bar, b1, eta_bar, M,
+  launch_chained(ffsl_sweep_vjp_kernel<T>, (d.nx * d.ny + tb - 1) / tb, tb, 0, st, d, c, 2, my, eta, out_bar, b1,
+                 eta_bar, M,
                                                                      Mb, 0, dt, 1, 0);
-  ffsl_sweep_vjp_kernel<T><<<(d.nx * d.nz + tb - 1) / tb, tb, 0, st>>>(d, c, 1, mx, v, b1, b2, v_bar, M, Mb, d.py,
+  launch_chained(ffsl_sweep_vjp_kernel<T>, (d.nx * d.nz + tb - 1) / tb, tb, 0, st, d, c, 1, mx, v, b1, b2, v_bar, M,
+                 Mb, d.py,
                                                                      dt, 0, 0);
-  ffsl_sweep_vjp_kernel<T><<<(d.ny * d.nz + tb - 1) / tb, tb, 0, st>>>(d, c, 0, mass, u, b2, field_bar, u_bar, M,
+  launch_chained(ffsl_sweep_vjp_kernel<T>, (d.ny * d.nz + tb - 1) / tb, tb, 0, st, d, c, 0, mass, u, b2, field_bar,
+                 u_bar, M,
                                                                      Mb, d.px, dt, 0, 1);
   return 6;  // kernels launched
 }
@@ -512,20 +524,21 @@ int launch_ffsl_vjp(const Dims& d, const Coef<T>& c, const T* field, const T* u,
 template <typename T>
 void launch_ffsl_lines_vjp(int N, int nlines, const T* scalar, const T* cfl, const T* out_bar, T* scalar_bar,
                            T* cfl_bar, double* M, double* Mb, int periodic, cudaStream_t st) {
-  ffsl_line_vjp_kernel<T><<<(nlines + 127) / 128, 128, 0, st>>>(N, nlines, scalar, cfl, out_bar, scalar_bar, cfl_bar,
+  launch_chained(ffsl_line_vjp_kernel<T>, (nlines + 127) / 128, 128, 0, st, N, nlines, scalar, cfl, out_bar,
+                 scalar_bar, cfl_bar,
                                                                 M, Mb, periodic);
 }
 
 template <typename T>
 void launch_ffsl_lines(int N, int nlines, const T* scalar, const T* cfl, T* out, double* M, int periodic,
                        cudaStream_t st) {
-  ffsl_line_kernel<T><<<(nlines + 127) / 128, 128, 0, st>>>(N, nlines, scalar, cfl, out, M, periodic);
+  launch_chained(ffsl_line_kernel<T>, (nlines + 127) / 128, 128, 0, st, N, nlines, scalar, cfl, out, M, periodic);
 }
 
 template <typename T>
 void launch_eos(const Dims& d, const Coef<T>& c, const T* th, const T* pi, T* rho, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  eos_kernel<T><<<box3(d, blk), blk, 0, st>>>(d, c, th, pi, rho);
+  launch_chained(eos_kernel<T>, box3(d, blk), blk, 0, st, d, c, th, pi, rho);
 }
 
 template int launch_ffsl<float>(const Dims&, const Coef<float>&, const float*, const float*, const float*,

@@ -228,6 +228,7 @@ __device__ __forceinline__ void dots_body(const T* __restrict__ Vb, size_t strid
 template <typename T>
 __global__ void dots_kernel(const T* __restrict__ Vb, size_t stride, int m, const T* __restrict__ w, size_t n,
                             double* partial, GState* gs, int mode, int gated) {
+  grid_chain();
   if (gated && gs->active == 0) return;
   dots_body<T>(Vb, stride, m, w, n, partial, gs, mode, blockIdx.x, gridDim.x);
 }
@@ -440,6 +441,7 @@ __device__ __forceinline__ void block_dots_body(const T* __restrict__ Vb, size_t
 template <typename T, int NT>
 __global__ void __launch_bounds__(GT, 2) block_dots_kernel(const T* __restrict__ Vb, size_t stride, int j0, int s,
                                                            size_t n, double* partial, GState* gs) {
+  grid_chain();
   if (gs->active == 0) return;
   block_dots_body<T, NT>(Vb, stride, j0, s, n, partial, gs, blockIdx.x, gridDim.x);
 }
@@ -734,6 +736,7 @@ __device__ __forceinline__ void block_update_body(T* Vb, size_t stride, int j0, 
 template <typename T, int S>
 __global__ void __launch_bounds__(GT, 2) block_update_kernel(T* Vb, size_t stride, int j0, size_t n, double* partial,
                                                              GState* gs) {
+  grid_chain();
   if (gs->active == 0) return;
   block_update_body<T, S>(Vb, stride, j0, n, partial, gs, blockIdx.x, gridDim.x);
 }
@@ -790,6 +793,7 @@ __device__ __forceinline__ void update_x64_body(const T* __restrict__ Vb, size_t
 template <typename T>
 __global__ void __launch_bounds__(256) update_x64_kernel(const T* __restrict__ Vb, size_t stride, int m,
                                                          double* __restrict__ x, size_t n, const GState* gs) {
+  grid_chain();
   update_x64_body<T>(Vb, stride, m, x, n, gs, blockIdx.x, gridDim.x);
 }
 
@@ -912,6 +916,7 @@ template <typename T>
 __global__ void __launch_bounds__(GT) update_kernel(const T* __restrict__ Vb, size_t stride, int m,
                                                     T* __restrict__ w, size_t n, double sign, double* partial,
                                                     GState* gs, int mode, int gated, int limit_kdone) {
+  grid_chain();
   if (gated && gs->active == 0) return;
   update_body<T>(Vb, stride, m, w, n, sign, partial, gs, mode, limit_kdone, blockIdx.x, gridDim.x);
 }
@@ -934,12 +939,14 @@ __device__ void setup_state(GState* gs, double eps, double tol, double atol_in, 
 }
 __global__ void setup_kernel(GState* gs, double eps, double tol, double atol_in, int restart, int method,
                              int columns) {
+  grid_chain();
   setup_state(gs, eps, tol, atol_in, restart, method, columns);
 }
 
 // Graph mode: after a residual, count the finished cycle and set the WHILE
 // condition: another cycle while ||M r|| > atol and cycles < maxiter.
 __global__ void gate_kernel(GState* gs, cudaGraphConditionalHandle h, int maxiter, int after_cycle) {
+  grid_chain();
   if (after_cycle) {
     gs->cycles += 1;
     gs->steps += gs->kdone;
@@ -957,14 +964,14 @@ __device__ void info_state(const GState* gs, GDevInfo* o) {
   o->atol = gs->atol;
   o->b_norm = gs->bnorm;
 }
-__global__ void info_kernel(const GState* gs, GDevInfo* o) { info_state(gs, o); }
+__global__ void info_kernel(const GState* gs, GDevInfo* o) { grid_chain(); info_state(gs, o); }
 
 __device__ void init_tol_state(GState* gs) {
   // atol = max(tol ||b||, atol); ptol = ||M b|| min(1, atol / ||b||)
   gs->atol = fmax(gs->tol * gs->bnorm, gs->atol_in);
   gs->ptol = gs->mbnorm * fmin(1.0, gs->atol / gs->bnorm);
 }
-__global__ void init_tol_kernel(GState* gs) { init_tol_state(gs); }
+__global__ void init_tol_kernel(GState* gs) { grid_chain(); init_tol_state(gs); }
 
 __device__ void begin_cycle_state(GState* gs) {
   const int R = gs->restart;
@@ -983,7 +990,10 @@ __device__ void begin_cycle_state(GState* gs) {
     gs->breakdown = 0;
   }
 }
-__global__ void begin_cycle_kernel(GState* gs) { begin_cycle_state(gs); }
+__global__ void begin_cycle_kernel(GState* gs) {
+  grid_chain();
+  begin_cycle_state(gs);
+}
 
 // y from the cycle's small problem; coef_i = y_i s_i, or B y in the block
 // form, whose triangular solves run on one warp (a row's inner product over
@@ -1081,9 +1091,13 @@ __device__ void small_solve_state(GState* gs) {
     gs->coef[k] = v;
   }
 }
-__global__ void small_solve_kernel(GState* gs) { small_solve_state(gs); }
+__global__ void small_solve_kernel(GState* gs) {
+  grid_chain();
+  small_solve_state(gs);
+}
 
 __global__ void snapshot_kernel(const GState* gs, GHostView* v) {
+  grid_chain();
   v->rnorm = gs->rnorm;
   v->atol = gs->atol;
   v->bnorm = gs->bnorm;
@@ -1102,6 +1116,7 @@ __device__ __forceinline__ T* gvec(const GroupMember<T>& g, int v) {
 template <typename T>
 __global__ void group_dots_kernel(GroupMember<T>* mem, const int* __restrict__ first, int M, int m, int wv,
                                   int mode, int gated) {
+  grid_chain();
   const int b = blockIdx.x;
   const int mi = group_find(first, M, b);
   const GroupMember<T>& g = mem[mi];
@@ -1113,6 +1128,7 @@ __global__ void group_dots_kernel(GroupMember<T>* mem, const int* __restrict__ f
 template <typename T, int NT>
 __global__ void __launch_bounds__(GT, 2) group_block_dots_kernel(GroupMember<T>* mem, const int* __restrict__ first,
                                                                  int M, int j0, int s) {
+  grid_chain();
   const int b = blockIdx.x;
   const int mi = group_find(first, M, b);
   const GroupMember<T>& g = mem[mi];
@@ -1123,6 +1139,7 @@ __global__ void __launch_bounds__(GT, 2) group_block_dots_kernel(GroupMember<T>*
 template <typename T, int S>
 __global__ void __launch_bounds__(GT, 2) group_block_update_kernel(GroupMember<T>* mem, const int* __restrict__ first,
                                                                    int M, int j0) {
+  grid_chain();
   const int b = blockIdx.x;
   const int mi = group_find(first, M, b);
   const GroupMember<T>& g = mem[mi];
@@ -1135,6 +1152,7 @@ __global__ void __launch_bounds__(GT, 2) group_block_update_kernel(GroupMember<T
 template <typename T>
 __global__ void __launch_bounds__(GT) group_update_kernel(GroupMember<T>* mem, const int* __restrict__ first, int M,
                                                           int m, int final_x) {
+  grid_chain();
   const int b = blockIdx.x;
   const int mi = group_find(first, M, b);
   const GroupMember<T>& g = mem[mi];
@@ -1152,6 +1170,7 @@ __global__ void __launch_bounds__(GT) group_update_kernel(GroupMember<T>* mem, c
 template <typename T>
 __global__ void __launch_bounds__(256) group_update_x64_kernel(GroupMember<T>* mem, const int* __restrict__ first,
                                                                int M, int m) {
+  grid_chain();
   const int b = blockIdx.x;
   const int mi = group_find(first, M, b);
   const GroupMember<T>& g = mem[mi];
@@ -1166,6 +1185,7 @@ __global__ void __launch_bounds__(256) group_update_x64_kernel(GroupMember<T>* m
 template <typename T>
 __global__ void __launch_bounds__(256) group_convert_kernel(GroupMember<T>* mem, const int* __restrict__ first,
                                                             int M, int mode) {
+  grid_chain();
   const int b = blockIdx.x;
   const int mi = group_find(first, M, b);
   const GroupMember<T>& g = mem[mi];
@@ -1197,6 +1217,7 @@ __global__ void __launch_bounds__(256) group_convert_kernel(GroupMember<T>* mem,
 // one thread per member
 template <typename T>
 __global__ void group_setup_kernel(GroupMember<T>* mem, int M, int R, int method, int transpose, int columns) {
+  grid_chain();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= M) return;
   GroupMember<T>& g = mem[m];
@@ -1205,22 +1226,26 @@ __global__ void group_setup_kernel(GroupMember<T>* mem, int M, int R, int method
 }
 template <typename T>
 __global__ void group_init_tol_kernel(GroupMember<T>* mem, int M) {
+  grid_chain();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m < M) init_tol_state(mem[m].gs);
 }
 template <typename T>
 __global__ void group_info_kernel(GroupMember<T>* mem, int M, int solve) {
+  grid_chain();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m < M && mem[m].info[solve]) info_state(mem[m].gs, mem[m].info[solve]);
 }
 // one block per member
 template <typename T>
 __global__ void group_begin_cycle_kernel(GroupMember<T>* mem) {
+  grid_chain();
   const GroupMember<T>& g = mem[blockIdx.x];
   if (g.running) begin_cycle_state(g.gs);
 }
 template <typename T>
 __global__ void group_small_solve_kernel(GroupMember<T>* mem) {
+  grid_chain();
   const GroupMember<T>& g = mem[blockIdx.x];
   if (g.running) small_solve_state(g.gs);
 }
@@ -1228,6 +1253,7 @@ __global__ void group_small_solve_kernel(GroupMember<T>* mem) {
 // members continue, set the WHILE condition while any does
 template <typename T>
 __global__ void group_gate_kernel(GroupMember<T>* mem, int M, cudaGraphConditionalHandle h, int after_cycle) {
+  grid_chain();
   int any = 0;
   for (int m = threadIdx.x; m < M; m += blockDim.x) {
     GroupMember<T>& g = mem[m];
@@ -1330,7 +1356,7 @@ void gm_block_dots(const T* Vb, size_t stride, int j0, int s, size_t n, double* 
                    cudaStream_t st) {
   const int g = gm_block_dots_blocks<T>(n);
   with_row_tiles(j0 + 1 + s, [&](auto nt) {
-    block_dots_kernel<T, decltype(nt)::value><<<g, GT, 0, st>>>(Vb, stride, j0, s, n, partial, gs);
+    launch_chained(block_dots_kernel<T, decltype(nt)::value>, g, GT, 0, st, Vb, stride, j0, s, n, partial, gs);
   });
 }
 
@@ -1338,7 +1364,7 @@ template <typename T>
 void gm_block_update(T* Vb, size_t stride, int j0, int s, size_t n, double* partial, GState* gs, cudaStream_t st) {
   const int g = gm_block_update_blocks<T>(n);
   with_columns(s, [&](auto sc) {
-    block_update_kernel<T, decltype(sc)::value><<<g, GT, 0, st>>>(Vb, stride, j0, n, partial, gs);
+    launch_chained(block_update_kernel<T, decltype(sc)::value>, g, GT, 0, st, Vb, stride, j0, n, partial, gs);
   });
 }
 
@@ -1355,7 +1381,7 @@ void gm_dots(const T* Vb, size_t stride, int m, const T* w, size_t n, double* pa
   constexpr int E = CH * V16<T>::n;
   const size_t smem = (size_t)(m + 1) * (nt / 32) * sizeof(double);
   const int g = resident_grid((const void*)dots_kernel<T>, nt, smem, n, nt * E);
-  dots_kernel<T><<<g, nt, smem, st>>>(Vb, stride, m, w, n, partial, gs, mode, gated);
+  launch_chained(dots_kernel<T>, g, nt, smem, st, Vb, stride, m, w, n, partial, gs, mode, gated);
 }
 
 template <typename T>
@@ -1363,31 +1389,32 @@ void gm_update(const T* Vb, size_t stride, int m, T* w, size_t n, double sign, d
                int mode, int gated, int limit_kdone, cudaStream_t st) {
   constexpr int E = CH * V16<T>::n;
   const int g = resident_grid((const void*)update_kernel<T>, GT, 0, n, GT * E);
-  update_kernel<T><<<g, GT, 0, st>>>(Vb, stride, m, w, n, sign, partial, gs, mode, gated, limit_kdone);
+  launch_chained(update_kernel<T>, g, GT, 0, st, Vb, stride, m, w, n, sign, partial, gs, mode, gated, limit_kdone);
 }
 
 template <typename T>
 void gm_update_x64(const T* Vb, size_t stride, int m, double* x, size_t n, const GState* gs, cudaStream_t st) {
-  update_x64_kernel<T><<<gm_x64_blocks_t<T>(n), 256, 0, st>>>(Vb, stride, m, x, n, gs);
+  launch_chained(update_x64_kernel<T>, gm_x64_blocks_t<T>(n), 256, 0, st, Vb, stride, m, x, n, gs);
 }
 
 void gm_setup(GState* gs, double eps, double tol, double atol_in, int restart, int method, int columns,
               cudaStream_t st) {
-  setup_kernel<<<1, 1, 0, st>>>(gs, eps, tol, atol_in, restart, method, columns);
+  launch_chained(setup_kernel, 1, 1, 0, st, gs, eps, tol, atol_in, restart, method, columns);
 }
-void gm_init_tol(GState* gs, cudaStream_t st) { init_tol_kernel<<<1, 1, 0, st>>>(gs); }
+void gm_init_tol(GState* gs, cudaStream_t st) { launch_chained(init_tol_kernel, 1, 1, 0, st, gs); }
 void gm_gate(GState* gs, cudaGraphConditionalHandle h, int maxiter, int after_cycle, cudaStream_t st) {
-  gate_kernel<<<1, 1, 0, st>>>(gs, h, maxiter, after_cycle);
+  launch_chained(gate_kernel, 1, 1, 0, st, gs, h, maxiter, after_cycle);
 }
-void gm_info(const GState* gs, GDevInfo* o, cudaStream_t st) { info_kernel<<<1, 1, 0, st>>>(gs, o); }
-void gm_begin_cycle(GState* gs, cudaStream_t st) { begin_cycle_kernel<<<1, 256, 0, st>>>(gs); }
+void gm_info(const GState* gs, GDevInfo* o, cudaStream_t st) { launch_chained(info_kernel, 1, 1, 0, st, gs, o); }
+void gm_begin_cycle(GState* gs, cudaStream_t st) { launch_chained(begin_cycle_kernel, 1, 256, 0, st, gs); }
 void gm_small_solve(GState* gs, int restart, cudaStream_t st) {
   const size_t smem = (size_t)restart * restart * sizeof(double);
   static SmemLimit attr_bytes;
   ensure_smem_limit((const void*)small_solve_kernel, attr_bytes, (size_t)GM_MAXR * GM_MAXR * sizeof(double));
-  small_solve_kernel<<<1, 256, smem, st>>>(gs);
+  launch_chained(small_solve_kernel, 1, 256, smem, st, gs);
 }
-void gm_snapshot(const GState* gs, GHostView* v, cudaStream_t st) { snapshot_kernel<<<1, 1, 0, st>>>(gs, v); }
+void gm_snapshot(const GState* gs, GHostView* v, cudaStream_t st) { launch_chained(snapshot_kernel, 1, 1, 0, st, gs,
+    v); }
 
 // ---------------------------------------------------------------------------
 // grouped host wrappers
@@ -1415,7 +1442,7 @@ int group_convert_blocks(size_t n) { return flat_grid(n, 256 * 8) < 296 ? flat_g
 
 template <typename T>
 void grp_setup(const GroupLaunch<T>& g, int transpose, cudaStream_t st) {
-  group_setup_kernel<T><<<(g.M + 127) / 128, 128, 0, st>>>(g.mem, g.M, g.R, g.method, transpose, g.S);
+  launch_chained(group_setup_kernel<T>, (g.M + 127) / 128, 128, 0, st, g.mem, g.M, g.R, g.method, transpose, g.S);
 }
 template <typename T>
 void grp_dots(const GroupLaunch<T>& g, int m, int w, int mode, int gated, cudaStream_t st) {
@@ -1423,56 +1450,58 @@ void grp_dots(const GroupLaunch<T>& g, int m, int w, int mode, int gated, cudaSt
   ensure_smem_limit((const void*)group_dots_kernel<T>, attr_bytes, (size_t)DOTS_SMEM_MAX);
   const int nt = gm_dots_threads<T>(m);
   const size_t smem = (size_t)(m + 1) * (nt / 32) * sizeof(double);
-  group_dots_kernel<T><<<g.blocks(GT_DOTS0 + m), nt, smem, st>>>(g.mem, g.row(GT_DOTS0 + m), g.M, m, w, mode, gated);
+  launch_chained(group_dots_kernel<T>, g.blocks(GT_DOTS0 + m), nt, smem, st, g.mem, g.row(GT_DOTS0 + m), g.M, m, w,
+                 mode, gated);
 }
 template <typename T>
 void grp_block_dots(const GroupLaunch<T>& g, int j0, int s, cudaStream_t st) {
   with_row_tiles(j0 + 1 + s, [&](auto nt) {
-    group_block_dots_kernel<T, decltype(nt)::value>
-        <<<g.blocks(GT_BDOT), GT, 0, st>>>(g.mem, g.row(GT_BDOT), g.M, j0, s);
+    launch_chained(group_block_dots_kernel<T, decltype(nt)::value>, g.blocks(GT_BDOT), GT, 0, st, g.mem,
+                   g.row(GT_BDOT), g.M, j0, s);
   });
 }
 template <typename T>
 void grp_block_update(const GroupLaunch<T>& g, int j0, int s, cudaStream_t st) {
   with_columns(s, [&](auto sc) {
-    group_block_update_kernel<T, decltype(sc)::value>
-        <<<g.blocks(GT_BUPD), GT, 0, st>>>(g.mem, g.row(GT_BUPD), g.M, j0);
+    launch_chained(group_block_update_kernel<T, decltype(sc)::value>, g.blocks(GT_BUPD), GT, 0, st, g.mem,
+                   g.row(GT_BUPD), g.M, j0);
   });
 }
 template <typename T>
 void grp_update_arnoldi(const GroupLaunch<T>& g, int m, cudaStream_t st) {
-  group_update_kernel<T><<<g.blocks(GT_UPD), GT, 0, st>>>(g.mem, g.row(GT_UPD), g.M, m, 0);
+  launch_chained(group_update_kernel<T>, g.blocks(GT_UPD), GT, 0, st, g.mem, g.row(GT_UPD), g.M, m, 0);
 }
 template <typename T>
 void grp_update_x(const GroupLaunch<T>& g, cudaStream_t st) {
-  if (g.refine) group_update_x64_kernel<T><<<g.blocks(GT_X64), 256, 0, st>>>(g.mem, g.row(GT_X64), g.M, g.R);
-  else group_update_kernel<T><<<g.blocks(GT_UPD), GT, 0, st>>>(g.mem, g.row(GT_UPD), g.M, g.R, 1);
+  if (g.refine) launch_chained(group_update_x64_kernel<T>, g.blocks(GT_X64), 256, 0, st, g.mem, g.row(GT_X64), g.M,
+                               g.R);
+  else launch_chained(group_update_kernel<T>, g.blocks(GT_UPD), GT, 0, st, g.mem, g.row(GT_UPD), g.M, g.R, 1);
 }
 template <typename T>
 void grp_convert(const GroupLaunch<T>& g, int mode, cudaStream_t st) {
-  group_convert_kernel<T><<<g.blocks(GT_CVT), 256, 0, st>>>(g.mem, g.row(GT_CVT), g.M, mode);
+  launch_chained(group_convert_kernel<T>, g.blocks(GT_CVT), 256, 0, st, g.mem, g.row(GT_CVT), g.M, mode);
 }
 template <typename T>
 void grp_init_tol(const GroupLaunch<T>& g, cudaStream_t st) {
-  group_init_tol_kernel<T><<<(g.M + 127) / 128, 128, 0, st>>>(g.mem, g.M);
+  launch_chained(group_init_tol_kernel<T>, (g.M + 127) / 128, 128, 0, st, g.mem, g.M);
 }
 template <typename T>
 void grp_begin_cycle(const GroupLaunch<T>& g, cudaStream_t st) {
-  group_begin_cycle_kernel<T><<<g.M, 256, 0, st>>>(g.mem);
+  launch_chained(group_begin_cycle_kernel<T>, g.M, 256, 0, st, g.mem);
 }
 template <typename T>
 void grp_small_solve(const GroupLaunch<T>& g, cudaStream_t st) {
   static SmemLimit attr_bytes;
   ensure_smem_limit((const void*)group_small_solve_kernel<T>, attr_bytes, (size_t)GM_MAXR * GM_MAXR * sizeof(double));
-  group_small_solve_kernel<T><<<g.M, 256, (size_t)g.R * g.R * sizeof(double), st>>>(g.mem);
+  launch_chained(group_small_solve_kernel<T>, g.M, 256, (size_t)g.R * g.R * sizeof(double), st, g.mem);
 }
 template <typename T>
 void grp_gate(const GroupLaunch<T>& g, cudaGraphConditionalHandle h, int after_cycle, cudaStream_t st) {
-  group_gate_kernel<T><<<1, 256, 0, st>>>(g.mem, g.M, h, after_cycle);
+  launch_chained(group_gate_kernel<T>, 1, 256, 0, st, g.mem, g.M, h, after_cycle);
 }
 template <typename T>
 void grp_info(const GroupLaunch<T>& g, int solve, cudaStream_t st) {
-  group_info_kernel<T><<<(g.M + 127) / 128, 128, 0, st>>>(g.mem, g.M, solve);
+  launch_chained(group_info_kernel<T>, (g.M + 127) / 128, 128, 0, st, g.mem, g.M, solve);
 }
 
 #define SISL_GROUP_INST(T)                                                                           \

@@ -231,6 +231,7 @@ template <typename T, int LV>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (LV == 1 ? 6 : 4) : (LV == 1 ? 4 : 3)) matvec_kernel(Dims d, Coef<T> c, CVec5<T> x,
                                                                             const double* xscale,
                                                      CVec5<T> b, Vec5<T> out, const int* active) {
+  grid_chain();
   if (active && *active == 0) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -463,6 +464,7 @@ template <typename T>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 2) matvec_march_kernel(Dims d, Coef<T> c, CVec5<T> x,
                                                                                   const double* xscale, CVec5<T> b,
                                                                                   Vec5<T> out, const int* active) {
+  grid_chain();
   if (active && *active == 0) return;
   matvec_march_block<T>(d, c, x, xscale, b, out, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.z);
 }
@@ -517,6 +519,7 @@ __device__ __forceinline__ PrecondW<T> precond_wlevel(const Dims& d, const Coef<
 template <typename T, int PT, int PC>
 __global__ void __launch_bounds__(PT) precond_tile_kernel(Dims d, Coef<T> c, CVec5<T> r, Vec5<T> out,
                                                           const int* active) {
+  grid_chain();
   if (active && *active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
@@ -625,6 +628,7 @@ __global__ void __launch_bounds__(PT) precond_tile_kernel(Dims d, Coef<T> c, CVe
 template <typename T, int PT, int PC, int PU>
 __global__ void __launch_bounds__(PT) precond_tile_batched_kernel(Dims d, Coef<T> c, CVec5<T> r, Vec5<T> out,
                                                                   const int* active) {
+  grid_chain();
   if (active && *active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
@@ -823,20 +827,20 @@ void launch_matvec(const Dims& d, const Coef<T>& c, CVec5<T> x, const double* xs
   if (d.tune_mv >= 6 && d.nz >= 2) {  // column march in 1, 2 or 4 z chunks
     const dim3 blk(32, 4, 1);
     dim3 grd((d.nx + 1 + 31) / 32, (d.ny + 1 + 3) / 4, d.tune_mv == 7 ? 2 : (d.tune_mv == 8 ? 4 : 1));
-    matvec_march_kernel<T><<<grd, blk, 0, st>>>(d, c, x, xscale, b, out, active);
+    launch_chained(matvec_march_kernel<T>, grd, blk, 0, st, d, c, x, xscale, b, out, active);
     return;
   }
   if (d.tune_mv == 4 || d.tune_mv == 5) {  // two or four levels per thread
     const dim3 blk(32, 8, 1);
     const int lv = d.tune_mv == 4 ? 2 : 4;
     dim3 grd((d.nx + 1 + 31) / 32, (d.ny + 1 + 7) / 8, (d.nz + lv) / lv);
-    if (lv == 2) matvec_kernel<T, 2><<<grd, blk, 0, st>>>(d, c, x, xscale, b, out, active);
-    else matvec_kernel<T, 4><<<grd, blk, 0, st>>>(d, c, x, xscale, b, out, active);
+    if (lv == 2) launch_chained(matvec_kernel<T, 2>, grd, blk, 0, st, d, c, x, xscale, b, out, active);
+    else launch_chained(matvec_kernel<T, 4>, grd, blk, 0, st, d, c, x, xscale, b, out, active);
     return;
   }
   const dim3 blk = stencil_block(d.tune_mv);
   dim3 grd((d.nx + 1 + blk.x - 1) / blk.x, (d.ny + 1 + blk.y - 1) / blk.y, (d.nz + 1 + blk.z - 1) / blk.z);
-  matvec_kernel<T, 1><<<grd, blk, 0, st>>>(d, c, x, xscale, b, out, active);
+  launch_chained(matvec_kernel<T, 1>, grd, blk, 0, st, d, c, x, xscale, b, out, active);
 }
 
 // ---------------------------------------------------------------------------
@@ -853,6 +857,7 @@ void launch_matvec(const Dims& d, const Coef<T>& c, CVec5<T> x, const double* xs
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT) precond_march_kernel(Dims d, Coef<T> c, CVec5<T> r, Vec5<T> out,
                                                            const int* active) {
+  grid_chain();
   if (active && *active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* s_d = reinterpret_cast<T*>(smem_raw);  // [nz][NT]
@@ -928,7 +933,7 @@ void launch_precond_march(const Dims& d, const Coef<T>& c, CVec5<T> r, Vec5<T> o
     cudaMemcpyAsync(out.f[0], r.f[0], sizeof(T) * field_size(d, LOC_U), cudaMemcpyDeviceToDevice, st);
   if (out.f[1] != r.f[1])
     cudaMemcpyAsync(out.f[1], r.f[1], sizeof(T) * field_size(d, LOC_V), cudaMemcpyDeviceToDevice, st);
-  precond_march_kernel<T, NT><<<dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st>>>(d, c, r, out, active);
+  launch_chained(precond_march_kernel<T, NT>, dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st, d, c, r, out, active);
 }
 
 // ---------------------------------------------------------------------------
@@ -1092,6 +1097,7 @@ __device__ __forceinline__ void precond_pipe_block(const Dims& d, const Coef<T>&
 template <typename T, int NT, int HINT>
 __global__ void __launch_bounds__(NT) precond_pipe_kernel(Dims d, Coef<T> c, CVec5<T> r, Vec5<T> out,
                                                           const int* active) {
+  grid_chain();
   if (active && *active == 0) return;
   precond_pipe_block<T, NT, HINT>(d, c, r, out, blockIdx.x, blockIdx.y);
 }
@@ -1107,6 +1113,7 @@ __global__ void __launch_bounds__(NT) precond_pipe_kernel(Dims d, Coef<T> c, CVe
 template <typename T, int NT, int S>
 __global__ void __launch_bounds__(NT) precond_async_kernel(Dims d, Coef<T> c, CVec5<T> r, Vec5<T> out,
                                                            const int* active) {
+  grid_chain();
   if (active && *active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nz = d.nz;
@@ -1229,7 +1236,8 @@ void launch_precond_async(const Dims& d, const Coef<T>& c, CVec5<T> r, Vec5<T> o
     cudaMemcpyAsync(out.f[0], r.f[0], sizeof(T) * field_size(d, LOC_U), cudaMemcpyDeviceToDevice, st);
   if (out.f[1] != r.f[1])
     cudaMemcpyAsync(out.f[1], r.f[1], sizeof(T) * field_size(d, LOC_V), cudaMemcpyDeviceToDevice, st);
-  precond_async_kernel<T, NT, S><<<dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st>>>(d, c, r, out, active);
+  launch_chained(precond_async_kernel<T, NT, S>, dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st, d, c, r, out,
+                 active);
 }
 
 template <typename T, int NT, int HINT>
@@ -1243,7 +1251,8 @@ void launch_precond_pipe(const Dims& d, const Coef<T>& c, CVec5<T> r, Vec5<T> ou
     cudaMemcpyAsync(out.f[0], r.f[0], sizeof(T) * field_size(d, LOC_U), cudaMemcpyDeviceToDevice, st);
   if (out.f[1] != r.f[1])
     cudaMemcpyAsync(out.f[1], r.f[1], sizeof(T) * field_size(d, LOC_V), cudaMemcpyDeviceToDevice, st);
-  precond_pipe_kernel<T, NT, HINT><<<dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st>>>(d, c, r, out, active);
+  launch_chained(precond_pipe_kernel<T, NT, HINT>, dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st, d, c, r, out,
+                 active);
 }
 
 template <typename T, int PT, int PC>
@@ -1253,7 +1262,7 @@ void launch_precond_tile(const Dims& d, const Coef<T>& c, CVec5<T> r, Vec5<T> ou
   static SmemLimit attr_bytes;  // per instantiation
   ensure_smem_limit((const void*)precond_tile_kernel<T, PT, PC>, attr_bytes, smem);
   dim3 grd((d.nx + PC - 1) / PC, d.ny);
-  precond_tile_kernel<T, PT, PC><<<grd, PT, smem, st>>>(d, c, r, out, active);
+  launch_chained(precond_tile_kernel<T, PT, PC>, grd, PT, smem, st, d, c, r, out, active);
 }
 
 template <typename T, int PT, int PC, int PU>
@@ -1263,7 +1272,7 @@ void launch_precond_tile_batched(const Dims& d, const Coef<T>& c, CVec5<T> r, Ve
   static SmemLimit attr_bytes;  // per instantiation
   ensure_smem_limit((const void*)precond_tile_batched_kernel<T, PT, PC, PU>, attr_bytes, smem);
   dim3 grd((d.nx + PC - 1) / PC, d.ny);
-  precond_tile_batched_kernel<T, PT, PC, PU><<<grd, PT, smem, st>>>(d, c, r, out, active);
+  launch_chained(precond_tile_batched_kernel<T, PT, PC, PU>, grd, PT, smem, st, d, c, r, out, active);
 }
 
 template <typename T>
@@ -1298,6 +1307,7 @@ template <typename T, typename U>
 __global__ void __launch_bounds__(128, sizeof(U) == 4 ? 3 : 2) group_matvec_kernel(GroupMember<T>* mem,
                                                                                   const int* __restrict__ first,
                                                                                   int M, int mode, int j) {
+  grid_chain();
   const int b = blockIdx.x;
   const int mi = group_find(first, M, b);
   const GroupMember<T>& g = mem[mi];
@@ -1340,6 +1350,7 @@ __global__ void __launch_bounds__(128, sizeof(U) == 4 ? 3 : 2) group_matvec_kern
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT) group_precond_kernel(GroupMember<T>* mem, const int* __restrict__ first, int M,
                                                            int mode, int tv, int gated) {
+  grid_chain();
   const int b = blockIdx.x;
   const int mi = group_find(first, M, b);
   const GroupMember<T>& g = mem[mi];
@@ -1369,10 +1380,11 @@ template <typename T>
 void grp_matvec(const GroupLaunch<T>& g, int mode, int j, cudaStream_t st) {
   const int nb = g.blocks(GT_MV);
   if (mode == 2) {
-    if constexpr (sizeof(T) == 4) group_matvec_kernel<T, double><<<nb, dim3(32, 4), 0, st>>>(g.mem, g.row(GT_MV), g.M, 2, 0);
+    if constexpr (sizeof(T) == 4) launch_chained(group_matvec_kernel<T, double>, nb, dim3(32, 4), 0, st, g.mem,
+                                                 g.row(GT_MV), g.M, 2, 0);
     return;
   }
-  group_matvec_kernel<T, T><<<nb, dim3(32, 4), 0, st>>>(g.mem, g.row(GT_MV), g.M, mode, j);
+  launch_chained(group_matvec_kernel<T, T>, nb, dim3(32, 4), 0, st, g.mem, g.row(GT_MV), g.M, mode, j);
 }
 
 template <typename T>
@@ -1382,7 +1394,8 @@ void grp_precond(const GroupLaunch<T>& g, int mode, int t, int gated, cudaStream
   const size_t smem = (size_t)nz_max * GROUP_PC_NT * sizeof(T);
   static SmemLimit attr_bytes;
   ensure_smem_limit((const void*)group_precond_kernel<T, GROUP_PC_NT>, attr_bytes, smem);
-  group_precond_kernel<T, GROUP_PC_NT><<<g.blocks(GT_PC), GROUP_PC_NT, smem, st>>>(g.mem, g.row(GT_PC), g.M, mode, t,
+  launch_chained(group_precond_kernel<T, GROUP_PC_NT>, g.blocks(GT_PC), GROUP_PC_NT, smem, st, g.mem, g.row(GT_PC),
+                 g.M, mode, t,
                                                                                    gated);
 }
 

@@ -65,6 +65,7 @@ __device__ __forceinline__ double rho_at(const Scalars& s, const Base64& b, int 
 // One thread per point of the (nx+1, ny+1, nz+1) union box.
 template <typename T>
 __global__ void prep_points(Dims d, Scalars s, Base64 b, PtrTable<T> out) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -181,6 +182,7 @@ __global__ void prep_points(Dims d, Scalars s, Base64 b, PtrTable<T> out) {
 //   c'(k) = upper(k) / pivot(k).
 template <typename T>
 __global__ void prep_thomas(Dims d, Scalars s, Base64 b, PtrTable<T> out) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -216,8 +218,8 @@ template <typename T>
 void launch_prepare(const Dims& d, const Scalars& s, const Base64& b, PtrTable<T> out, cudaStream_t st) {
   dim3 blk(32, 4, 2);
   dim3 grd((d.nx + 1 + blk.x - 1) / blk.x, (d.ny + 1 + blk.y - 1) / blk.y, (d.nz + 1 + blk.z - 1) / blk.z);
-  prep_points<T><<<grd, blk, 0, st>>>(d, s, b, out);
-  prep_thomas<T><<<dim3((d.nx + 127) / 128, d.ny), 128, 0, st>>>(d, s, b, out);
+  launch_chained(prep_points<T>, grd, blk, 0, st, d, s, b, out);
+  launch_chained(prep_thomas<T>, dim3((d.nx + 127) / 128, d.ny), 128, 0, st, d, s, b, out);
 }
 
 template Coef<float> make_coef<float>(float* const*, const Scalars&);

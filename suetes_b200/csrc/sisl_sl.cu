@@ -27,6 +27,7 @@ __global__ void traj_velocity_kernel(Dims d, Coef<T> c, const T* __restrict__ u,
                                      const T* __restrict__ e, const T* __restrict__ up,
                                      const T* __restrict__ vp, const T* __restrict__ ep, int extrap,
                                      PtrTable<T> vel) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -249,6 +250,7 @@ __device__ __forceinline__ T tricubic_rel(const T* __restrict__ f, const Ext& e,
 template <typename T>
 __global__ void departure_kernel(Dims d, int loc, T dt, const T* __restrict__ vx, const T* __restrict__ vy,
                                  const T* __restrict__ vz, int iters, T* cx, T* cy, T* cz, int relative) {
+  grid_chain();
   const Ext e = loc_ext(d, loc);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -267,6 +269,7 @@ template <typename T>
 __global__ void tricubic_kernel(Ext src, Ext dst, const T* __restrict__ f, const T* __restrict__ cx,
                                 const T* __restrict__ cy, const T* __restrict__ cz, T* out, int limiter,
                                 T scale) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -278,6 +281,7 @@ __global__ void tricubic_kernel(Ext src, Ext dst, const T* __restrict__ f, const
 template <typename T>
 __global__ void trilinear_kernel(Ext src, Ext dst, const T* __restrict__ f, const T* __restrict__ cx,
                                  const T* __restrict__ cy, const T* __restrict__ cz, T* out) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -292,6 +296,7 @@ template <typename T>
 __global__ void sl_advect_kernel(Dims d, int loc, T dt, const T* __restrict__ vx, const T* __restrict__ vy,
                                  const T* __restrict__ vz, int iters, int nf, const T* __restrict__ f0,
                                  const T* __restrict__ f1, T* o0, T* o1, T s0, T s1, int limiter) {
+  grid_chain();
   const Ext e = loc_ext(d, loc);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -314,7 +319,7 @@ template <typename T>
 void launch_traj_velocity(const Dims& d, const Coef<T>& c, const T* u, const T* v, const T* eta, const T* up,
                           const T* vp, const T* etap, int extrapolate, PtrTable<T> vel, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  traj_velocity_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(
+  launch_chained(traj_velocity_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st,
       d, c, u, v, eta, up, vp, etap, extrapolate, vel);
 }
 
@@ -322,7 +327,7 @@ template <typename T>
 void launch_departure(const Dims& d, int loc, double dt, const T* const* vel3, int iterations, T* const* coords3,
                       int relative, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  departure_kernel<T><<<box_grid(ext_x(d, loc), ext_y(d, loc), ext_z(d, loc), blk), blk, 0, st>>>(
+  launch_chained(departure_kernel<T>, box_grid(ext_x(d, loc), ext_y(d, loc), ext_z(d, loc), blk), blk, 0, st,
       d, loc, (T)dt, vel3[0], vel3[1], vel3[2], iterations, coords3[0], coords3[1], coords3[2], relative);
 }
 
@@ -330,7 +335,7 @@ template <typename T>
 void launch_tricubic_ext(int sx, int sy, int sz, int dx, int dy, int dz, const T* field, const T* const* coords3,
                          T* out, int use_limiter, T scale, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  tricubic_kernel<T><<<box_grid(dx, dy, dz, blk), blk, 0, st>>>(Ext{sx, sy, sz}, Ext{dx, dy, dz}, field,
+  launch_chained(tricubic_kernel<T>, box_grid(dx, dy, dz, blk), blk, 0, st, Ext{sx, sy, sz}, Ext{dx, dy, dz}, field,
                                                                coords3[0], coords3[1], coords3[2], out,
                                                                use_limiter, scale);
 }
@@ -339,7 +344,7 @@ template <typename T>
 void launch_trilinear_ext(int sx, int sy, int sz, int dx, int dy, int dz, const T* field, const T* const* coords3,
                           T* out, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  trilinear_kernel<T><<<box_grid(dx, dy, dz, blk), blk, 0, st>>>(Ext{sx, sy, sz}, Ext{dx, dy, dz}, field,
+  launch_chained(trilinear_kernel<T>, box_grid(dx, dy, dz, blk), blk, 0, st, Ext{sx, sy, sz}, Ext{dx, dy, dz}, field,
                                                                 coords3[0], coords3[1], coords3[2], out);
 }
 
@@ -347,7 +352,7 @@ template <typename T>
 void launch_sl_advect(const Dims& d, int loc, double dt, const T* const* vel3, int iterations, int nf,
                       const T* const* fields, T* const* outs, const T* scales, int use_limiter, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  sl_advect_kernel<T><<<box_grid(ext_x(d, loc), ext_y(d, loc), ext_z(d, loc), blk), blk, 0, st>>>(
+  launch_chained(sl_advect_kernel<T>, box_grid(ext_x(d, loc), ext_y(d, loc), ext_z(d, loc), blk), blk, 0, st,
       d, loc, (T)dt, vel3[0], vel3[1], vel3[2], iterations, nf, fields[0], nf > 1 ? fields[1] : nullptr,
       outs[0], nf > 1 ? outs[1] : nullptr, scales[0], nf > 1 ? scales[1] : T(0), use_limiter);
 }

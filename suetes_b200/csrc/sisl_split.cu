@@ -34,6 +34,7 @@ __device__ __forceinline__ T kinematic(const Dims& d, const Coef<T>& c, const Wi
 template <typename T>
 __global__ void split_diag_kernel(Dims d, Coef<T> c, const T* __restrict__ u, const T* __restrict__ v,
                                   const T* w_in, T* eta_out, T* w_out) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -103,6 +104,7 @@ template <typename T>
 __global__ void __launch_bounds__(AX * AY, sizeof(T) == 4 ? 3 : 2) split_adv_kernel(
     Dims d, Coef<T> c, const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ w,
     const T* __restrict__ eta, const T* __restrict__ th, T eps_l, PtrTable<T> out, int chunk) {
+  grid_chain();
   __shared__ T Qt[2][4][AY + 4][AX + 4];
   const int i0 = blockIdx.x * AX, j0 = blockIdx.y * AY;
   const int tx = threadIdx.x, ty = threadIdx.y;
@@ -185,6 +187,7 @@ __global__ void __launch_bounds__(AX * AY, sizeof(T) == 4 ? 3 : 2) split_adv_ker
 // adv4 at mass points averaged to the u faces, v faces and w levels
 template <typename T>
 __global__ void split_slow_kernel(Dims d, PtrTable<T> t, PtrTable<T> sf) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -218,6 +221,7 @@ __global__ void split_slow_kernel(Dims d, PtrTable<T> t, PtrTable<T> sf) {
 
 template <typename T>
 __global__ void split_init_kernel(Dims d, SplitArgs<T> a) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -279,6 +283,7 @@ __device__ __forceinline__ void div_tile(const Dims& d, const Coef<T>& c, const 
 // previous corrector (gx0_ready) on the others.
 template <typename T>
 __global__ void __launch_bounds__(SX * SY) split_predict_kernel(Dims d, Coef<T> c, SplitArgs<T> a) {
+  grid_chain();
   __shared__ T Dt[SY + 1][SX + 1];
   const int i0 = blockIdx.x * SX, j0 = blockIdx.y * SY, k = blockIdx.z;
   const int tx = threadIdx.x, ty = threadIdx.y;
@@ -339,6 +344,7 @@ __global__ void __launch_bounds__(SX * SY) split_predict_kernel(Dims d, Coef<T> 
 // gradient of delta pi.  One thread per column; cpr/dpr hold the sweep.
 template <typename T>
 __global__ void __launch_bounds__(128) split_column_kernel(Dims d, Coef<T> c, SplitArgs<T> a, T a2cp, T adcp) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -422,6 +428,7 @@ __global__ void __launch_bounds__(128) split_column_kernel(Dims d, Coef<T> c, Sp
 template <typename T, int PT, int PC>
 __global__ void __launch_bounds__(PT) split_column_tile_kernel(Dims d, Coef<T> c, SplitArgs<T> a, T a2cp,
                                                                T adcp) {
+  grid_chain();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
   const int nx = d.nx, nz = d.nz;
@@ -523,6 +530,7 @@ __global__ void __launch_bounds__(PT) split_column_tile_kernel(Dims d, Coef<T> c
 template <typename T>
 __global__ void __launch_bounds__(SX * SY) split_correct_kernel(Dims d, Coef<T> c, SplitArgs<T> a,
                                                                 T* __restrict__ upp2, T* __restrict__ vpp2) {
+  grid_chain();
   __shared__ T Dt[SY + 1][SX + 1];
   const int i0 = blockIdx.x * SX, j0 = blockIdx.y * SY, k = blockIdx.z;
   const int tx = threadIdx.x, ty = threadIdx.y;
@@ -570,6 +578,7 @@ __global__ void __launch_bounds__(SX * SY) split_correct_kernel(Dims d, Coef<T> 
 
 template <typename T>
 __global__ void split_end_kernel(Dims d, SplitArgs<T> a, T dtns, T* u, T* v, T* w, T* eta, T* pp, T* th) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -596,6 +605,7 @@ __global__ void split_end_kernel(Dims d, SplitArgs<T> a, T dtns, T* u, T* v, T* 
 
 template <typename T>
 __global__ void split_axpy_kernel(size_t n, const T* __restrict__ b, T* a) {
+  grid_chain();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
     a[q] = a[q] + b[q];
 }
@@ -606,7 +616,7 @@ template <typename T>
 void launch_split_diag(const Dims& d, const Coef<T>& c, const T* u, const T* v, const T* w_in, T* eta_out,
                        T* w_out, cudaStream_t st) {
   const dim3 blk(32, 4, 2);
-  split_diag_kernel<T><<<box(d.nx, d.ny, d.nz + 1, blk), blk, 0, st>>>(d, c, u, v, w_in, eta_out, w_out);
+  launch_chained(split_diag_kernel<T>, box(d.nx, d.ny, d.nz + 1, blk), blk, 0, st, d, c, u, v, w_in, eta_out, w_out);
 }
 
 template <typename T>
@@ -618,7 +628,8 @@ void launch_split_adv(const Dims& d, const Coef<T>& c, const T* u, const T* v, c
   // 16 levels a block where that leaves two blocks an SM, else 8: a chunk's start reads four levels more
   const int tiles = ((d.nx + AX - 1) / AX) * ((d.ny + AY - 1) / AY);
   const int chunk = tiles * ((d.nz + 15) / 16) >= 2 * 148 ? 16 : 8;
-  split_adv_kernel<T><<<dim3((d.nx + AX - 1) / AX, (d.ny + AY - 1) / AY, (d.nz + chunk - 1) / chunk), blk, 0, st>>>(
+  launch_chained(split_adv_kernel<T>, dim3((d.nx + AX - 1) / AX, (d.ny + AY - 1) / AY, (d.nz + chunk - 1) / chunk),
+                 blk, 0, st,
       d, c, u, v, w, eta, th, eps_l, o, chunk);
 }
 
@@ -629,19 +640,19 @@ void launch_split_slow(const Dims& d, const T* const* tend6, const T* const* adv
   for (int q = 0; q < 6; ++q) t.p[q] = const_cast<T*>(tend6[q]);
   for (int q = 0; q < 4; ++q) t.p[6 + q] = const_cast<T*>(adv4[q]);
   for (int q = 0; q < 5; ++q) s.p[q] = sf5[q];
-  split_slow_kernel<T><<<box(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, t, s);
+  launch_chained(split_slow_kernel<T>, box(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, t, s);
 }
 
 template <typename T>
 void launch_split_init(const Dims& d, const SplitArgs<T>& a, cudaStream_t st) {
   const dim3 blk(32, 4, 2);
-  split_init_kernel<T><<<box(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, a);
+  launch_chained(split_init_kernel<T>, box(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, a);
 }
 
 template <typename T>
 void launch_split_predict(const Dims& d, const Coef<T>& c, const SplitArgs<T>& a, cudaStream_t st) {
   const dim3 blk(SX, SY, 1);
-  split_predict_kernel<T><<<box(d.nx + 1, d.ny + 1, d.nz, blk), blk, 0, st>>>(d, c, a);
+  launch_chained(split_predict_kernel<T>, box(d.nx + 1, d.ny + 1, d.nz, blk), blk, 0, st, d, c, a);
 }
 
 template <typename T>
@@ -653,17 +664,18 @@ void launch_split_column(const Dims& d, const Coef<T>& c, const SplitArgs<T>& a,
   if (smem <= 200 * 1024) {  // tiles of 32 columns; the one-thread-per-column march beyond
     static SmemLimit attr_bytes;  // per instantiation
     ensure_smem_limit((const void*)split_column_tile_kernel<T, PT, PC>, attr_bytes, smem);
-    split_column_tile_kernel<T, PT, PC><<<dim3((d.nx + PC - 1) / PC, d.ny), PT, smem, st>>>(d, c, a, a2cp, adcp);
+    launch_chained(split_column_tile_kernel<T, PT, PC>, dim3((d.nx + PC - 1) / PC, d.ny), PT, smem, st, d, c, a,
+                   a2cp, adcp);
     return;
   }
-  split_column_kernel<T><<<dim3((d.nx + 127) / 128, d.ny), 128, 0, st>>>(d, c, a, a2cp, adcp);
+  launch_chained(split_column_kernel<T>, dim3((d.nx + 127) / 128, d.ny), 128, 0, st, d, c, a, a2cp, adcp);
 }
 
 template <typename T>
 void launch_split_correct(const Dims& d, const Coef<T>& c, const SplitArgs<T>& a, T* upp2, T* vpp2,
                           cudaStream_t st) {
   const dim3 blk(SX, SY, 1);
-  split_correct_kernel<T><<<box(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, c, a, upp2, vpp2);
+  launch_chained(split_correct_kernel<T>, box(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, c, a, upp2, vpp2);
 }
 
 template <typename T>
@@ -671,12 +683,13 @@ void launch_split_end(const Dims& d, const SplitArgs<T>& a, int nsteps, T* u, T*
                       cudaStream_t st) {
   const dim3 blk(32, 4, 2);
   const T dtns = (T)((double)a.dtau * nsteps);
-  split_end_kernel<T><<<box(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, a, dtns, u, v, w, eta, p, th);
+  launch_chained(split_end_kernel<T>, box(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, a, dtns, u, v, w, eta,
+                 p, th);
 }
 
 template <typename T>
 void launch_split_axpy(size_t n, const T* b, T* a, cudaStream_t st) {
-  split_axpy_kernel<T><<<(unsigned)std::min<size_t>((n + 255) / 256, 148 * 16), 256, 0, st>>>(n, b, a);
+  launch_chained(split_axpy_kernel<T>, (unsigned)std::min<size_t>((n + 255) / 256, 148 * 16), 256, 0, st, n, b, a);
 }
 
 #define SISL_INST_SPLIT(T)                                                                                       \

@@ -25,6 +25,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) stagger_kernel(Shape3 in, Shape3 out, int axis, int to_face, int periodic,
                                                       T c0, T c1, const T* __restrict__ mult,
                                                       const T* __restrict__ f, T* __restrict__ o) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(256) stagger_t_kernel(Shape3 in, Shape3 out, i
                                                         int periodic, int stop_grad, T c0, T c1,
                                                         const T* __restrict__ mult, const T* __restrict__ g,
                                                         T* __restrict__ gin) {
+  grid_chain();
   // one thread per INPUT point; g has the output shape
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -110,9 +112,11 @@ void launch_stagger(const int in_shape[3], int axis, int to_face, int periodic, 
   out.e[axis] += to_face ? 1 : -1;
   dim3 blk(32, 4, 2);
   if (!transpose)
-    stagger_kernel<T><<<sgrid(out, blk), blk, 0, st>>>(in, out, axis, to_face, periodic, c0, c1, mult, src, dst);
+    launch_chained(stagger_kernel<T>, sgrid(out, blk), blk, 0, st, in, out, axis, to_face, periodic, c0, c1, mult,
+                   src, dst);
   else
-    stagger_t_kernel<T><<<sgrid(in, blk), blk, 0, st>>>(in, out, axis, to_face, periodic, stop_grad, c0, c1, mult,
+    launch_chained(stagger_t_kernel<T>, sgrid(in, blk), blk, 0, st, in, out, axis, to_face, periodic, stop_grad, c0,
+                   c1, mult,
                                                         src, dst);
 }
 

@@ -113,6 +113,7 @@ __device__ __forceinline__ void radd(T* p, int i, T v) {
 // field[q] += sum * 2^-e for every registered field (one rounding per element)
 template <typename T>
 __global__ void det_finish_kernel(DetSink<T> s) {
+  grid_chain();
   for (int f = 0; f < s.n; ++f) {
     const unsigned gb = s.gmax[f];
     if (gb == 0u) continue;  // no contribution
@@ -455,6 +456,7 @@ __device__ __forceinline__ void explicit_vjp_point(const Dims& d, const Coef<T>&
 template <typename T>
 __global__ void __launch_bounds__(256) explicit_vjp_kernel(Dims d, Coef<T> c, ExplicitIn<T> in, ExplicitBar<T> bi,
                                                            StateBar<T> bo, int mode, DetSink<T> sink) {
+  grid_chain();
   det_begin(sink);
   explicit_vjp_point(d, c, in, bi, bo, mode);
   det_end<T>();
@@ -553,6 +555,7 @@ __device__ __forceinline__ void corrector_vjp_point(const Dims& d, const Coef<T>
 template <typename T>
 __global__ void __launch_bounds__(256) corrector_vjp_kernel(Dims d, Coef<T> c, CorrectorIn<T> in,
                                                             CorrectorBar<T> cb, DetSink<T> sink) {
+  grid_chain();
   det_begin(sink);
   corrector_vjp_point(d, c, in, cb);
   det_end<T>();
@@ -562,6 +565,7 @@ __global__ void __launch_bounds__(256) corrector_vjp_kernel(Dims d, Coef<T> c, C
 template <typename T>
 __global__ void corrector_theta_vjp_kernel(Dims d, Coef<T> c, const T* __restrict__ tb, T* thab, T* tthb, T* wnb,
                                            T* wxb) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -589,6 +593,7 @@ __global__ void corrector_theta_vjp_kernel(Dims d, Coef<T> c, const T* __restric
 // and lid rows are zero
 template <typename T>
 __global__ void fixup_vjp_kernel(Dims d, T* rub, T* rvb, T* ub, T* vb, T* reb) {
+  grid_chain();
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
   const int k = blockIdx.z;
@@ -625,6 +630,7 @@ __global__ void fixup_vjp_kernel(Dims d, T* rub, T* rvb, T* ub, T* vb, T* reb) {
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256) finalize_vjp_kernel(Dims d, Coef<T> c, FinalizeBar<T> fb) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -676,6 +682,7 @@ __global__ void __launch_bounds__(256) finalize_vjp_kernel(Dims d, Coef<T> c, Fi
 // the divergence padded (stop_gradient) on non-periodic edges
 template <typename T>
 __global__ void div_t_kernel(Dims d, Coef<T> c, const T* __restrict__ ub, const T* __restrict__ vb, T* divb) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -695,6 +702,7 @@ __global__ void div_t_kernel(Dims d, Coef<T> c, const T* __restrict__ ub, const 
 // winds += D_centre^T(div_bar), div = m (du/dx + dv/dy)
 template <typename T>
 __global__ void div_winds_t_kernel(Dims d, Coef<T> c, const T* __restrict__ divb, T* ub, T* vb) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -721,6 +729,7 @@ __global__ void div_winds_t_kernel(Dims d, Coef<T> c, const T* __restrict__ divb
 template <typename T>
 __global__ void __launch_bounds__(256) lap_t_faces_kernel(Dims d, Coef<T> c, PtrTable<T> bt, PtrTable<T> gxb,
                                                           PtrTable<T> gyb, T scale) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int kz = blockIdx.z * blockDim.z + threadIdx.z;
@@ -759,6 +768,7 @@ __global__ void __launch_bounds__(256) lap_t_faces_kernel(Dims d, Coef<T> c, Ptr
 template <typename T>
 __global__ void __launch_bounds__(256) lap_t_mass_kernel(Dims d, Coef<T> c, PtrTable<T> gxb, PtrTable<T> gyb,
                                                          PtrTable<T> out) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int kz = blockIdx.z * blockDim.z + threadIdx.z;
@@ -798,6 +808,7 @@ __global__ void __launch_bounds__(256) lap_t_mass_kernel(Dims d, Coef<T> c, PtrT
 // state cotangents += transpose of the mass-point copies (hyper_src_kernel)
 template <typename T>
 __global__ void hyper_src_t_kernel(Dims d, PtrTable<T> s, T* ub, T* vb, T* wb, T* thb) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -852,6 +863,7 @@ __device__ __forceinline__ void kinematic_adj(const Dims& d, const Coef<T>& c, c
 template <typename T>
 __global__ void __launch_bounds__(256) split_diag_vjp_kernel(Dims d, Coef<T> c, T* wb, T* eb, T* ub, T* vb,
                                                              DetSink<T> sink) {
+  grid_chain();
   det_begin(sink);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -941,6 +953,7 @@ struct FaceBar {
 constexpr int VJP_KC = 4;
 template <typename T, bool PRED>
 __global__ void __launch_bounds__(256) split_faces_vjp_kernel(Dims d, Coef<T> c, SplitBar<T> b) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -1048,6 +1061,7 @@ __device__ __forceinline__ T col_flux_bar(const Dims& d, const Coef<T>& c, T dta
 // s2 for the faces' kernel.
 template <typename T>
 __global__ void __launch_bounds__(128) split_column_vjp_kernel(Dims d, Coef<T> c, SplitBar<T> b, T a2cp, T adcp) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -1119,6 +1133,7 @@ __global__ void __launch_bounds__(128) split_column_vjp_kernel(Dims d, Coef<T> c
 template <typename T, int PT, int PC>
 __global__ void __launch_bounds__(PT) split_column_vjp_tile_kernel(Dims d, Coef<T> c, SplitBar<T> b, T a2cp,
                                                                    T adcp) {
+  grid_chain();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nx = d.nx, nz = d.nz;
   T* s_x = reinterpret_cast<T*>(smem_raw);  // [nz][PC] x_bar -> r
@@ -1209,6 +1224,7 @@ __global__ void __launch_bounds__(PT) split_column_vjp_tile_kernel(Dims d, Coef<
 // per column of the union box and VJP_KC levels.
 template <typename T>
 __global__ void __launch_bounds__(256) split_column_faces_vjp_kernel(Dims d, Coef<T> c, SplitBar<T> b) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -1271,6 +1287,7 @@ __global__ void __launch_bounds__(256) split_column_faces_vjp_kernel(Dims d, Coe
 template <typename T>
 __global__ void split_end_vjp_kernel(Dims d, PtrTable<T> o, PtrTable<T> cb, T* th0b, T* upp, T* vpp, T* wpp, T* ppp,
                                      T* sfth, T dtns) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -1309,6 +1326,7 @@ template <typename T>
 __global__ void split_init_vjp_kernel(Dims d, const T* __restrict__ upp, const T* __restrict__ vpp,
                                       const T* __restrict__ wpp, const T* __restrict__ ppp, PtrTable<T> s,
                                       PtrTable<T> cb) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -1341,6 +1359,7 @@ __global__ void split_init_vjp_kernel(Dims d, const T* __restrict__ upp, const T
 template <typename T>
 __global__ void __launch_bounds__(256) split_slow_vjp_kernel(Dims d, PtrTable<T> sf, PtrTable<T> t, PtrTable<T> a,
                                                              DetSink<T> sink) {
+  grid_chain();
   det_begin(sink);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1449,6 +1468,7 @@ struct AdvBar {
 template <typename T>
 __global__ void __launch_bounds__(256) split_adv_vjp_mass_kernel(Dims d, Coef<T> c, AdvIn<T> in, PtrTable<T> qb,
                                                                  T* thb) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -1501,6 +1521,7 @@ __global__ void __launch_bounds__(256) split_adv_vjp_mass_kernel(Dims d, Coef<T>
 template <typename T>
 __global__ void __launch_bounds__(256) split_adv_vjp_faces_kernel(Dims d, Coef<T> c, AdvIn<T> in, PtrTable<T> qb,
                                                                   T* ub, T* vb, T* wb, T* eb) {
+  grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
@@ -1623,7 +1644,7 @@ void det_run(DetSink<T> s, Launch&& launch, cudaStream_t st) {
     cudaMemsetAsync(s.acc[f], 0, (sizeof(T) == 8 ? 2 : 1) * sizeof(unsigned long long) * (size_t)s.len[f], st);
   s.mode = 2;
   launch(s);
-  det_finish_kernel<T><<<148 * 8, 256, 0, st>>>(s);
+  launch_chained(det_finish_kernel<T>, 148 * 8, 256, 0, st, s);
 }
 }  // namespace
 
@@ -1635,7 +1656,8 @@ void launch_explicit_vjp(const Dims& d, const Coef<T>& c, const ExplicitIn<T>& i
   T* dst[10] = {bo.u, bo.v, bo.w, bo.eta, bo.pi, bo.th, bo.hyper[0], bo.hyper[1], bo.hyper[2], bo.hyper[3]};
   const unsigned len[10] = {(unsigned)field_size(d, LOC_U), (unsigned)field_size(d, LOC_V), w, w, m, m, m, m, m, m};
   det_run<T>(det_make<T>(det_scratch, dst, len, 10), [&](const DetSink<T>& s) {
-    explicit_vjp_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, c, in, bi, bo, mode, s);
+    launch_chained(explicit_vjp_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, c, in, bi, bo,
+                   mode, s);
   }, st);
 }
 
@@ -1648,7 +1670,7 @@ void launch_corrector_vjp(const Dims& d, const Coef<T>& c, const CorrectorIn<T>&
   T* dst[12] = {cb.rhs_u, cb.rhs_v, cb.rhs_w, cb.rhs_pi, cb.reta, cb.th, cb.pg, cb.gu, cb.gv, cb.geta, cb.ug, cb.vg};
   const unsigned len[12] = {fu, fv, w, m, w, m, m, fu, fv, w, fu, fv};
   det_run<T>(det_make<T>(det_scratch, dst, len, 12), [&](const DetSink<T>& s) {
-    corrector_vjp_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, c, in, cb, s);
+    launch_chained(corrector_vjp_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, c, in, cb, s);
   }, st);
 }
 
@@ -1656,7 +1678,8 @@ template <typename T>
 void launch_corrector_theta_vjp(const Dims& d, const Coef<T>& c, const T* thn_bar, T* tha_bar, T* tth_bar,
                                 T* w_now_bar, T* w_next_bar, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  corrector_theta_vjp_kernel<T><<<box_grid(d.nx, d.ny, d.nz + 1, blk), blk, 0, st>>>(d, c, thn_bar, tha_bar,
+  launch_chained(corrector_theta_vjp_kernel<T>, box_grid(d.nx, d.ny, d.nz + 1, blk), blk, 0, st, d, c, thn_bar,
+                 tha_bar,
                                                                                    tth_bar, w_now_bar, w_next_bar);
 }
 
@@ -1664,16 +1687,18 @@ template <typename T>
 void launch_fixup_vjp(const Dims& d, T* ru_bar, T* rv_bar, T* u_bar, T* v_bar, T* reta_bar, cudaStream_t st) {
   const int na = (d.nx > d.ny ? d.nx : d.ny);
   const int nk = (d.nz > d.ny ? d.nz : d.ny);
-  fixup_vjp_kernel<T><<<dim3((na + 127) / 128, 3, nk), 128, 0, st>>>(d, ru_bar, rv_bar, u_bar, v_bar, reta_bar);
+  launch_chained(fixup_vjp_kernel<T>, dim3((na + 127) / 128, 3, nk), 128, 0, st, d, ru_bar, rv_bar, u_bar, v_bar,
+                 reta_bar);
 }
 
 template <typename T>
 void launch_finalize_vjp(const Dims& d, const Coef<T>& c, const FinalizeBar<T>& fb, T* div_bar, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  finalize_vjp_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, c, fb);
+  launch_chained(finalize_vjp_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, c, fb);
   if (c.s.nu_div != 0.0) {
-    div_t_kernel<T><<<box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st>>>(d, c, fb.x2u, fb.x2v, div_bar);
-    div_winds_t_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz, blk), blk, 0, st>>>(d, c, div_bar, fb.x2u, fb.x2v);
+    launch_chained(div_t_kernel<T>, box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st, d, c, fb.x2u, fb.x2v, div_bar);
+    launch_chained(div_winds_t_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz, blk), blk, 0, st, d, c, div_bar, fb.x2u,
+                   fb.x2v);
   }
 }
 
@@ -1684,11 +1709,12 @@ void launch_hyper_vjp(const Dims& d, const Coef<T>& c, PtrTable<T> hyp_bar, PtrT
   const dim3 gf = box_grid(d.nx + 1, d.ny + 1, 4 * d.nz, blk);
   const dim3 gm = box_grid(d.nx, d.ny, 4 * d.nz, blk);
   // hyp = -nu_h lap(lap(src)): src_bar = lap^T(lap^T(-nu_h hyp_bar))
-  lap_t_faces_kernel<T><<<gf, blk, 0, st>>>(d, c, hyp_bar, gx4, gy4, (T)(-c.s.nu_h));
-  lap_t_mass_kernel<T><<<gm, blk, 0, st>>>(d, c, gx4, gy4, tmp4);
-  lap_t_faces_kernel<T><<<gf, blk, 0, st>>>(d, c, tmp4, gx4, gy4, T(1));
-  lap_t_mass_kernel<T><<<gm, blk, 0, st>>>(d, c, gx4, gy4, hyp_bar);
-  hyper_src_t_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, hyp_bar, u_bar, v_bar,
+  launch_chained(lap_t_faces_kernel<T>, gf, blk, 0, st, d, c, hyp_bar, gx4, gy4, (T)(-c.s.nu_h));
+  launch_chained(lap_t_mass_kernel<T>, gm, blk, 0, st, d, c, gx4, gy4, tmp4);
+  launch_chained(lap_t_faces_kernel<T>, gf, blk, 0, st, d, c, tmp4, gx4, gy4, T(1));
+  launch_chained(lap_t_mass_kernel<T>, gm, blk, 0, st, d, c, gx4, gy4, hyp_bar);
+  launch_chained(hyper_src_t_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, hyp_bar, u_bar,
+                 v_bar,
                                                                                      w_bar, th_bar);
 }
 
@@ -1702,7 +1728,8 @@ void launch_split_diag_vjp(const Dims& d, const Coef<T>& c, T* wb, T* eb, T* ub,
   T* dst[2] = {ub, vb};
   const unsigned len[2] = {(unsigned)field_size(d, LOC_U), (unsigned)field_size(d, LOC_V)};
   det_run<T>(det_make<T>(det_scratch, dst, len, 2), [&](const DetSink<T>& s) {
-    split_diag_vjp_kernel<T><<<box_grid(d.nx, d.ny, d.nz + 1, blk), blk, 0, st>>>(d, c, wb, eb, ub, vb, s);
+    launch_chained(split_diag_vjp_kernel<T>, box_grid(d.nx, d.ny, d.nz + 1, blk), blk, 0, st, d, c, wb, eb, ub, vb,
+                   s);
   }, st);
 }
 
@@ -1710,7 +1737,7 @@ template <typename T>
 void launch_split_substep_vjp(const Dims& d, const Coef<T>& c, const SplitBar<T>& b, cudaStream_t st) {
   const dim3 blk(32, 8, 1);
   const dim3 grd((d.nx + 32) / 32, (d.ny + 8) / 8, (d.nz + VJP_KC) / VJP_KC);
-  split_faces_vjp_kernel<T, false><<<grd, blk, 0, st>>>(d, c, b);  // corrector^T
+  launch_chained(split_faces_vjp_kernel<T, false>, grd, blk, 0, st, d, c, b);  // corrector^T
   {  // column^T, with the forward's alpha dtau products
     const double ad = (double)b.alpha * (double)b.dtau;
     const T a2cp = (T)(ad * ad * c.s.cp), adcp = (T)(ad * c.s.cp);
@@ -1719,14 +1746,14 @@ void launch_split_substep_vjp(const Dims& d, const Coef<T>& c, const SplitBar<T>
     if (smem <= 200 * 1024) {  // tiles of 32 columns; the one-thread-per-column march beyond
       static SmemLimit attr_bytes;  // per instantiation
       ensure_smem_limit((const void*)split_column_vjp_tile_kernel<T, PT, PC>, attr_bytes, smem);
-      split_column_vjp_tile_kernel<T, PT, PC>
-          <<<dim3((d.nx + PC - 1) / PC, d.ny), PT, smem, st>>>(d, c, b, a2cp, adcp);
+      launch_chained(split_column_vjp_tile_kernel<T, PT, PC>, dim3((d.nx + PC - 1) / PC, d.ny), PT, smem, st, d, c,
+                     b, a2cp, adcp);
     } else {
-      split_column_vjp_kernel<T><<<dim3((d.nx + 127) / 128, d.ny), 128, 0, st>>>(d, c, b, a2cp, adcp);
+      launch_chained(split_column_vjp_kernel<T>, dim3((d.nx + 127) / 128, d.ny), 128, 0, st, d, c, b, a2cp, adcp);
     }
-    split_column_faces_vjp_kernel<T><<<grd, blk, 0, st>>>(d, c, b);
+    launch_chained(split_column_faces_vjp_kernel<T>, grd, blk, 0, st, d, c, b);
   }
-  split_faces_vjp_kernel<T, true><<<grd, blk, 0, st>>>(d, c, b);  // predictor^T
+  launch_chained(split_faces_vjp_kernel<T, true>, grd, blk, 0, st, d, c, b);  // predictor^T
 }
 
 template <typename T>
@@ -1738,7 +1765,8 @@ void launch_split_end_vjp(const Dims& d, const T* const* out6, T* const* c6, T* 
     o.p[q] = const_cast<T*>(out6[q]);
     cb.p[q] = c6[q];
   }
-  split_end_vjp_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, o, cb, th0b, upp, vpp,
+  launch_chained(split_end_vjp_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, o, cb, th0b,
+                 upp, vpp,
                                                                                      wpp, ppp, sfth, dtns);
 }
 
@@ -1751,7 +1779,8 @@ void launch_split_init_vjp(const Dims& d, const T* upp, const T* vpp, const T* w
     s.p[q] = s6[q];
     cb.p[q] = c6[q];
   }
-  split_init_vjp_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, upp, vpp, wpp, ppp, s,
+  launch_chained(split_init_vjp_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, upp, vpp, wpp,
+                 ppp, s,
                                                                                       cb);
 }
 
@@ -1766,7 +1795,7 @@ void launch_split_slow_vjp(const Dims& d, const T* const* sf5, T* const* tend6, 
   const unsigned fm = (unsigned)field_size(d, LOC_M);
   const unsigned len[4] = {fm, fm, fm, fm};
   det_run<T>(det_make<T>(det_scratch, a.p, len, 4), [&](const DetSink<T>& s) {
-    split_slow_vjp_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, sf, t, a, s);
+    launch_chained(split_slow_vjp_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, sf, t, a, s);
   }, st);
 }
 
@@ -1778,8 +1807,9 @@ void launch_split_adv_vjp(const Dims& d, const Coef<T>& c, const T* u, const T* 
   AdvIn<T> in{u, v, w, eta, th, {adv4[0], adv4[1], adv4[2], adv4[3]}, eps_l};
   PtrTable<T> qb{};
   for (int q = 0; q < 4; ++q) qb.p[q] = tmp4[q];
-  split_adv_vjp_mass_kernel<T><<<box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st>>>(d, c, in, qb, thb);
-  split_adv_vjp_faces_kernel<T><<<box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st>>>(d, c, in, qb, ub, vb, wb,
+  launch_chained(split_adv_vjp_mass_kernel<T>, box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st, d, c, in, qb, thb);
+  launch_chained(split_adv_vjp_faces_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, c, in,
+                 qb, ub, vb, wb,
                                                                                            eb);
 }
 
