@@ -19,71 +19,81 @@ __device__ __forceinline__ Ext loc_ext(const Dims& d, int loc) {
 }
 
 // ---------------------------------------------------------------------------
-// index velocities of every stagger, one thread per union-box point
+// index velocities of every stagger, TV_LV levels of a union-box column per
+// thread: their loads are in flight together and the levels share eta_dot.
+// EX: extrapolate (1.5 x - 0.5 x_prev); a run-time flag there put a wait
+// between the loads (384x384x96 float32, mass points only: 100 us).
 // vel[loc*3 + 0..2] = (u * m / dx, v * m / dy, eta_dot) averaged to loc.
 // ---------------------------------------------------------------------------
 template <typename T>
+constexpr int TV_LV = sizeof(T) == 4 ? 4 : 1;
+template <typename T, bool EX>
 __global__ void traj_velocity_kernel(Dims d, Coef<T> c, const T* __restrict__ u, const T* __restrict__ v,
                                      const T* __restrict__ e, const T* __restrict__ up,
-                                     const T* __restrict__ vp, const T* __restrict__ ep, int extrap,
+                                     const T* __restrict__ vp, const T* __restrict__ ep,
                                      PtrTable<T> vel) {
   grid_chain();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z * blockDim.z + threadIdx.z;
+  const int k0 = (blockIdx.z * blockDim.z + threadIdx.z) * TV_LV<T>;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  if (i > nx || j > ny || k > nz) return;
+  if (i > nx || j > ny) return;
   const T idx = (T)(1.0 / d.dx), idy = (T)(1.0 / d.dy);
   auto U = [&](int a, int b, int cc) {
     const int p = iu(d, a, b, cc);
-    return extrap ? T(1.5) * ld(u, p) - T(0.5) * ld(up, p) : ld(u, p);
+    return EX ? T(1.5) * ld(u, p) - T(0.5) * ld(up, p) : ld(u, p);
   };
   auto V = [&](int a, int b, int cc) {
     const int p = iv(d, a, b, cc);
-    return extrap ? T(1.5) * ld(v, p) - T(0.5) * ld(vp, p) : ld(v, p);
+    return EX ? T(1.5) * ld(v, p) - T(0.5) * ld(vp, p) : ld(v, p);
   };
   auto E = [&](int a, int b, int cc) {
     const int p = iw(d, a, b, cc);
-    return extrap ? T(1.5) * ld(e, p) - T(0.5) * ld(ep, p) : ld(e, p);
+    return EX ? T(1.5) * ld(e, p) - T(0.5) * ld(ep, p) : ld(e, p);
   };
   auto Um = [&](int a, int b, int cc) { return T(0.5) * (U(a, b, cc) + U(a + 1, b, cc)); };
   auto Vm = [&](int a, int b, int cc) { return T(0.5) * (V(a, b, cc) + V(a, b + 1, cc)); };
   auto Em = [&](int a, int b, int cc) { return T(0.5) * (E(a, b, cc) + E(a, b, cc + 1)); };
 
   // a null first pointer skips a stagger
-  if (vel.p[0] && i < nx && j < ny && k < nz) {  // m
-    const int p = im(d, i, j, k);
-    const T m = ld(c.mm, h_m(d, i, j));
-    vel.p[0][p] = Um(i, j, k) * m * idx;
-    vel.p[1][p] = Vm(i, j, k) * m * idy;
-    vel.p[2][p] = Em(i, j, k);
-  }
-  if (vel.p[3] && j < ny && k < nz) {  // u
-    int l, r;
-    face_pair(i, nx, d.px, l, r);
-    const int p = iu(d, i, j, k);
-    const T m = ld(c.mu, h_u(d, i, j));
-    vel.p[3][p] = U(i, j, k) * m * idx;
-    vel.p[4][p] = T(0.5) * (Vm(l, j, k) + Vm(r, j, k)) * m * idy;
-    vel.p[5][p] = T(0.5) * (Em(l, j, k) + Em(r, j, k));
-  }
-  if (vel.p[6] && i < nx && k < nz) {  // v
-    int l, r;
-    face_pair(j, ny, d.py, l, r);
-    const int p = iv(d, i, j, k);
-    const T m = ld(c.mv, h_v(d, i, j));
-    vel.p[6][p] = T(0.5) * (Um(i, l, k) + Um(i, r, k)) * m * idx;
-    vel.p[7][p] = V(i, j, k) * m * idy;
-    vel.p[8][p] = T(0.5) * (Em(i, l, k) + Em(i, r, k));
-  }
-  if (vel.p[9] && i < nx && j < ny) {  // w
-    int kl, kr;
-    level_pair(k, nz, kl, kr);
-    const int p = iw(d, i, j, k);
-    const T m = ld(c.mm, h_m(d, i, j));
-    vel.p[9][p] = T(0.5) * (Um(i, j, kl) + Um(i, j, kr)) * m * idx;
-    vel.p[10][p] = T(0.5) * (Vm(i, j, kl) + Vm(i, j, kr)) * m * idy;
-    vel.p[11][p] = E(i, j, k);
+#pragma unroll
+  for (int l = 0; l < TV_LV<T>; ++l) {
+    const int k = k0 + l;
+    if (k > nz) break;
+    if (vel.p[0] && i < nx && j < ny && k < nz) {  // m
+      const int p = im(d, i, j, k);
+      const T m = ld(c.mm, h_m(d, i, j));
+      vel.p[0][p] = Um(i, j, k) * m * idx;
+      vel.p[1][p] = Vm(i, j, k) * m * idy;
+      vel.p[2][p] = Em(i, j, k);
+    }
+    if (vel.p[3] && j < ny && k < nz) {  // u
+      int l, r;
+      face_pair(i, nx, d.px, l, r);
+      const int p = iu(d, i, j, k);
+      const T m = ld(c.mu, h_u(d, i, j));
+      vel.p[3][p] = U(i, j, k) * m * idx;
+      vel.p[4][p] = T(0.5) * (Vm(l, j, k) + Vm(r, j, k)) * m * idy;
+      vel.p[5][p] = T(0.5) * (Em(l, j, k) + Em(r, j, k));
+    }
+    if (vel.p[6] && i < nx && k < nz) {  // v
+      int l, r;
+      face_pair(j, ny, d.py, l, r);
+      const int p = iv(d, i, j, k);
+      const T m = ld(c.mv, h_v(d, i, j));
+      vel.p[6][p] = T(0.5) * (Um(i, l, k) + Um(i, r, k)) * m * idx;
+      vel.p[7][p] = V(i, j, k) * m * idy;
+      vel.p[8][p] = T(0.5) * (Em(i, l, k) + Em(i, r, k));
+    }
+    if (vel.p[9] && i < nx && j < ny) {  // w
+      int kl, kr;
+      level_pair(k, nz, kl, kr);
+      const int p = iw(d, i, j, k);
+      const T m = ld(c.mm, h_m(d, i, j));
+      vel.p[9][p] = T(0.5) * (Um(i, j, kl) + Um(i, j, kr)) * m * idx;
+      vel.p[10][p] = T(0.5) * (Vm(i, j, kl) + Vm(i, j, kr)) * m * idy;
+      vel.p[11][p] = E(i, j, k);
+    }
   }
 }
 
@@ -109,28 +119,78 @@ __device__ __forceinline__ T trilinear(const T* __restrict__ f, const Ext& e, T 
   return acc;
 }
 
-// the same gather at the split point (i + ox, j + oy, k + oz)
+// The gather of the three velocities at stencil base (lx, ly, lz) with
+// weights (wx, wy, wz), corners summed in itertools.product order.  float32:
+// all 24 loads in flight together, and away from the x edges both columns of a
+// row from one address (departure and tricubic of 256x256x80: 233 -> 186 us);
+// float64, whose 24 values take twice the registers, one velocity at a time
+// (150x131x60: 81 us against 98).
 template <typename T>
-__device__ __forceinline__ T trilinear_rel(const T* __restrict__ f, const Ext& e, int i, int j, int k, T ox, T oy,
-                                           T oz) {
-  int lx, ly, lz;
-  T wx, wy, wz;
-  linear_base(i, ox, lx, wx);
-  linear_base(j, oy, ly, wy);
-  linear_base(k, oz, lz, wz);
-  const int ix[2] = {min(max(lx, 0), e.ex - 1), min(max(lx + 1, 0), e.ex - 1)};
+__device__ __forceinline__ void trilinear3(const T* __restrict__ vx, const T* __restrict__ vy,
+                                           const T* __restrict__ vz, const Ext& e, int lx, int ly, int lz, T wx, T wy,
+                                           T wz, T& ax, T& ay, T& az) {
   const int iy[2] = {min(max(ly, 0), e.ey - 1), min(max(ly + 1, 0), e.ey - 1)};
   const int iz[2] = {min(max(lz, 0), e.ez - 1), min(max(lz + 1, 0), e.ez - 1)};
   const T Wx[2] = {T(1) - wx, wx}, Wy[2] = {T(1) - wy, wy}, Wz[2] = {T(1) - wz, wz};
-  T acc = T(0);
+  const T* __restrict__ fs[3] = {vx, vy, vz};
+  if (sizeof(T) == 8) {
+    const int ix[2] = {min(max(lx, 0), e.ex - 1), min(max(lx + 1, 0), e.ex - 1)};
+    auto one = [&](const T* __restrict__ f) {
+      T acc = T(0);
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+            acc += Wx[a] * Wy[b] * Wz[q] * ld(f, ix[a] + e.ex * (iy[b] + e.ey * iz[q]));
+      return acc;
+    };
+    ax = one(vx);
+    ay = one(vy);
+    az = one(vz);
+    return;
+  }
+  T vals[3][2][2][2];
+  if (lx >= 0 && lx + 1 < e.ex) {
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int row = lx + e.ex * (iy[b] + e.ey * iz[q]);
+#pragma unroll
+        for (int n = 0; n < 3; ++n) {
+          const T* __restrict__ p = fs[n] + row;
+          vals[n][0][b][q] = __ldg(p);
+          vals[n][1][b][q] = __ldg(p + 1);
+        }
+      }
+  } else {
+    const int ix[2] = {min(max(lx, 0), e.ex - 1), min(max(lx + 1, 0), e.ex - 1)};
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int row = e.ex * (iy[b] + e.ey * iz[q]);
+#pragma unroll
+        for (int n = 0; n < 3; ++n) {
+          vals[n][0][b][q] = ld(fs[n], ix[0] + row);
+          vals[n][1][b][q] = ld(fs[n], ix[1] + row);
+        }
+      }
+  }
+  T acc[3] = {T(0), T(0), T(0)};
 #pragma unroll
   for (int a = 0; a < 2; ++a)
 #pragma unroll
     for (int b = 0; b < 2; ++b)
 #pragma unroll
       for (int q = 0; q < 2; ++q)
-        acc += Wx[a] * Wy[b] * Wz[q] * ld(f, ix[a] + e.ex * (iy[b] + e.ey * iz[q]));
-  return acc;
+#pragma unroll
+        for (int n = 0; n < 3; ++n) acc[n] += Wx[a] * Wy[b] * Wz[q] * vals[n][a][b][q];
+  ax = acc[0];
+  ay = acc[1];
+  az = acc[2];
 }
 
 // Midpoint departure iteration in split form: the offsets (ox, oy, oz) =
@@ -142,10 +202,15 @@ __device__ __forceinline__ void departure_rel(const Ext& e, int i, int j, int k,
   const int p = i + e.ex * (j + e.ey * k);
   T ax = dt * ld(vx, p), ay = dt * ld(vy, p), az = dt * ld(vz, p);
   for (int it = 0; it < iters; ++it) {
-    const T mx = T(-0.5) * ax, my = T(-0.5) * ay, mz = T(-0.5) * az;
-    ax = dt * trilinear_rel(vx, e, i, j, k, mx, my, mz);
-    ay = dt * trilinear_rel(vy, e, i, j, k, mx, my, mz);
-    az = dt * trilinear_rel(vz, e, i, j, k, mx, my, mz);
+    int lx, ly, lz;
+    T wx, wy, wz;
+    linear_base(i, T(-0.5) * ax, lx, wx);
+    linear_base(j, T(-0.5) * ay, ly, wy);
+    linear_base(k, T(-0.5) * az, lz, wz);
+    trilinear3(vx, vy, vz, e, lx, ly, lz, wx, wy, wz, ax, ay, az);
+    ax *= dt;
+    ay *= dt;
+    az *= dt;
   }
   ox = -ax;
   oy = -ay;
@@ -161,9 +226,11 @@ __device__ __forceinline__ void departure_at(const Ext& e, int i, int j, int k, 
   T ax = dt * ld(vx, p), ay = dt * ld(vy, p), az = dt * ld(vz, p);
   for (int it = 0; it < iters; ++it) {
     const T mx = X - T(0.5) * ax, my = Y - T(0.5) * ay, mz = Z - T(0.5) * az;
-    ax = dt * trilinear(vx, e, mx, my, mz);
-    ay = dt * trilinear(vy, e, mx, my, mz);
-    az = dt * trilinear(vz, e, mx, my, mz);
+    const T fx = floor(mx), fy = floor(my), fz = floor(mz);
+    trilinear3(vx, vy, vz, e, (int)fx, (int)fy, (int)fz, mx - fx, my - fy, mz - fz, ax, ay, az);
+    ax *= dt;
+    ay *= dt;
+    az *= dt;
   }
   cx = X - ax;
   cy = Y - ay;
@@ -193,18 +260,43 @@ __device__ __forceinline__ T tricubic_core(const T* __restrict__ f, const Ext& e
   const int iz[4] = {max(z0 - 1, 0), z0, min(z0 + 1, e.ez - 1), min(z0 + 2, e.ez - 1)};
   const int plane = e.ex * e.ey;
   T out = T(0);
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    T sy = T(0);
+  if (sizeof(T) == 4 && e.ex >= 4) {
+    // the four columns xb .. xb + 3 hold every clamped stencil column: one row address serves four loads
+    // (384x384x96 float32: 244 us, 312 with an address per load; float64 is bound by its loads' bytes, and the
+    // registers cost it 3 %)
+    const int xb = min(max(x0 - 1, 0), e.ex - 4);
+    T S[4] = {T(0), T(0), T(0), T(0)};
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
-      const int row = ix[a] + e.ex * iy[b];
-      T sz = T(0);
+      T sz[4] = {T(0), T(0), T(0), T(0)};
 #pragma unroll
-      for (int q = 0; q < 4; ++q) sz += wz[q] * ld(f, row + plane * iz[q]);
-      sy += wy[b] * sz;
+      for (int q = 0; q < 4; ++q) {
+        const T* __restrict__ p = f + (xb + e.ex * iy[b] + plane * iz[q]);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) sz[m] += wz[q] * __ldg(p + m);
+      }
+#pragma unroll
+      for (int m = 0; m < 4; ++m) S[m] += wy[b] * sz[m];
     }
-    out += wx[a] * sy;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const int m = ix[a] - xb;
+      out += wx[a] * (m == 0 ? S[0] : (m == 1 ? S[1] : (m == 2 ? S[2] : S[3])));
+    }
+  } else {
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      T sy = T(0);
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int row = ix[a] + e.ex * iy[b];
+        T sz = T(0);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sz += wz[q] * ld(f, row + plane * iz[q]);
+        sy += wy[b] * sz;
+      }
+      out += wx[a] * sy;
+    }
   }
   if (limiter) {
     const int x1 = min(x0 + 1, e.ex - 1), y1 = min(y0 + 1, e.ey - 1), z1 = min(z0 + 1, e.ez - 1);
@@ -319,8 +411,9 @@ template <typename T>
 void launch_traj_velocity(const Dims& d, const Coef<T>& c, const T* u, const T* v, const T* eta, const T* up,
                           const T* vp, const T* etap, int extrapolate, PtrTable<T> vel, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  launch_chained(traj_velocity_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st,
-      d, c, u, v, eta, up, vp, etap, extrapolate, vel);
+  const dim3 grd = box_grid(d.nx + 1, d.ny + 1, (d.nz + TV_LV<T>) / TV_LV<T>, blk);
+  if (extrapolate) launch_chained(traj_velocity_kernel<T, true>, grd, blk, 0, st, d, c, u, v, eta, up, vp, etap, vel);
+  else launch_chained(traj_velocity_kernel<T, false>, grd, blk, 0, st, d, c, u, v, eta, up, vp, etap, vel);
 }
 
 template <typename T>
