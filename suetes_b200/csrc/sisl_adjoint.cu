@@ -103,7 +103,7 @@ __device__ __forceinline__ void at_main_block(const Dims& d, const Coef<T>& c, c
   if (i > nx || j > ny || k > nz) return;
   const T ys = yscale ? (T)(*yscale) : T(1);
   const T adt = (T)(c.s.alpha * c.s.dt), cp = (T)c.s.cp, a = (T)c.s.alpha, ps = (T)c.s.ps;
-  const T idx = (T)(1.0 / d.dx), idy = (T)(1.0 / d.dy);
+  const T idx = (T)d.rdx, idy = (T)d.rdy;
   const T* __restrict__ yu = y.f[0];
   const T* __restrict__ yv = y.f[1];
   const T* __restrict__ yw = y.f[2];
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(TPT) pt_column_kernel(Dims d, Coef<T> c, CVec5
   const int j = blockIdx.y;
   const int tid = threadIdx.x;
   const int pm = nx * ny;
-  const T ps = (T)c.s.ps, ips = (T)(1.0 / c.s.ps), inva = T(1) / (T)c.s.alpha;
+  const T ps = (T)c.s.ps, ips = (T)c.s.rps, inva = T(1) / (T)c.s.alpha;
   const T* __restrict__ yw = y.f[2];
   const T* __restrict__ yp = y.f[3];
   const T* __restrict__ yW = y.f[4];
@@ -389,7 +389,7 @@ __device__ __forceinline__ void pt_column_batched_block(const Dims& d, const Coe
   const int tid = threadIdx.x;
   const int pm = nx * ny;
   const int nm = nz * TPC, nw = (nz + 1) * TPC;
-  const T ps = (T)c.s.ps, ips = (T)(1.0 / c.s.ps), inva = T(1) / (T)c.s.alpha;
+  const T ps = (T)c.s.ps, ips = (T)c.s.rps, inva = T(1) / (T)c.s.alpha;
   const T* __restrict__ yw = y.f[2];
   const T* __restrict__ yp = y.f[3];
   const T* __restrict__ yW = y.f[4];
@@ -919,7 +919,7 @@ __device__ __forceinline__ void pt_march_block(const Dims& d, const Coef<T>& c, 
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   if (i >= nx) return;
   const int pm = nx * ny, h = i + nx * j;
-  const T ps = (T)c.s.ps, ips = (T)(1.0 / c.s.ps), inva = T(1) / (T)c.s.alpha;
+  const T ps = (T)c.s.ps, ips = (T)c.s.rps, inva = T(1) / (T)c.s.alpha;
   const T* __restrict__ yw = y.f[2];
   const T* __restrict__ yp = y.f[3];
   const T* __restrict__ yW = y.f[4];

@@ -84,6 +84,10 @@ struct Dims {
   // (sisl_autotune): the Helmholtz matvec, its transpose (stencil block), the
   // column preconditioner and its transpose (column tile)
   int tune_mv = 6, tune_pc = 6, tune_mvt = 0, tune_pct = 0;
+  // reciprocals, formed once on the host: a float64 division per thread and
+  // axis weighed on every point kernel (256x256x80 float32 explicit tendencies
+  // 324 us against 258, the float64 residual 315 against 298)
+  double rdx = 1.0 / dx, rdy = 1.0 / dy;
 };
 
 // block shapes of the 3-D stencil kernels (256 threads each)

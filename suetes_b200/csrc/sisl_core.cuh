@@ -19,6 +19,7 @@ struct Base64 {
 // Physical and solver scalars.
 struct Scalars {
   double dt, alpha, g, cp, Rd, cvd, p0, ps, nu_div, nu_h;
+  double rps = 1.0 / ps;
 };
 
 // Derived coefficient arrays in working precision T.  Every array is

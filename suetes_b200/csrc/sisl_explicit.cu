@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(LX * LY, 2) hyper_lap_kernel(Dims d, Coef<T> c
       zl[n][f] = df[n][f] * iz;
     }
   }
-  const T idx = (T)(1.0 / d.dx), idy = (T)(1.0 / d.dy);
+  const T idx = (T)d.rdx, idy = (T)d.rdy;
   const T mu0 = ld(c.mu, h_u(d, i, j)), mu1 = ld(c.mu, h_u(d, i + 1, j));
   const T mv0 = ld(c.mv, h_v(d, i, j)), mv1 = ld(c.mv, h_v(d, i, j + 1)), m = ld(c.mm, h_m(d, i, j));
   // tile positions of the two cells of each face; an open boundary face repeats its neighbour's pair (face_pair)
@@ -342,8 +342,8 @@ __global__ void hdiv_kernel(Dims d, Coef<T> c, const T* __restrict__ u, const T*
   const int k = blockIdx.z * blockDim.z + threadIdx.z;
   if (i >= d.nx || j >= d.ny || k >= d.nz) return;
   const T m = ld(c.mm, h_m(d, i, j));
-  const T dux = (ld(u, iu(d, i + 1, j, k)) - ld(u, iu(d, i, j, k))) * (T)(1.0 / d.dx) * m;
-  const T dvy = (ld(v, iv(d, i, j + 1, k)) - ld(v, iv(d, i, j, k))) * (T)(1.0 / d.dy) * m;
+  const T dux = (ld(u, iu(d, i + 1, j, k)) - ld(u, iu(d, i, j, k))) * (T)d.rdx * m;
+  const T dvy = (ld(v, iv(d, i, j + 1, k)) - ld(v, iv(d, i, j, k))) * (T)d.rdy * m;
   div[im(d, i, j, k)] = dux + dvy;
 }
 
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(256) finalize_kernel(Dims d, Coef<T> c, Finali
     if (fa.div) {
       int l, r;
       face_pair(i, nx, d.px, l, r);
-      val += nud * (ld(fa.div, im(d, r, j, k)) - ld(fa.div, im(d, l, j, k))) * (T)(1.0 / d.dx) *
+      val += nud * (ld(fa.div, im(d, r, j, k)) - ld(fa.div, im(d, l, j, k))) * (T)d.rdx *
              ld(c.mu, h_u(d, i, j));
     }
     if (R.on & RELAX_U) val = blend(val, R.mask_u, h_u(d, i, j), R.ext_field[0] ? ld(R.ext_field[0], p) : R.ext[0]);
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(256) finalize_kernel(Dims d, Coef<T> c, Finali
     if (fa.div) {
       int l, r;
       face_pair(j, ny, d.py, l, r);
-      val += nud * (ld(fa.div, im(d, i, r, k)) - ld(fa.div, im(d, i, l, k))) * (T)(1.0 / d.dy) *
+      val += nud * (ld(fa.div, im(d, i, r, k)) - ld(fa.div, im(d, i, l, k))) * (T)d.rdy *
              ld(c.mv, h_v(d, i, j));
     }
     if (R.on & RELAX_V) val = blend(val, R.mask_v, h_v(d, i, j), R.ext_field[1] ? ld(R.ext_field[1], p) : R.ext[1]);

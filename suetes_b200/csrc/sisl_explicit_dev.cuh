@@ -26,13 +26,13 @@ struct Grad {
   __device__ __forceinline__ T gx(int i, int j, int k) const {
     int l, r;
     face_pair(i, d.nx, d.px, l, r);
-    const T g = (Q(r, j, k) - Q(l, j, k)) * (T)(1.0 / d.dx) * ld(c.mu, h_u(d, i, j));
+    const T g = (Q(r, j, k) - Q(l, j, k)) * (T)d.rdx * ld(c.mu, h_u(d, i, j));
     return g - ld(c.zxu, iu(d, i, j, k)) * T(0.5) * (gzm(l, j, k) + gzm(r, j, k));
   }
   __device__ __forceinline__ T gy(int i, int j, int k) const {
     int l, r;
     face_pair(j, d.ny, d.py, l, r);
-    const T g = (Q(i, r, k) - Q(i, l, k)) * (T)(1.0 / d.dy) * ld(c.mv, h_v(d, i, j));
+    const T g = (Q(i, r, k) - Q(i, l, k)) * (T)d.rdy * ld(c.mv, h_v(d, i, j));
     return g - ld(c.zev, iv(d, i, j, k)) * T(0.5) * (gzm(i, l, k) + gzm(i, r, k));
   }
 };
@@ -103,7 +103,7 @@ __device__ __forceinline__ T divergence(const Dims& d, const Coef<T>& c, const T
   const T fz0 = (k == 0) ? T(0) : ld(eta, w0) * ld(c.dzw, w0) * ld(c.rhow, w0) * thw(i, j, k);
   const T fz1 = (k + 1 == d.nz) ? T(0) : ld(eta, w1) * ld(c.dzw, w1) * ld(c.rhow, w1) * thw(i, j, k + 1);
   const T m = ld(c.mm, h_m(d, i, j));
-  const T divh = m * m * ((fx1 - fx0) * (T)(1.0 / d.dx) + (fy1 - fy0) * (T)(1.0 / d.dy));
+  const T divh = m * m * ((fx1 - fx0) * (T)d.rdx + (fy1 - fy0) * (T)d.rdy);
   return -ld(c.cpidz, im(d, i, j, k)) * (divh + (fz1 - fz0));
 }
 
@@ -124,13 +124,13 @@ struct HLap {
   __device__ __forceinline__ T Gx(int fi, int j, int k) const {  // at u face fi
     int l, r;
     face_pair(fi, d.nx, d.px, l, r);
-    const T dxi = (F(r, j, k) - F(l, j, k)) * (T)(1.0 / d.dx) * ld(c.mu, h_u(d, fi, j));
+    const T dxi = (F(r, j, k) - F(l, j, k)) * (T)d.rdx * ld(c.mu, h_u(d, fi, j));
     return dxi - ld(c.zxu, iu(d, fi, j, k)) * T(0.5) * (dzm(l, j, k) + dzm(r, j, k));
   }
   __device__ __forceinline__ T Gy(int i, int fj, int k) const {  // at v face fj
     int l, r;
     face_pair(fj, d.ny, d.py, l, r);
-    const T deta = (F(i, r, k) - F(i, l, k)) * (T)(1.0 / d.dy) * ld(c.mv, h_v(d, i, fj));
+    const T deta = (F(i, r, k) - F(i, l, k)) * (T)d.rdy * ld(c.mv, h_v(d, i, fj));
     return deta - ld(c.zev, iv(d, i, fj, k)) * T(0.5) * (dzm(i, l, k) + dzm(i, r, k));
   }
 };

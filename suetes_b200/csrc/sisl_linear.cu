@@ -59,7 +59,7 @@ template <typename T>
 __device__ __forceinline__ void mv_rows(const Dims& d, const Coef<T>& c, const MvIn<T>& q, T xs, bool u_lock,
                                         bool v_lock, bool wb, T (&L)[5]) {
   const T adt = (T)(c.s.alpha * c.s.dt), cp = (T)c.s.cp, a = (T)c.s.alpha, ps = (T)c.s.ps;
-  const T idx = (T)(1.0 / d.dx), idy = (T)(1.0 / d.dy);
+  const T idx = (T)d.rdx, idy = (T)d.rdy;
   const T vat = T(0.25) * (q.vX0 + q.vX1 + q.vO0 + q.vO1) * xs;
   const T tend_u = -cp * q.thu * ((q.PO - q.PX) * idx * q.mu_f - q.zxu * T(0.5) * (q.gmX + q.gmO)) + q.fu_f * vat;
   L[0] = u_lock ? q.xu_f * xs : q.xu_f * xs - adt * tend_u;
@@ -119,7 +119,7 @@ __device__ __forceinline__ void matvec_point(const Dims& d, const Coef<T>& c, co
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const T adt = (T)(c.s.alpha * c.s.dt), cp = (T)c.s.cp, a = (T)c.s.alpha, ps = (T)c.s.ps;
   const T sp = xs / ps;
-  const T idx = (T)(1.0 / d.dx), idy = (T)(1.0 / d.dy);
+  const T idx = (T)d.rdx, idy = (T)d.rdy;
   const int pm = nx * ny, pu = (nx + 1) * ny, pv = nx * (ny + 1);
   const T* __restrict__ xu = x.f[0];
   const T* __restrict__ xv = x.f[1];
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(PT) precond_tile_kernel(Dims d, Coef<T> c, CVe
   T* __restrict__ op = out.f[3];
   T* __restrict__ oW = out.f[4];
   const T inva = T(1) / (T)c.s.alpha;
-  const T ips = (T)(1.0 / c.s.ps);
+  const T ips = (T)c.s.rps;
   const T ps = (T)c.s.ps;
   const int pm = nx * ny;
 
@@ -650,7 +650,7 @@ __global__ void __launch_bounds__(PT) precond_tile_batched_kernel(Dims d, Coef<T
   T* __restrict__ op = out.f[3];
   T* __restrict__ oW = out.f[4];
   const T inva = T(1) / (T)c.s.alpha;
-  const T ips = (T)(1.0 / c.s.ps);
+  const T ips = (T)c.s.rps;
   const T ps = (T)c.s.ps;
   const int pm = nx * ny;
   const int nm = nz * PC, nw = (nz + 1) * PC;
@@ -867,7 +867,7 @@ __global__ void __launch_bounds__(NT) precond_march_kernel(Dims d, Coef<T> c, CV
   if (i >= nx) return;
   const int pm = nx * ny, h = i + nx * j;
   const int pu = (nx + 1) * ny, pv = nx * (ny + 1);
-  const T inva = T(1) / (T)c.s.alpha, ips = (T)(1.0 / c.s.ps), ps = (T)c.s.ps;
+  const T inva = T(1) / (T)c.s.alpha, ips = (T)c.s.rps, ps = (T)c.s.ps;
   const T* __restrict__ ru = r.f[0];
   const T* __restrict__ rv = r.f[1];
   const T* __restrict__ rw = r.f[2];
@@ -1003,7 +1003,7 @@ __device__ __forceinline__ void precond_pipe_block(const Dims& d, const Coef<T>&
   if (i >= nx) return;
   const int pm = nx * ny, h = i + nx * j;
   const int pu = (nx + 1) * ny, pv = nx * (ny + 1);
-  const T inva = T(1) / (T)c.s.alpha, ips = (T)(1.0 / c.s.ps), ps = (T)c.s.ps;
+  const T inva = T(1) / (T)c.s.alpha, ips = (T)c.s.rps, ps = (T)c.s.ps;
   const T* __restrict__ ru = r.f[0];
   const T* __restrict__ rv = r.f[1];
   const T* __restrict__ rw = r.f[2];
@@ -1125,7 +1125,7 @@ __global__ void __launch_bounds__(NT) precond_async_kernel(Dims d, Coef<T> c, CV
   if (i >= nx) return;
   const int pm = nx * ny, h = i + nx * j;
   const int pu = (nx + 1) * ny, pv = nx * (ny + 1);
-  const T inva = T(1) / (T)c.s.alpha, ips = (T)(1.0 / c.s.ps), ps = (T)c.s.ps;
+  const T inva = T(1) / (T)c.s.alpha, ips = (T)c.s.rps, ps = (T)c.s.ps;
   const T* __restrict__ ru = r.f[0];
   const T* __restrict__ rv = r.f[1];
   const T* __restrict__ rw = r.f[2];

@@ -38,7 +38,7 @@ __global__ void traj_velocity_kernel(Dims d, Coef<T> c, const T* __restrict__ u,
   const int k0 = (blockIdx.z * blockDim.z + threadIdx.z) * TV_LV<T>;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   if (i > nx || j > ny) return;
-  const T idx = (T)(1.0 / d.dx), idy = (T)(1.0 / d.dy);
+  const T idx = (T)d.rdx, idy = (T)d.rdy;
   auto U = [&](int a, int b, int cc) {
     const int p = iu(d, a, b, cc);
     return EX ? T(1.5) * ld(u, p) - T(0.5) * ld(up, p) : ld(u, p);

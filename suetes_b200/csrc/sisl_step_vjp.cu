@@ -171,7 +171,7 @@ struct GradAdj {
     if (face_padded(i, d.nx, d.px)) return;
     int l, r;
     face_pair(i, d.nx, d.px, l, r);
-    const T s = x * (T)(1.0 / d.dx) * ld(c.mu, h_u(d, i, j));
+    const T s = x * (T)d.rdx * ld(c.mu, h_u(d, i, j));
     radd(qb, im(d, r, j, k), s);
     radd(qb, im(d, l, j, k), -s);
     const T y = -ld(c.zxu, iu(d, i, j, k)) * T(0.5) * x;
@@ -182,7 +182,7 @@ struct GradAdj {
     if (face_padded(j, d.ny, d.py)) return;
     int l, r;
     face_pair(j, d.ny, d.py, l, r);
-    const T s = x * (T)(1.0 / d.dy) * ld(c.mv, h_v(d, i, j));
+    const T s = x * (T)d.rdy * ld(c.mv, h_v(d, i, j));
     radd(qb, im(d, i, r, k), s);
     radd(qb, im(d, i, l, k), -s);
     const T y = -ld(c.zev, iv(d, i, j, k)) * T(0.5) * x;
@@ -257,7 +257,7 @@ __device__ __forceinline__ void divergence_adj(const Dims& d, const Coef<T>& c, 
   if (x == T(0)) return;
   const T s = -ld(c.cpidz, im(d, i, j, k)) * x;
   const T m = ld(c.mm, h_m(d, i, j));
-  const T hx = m * m * s * (T)(1.0 / d.dx), hy = m * m * s * (T)(1.0 / d.dy);
+  const T hx = m * m * s * (T)d.rdx, hy = m * m * s * (T)d.rdy;
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
     const T wgt = q ? hx : -hx;
@@ -692,10 +692,10 @@ __global__ void div_t_kernel(Dims d, Coef<T> c, const T* __restrict__ ub, const 
   T acc = T(0);
   int n = adj_faces(i, d.nx, d.px, f, s);
   for (int q = 0; q < n; ++q)
-    acc += (T)s[q] * ld(c.mu, h_u(d, f[q], j)) * (T)(1.0 / d.dx) * ld(ub, iu(d, f[q], j, k));
+    acc += (T)s[q] * ld(c.mu, h_u(d, f[q], j)) * (T)d.rdx * ld(ub, iu(d, f[q], j, k));
   n = adj_faces(j, d.ny, d.py, f, s);
   for (int q = 0; q < n; ++q)
-    acc += (T)s[q] * ld(c.mv, h_v(d, i, f[q])) * (T)(1.0 / d.dy) * ld(vb, iv(d, i, f[q], k));
+    acc += (T)s[q] * ld(c.mv, h_v(d, i, f[q])) * (T)d.rdy * ld(vb, iv(d, i, f[q], k));
   divb[im(d, i, j, k)] = nud * acc;
 }
 
@@ -711,13 +711,13 @@ __global__ void div_winds_t_kernel(Dims d, Coef<T> c, const T* __restrict__ divb
     T acc = T(0);
     if (i >= 1) acc += ld(c.mm, h_m(d, i - 1, j)) * ld(divb, im(d, i - 1, j, k));
     if (i <= d.nx - 1) acc -= ld(c.mm, h_m(d, i, j)) * ld(divb, im(d, i, j, k));
-    ub[iu(d, i, j, k)] += acc * (T)(1.0 / d.dx);
+    ub[iu(d, i, j, k)] += acc * (T)d.rdx;
   }
   if (i < d.nx) {
     T acc = T(0);
     if (j >= 1) acc += ld(c.mm, h_m(d, i, j - 1)) * ld(divb, im(d, i, j - 1, k));
     if (j <= d.ny - 1) acc -= ld(c.mm, h_m(d, i, j)) * ld(divb, im(d, i, j, k));
-    vb[iv(d, i, j, k)] += acc * (T)(1.0 / d.dy);
+    vb[iv(d, i, j, k)] += acc * (T)d.rdy;
   }
 }
 
@@ -751,14 +751,14 @@ __global__ void __launch_bounds__(256) lap_t_faces_kernel(Dims d, Coef<T> c, Ptr
   };
   if (j < ny) {  // u face i
     T acc = T(0);
-    if (i >= 1) acc += ld(c.mm, h_m(d, i - 1, j)) * (T)(1.0 / d.dx) * B(i - 1, j, k) + T(0.5) * gmb(c.zxm, i - 1, j, k);
-    if (i <= nx - 1) acc += -ld(c.mm, h_m(d, i, j)) * (T)(1.0 / d.dx) * B(i, j, k) + T(0.5) * gmb(c.zxm, i, j, k);
+    if (i >= 1) acc += ld(c.mm, h_m(d, i - 1, j)) * (T)d.rdx * B(i - 1, j, k) + T(0.5) * gmb(c.zxm, i - 1, j, k);
+    if (i <= nx - 1) acc += -ld(c.mm, h_m(d, i, j)) * (T)d.rdx * B(i, j, k) + T(0.5) * gmb(c.zxm, i, j, k);
     gxb.p[f][iu(d, i, j, k)] = acc;
   }
   if (i < nx) {  // v face j
     T acc = T(0);
-    if (j >= 1) acc += ld(c.mm, h_m(d, i, j - 1)) * (T)(1.0 / d.dy) * B(i, j - 1, k) + T(0.5) * gmb(c.zem, i, j - 1, k);
-    if (j <= ny - 1) acc += -ld(c.mm, h_m(d, i, j)) * (T)(1.0 / d.dy) * B(i, j, k) + T(0.5) * gmb(c.zem, i, j, k);
+    if (j >= 1) acc += ld(c.mm, h_m(d, i, j - 1)) * (T)d.rdy * B(i, j - 1, k) + T(0.5) * gmb(c.zem, i, j - 1, k);
+    if (j <= ny - 1) acc += -ld(c.mm, h_m(d, i, j)) * (T)d.rdy * B(i, j, k) + T(0.5) * gmb(c.zem, i, j, k);
     gyb.p[f][iv(d, i, j, k)] = acc;
   }
 }
@@ -795,9 +795,9 @@ __global__ void __launch_bounds__(256) lap_t_mass_kernel(Dims d, Coef<T> c, PtrT
   };
   T acc = T(0);
   for (int q = 0; q < nfx; ++q)
-    acc += (T)sx[q] * ld(c.mu, h_u(d, fx[q], j)) * (T)(1.0 / d.dx) * ld(GX, iu(d, fx[q], j, k));
+    acc += (T)sx[q] * ld(c.mu, h_u(d, fx[q], j)) * (T)d.rdx * ld(GX, iu(d, fx[q], j, k));
   for (int q = 0; q < nfy; ++q)
-    acc += (T)sy[q] * ld(c.mv, h_v(d, i, fy[q])) * (T)(1.0 / d.dy) * ld(GY, iv(d, i, fy[q], k));
+    acc += (T)sy[q] * ld(c.mv, h_v(d, i, fy[q])) * (T)d.rdy * ld(GY, iv(d, i, fy[q], k));
   // dzw(kw) = (F(kw) - F(kw-1)) / dz_w at interior levels, dzm = avg of dzw
   const T m0 = dzmb(k);
   if (k >= 1) acc += T(0.5) * (dzmb(k - 1) + m0) * ld(c.idzw, iw(d, i, j, k));
@@ -1033,9 +1033,9 @@ __global__ void __launch_bounds__(256) split_faces_vjp_kernel(Dims d, Coef<T> c,
     if (k < nz) {  // pi'' of the pressure gradient; the edge levels of the vertical one are padded copies
       const double y1 = k + 1 < nz ? F.slope(i, j, k + 1) : 0.0;
       double a = ((double)(F.hu(i, j, k) * ld(c.mu, h_u(d, i, j))) -
-                  (double)(F.hu(i + 1, j, k) * ld(c.mu, h_u(d, F.fu(i + 1), j)))) * (1.0 / d.dx) +
+                  (double)(F.hu(i + 1, j, k) * ld(c.mu, h_u(d, F.fu(i + 1), j)))) * d.rdx +
                  ((double)(F.hv(i, j, k) * ld(c.mv, h_v(d, i, j))) -
-                  (double)(F.hv(i, j + 1, k) * ld(c.mv, h_v(d, i, F.fv(j + 1))))) * (1.0 / d.dy);
+                  (double)(F.hv(i, j + 1, k) * ld(c.mv, h_v(d, i, F.fv(j + 1))))) * d.rdy;
       if (k > 0) a += 0.5 * (ym + y0) * (double)ld(c.idzw, iw(d, i, j, k));
       if (k + 1 < nz) a -= 0.5 * (y0 + y1) * (double)ld(c.idzw, iw(d, i, j, k + 1));
       const int p = im(d, i, j, k);
