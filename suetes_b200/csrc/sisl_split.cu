@@ -242,37 +242,49 @@ __global__ void split_init_kernel(Dims d, SplitArgs<T> a) {
   }
 }
 
-// horizontal divergence of the total winds (stage + u'') at a cell
-template <typename T>
-__device__ __forceinline__ T cell_div(const Dims& d, const Coef<T>& c, const T* uc, const T* up, const T* vc,
-                                      const T* vp, int i, int j, int k) {
-  const T mm = ld(c.mm, h_m(d, i, j));
-  const int u0 = iu(d, i, j, k), v0 = iv(d, i, j, k);
-  const T du = ((uc[u0 + 1] + up[u0 + 1]) - (uc[u0] + up[u0])) / (T)d.dx * mm;
-  const T dv = ((vc[v0 + d.nx] + vp[v0 + d.nx]) - (vc[v0] + vp[v0])) / (T)d.dy * mm;
-  return du + dv;
-}
-
 // Blocks of the predictor and corrector: SX x SY faces of one level.
 constexpr int SX = 32, SY = 8;
 
-// The horizontal divergence of the total winds (stage + perturbation) of the
-// cells (i0 - 1 + x, j0 - 1 + y), x <= SX, y <= SY, at level k, into Dt.
-// Cell indices beyond the grid wrap on a periodic axis and are clamped on an
-// open one, so every interior face (i, j) of the block finds the two cells
-// of its divergence-damping gradient at tile columns i - i0, i - i0 + 1
-// (rows j - j0, j - j0 + 1), as face_pair gives them, and the periodic
-// duplicate face n its wrapped pair; the open boundary faces take no
-// gradient (the divergence-damping gradient, steppers.py:1528-1538).  One cell divergence per cell of the tile instead of two per
-// face and axis.
+// What the faces (i, j) of a block read of the cells (i0 - 1 + x, j0 - 1 + y),
+// x <= SX, y <= SY, formed once per cell: the horizontal divergence of the
+// total winds (stage + perturbation), pi'' and its vertical derivative at the
+// mass level (Grad::gzm).  Cell indices beyond the grid wrap on a periodic
+// axis and are clamped on an open one, so every interior face (i, j) of
+// the block finds the two cells of its gradients at tile columns i - i0,
+// i - i0 + 1 (rows j - j0, j - j0 + 1), as face_pair gives them, and the
+// periodic duplicate face n its wrapped pair; the open boundary faces take no
+// gradient (steppers.py:1528-1538).
 template <typename T>
-__device__ __forceinline__ void div_tile(const Dims& d, const Coef<T>& c, const T* uc, const T* up, const T* vc,
-                                         const T* vp, int i0, int j0, int k, T (*Dt)[SX + 1]) {
-  const int t = threadIdx.x + SX * threadIdx.y;
-  for (int q = t; q < (SX + 1) * (SY + 1); q += SX * SY) {
+struct FaceTile {
+  T div[SY + 1][SX + 1], p[SY + 1][SX + 1], gz[SY + 1][SX + 1];
+};
+// 1/dx and the map factor in one product, rounded once
+template <typename T>
+__device__ __forceinline__ T over(T m, double inv) {
+  return (T)((double)m * inv);
+}
+
+template <typename T>
+__device__ __forceinline__ void fill_tile(const Dims& d, const Coef<T>& c, const T* __restrict__ uc,
+                                          const T* __restrict__ up, const T* __restrict__ vc,
+                                          const T* __restrict__ vp, const T* __restrict__ pp, bool grad, int i0, int j0,
+                                          int k, FaceTile<T>& t) {
+  const int nx = d.nx, ny = d.ny, nz = d.nz, pm = nx * ny;
+  const int kl = k > 0 ? k - 1 : 0, kh = k + 1 < nz ? k + 1 : nz - 1;
+  for (int q = threadIdx.x + SX * threadIdx.y; q < (SX + 1) * (SY + 1); q += SX * SY) {
     const int x = q % (SX + 1), y = q / (SX + 1);
-    const int ci = wrap_or_clamp(i0 - 1 + x, d.nx, d.px), cj = wrap_or_clamp(j0 - 1 + y, d.ny, d.py);
-    Dt[y][x] = cell_div(d, c, uc, up, vc, vp, ci, cj, k);
+    const int ci = wrap_or_clamp(i0 - 1 + x, nx, d.px), cj = wrap_or_clamp(j0 - 1 + y, ny, d.py);
+    const int u0 = iu(d, ci, cj, k), v0 = iv(d, ci, cj, k), h = ci + nx * cj;
+    const T ca = ld(uc, u0), cb = ld(uc, u0 + 1), ua = ld(up, u0), ub = ld(up, u0 + 1);
+    const T da = ld(vc, v0), db = ld(vc, v0 + nx), va = ld(vp, v0), vb = ld(vp, v0 + nx);
+    const T mm = ld(c.mm, h);
+    if (grad) {
+      const T P0 = ld(pp, h + k * pm), Pl = ld(pp, h + kl * pm), Ph = ld(pp, h + kh * pm);
+      const T z0 = ld(c.idzw, h + k * pm), z1 = ld(c.idzw, h + (k + 1) * pm);
+      t.p[y][x] = P0;
+      t.gz[y][x] = T(0.5) * ((k == 0 ? Ph - P0 : P0 - Pl) * z0 + (k + 1 == nz ? P0 - Pl : Ph - P0) * z1);
+    }
+    t.div[y][x] = ((cb + ub) - (ca + ua)) * over(mm, d.rdx) + ((db + vb) - (da + va)) * over(mm, d.rdy);
   }
 }
 
@@ -281,58 +293,64 @@ __device__ __forceinline__ void div_tile(const Dims& d, const Coef<T>& c, const 
 // first face (periodic duplicate).  The pressure gradient of the old pi''
 // is formed here on the first sub-step of a stage and taken from the
 // previous corrector (gx0_ready) on the others.
+//
+// Predictor and corrector are bound by the issue of their loads; the cell
+// tile took two gradients' 28 loads per point to 6.  256x256x64 float32, us:
+// predictor 76 -> 74 (gradient ready), corrector 116 -> 90 (walking four levels
+// a block, for hoisted indices, costs more in barriers: 80 and 130).
 template <typename T>
 __global__ void __launch_bounds__(SX * SY) split_predict_kernel(Dims d, Coef<T> c, SplitArgs<T> a) {
   grid_chain();
-  __shared__ T Dt[SY + 1][SX + 1];
+  __shared__ FaceTile<T> t;
   const int i0 = blockIdx.x * SX, j0 = blockIdx.y * SY, k = blockIdx.z;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int i = i0 + tx, j = j0 + ty;
   const int nx = d.nx, ny = d.ny;
-  div_tile<T>(d, c, a.uc, a.upp, a.vc, a.vpp, i0, j0, k, Dt);
+  const bool ready = a.gx0_ready;
+  fill_tile<T>(d, c, a.uc, a.upp, a.vc, a.vpp, a.ppp, !ready, i0, j0, k, t);
   __syncthreads();
   if (i > nx || j > ny) return;
   const T cp = (T)c.s.cp, hdt = T(0.5) * a.dtau;
-  const Grad<T> G{d, c, a.ppp};
+  const T idx = (T)d.rdx, idy = (T)d.rdy;
   if (j < ny) {
     const int p = iu(d, i, j, k);
     const int ie = (d.px && i == nx) ? 0 : i, pe = iu(d, ie, j, k);
-    T val;
     if (!d.px && (i == 0 || i == nx)) {
-      val = a.u0[p] - a.uc[p];
+      a.uh[p] = ld(a.u0, p) - ld(a.uc, p);
     } else {
+      const T mu = ld(c.mu, h_u(d, ie, j)), th = ld(c.thu, pe), sf = ld(a.sfu, pe), old = ld(a.upp, pe);
       T g0;
-      if (a.gx0_ready) {
-        g0 = a.gx0[p];
+      if (ready) {
+        g0 = ld(a.gx0, p);
       } else {
-        g0 = G.gx(ie, j, k);
+        const T g = (t.p[ty + 1][tx + 1] - t.p[ty + 1][tx]) * idx * mu;
+        g0 = g - ld(c.zxu, pe) * T(0.5) * (t.gz[ty + 1][tx] + t.gz[ty + 1][tx + 1]);
         a.gx0[p] = g0;
       }
-      const T dgx = (Dt[ty + 1][tx + 1] - Dt[ty + 1][tx]) / (T)d.dx * ld(c.mu, h_u(d, ie, j));
-      const T rhs = a.sfu[pe] - cp * ld(c.thu, pe) * g0 + a.nu_div * dgx;
-      val = a.upp[pe] + hdt * rhs;
+      const T dgx = (t.div[ty + 1][tx + 1] - t.div[ty + 1][tx]) * over(mu, d.rdx);
+      const T rhs = sf - cp * th * g0 + a.nu_div * dgx;
+      a.uh[p] = old + hdt * rhs;
     }
-    a.uh[p] = val;
   }
   if (i < nx) {
     const int p = iv(d, i, j, k);
     const int je = (d.py && j == ny) ? 0 : j, pe = iv(d, i, je, k);
-    T val;
     if (!d.py && (j == 0 || j == ny)) {
-      val = a.v0[p] - a.vc[p];
+      a.vh[p] = ld(a.v0, p) - ld(a.vc, p);
     } else {
+      const T mv = ld(c.mv, h_v(d, i, je)), th = ld(c.thv, pe), sf = ld(a.sfv, pe), old = ld(a.vpp, pe);
       T g0;
-      if (a.gx0_ready) {
-        g0 = a.gy0[p];
+      if (ready) {
+        g0 = ld(a.gy0, p);
       } else {
-        g0 = G.gy(i, je, k);
+        const T g = (t.p[ty + 1][tx + 1] - t.p[ty][tx + 1]) * idy * mv;
+        g0 = g - ld(c.zev, pe) * T(0.5) * (t.gz[ty][tx + 1] + t.gz[ty + 1][tx + 1]);
         a.gy0[p] = g0;
       }
-      const T dgy = (Dt[ty + 1][tx + 1] - Dt[ty][tx + 1]) / (T)d.dy * ld(c.mv, h_v(d, i, je));
-      const T rhs = a.sfv[pe] - cp * ld(c.thv, pe) * g0 + a.nu_div * dgy;
-      val = a.vpp[pe] + hdt * rhs;
+      const T dgy = (t.div[ty + 1][tx + 1] - t.div[ty][tx + 1]) * over(mv, d.rdy);
+      const T rhs = sf - cp * th * g0 + a.nu_div * dgy;
+      a.vh[p] = old + hdt * rhs;
     }
-    a.vh[p] = val;
   }
 }
 
@@ -417,66 +435,119 @@ __global__ void __launch_bounds__(128) split_column_kernel(Dims d, Coef<T> c, Sp
 }
 
 // The same column solve on tiles of PC columns (one block per tile and
-// row j) so that every thread works outside the recurrence: A1 the w-level
-// terms (explicit w'', the eta_dot flux, the coupling gamma) and A2 the
-// right-hand sides at every (level, column) pair, B one warp runs the
-// Thomas sweeps in shared memory, forming each row (lower, upper, main)
-// from gamma and C_pi / dz_m, C the pi'' and w'' updates.  Arithmetic is
-// term for term that of split_column_kernel.  Shared memory: (4 nz + 2) PC
-// values (c' overwrites the eta_dot fluxes once the right-hand sides are
-// formed).
+// row j) so that every thread works outside the recurrence, each phase's
+// loads batched (PU items in flight per thread): A0 the horizontal flux
+// divergence and the winds at the mass levels, A1 the w-level terms (explicit
+// w'', the eta_dot flux, the coupling gamma), A2 the right-hand sides, B one
+// warp runs the Thomas sweeps in shared memory, forming each row (lower,
+// upper, main) from gamma and C_pi / dz_m, C the pi'' and w'' updates.  dz_m
+// cancels between the divergence and C_pi / dz_m.  Shared memory: (6 nz + 2)
+// PC values (c' overwrites the eta_dot fluxes once the right-hand sides are
+// formed).  Bound by memory latency: 256x256x64 float32 157 us with a load
+// at a time and six divisions a point, 116 here.
 template <typename T, int PT, int PC>
-__global__ void __launch_bounds__(PT) split_column_tile_kernel(Dims d, Coef<T> c, SplitArgs<T> a, T a2cp,
-                                                               T adcp) {
+__global__ void __launch_bounds__(PT, sizeof(T) == 4 ? 4 : 2) split_column_tile_kernel(Dims d, Coef<T> c,
+                                                                                      SplitArgs<T> a, T a2cp,
+                                                                                      T adcp) {
   grid_chain();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
-  const int nx = d.nx, nz = d.nz;
+  const int nx = d.nx, ny = d.ny, nz = d.nz, pm = nx * ny;
   T* s_fz = sm;                      // [nz+1][PC]  eta_dot flux -> c'
   T* s_gam = s_fz + (nz + 1) * PC;   // [nz+1][PC]  gamma
-  T* s_x = s_gam + (nz + 1) * PC;    // [nz][PC]    rhs -> d' -> delta pi
+  T* s_x = s_gam + (nz + 1) * PC;    // [nz][PC]    flux divergence -> rhs -> d' -> delta pi
   T* s_cz = s_x + nz * PC;           // [nz][PC]    C_pi / dz_m
-  const int i0 = blockIdx.x * PC, j = blockIdx.y, tid = threadIdx.x;
+  T* s_um = s_cz + nz * PC;          // [nz][PC]    winds at mass levels
+  T* s_vm = s_um + nz * PC;          // [nz][PC]
+  const int j = blockIdx.y, tid = threadIdx.x;
+  const int lane = tid % PC, kt = tid / PC;
+  constexpr int KS = PT / PC;  // levels per pass of the block
+  const int i = blockIdx.x * PC + lane, ic = min(i, nx - 1);
+  const bool live = i < nx;
+  const int h = ic + nx * j;
   const T al = a.alpha, dtau = a.dtau, cp = (T)c.s.cp;
-  const T dx = (T)d.dx, dy = (T)d.dy;
-  const Winds<T> W{d, c, a.uh, a.vh};
-  const Grad<T> G{d, c, a.ppp};
-  for (int q = tid; q < (nz + 1) * PC; q += PT) {  // A1
-    const int k = q / PC, i = i0 + q % PC;
-    T fz = T(0), gam = T(0);
-    if (i < nx && k > 0 && k < nz) {
-      const int pw = iw(d, i, j, k);
-      const T thw = ld(c.thw, pw), rw = ld(c.rhow, pw);
-      const T wold = a.wpp[pw];
-      const T wex = wold + dtau * (a.sfw[pw] - cp * thw * G.gzw(i, j, k));
-      const T wav = (T(1) - al) * wold + al * wex;
-      fz = (wav - kinematic(d, c, W, i, j, k)) * rw * thw;
-      gam = a2cp * thw * rw * thw / ld(c.dzw, pw);
-      a.wpp[pw] = wex;
+  const T mm = ld(c.mm, h), m2x = over(mm * mm, d.rdx), m2y = over(mm * mm, d.rdy);
+  {  // A0
+    constexpr int PU = 2;
+    const T* __restrict__ uh = a.uh;
+    const T* __restrict__ vh = a.vh;
+    for (int k0 = kt; k0 < nz; k0 += PU * KS) {
+      T u0[PU], u1[PU], v0[PU], v1[PU], ru0[PU], ru1[PU], rv0[PU], rv1[PU], tu0[PU], tu1[PU], tv0[PU], tv1[PU], cz[PU];
+#pragma unroll
+      for (int n = 0; n < PU; ++n) {
+        const int k = min(k0 + n * KS, nz - 1), pu = iu(d, ic, j, k), pv = iv(d, ic, j, k);
+        u0[n] = ld(uh, pu);
+        u1[n] = ld(uh, pu + 1);
+        v0[n] = ld(vh, pv);
+        v1[n] = ld(vh, pv + nx);
+        ru0[n] = ld(c.rdu, pu);
+        ru1[n] = ld(c.rdu, pu + 1);
+        tu0[n] = ld(c.thu, pu);
+        tu1[n] = ld(c.thu, pu + 1);
+        rv0[n] = ld(c.rdv, pv);
+        rv1[n] = ld(c.rdv, pv + nx);
+        tv0[n] = ld(c.thv, pv);
+        tv1[n] = ld(c.thv, pv + nx);
+        cz[n] = ld(c.cpidz, h + k * pm);
+      }
+#pragma unroll
+      for (int n = 0; n < PU; ++n) {
+        const int k = k0 + n * KS;
+        if (k >= nz) break;
+        const int q = k * PC + lane;
+        s_um[q] = T(0.5) * (u0[n] + u1[n]);
+        s_vm[q] = T(0.5) * (v0[n] + v1[n]);
+        s_x[q] = (u1[n] * ru1[n] * tu1[n] - u0[n] * ru0[n] * tu0[n]) * m2x +
+                 (v1[n] * rv1[n] * tv1[n] - v0[n] * rv0[n] * tv0[n]) * m2y;
+        s_cz[q] = live ? cz[n] : T(0);
+      }
     }
-    s_fz[q] = fz;
-    s_gam[q] = gam;
   }
   __syncthreads();
-  for (int q = tid; q < nz * PC; q += PT) {  // A2
-    const int k = q / PC, i = i0 + q % PC;
-    if (i >= nx) {  // a trivial row: lower = upper = 0, main = 1
-      s_x[q] = T(0);
-      s_cz[q] = T(0);
-      continue;
+  {  // A1
+    constexpr int PU = 2;
+    const T* __restrict__ pp = a.ppp;
+    for (int k0 = kt; k0 <= nz; k0 += PU * KS) {
+      T th[PU], rw[PU], wo[PU], sf[PU], iz[PU], dz[PU], zx[PU], ze[PU], pl[PU], ph[PU];
+#pragma unroll
+      for (int n = 0; n < PU; ++n) {
+        const int k = min(k0 + n * KS, nz), pw = h + k * pm;  // an end level's own values: nobody writes them here
+        th[n] = ld(c.thw, pw);
+        rw[n] = ld(c.rhow, pw);
+        wo[n] = a.wpp[pw];
+        sf[n] = ld(a.sfw, pw);
+        iz[n] = ld(c.idzw, pw);
+        dz[n] = ld(c.dzw, pw);
+        zx[n] = ld(c.zxw, pw);
+        ze[n] = ld(c.zew, pw);
+        pl[n] = ld(pp, h + max(k - 1, 0) * pm);
+        ph[n] = ld(pp, h + min(k, nz - 1) * pm);
+      }
+#pragma unroll
+      for (int n = 0; n < PU; ++n) {
+        const int k = k0 + n * KS;
+        if (k > nz) break;
+        const int q = k * PC + lane;
+        T fz = T(0), gam = T(0);
+        if (live && k > 0 && k < nz) {
+          const T wex = wo[n] + dtau * (sf[n] - cp * th[n] * ((ph[n] - pl[n]) * iz[n]));
+          const T wav = (T(1) - al) * wo[n] + al * wex;
+          const T kin = mm * (T(0.5) * (s_um[q - PC] + s_um[q]) * zx[n] + T(0.5) * (s_vm[q - PC] + s_vm[q]) * ze[n]);
+          fz = (wav - kin) * rw[n] * th[n];
+          gam = a2cp * th[n] * rw[n] * th[n] / dz[n];
+          a.wpp[h + k * pm] = wex;
+        }
+        s_fz[q] = fz;
+        s_gam[q] = gam;
+      }
     }
-    const int p = im(d, i, j, k);
-    const T mm = ld(c.mm, h_m(d, i, j));
-    const T dzm = ld(c.dzm, p), cpidz = ld(c.cpidz, p);
-    const int u0 = iu(d, i, j, k), v0 = iv(d, i, j, k);
-    const T fx0 = a.uh[u0] * ld(c.rdu, u0) * ld(c.thu, u0);
-    const T fx1 = a.uh[u0 + 1] * ld(c.rdu, u0 + 1) * ld(c.thu, u0 + 1);
-    const T fy0 = a.vh[v0] * ld(c.rdv, v0) * ld(c.thv, v0);
-    const T fy1 = a.vh[v0 + nx] * ld(c.rdv, v0 + nx) * ld(c.thv, v0 + nx);
-    const T div_h = mm * ((fx1 - fx0) / dx * mm / dzm + (fy1 - fy0) / dy * mm / dzm);
-    const T div_z = (s_fz[q + PC] - s_fz[q]) / dzm;
-    s_x[q] = dtau * (a.sfp[p] - cpidz * dzm * (div_h + div_z));
-    s_cz[q] = cpidz;
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int k = kt; k < nz; k += KS) {  // A2; a column past the grid: a trivial row, lower = upper = 0, main = 1
+    const int q = k * PC + lane;
+    const T sp = ld(a.sfp, h + k * pm);
+    s_x[q] = live ? dtau * (sp - s_cz[q] * (s_x[q] + (s_fz[q + PC] - s_fz[q]))) : T(0);
   }
   __syncthreads();
   if (tid < PC) {  // B
@@ -509,18 +580,33 @@ __global__ void __launch_bounds__(PT) split_column_tile_kernel(Dims d, Coef<T> c
     }
   }
   __syncthreads();
-  for (int q = tid; q < (nz + 1) * PC; q += PT) {  // C
-    const int k = q / PC, i = i0 + q % PC;
-    if (i >= nx) continue;
-    const int pw = iw(d, i, j, k);
-    if (k == 0) {
-      a.wpp[pw] = kinematic(d, c, W, i, j, 0);
-    } else if (k == nz) {
-      a.wpp[pw] = T(0);
-    } else {
-      a.wpp[pw] = a.wpp[pw] - adcp * ld(c.thw, pw) * ((s_x[q] - s_x[q - PC]) * ld(c.idzw, pw));
+  if (!live) return;
+  constexpr int PU = 4;
+  for (int k0 = kt; k0 <= nz; k0 += PU * KS) {  // C
+    T wx[PU], th[PU], iz[PU], po[PU];
+#pragma unroll
+    for (int n = 0; n < PU; ++n) {
+      const int k = min(k0 + n * KS, nz), pw = h + k * pm;
+      wx[n] = a.wpp[pw];
+      th[n] = ld(c.thw, pw);
+      iz[n] = ld(c.idzw, pw);
+      po[n] = a.ppp[h + min(k, nz - 1) * pm];
     }
-    if (k < nz) a.ppp[pw] = a.ppp[pw] + s_x[q];
+#pragma unroll
+    for (int n = 0; n < PU; ++n) {
+      const int k = k0 + n * KS;
+      if (k > nz) break;
+      const int pw = h + k * pm, q = k * PC + lane;
+      if (k == 0) {  // the kinematic ground value: both levels of the padded pair
+        const T uw = T(0.5) * (s_um[lane] + s_um[PC + lane]), vw = T(0.5) * (s_vm[lane] + s_vm[PC + lane]);
+        a.wpp[pw] = mm * (uw * ld(c.zxw, pw) + vw * ld(c.zew, pw));
+      } else if (k == nz) {
+        a.wpp[pw] = T(0);
+      } else {
+        a.wpp[pw] = wx[n] - adcp * th[n] * ((s_x[q] - s_x[q - PC]) * iz[n]);
+      }
+      if (k < nz) a.ppp[pw] = po[n] + s_x[q];
+    }
   }
 }
 
@@ -531,47 +617,49 @@ template <typename T>
 __global__ void __launch_bounds__(SX * SY) split_correct_kernel(Dims d, Coef<T> c, SplitArgs<T> a,
                                                                 T* __restrict__ upp2, T* __restrict__ vpp2) {
   grid_chain();
-  __shared__ T Dt[SY + 1][SX + 1];
+  __shared__ FaceTile<T> t;
   const int i0 = blockIdx.x * SX, j0 = blockIdx.y * SY, k = blockIdx.z;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int i = i0 + tx, j = j0 + ty;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  if (k < nz) div_tile<T>(d, c, a.uc, a.uh, a.vc, a.vh, i0, j0, k, Dt);
+  if (k < nz) fill_tile<T>(d, c, a.uc, a.uh, a.vc, a.vh, a.ppp, true, i0, j0, k, t);
   __syncthreads();
   if (i > nx || j > ny) return;
   const T cp = (T)c.s.cp, dtau = a.dtau;
-  const Grad<T> G{d, c, a.ppp};
+  const T idx = (T)d.rdx, idy = (T)d.rdy;
   if (j < ny && k < nz) {
     const int p = iu(d, i, j, k);
-    T val;
     if (!d.px && (i == 0 || i == nx)) {
-      val = a.u0[p] - a.uc[p];
+      upp2[p] = ld(a.u0, p) - ld(a.uc, p);
     } else {
       const int ie = (d.px && i == nx) ? 0 : i, pe = iu(d, ie, j, k);
-      const T g1 = G.gx(ie, j, k);
+      const T mu = ld(c.mu, h_u(d, ie, j)), zx = ld(c.zxu, pe), th = ld(c.thu, pe), sf = ld(a.sfu, pe), old = ld(a.upp, pe),
+              g0 = ld(a.gx0, pe);
+      const T g = (t.p[ty + 1][tx + 1] - t.p[ty + 1][tx]) * idx * mu;
+      const T g1 = g - zx * T(0.5) * (t.gz[ty + 1][tx] + t.gz[ty + 1][tx + 1]);
+      const T dgx = (t.div[ty + 1][tx + 1] - t.div[ty + 1][tx]) * over(mu, d.rdx);
+      upp2[p] = old + dtau * (sf - T(0.5) * cp * th * (g0 + g1) + a.nu_div * dgx);
       if (a.gx1) a.gx1[p] = g1;
-      const T dgx = (Dt[ty + 1][tx + 1] - Dt[ty + 1][tx]) / (T)d.dx * ld(c.mu, h_u(d, ie, j));
-      val = a.upp[pe] + dtau * (a.sfu[pe] - T(0.5) * cp * ld(c.thu, pe) * (a.gx0[pe] + g1) + a.nu_div * dgx);
     }
-    upp2[p] = val;
   }
   if (i < nx && k < nz) {
     const int p = iv(d, i, j, k);
-    T val;
     if (!d.py && (j == 0 || j == ny)) {
-      val = a.v0[p] - a.vc[p];
+      vpp2[p] = ld(a.v0, p) - ld(a.vc, p);
     } else {
       const int je = (d.py && j == ny) ? 0 : j, pe = iv(d, i, je, k);
-      const T g1 = G.gy(i, je, k);
+      const T mv = ld(c.mv, h_v(d, i, je)), ze = ld(c.zev, pe), th = ld(c.thv, pe), sf = ld(a.sfv, pe), old = ld(a.vpp, pe),
+              g0 = ld(a.gy0, pe);
+      const T g = (t.p[ty + 1][tx + 1] - t.p[ty][tx + 1]) * idy * mv;
+      const T g1 = g - ze * T(0.5) * (t.gz[ty][tx + 1] + t.gz[ty + 1][tx + 1]);
+      const T dgy = (t.div[ty + 1][tx + 1] - t.div[ty][tx + 1]) * over(mv, d.rdy);
+      vpp2[p] = old + dtau * (sf - T(0.5) * cp * th * (g0 + g1) + a.nu_div * dgy);
       if (a.gy1) a.gy1[p] = g1;
-      const T dgy = (Dt[ty + 1][tx + 1] - Dt[ty][tx + 1]) / (T)d.dy * ld(c.mv, h_v(d, i, je));
-      val = a.vpp[pe] + dtau * (a.sfv[pe] - T(0.5) * cp * ld(c.thv, pe) * (a.gy0[pe] + g1) + a.nu_div * dgy);
     }
-    vpp2[p] = val;
   }
   if (i < nx && j < ny) {
     const int p = iw(d, i, j, k);
-    const T wc = a.wc[p];
+    const T wc = ld(a.wc, p);
     a.wpp[p] = (wc + a.wpp[p]) / (T(1) + dtau * ld(a.tau, p)) - wc;
   }
 }
@@ -655,17 +743,27 @@ void launch_split_predict(const Dims& d, const Coef<T>& c, const SplitArgs<T>& a
   launch_chained(split_predict_kernel<T>, box(d.nx + 1, d.ny + 1, d.nz, blk), blk, 0, st, d, c, a);
 }
 
+template <typename T, int PC>
+static void launch_column_tile(const Dims& d, const Coef<T>& c, const SplitArgs<T>& a, T a2cp, T adcp, size_t smem,
+                               cudaStream_t st) {
+  constexpr int PT = 256;
+  static SmemLimit attr_bytes;  // per instantiation
+  ensure_smem_limit((const void*)split_column_tile_kernel<T, PT, PC>, attr_bytes, smem);
+  launch_chained(split_column_tile_kernel<T, PT, PC>, dim3((d.nx + PC - 1) / PC, d.ny), PT, smem, st, d, c, a, a2cp,
+                 adcp);
+}
+
 template <typename T>
 void launch_split_column(const Dims& d, const Coef<T>& c, const SplitArgs<T>& a, cudaStream_t st) {
   const double ad = (double)a.alpha * (double)a.dtau;
   const T a2cp = (T)(ad * ad * c.s.cp), adcp = (T)(ad * c.s.cp);
-  constexpr int PT = 256, PC = 32;
-  const size_t smem = (size_t)(4 * d.nz + 2) * PC * sizeof(T);
-  if (smem <= 200 * 1024) {  // tiles of 32 columns; the one-thread-per-column march beyond
-    static SmemLimit attr_bytes;  // per instantiation
-    ensure_smem_limit((const void*)split_column_tile_kernel<T, PT, PC>, attr_bytes, smem);
-    launch_chained(split_column_tile_kernel<T, PT, PC>, dim3((d.nx + PC - 1) / PC, d.ny), PT, smem, st, d, c, a,
-                   a2cp, adcp);
+  const size_t level = (size_t)(6 * d.nz + 2) * sizeof(T);  // shared memory of a column
+  if (32 * level <= 200 * 1024) {
+    launch_column_tile<T, 32>(d, c, a, a2cp, adcp, 32 * level, st);
+    return;
+  }
+  if (16 * level <= 200 * 1024) {  // many levels: half the columns; the one-thread-per-column march beyond
+    launch_column_tile<T, 16>(d, c, a, a2cp, adcp, 16 * level, st);
     return;
   }
   launch_chained(split_column_kernel<T>, dim3((d.nx + 127) / 128, d.ny), 128, 0, st, d, c, a, a2cp, adcp);

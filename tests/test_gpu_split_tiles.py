@@ -27,3 +27,9 @@ def test_step_is_the_oracles(shape, periodic):
     out = pst.step(to_cuda(s0), 0.0, None, lambda s, f: s)
     errs = {k: rel_l2(out[k], ref[k]) for k in ("u", "v", "w", "eta_dot", "pi", "th_v", "rho")}
     assert max(errs.values()) < 1e-10, errs
+
+
+# past the shared memory of a tile of 32 columns (133 levels in float64), of 16 (266), and into the march
+@pytest.mark.parametrize("nz", [133, 134, 266, 267])
+def test_column_solve_at_many_levels(nz):
+    test_step_is_the_oracles((17, 2, nz), ())
