@@ -996,58 +996,102 @@ __global__ void begin_cycle_kernel(GState* gs) {
 }
 
 // y from the cycle's small problem; coef_i = y_i s_i, or B y in the block
-// form, whose triangular solves run on one warp (a row's inner product over
-// the lanes).
+// form, whose triangular solves run on one warp.
+// Columns of H the least-squares solve stages at a time.
+constexpr int SS_C = 32;
+// the factorisation of a restart of 100 has work for 32 warps, one of 30 for 8
+inline int small_solve_threads(int R) { return R > 32 ? 1024 : 256; }
+inline size_t small_solve_smem(int R) { return ((size_t)R * R + (size_t)SS_C * (R | 1)) * sizeof(double); }
+
+// One warp: x <- the solution of T^T x = x for the lower triangle T (row
+// stride ld, n <= GM_MAXR rows) with reciprocal diagonal rd, from the last row
+// up; a lane keeps every 32nd element, and each solved one is subtracted
+// from all the others at once (its row of T is read ahead of it).
+__device__ __forceinline__ void triangle_back(const double* t, int ld, int n, const double* rd, double* x) {
+  const int lane = threadIdx.x & 31;
+  double v[GM_MAXR / 32];
+#pragma unroll
+  for (int q = 0; q < GM_MAXR / 32; ++q) v[q] = lane + 32 * q < n ? x[lane + 32 * q] : 0.0;
+#pragma unroll
+  for (int q = GM_MAXR / 32 - 1; q >= 0; --q) {
+    for (int i = min(n, 32 * (q + 1)) - 1; i >= 32 * q; --i) {
+      const double xi = __shfl_sync(0xffffffffu, v[q], i & 31) * rd[i];
+#pragma unroll
+      for (int m = 0; m <= q; ++m) {
+        const int k = lane + 32 * m;
+        if (k < i) v[m] -= t[i * ld + k] * xi;
+      }
+      if (lane == (i & 31)) v[q] = xi;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < GM_MAXR / 32; ++q)
+    if (lane + 32 * q < n) x[lane + 32 * q] = v[q];
+}
+
+// The cycle's least-squares problem, one block.  Bound by its serial chain:
+// what each pivot and each solved unknown waits for.  Restart 100, batched: 530
+// us with strided reads of H, an integer division per updated element and two
+// warp sums per unknown, 151 us here (186 with 8 warps); restart 30,
+// incremental: 22.5 -> 6.2 us.
 __device__ void small_solve_state(GState* gs) {
-  extern __shared__ double a2[];  // R * R
-  const int R = gs->restart, kd = gs->kdone, lane = threadIdx.x & 31;
+  extern __shared__ double a2[];  // R * R, then a chunk of columns of H
+  const int R = gs->restart, kd = gs->kdone, tid = threadIdx.x, lane = tid & 31, wp = tid >> 5, nw = blockDim.x >> 5;
   __shared__ double b2[GM_MAXR];
   __shared__ double y[GM_MAXR];
+  __shared__ double rd[GM_MAXR];  // reciprocal diagonal of a triangular solve
   if (gs->method == 0) {
-    // _lstsq(H.T, beta): normal equations (H H^T) y = H beta, Cholesky solve
-    for (int q = threadIdx.x; q < R * R; q += blockDim.x) {
-      const int p = q / R, r = q % R;
-      double s = 0.0;
-      for (int c = 0; c <= R; ++c) s += gs->H[p][c] * gs->H[r][c];
-      a2[q] = s;
-    }
-    for (int p = threadIdx.x; p < R; p += blockDim.x) {
-      double s = 0.0;
-      for (int c = 0; c <= R; ++c) s += gs->H[p][c] * gs->beta[c];
-      b2[p] = s;
+    // _lstsq(H.T, beta): normal equations (H H^T) y = H beta, Cholesky solve.  Row p of H ends at column p + 1, and
+    // the lower triangle is enough.
+    const int P = R | 1;
+    double* ht = a2 + (size_t)R * R;  // [SS_C][P]: columns c0 .. of H, transposed
+    for (int q = tid; q < R * R; q += blockDim.x) a2[q] = 0.0;
+    for (int p = tid; p < R; p += blockDim.x) b2[p] = 0.0;
+    for (int c0 = 0; c0 <= R; c0 += SS_C) {
+      const int nc = min(SS_C, R + 1 - c0);
+      __syncthreads();
+      for (int q = tid; q < R * SS_C; q += blockDim.x) {
+        const int r = q / SS_C, c = q % SS_C;
+        if (c < nc) ht[c * P + r] = gs->H[r][c0 + c];
+      }
+      __syncthreads();
+      for (int p = max(c0 - 1, 0) + wp; p < R; p += nw)
+        for (int r = max(c0 - 1, 0) + lane; r <= p; r += 32) {
+          double v = a2[p * R + r];
+          for (int c = 0; c < min(nc, r + 2 - c0); ++c) v += ht[c * P + p] * ht[c * P + r];
+          a2[p * R + r] = v;
+        }
+      for (int p = tid; p < R; p += blockDim.x) {
+        double v = b2[p];
+        for (int c = 0; c < min(nc, p + 2 - c0); ++c) v += ht[c * P + p] * gs->beta[c0 + c];
+        b2[p] = v;
+      }
     }
     __syncthreads();
-    // right-looking Cholesky, lower factor stored in a2
+    // right-looking Cholesky, lower factor stored in a2; with several columns per block the right-hand side rides
+    // along as one more row, which leaves L^-1 b2 in y
+    const bool carry = gs->columns > 1;
     for (int k = 0; k < R; ++k) {
-      if (threadIdx.x == 0) a2[k * R + k] = sqrt(a2[k * R + k]);
-      __syncthreads();
-      const double dkk = a2[k * R + k];
-      for (int i = k + 1 + threadIdx.x; i < R; i += blockDim.x) a2[i * R + k] /= dkk;
-      __syncthreads();
-      for (int q = threadIdx.x; q < (R - k - 1) * (R - k - 1); q += blockDim.x) {
-        const int i = k + 1 + q / (R - k - 1), jj = k + 1 + q % (R - k - 1);
-        if (jj <= i) a2[i * R + jj] -= a2[i * R + k] * a2[jj * R + k];
+      const double dkk = sqrt(a2[k * R + k]);
+      __syncthreads();  // every thread has the pivot
+      for (int i = k + 1 + tid; i < R; i += blockDim.x) a2[i * R + k] /= dkk;
+      if (tid == 0) {
+        a2[k * R + k] = dkk;
+        rd[k] = 1.0 / dkk;
+        if (carry) y[k] = b2[k] / dkk;
       }
+      __syncthreads();
+      for (int i = k + 1 + wp; i < R; i += nw) {
+        const double lik = a2[i * R + k];
+        for (int jj = k + 1 + lane; jj <= i; jj += 32) a2[i * R + jj] -= lik * a2[jj * R + k];
+      }
+      if (carry)
+        for (int i = k + 1 + tid; i < R; i += blockDim.x) b2[i] -= a2[i * R + k] * y[k];
       __syncthreads();
     }
-    if (gs->columns > 1) {
-      if (threadIdx.x < 32) {
-        for (int i = 0; i < R; ++i) {  // L z = b2
-          double s = 0.0;
-          for (int k = lane; k < i; k += 32) s += a2[i * R + k] * y[k];
-          s = warp_sum(s);
-          if (lane == 0) y[i] = (b2[i] - s) / a2[i * R + i];
-          __syncwarp();
-        }
-        for (int i = R - 1; i >= 0; --i) {  // L^T y = z
-          double s = 0.0;
-          for (int k = i + 1 + lane; k < R; k += 32) s += a2[k * R + i] * y[k];
-          s = warp_sum(s);
-          if (lane == 0) y[i] = (y[i] - s) / a2[i * R + i];
-          __syncwarp();
-        }
-      }
-    } else if (threadIdx.x == 0) {
+    if (carry) {
+      if (wp == 0) triangle_back(a2, R, R, rd, y);  // L^T y = z
+    } else if (tid == 0) {
       for (int i = 0; i < R; ++i) {  // L z = b2
         double s = b2[i];
         for (int k = 0; k < i; ++k) s -= a2[i * R + k] * y[k];
@@ -1063,14 +1107,16 @@ __device__ void small_solve_state(GState* gs) {
   } else {
     // back substitution with the rotated rows: sum_j R[j][i] y_j = beta_i
     if (gs->columns > 1) {
-      if (threadIdx.x < 32)
-        for (int i = kd - 1; i >= 0; --i) {
-          double s = 0.0;
-          for (int jj = i + 1 + lane; jj < kd; jj += 32) s += gs->H[jj][i] * y[jj];
-          s = warp_sum(s);
-          if (lane == 0) y[i] = (gs->beta[i] - s) / gs->H[i][i];
-          __syncwarp();
-        }
+      for (int q = tid; q < kd * R; q += blockDim.x) {
+        const int i = q / R, k = q % R;
+        if (k < i) a2[i * R + k] = gs->H[i][k];
+      }
+      for (int i = tid; i < kd; i += blockDim.x) {
+        rd[i] = 1.0 / gs->H[i][i];
+        y[i] = gs->beta[i];
+      }
+      __syncthreads();
+      if (wp == 0) triangle_back(a2, R, kd, rd, y);
     } else if (threadIdx.x == 0) {
       for (int i = kd - 1; i >= 0; --i) {
         double s = gs->beta[i];
@@ -1091,7 +1137,7 @@ __device__ void small_solve_state(GState* gs) {
     gs->coef[k] = v;
   }
 }
-__global__ void small_solve_kernel(GState* gs) {
+__global__ void __launch_bounds__(1024) small_solve_kernel(GState* gs) {
   grid_chain();
   small_solve_state(gs);
 }
@@ -1244,7 +1290,7 @@ __global__ void group_begin_cycle_kernel(GroupMember<T>* mem) {
   if (g.running) begin_cycle_state(g.gs);
 }
 template <typename T>
-__global__ void group_small_solve_kernel(GroupMember<T>* mem) {
+__global__ void __launch_bounds__(1024) group_small_solve_kernel(GroupMember<T>* mem) {
   grid_chain();
   const GroupMember<T>& g = mem[blockIdx.x];
   if (g.running) small_solve_state(g.gs);
@@ -1408,10 +1454,10 @@ void gm_gate(GState* gs, cudaGraphConditionalHandle h, int maxiter, int after_cy
 void gm_info(const GState* gs, GDevInfo* o, cudaStream_t st) { launch_chained(info_kernel, 1, 1, 0, st, gs, o); }
 void gm_begin_cycle(GState* gs, cudaStream_t st) { launch_chained(begin_cycle_kernel, 1, 256, 0, st, gs); }
 void gm_small_solve(GState* gs, int restart, cudaStream_t st) {
-  const size_t smem = (size_t)restart * restart * sizeof(double);
+  const size_t smem = small_solve_smem(restart);
   static SmemLimit attr_bytes;
-  ensure_smem_limit((const void*)small_solve_kernel, attr_bytes, (size_t)GM_MAXR * GM_MAXR * sizeof(double));
-  launch_chained(small_solve_kernel, 1, 256, smem, st, gs);
+  ensure_smem_limit((const void*)small_solve_kernel, attr_bytes, small_solve_smem(GM_MAXR));
+  launch_chained(small_solve_kernel, 1, small_solve_threads(restart), smem, st, gs);
 }
 void gm_snapshot(const GState* gs, GHostView* v, cudaStream_t st) { launch_chained(snapshot_kernel, 1, 1, 0, st, gs,
     v); }
@@ -1492,8 +1538,8 @@ void grp_begin_cycle(const GroupLaunch<T>& g, cudaStream_t st) {
 template <typename T>
 void grp_small_solve(const GroupLaunch<T>& g, cudaStream_t st) {
   static SmemLimit attr_bytes;
-  ensure_smem_limit((const void*)group_small_solve_kernel<T>, attr_bytes, (size_t)GM_MAXR * GM_MAXR * sizeof(double));
-  launch_chained(group_small_solve_kernel<T>, g.M, 256, (size_t)g.R * g.R * sizeof(double), st, g.mem);
+  ensure_smem_limit((const void*)group_small_solve_kernel<T>, attr_bytes, small_solve_smem(GM_MAXR));
+  launch_chained(group_small_solve_kernel<T>, g.M, small_solve_threads(g.R), small_solve_smem(g.R), st, g.mem);
 }
 template <typename T>
 void grp_gate(const GroupLaunch<T>& g, cudaGraphConditionalHandle h, int after_cycle, cudaStream_t st) {
