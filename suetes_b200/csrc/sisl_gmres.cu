@@ -351,8 +351,11 @@ __device__ __forceinline__ void block_coefs(GState* gs, const double* w, double*
 //
 // Bound by reading the m + s vectors: the tensor work of a pass (8 of 8
 // columns for 6 vectors) stays below the loads' time.  256x256x80 float32,
-// the inner products of a cycle of 30: 9.1 ms in one-step form, 2.71 ms here
-// (3.7 TB/s of the rows read once; the float64 tensor pipe 60 % busy).
+// the inner products of a cycle of 30: 9.1 ms in one-step form, 2.14 ms here
+// (4.7 TB/s of the rows read once), 2.71 with four row tiles loaded and then
+// multiplied.  One tile ahead is enough and keeps two blocks' registers: four
+// ahead spill (31 rows 893 us against 577), two ahead 807; three blocks an SM
+// help only the shortest (7 rows 198 against 263, 31 rows 623).
 //
 // The partial tiles are summed in two levels (groups of GM_GROUP blocks, then
 // the groups), in a fixed order: the same bits on every run.
@@ -361,7 +364,7 @@ __device__ __forceinline__ void block_dots_body(const T* __restrict__ Vb, size_t
                                                 double* partial, GState* gs, int bid, int nblk) {
   constexpr int VN = V16<T>::n;
   constexpr int KW = 8 * VN;  // elements of every row a warp takes per pass: two 16-byte pieces per lane
-  constexpr int GRP = NT < 4 ? NT : 4;
+  constexpr int GRP = NT < 4 ? NT : 4;  // tiles summed over the warps at a time
   __shared__ double red[8][GRP * 64];
   __shared__ double w[NT * 64], r1s[NT * 64];
   const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
@@ -373,28 +376,36 @@ __device__ __forceinline__ void block_dots_body(const T* __restrict__ Vb, size_t
   double acc[NT][2];
 #pragma unroll
   for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = 0.0;
-  for (size_t k = ((size_t)bid * 8 + wp) * KW; k < n; k += (size_t)nblk * 8 * KW) {
-    T z[2 * VN];
-    load16(zp + k, z);
-    load16(zp + k + 4 * VN, z + VN);
+  // a row tile's loads (at a pass's end the next pass's first ones) are issued while the tile before is multiplied
+  const size_t step = (size_t)nblk * 8 * KW;
+  T z[2 * VN], zn[2 * VN], a[2 * VN], an[2 * VN];
+  auto load = [&](const T* v, T* q) {
+    load16(v, q);
+    load16(v + 4 * VN, q + VN);
+  };
+  auto row = [&](int t) { return v0 + (size_t)min(8 * t + r, rows - 1) * stride; };
+  size_t k = ((size_t)bid * 8 + wp) * KW;
+  if (k < n) {
+    load(zp + k, z);
+    load(row(0) + k, a);
+  }
+  for (; k < n; k += step) {
+    const size_t kn = k + step < n ? k + step : k;  // the last pass repeats its own loads
 #pragma unroll
-    for (int t0 = 0; t0 < NT; t0 += GRP) {
-      T a[GRP][2 * VN];
-#pragma unroll
-      for (int t = 0; t < GRP; ++t) {
-        if (t0 + t >= NT) continue;
-        const T* v = v0 + (size_t)min(8 * (t0 + t) + r, rows - 1) * stride + k;
-        load16(v, a[t]);
-        load16(v + 4 * VN, a[t] + VN);
+    for (int t = 0; t < NT; ++t) {
+      if (t + 1 < NT) {
+        load(row(t + 1) + k, an);
+      } else {
+        load(zp + kn, zn);
+        load(row(0) + kn, an);
       }
 #pragma unroll
-      for (int e = 0; e < 2 * VN; ++e) {
-        const double zd = (double)z[e];
+      for (int e = 0; e < 2 * VN; ++e) dmma(acc[t], (double)a[e], (double)z[e]);
 #pragma unroll
-        for (int t = 0; t < GRP; ++t)
-          if (t0 + t < NT) dmma(acc[t0 + t], (double)a[t][e], zd);
-      }
+      for (int e = 0; e < 2 * VN; ++e) a[e] = an[e];
     }
+#pragma unroll
+    for (int e = 0; e < 2 * VN; ++e) z[e] = zn[e];
   }
   double* mine = partial + (size_t)bid * (NT * 64);
 #pragma unroll
