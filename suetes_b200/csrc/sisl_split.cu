@@ -5,12 +5,11 @@
 // v_m, w_m (split_adv_kernel) averaged to the staggers (split_slow_kernel);
 // then n acoustic sub-steps of three kernels: the horizontal predictor to
 // the midpoint (split_predict_kernel), the vertically implicit pi''/w''
-// column solve (split_column_kernel, one thread per column, Thomas in the
-// float arithmetic of the tridiagonal solve), and the centred corrector with
-// the backward w damping (split_correct_kernel); split_end_kernel assembles
-// the stage state and split_diag_kernel diagnoses eta_dot and the kinematic
-// w boundaries.  Every kernel is one thread per output point (columns for
-// the solve) and HBM-bound.
+// column solve (split_column_tile_kernel, Thomas in the float arithmetic of
+// the tridiagonal solve; split_column_kernel, one thread per column, past its
+// shared memory), and the centred corrector with the backward w damping
+// (split_correct_kernel); split_end_kernel assembles the stage state and
+// split_diag_kernel diagnoses eta_dot and the kinematic w boundaries.
 #include "sisl_explicit_dev.cuh"
 #include "sisl_split.cuh"
 
