@@ -260,7 +260,9 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
 // result.
 __device__ __forceinline__ void block_coefs(GState* gs, const double* w, double* r1s, int j0, int s) {
   __shared__ double g[GM_S][GM_S], r2[GM_S][GM_S], u[GM_S][GM_S];
+  __shared__ int keep_s;
   const int m = j0 + 1, tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+  if (tid < GM_S * GM_S) (&r2[0][0])[tid] = (&u[0][0])[tid] = 0.0;
   for (int q = tid; q < m * 8; q += GT) {
     const int l = q >> 3, i = q & 7;
     double v = 0.0;
@@ -285,8 +287,6 @@ __device__ __forceinline__ void block_coefs(GState* gs, const double* w, double*
   if (tid == 0) {
     int keep = s;
     const double lost = 32.0 * gs->eps;
-    for (int i = 0; i < GM_S; ++i)
-      for (int k = 0; k < GM_S; ++k) { r2[i][k] = 0.0; u[i][k] = 0.0; }
     for (int i = 0; i < keep; ++i) {
       double piv = g[i][i];
       for (int q = 0; q < i; ++q) {
@@ -307,19 +307,25 @@ __device__ __forceinline__ void block_coefs(GState* gs, const double* w, double*
         keep = i;
       }
     }
-    for (int i = 0; i < keep; ++i) {  // u = r2^-1
-      u[i][i] = 1.0 / r2[i][i];
-      for (int q = i - 1; q >= 0; --q) {
-        double v = 0.0;
-        for (int p = q + 1; p <= i; ++p) v -= r2[q][p] * u[p][i];
-        u[q][i] = v / r2[q][q];
-      }
-    }
     gs->bs = keep;
-    for (int i = 0; i < GM_S; ++i)
-      for (int k = 0; k < GM_S; ++k) { gs->r2[i][k] = r2[i][k]; gs->u[i][k] = u[i][k]; }
+    keep_s = keep;
   }
   __syncthreads();
+  if (tid < keep_s) {  // u = r2^-1, a column per thread
+    const int i = tid;
+    u[i][i] = 1.0 / r2[i][i];
+    for (int q = i - 1; q >= 0; --q) {
+      double v = 0.0;
+      for (int p = q + 1; p <= i; ++p) v -= r2[q][p] * u[p][i];
+      u[q][i] = v / r2[q][q];
+    }
+  }
+  __syncthreads();
+  if (tid < GM_S * GM_S) {
+    const int i = tid / GM_S, k = tid - i * GM_S;
+    gs->r2[i][k] = r2[i][k];
+    gs->u[i][k] = u[i][k];
+  }
   // r1 u, then back to the stored vectors: cv = B (r1 u)
   double t[GM_S];
   for (int l = tid; l < m; l += GT) {
@@ -477,10 +483,10 @@ __device__ __forceinline__ void block_finish(GState* gs, const double (&gram)[GM
   __shared__ int keep_s, done_s;
   const int m = j0 + 1, R = gs->restart, tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
   const bool rotate = gs->method != 0;
+  if (tid < GM_S * GM_S) (&rc[0][0])[tid] = (&ri[0][0])[tid] = (&t2[0][0])[tid] = 0.0;
+  __syncthreads();
   if (tid == 0) {
     int keep = gs->bs;
-    for (int i = 0; i < GM_S; ++i)
-      for (int k = 0; k < GM_S; ++k) { rc[i][k] = 0.0; ri[i][k] = 0.0; t2[i][k] = 0.0; }
     for (int i = 0; i < keep; ++i) {
       double piv = gram[i][i];
       for (int q = 0; q < i; ++q) {
@@ -498,20 +504,22 @@ __device__ __forceinline__ void block_finish(GState* gs, const double (&gram)[GM
       rc[i][i] = piv > 0.0 ? sqrt(piv) : 0.0;
       if (!(rc[i][i] > 0.0)) keep = i + 1;  // i = 0: nothing left of Z_1
     }
-    for (int i = 0; i < keep; ++i) {
-      ri[i][i] = rc[i][i] > 0.0 ? 1.0 / rc[i][i] : 0.0;
-      for (int q = i - 1; q >= 0; --q) {
-        double v = 0.0;
-        for (int p = q + 1; p <= i; ++p) v -= rc[q][p] * ri[p][i];
-        ri[q][i] = v * ri[q][q];
-      }
-      for (int q = 0; q <= i; ++q) {
-        double v = 0.0;
-        for (int p = q; p <= i; ++p) v += rc[q][p] * gs->r2[p][i];
-        t2[q][i] = v;
-      }
-    }
     keep_s = keep;
+  }
+  __syncthreads();
+  if (tid < keep_s) {  // ri = rc^-1 and t2 = rc r2, a column per thread
+    const int i = tid;
+    for (int q = 0; q <= i; ++q) {
+      double v = 0.0;
+      for (int p = q; p <= i; ++p) v += rc[q][p] * gs->r2[p][i];
+      t2[q][i] = v;
+    }
+    ri[i][i] = rc[i][i] > 0.0 ? 1.0 / rc[i][i] : 0.0;
+    for (int q = i - 1; q >= 0; --q) {
+      double v = 0.0;
+      for (int p = q + 1; p <= i; ++p) v -= rc[q][p] * ri[p][i];
+      ri[q][i] = v * (rc[q][q] > 0.0 ? 1.0 / rc[q][q] : 0.0);
+    }
   }
   for (int q = tid; q < 2 * j0; q += GT) (&gv[0][0])[q] = (&gs->givens[0][0])[q];
   __syncthreads();
