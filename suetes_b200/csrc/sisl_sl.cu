@@ -119,6 +119,10 @@ __device__ __forceinline__ T trilinear(const T* __restrict__ f, const Ext& e, T 
   return acc;
 }
 
+// Upper neighbour of stencil base l, clamped into [0, n): no sum that could
+// overflow, since a diverged wind puts l at either end of the integers.
+__device__ __forceinline__ int upper_index(int l, int n) { return l < n - 1 ? max(l + 1, 0) : n - 1; }
+
 // The gather of the three velocities at stencil base (lx, ly, lz) with
 // weights (wx, wy, wz), corners summed in itertools.product order.  float32:
 // all 24 loads in flight together, and away from the x edges both columns of a
@@ -129,12 +133,12 @@ template <typename T>
 __device__ __forceinline__ void trilinear3(const T* __restrict__ vx, const T* __restrict__ vy,
                                            const T* __restrict__ vz, const Ext& e, int lx, int ly, int lz, T wx, T wy,
                                            T wz, T& ax, T& ay, T& az) {
-  const int iy[2] = {min(max(ly, 0), e.ey - 1), min(max(ly + 1, 0), e.ey - 1)};
-  const int iz[2] = {min(max(lz, 0), e.ez - 1), min(max(lz + 1, 0), e.ez - 1)};
+  const int iy[2] = {min(max(ly, 0), e.ey - 1), upper_index(ly, e.ey)};
+  const int iz[2] = {min(max(lz, 0), e.ez - 1), upper_index(lz, e.ez)};
   const T Wx[2] = {T(1) - wx, wx}, Wy[2] = {T(1) - wy, wy}, Wz[2] = {T(1) - wz, wz};
   const T* __restrict__ fs[3] = {vx, vy, vz};
   if (sizeof(T) == 8) {
-    const int ix[2] = {min(max(lx, 0), e.ex - 1), min(max(lx + 1, 0), e.ex - 1)};
+    const int ix[2] = {min(max(lx, 0), e.ex - 1), upper_index(lx, e.ex)};
     auto one = [&](const T* __restrict__ f) {
       T acc = T(0);
 #pragma unroll
@@ -152,7 +156,7 @@ __device__ __forceinline__ void trilinear3(const T* __restrict__ vx, const T* __
     return;
   }
   T vals[3][2][2][2];
-  if (lx >= 0 && lx + 1 < e.ex) {
+  if ((unsigned)lx < (unsigned)(e.ex - 1)) {  // lx and lx + 1 are columns of the field
 #pragma unroll
     for (int b = 0; b < 2; ++b)
 #pragma unroll
@@ -166,7 +170,7 @@ __device__ __forceinline__ void trilinear3(const T* __restrict__ vx, const T* __
         }
       }
   } else {
-    const int ix[2] = {min(max(lx, 0), e.ex - 1), min(max(lx + 1, 0), e.ex - 1)};
+    const int ix[2] = {min(max(lx, 0), e.ex - 1), upper_index(lx, e.ex)};
 #pragma unroll
     for (int b = 0; b < 2; ++b)
 #pragma unroll

@@ -49,3 +49,29 @@ def test_departure_points_on_small_grids(shape, dtype, tol):
         out = PA(p[0], p[2], 100.0).compute_departure_indices(to_cuda(s, dtype), loc=loc)
         bound = tol * (1.0 if dtype == torch.float64 else max(8.0, float(max(shape))))  # a coordinate's own rounding
         assert max_abs(out, ref) < bound, (loc, max_abs(out, ref))
+
+
+# A diverged wind: the midpoints lie past the largest integer (or are not
+# numbers) and the gathers take the nearest edge.  Uniform winds interpolate
+# to themselves, so the points are known: index minus displacement, with the
+# rounding of four float products.
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-13), (torch.float32, 2e-6)])
+@pytest.mark.parametrize("wind", [1e12, -1e12, 3e30, -3e30, float("inf"), float("-inf"), float("nan")])
+def test_departure_points_of_a_diverged_wind(wind, dtype, tol):
+    from suetes_b200 import SemiLagrangianAdvector3D as PA
+    shape = (8, 5, 4)
+    p = build("cuda", *shape, 1000.0, 1000.0, 500.0, device="cuda", dt=100.0)
+    adv = PA(p[0], p[2], 100.0)
+    for axis in ("u", "v", "eta_dot"):
+        s = {k: torch.zeros(v, dtype=dtype, device="cuda") for k, v in shapes5(*shape).items()
+             if k in ("u", "v", "eta_dot")}
+        s[axis] += wind
+        for loc in ("m", "u", "v", "w"):
+            out = adv.compute_departure_indices(s, loc=loc)
+            if abs(wind) < float("inf"):
+                assert torch.isfinite(out).all()
+                if axis != "eta_dot":  # dt wind m / dx, the map factor 1 to 1e-6 on this grid
+                    along = out[0 if axis == "u" else 1].double() / (-0.1 * wind)
+                    assert float((along - 1.0).abs().max()) < tol + 1e-5
+            else:
+                assert not torch.isfinite(out).all()
