@@ -1060,27 +1060,29 @@ __device__ void small_solve_state(GState* gs) {
   __shared__ double y[GM_MAXR];
   __shared__ double rd[GM_MAXR];  // reciprocal diagonal of a triangular solve
   if (gs->method == 0) {
-    // _lstsq(H.T, beta): normal equations (H H^T) y = H beta, Cholesky solve.  Row p of H ends at column p + 1, and
-    // the lower triangle is enough.
+    // _lstsq(H.T, beta): normal equations (H H^T) y = H beta, Cholesky solve, over the cycle's kd steps.  A row past them
+    // is an identity row (begin_cycle): as an unknown it would meet the last step's subdiagonal equation for nothing
+    // and leave the square Hessenberg system in the least-squares problem's place.  Row p of H ends at column p + 1,
+    // and the lower triangle is enough.
     const int P = R | 1;
     double* ht = a2 + (size_t)R * R;  // [SS_C][P]: columns c0 .. of H, transposed
-    for (int q = tid; q < R * R; q += blockDim.x) a2[q] = 0.0;
-    for (int p = tid; p < R; p += blockDim.x) b2[p] = 0.0;
-    for (int c0 = 0; c0 <= R; c0 += SS_C) {
-      const int nc = min(SS_C, R + 1 - c0);
+    for (int q = tid; q < kd * R; q += blockDim.x) a2[q] = 0.0;
+    for (int p = tid; p < kd; p += blockDim.x) b2[p] = 0.0;
+    for (int c0 = 0; c0 <= kd; c0 += SS_C) {
+      const int nc = min(SS_C, kd + 1 - c0);
       __syncthreads();
-      for (int q = tid; q < R * SS_C; q += blockDim.x) {
+      for (int q = tid; q < kd * SS_C; q += blockDim.x) {
         const int r = q / SS_C, c = q % SS_C;
         if (c < nc) ht[c * P + r] = gs->H[r][c0 + c];
       }
       __syncthreads();
-      for (int p = max(c0 - 1, 0) + wp; p < R; p += nw)
+      for (int p = max(c0 - 1, 0) + wp; p < kd; p += nw)
         for (int r = max(c0 - 1, 0) + lane; r <= p; r += 32) {
           double v = a2[p * R + r];
           for (int c = 0; c < min(nc, r + 2 - c0); ++c) v += ht[c * P + p] * ht[c * P + r];
           a2[p * R + r] = v;
         }
-      for (int p = tid; p < R; p += blockDim.x) {
+      for (int p = tid; p < kd; p += blockDim.x) {
         double v = b2[p];
         for (int c = 0; c < min(nc, p + 2 - c0); ++c) v += ht[c * P + p] * gs->beta[c0 + c];
         b2[p] = v;
@@ -1090,38 +1092,38 @@ __device__ void small_solve_state(GState* gs) {
     // right-looking Cholesky, lower factor stored in a2; with several columns per block the right-hand side rides
     // along as one more row, which leaves L^-1 b2 in y
     const bool carry = gs->columns > 1;
-    for (int k = 0; k < R; ++k) {
+    for (int k = 0; k < kd; ++k) {
       const double dkk = sqrt(a2[k * R + k]);
       __syncthreads();  // every thread has the pivot
-      for (int i = k + 1 + tid; i < R; i += blockDim.x) a2[i * R + k] /= dkk;
+      for (int i = k + 1 + tid; i < kd; i += blockDim.x) a2[i * R + k] /= dkk;
       if (tid == 0) {
         a2[k * R + k] = dkk;
         rd[k] = 1.0 / dkk;
         if (carry) y[k] = b2[k] / dkk;
       }
       __syncthreads();
-      for (int i = k + 1 + wp; i < R; i += nw) {
+      for (int i = k + 1 + wp; i < kd; i += nw) {
         const double lik = a2[i * R + k];
         for (int jj = k + 1 + lane; jj <= i; jj += 32) a2[i * R + jj] -= lik * a2[jj * R + k];
       }
       if (carry)
-        for (int i = k + 1 + tid; i < R; i += blockDim.x) b2[i] -= a2[i * R + k] * y[k];
+        for (int i = k + 1 + tid; i < kd; i += blockDim.x) b2[i] -= a2[i * R + k] * y[k];
       __syncthreads();
     }
     if (carry) {
-      if (wp == 0) triangle_back(a2, R, R, rd, y);  // L^T y = z
+      if (wp == 0) triangle_back(a2, R, kd, rd, y);  // L^T y = z
     } else if (tid == 0) {
-      for (int i = 0; i < R; ++i) {  // L z = b2
+      for (int i = 0; i < kd; ++i) {  // L z = b2
         double s = b2[i];
         for (int k = 0; k < i; ++k) s -= a2[i * R + k] * y[k];
         y[i] = s / a2[i * R + i];
       }
-      for (int i = R - 1; i >= 0; --i) {  // L^T y = z
+      for (int i = kd - 1; i >= 0; --i) {  // L^T y = z
         double s = y[i];
-        for (int k = i + 1; k < R; ++k) s -= a2[k * R + i] * y[k];
+        for (int k = i + 1; k < kd; ++k) s -= a2[k * R + i] * y[k];
         y[i] = s / a2[i * R + i];
       }
-      for (int i = 0; i < R; ++i) gs->coef[i] = y[i] * gs->s[i];
+      for (int i = 0; i < R; ++i) gs->coef[i] = (i < kd) ? y[i] * gs->s[i] : 0.0;
     }
   } else {
     // back substitution with the rotated rows: sum_j R[j][i] y_j = beta_i
