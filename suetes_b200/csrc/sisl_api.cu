@@ -439,17 +439,63 @@ int block_columns(const SislCore* c, bool taped) {
   return radius >= 3.0 ? GM_S : 1;
 }
 
+// A conditional WHILE node at the tail of st's capture: gate(handle,
+// after_pass, stream) launches the kernel that sets its condition, before it
+// and after every pass; body(stream) records one pass, captured on side.
+template <typename Gate, typename Body>
+int capture_while(cudaStream_t st, cudaStream_t side, Gate&& gate, Body&& body) {
+  cudaStreamCaptureStatus cs;
+  cudaGraph_t gr;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t nd = 0;
+  if (cuda_failed(cudaStreamGetCaptureInfo(st, &cs, nullptr, &gr, &deps, &nd), "cudaStreamGetCaptureInfo") ||
+      cs != cudaStreamCaptureStatusActive)
+    return SISL_ERR_ARG;
+  cudaGraphConditionalHandle h;
+  if (cuda_failed(cudaGraphConditionalHandleCreate(&h, gr, 0, cudaGraphCondAssignDefault),
+                  "cudaGraphConditionalHandleCreate"))
+    return SISL_ERR_CUDA;
+  gate(h, 0, st);
+  if (cuda_failed(cudaStreamGetCaptureInfo(st, &cs, nullptr, &gr, &deps, &nd), "cudaStreamGetCaptureInfo"))
+    return SISL_ERR_CUDA;
+  cudaGraphNodeParams np{};
+  np.type = cudaGraphNodeTypeConditional;
+  np.conditional.handle = h;
+  np.conditional.type = cudaGraphCondTypeWhile;
+  np.conditional.size = 1;
+  cudaGraphNode_t node;
+  if (cuda_failed(cudaGraphAddNode(&node, gr, deps, nd, &np), "cudaGraphAddNode(conditional)")) return SISL_ERR_CUDA;
+  if (cuda_failed(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies),
+                  "cudaStreamUpdateCaptureDependencies"))
+    return SISL_ERR_CUDA;
+  if (cuda_failed(cudaStreamBeginCaptureToGraph(side, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                                cudaStreamCaptureModeRelaxed),
+                  "cudaStreamBeginCaptureToGraph"))
+    return SISL_ERR_CUDA;
+  body(side);
+  gate(h, 1, side);
+  cudaGraph_t body_out = nullptr;
+  if (cuda_failed(cudaStreamEndCapture(side, &body_out), "cudaStreamEndCapture(body)")) return SISL_ERR_CUDA;
+  return SISL_OK;
+}
+
 // Restarted GMRES on the packed vectors g.bg (rhs) and g.xg (initial guess).
 // transpose = 1 runs the same iteration on A^T with the preconditioner M^T
 // (the bwd_solve of steppers.py:473-481).
 //
+// A block that loses columns to rounding would end its cycle early, short of
+// the restart's steps.  Such a cycle is dropped (x is as before it, it counts
+// for nothing) and the solve goes on one column at a time: a cycle that
+// counts has taken all its steps, converged or broken down, as the reference's.
+//
 // Host mode (dev_info == nullptr): one device-to-host read of the residual
 // summary per restart cycle decides whether another cycle runs.
-// Graph mode (dev_info != nullptr, st capturing): the restart loop becomes a
-// CUDA-graph conditional WHILE node whose body is one restart cycle; a gate
-// kernel after every residual sets the condition (rnorm > atol and cycles <
-// maxiter) on the device, and the final statistics land in *dev_info.  No
-// host synchronisation: the whole solve replays inside one graph launch.
+// Graph mode (dev_info != nullptr, st capturing): the restart loop becomes
+// two CUDA-graph conditional WHILE nodes, cycles in blocks and then cycles of
+// single columns, whose body is one restart cycle; a gate kernel after every
+// residual sets the condition (rnorm > atol and cycles < maxiter) on the
+// device, and the final statistics land in *dev_info.  No host
+// synchronisation: the whole solve replays inside one graph launch.
 template <typename T>
 int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, SislSolveInfo* info,
               int transpose = 0, GDevInfo* dev_info = nullptr, bool taped = false) {
@@ -546,10 +592,10 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
       gm_dots<T>(g.V(0), n, 0, g.V(0), n, g.partial, gs, 3 /*RNORM*/, 0, s);
     }
   };
-  // one restart cycle: R Arnoldi steps in blocks, the small least-squares solve, x update
-  int cols[GM_MAXR];
-  const int nblocks = gm_block_plan(R, S, method, cols);
-  auto cycle = [&](cudaStream_t s) {
+  // one restart cycle: R Arnoldi steps in blocks of at most S columns, the small least-squares solve, x update
+  auto cycle = [&](cudaStream_t s, int S) {
+    int cols[GM_MAXR];
+    const int nblocks = gm_block_plan(R, S, method, cols);
     {
       KScope k(c, SISL_K_OTHER, s);
       gm_begin_cycle(gs, s);
@@ -605,46 +651,19 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
   if (dev_info) {  // ---- graph mode ----
     if (!c->cap_side) return SISL_ERR_ARG;
     residual(st);
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t gr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t nd = 0;
-    if (cuda_failed(cudaStreamGetCaptureInfo(st, &cs, nullptr, &gr, &deps, &nd), "cudaStreamGetCaptureInfo") ||
-        cs != cudaStreamCaptureStatusActive)
-      return SISL_ERR_ARG;
-    cudaGraphConditionalHandle h;
-    if (cuda_failed(cudaGraphConditionalHandleCreate(&h, gr, 0, cudaGraphCondAssignDefault),
-                    "cudaGraphConditionalHandleCreate"))
-      return SISL_ERR_CUDA;
-    {
-      KScope k(c, SISL_K_OTHER, st);
-      gm_gate(gs, h, maxiter, 0, st);
+    for (int form = S > 1 ? 1 : 0; form >= 0; --form) {
+      const int rc = capture_while(
+          st, c->cap_side,
+          [&](cudaGraphConditionalHandle h, int after, cudaStream_t s) {
+            KScope k(c, SISL_K_OTHER, s);
+            gm_gate(gs, h, maxiter, after, form, s);
+          },
+          [&](cudaStream_t s) {
+            cycle(s, form ? S : 1);
+            residual(s);
+          });
+      if (rc) return rc;
     }
-    if (cuda_failed(cudaStreamGetCaptureInfo(st, &cs, nullptr, &gr, &deps, &nd), "cudaStreamGetCaptureInfo"))
-      return SISL_ERR_CUDA;
-    cudaGraphNodeParams np{};
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = h;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    cudaGraphNode_t node;
-    if (cuda_failed(cudaGraphAddNode(&node, gr, deps, nd, &np), "cudaGraphAddNode(conditional)")) return SISL_ERR_CUDA;
-    cudaGraph_t body = np.conditional.phGraph_out[0];
-    if (cuda_failed(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies),
-                    "cudaStreamUpdateCaptureDependencies"))
-      return SISL_ERR_CUDA;
-    cudaStream_t sb = c->cap_side;
-    if (cuda_failed(cudaStreamBeginCaptureToGraph(sb, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed),
-                    "cudaStreamBeginCaptureToGraph"))
-      return SISL_ERR_CUDA;
-    cycle(sb);
-    residual(sb);
-    {
-      KScope k(c, SISL_K_OTHER, sb);
-      gm_gate(gs, h, maxiter, 1, sb);
-    }
-    cudaGraph_t body_out = nullptr;
-    if (cuda_failed(cudaStreamEndCapture(sb, &body_out), "cudaStreamEndCapture(body)")) return SISL_ERR_CUDA;
     {
       KScope k(c, SISL_K_OTHER, st);
       gm_info(gs, dev_info, st);
@@ -668,12 +687,16 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
   residual(st);
   int rc = read();
   if (rc) return rc;
-  int cycles = 0, steps = 0;
+  int cycles = 0, steps = 0, form = S;
   while (cycles < maxiter && hv->rnorm > hv->atol) {
-    cycle(st);
+    cycle(st, form);
     residual(st);
     rc = read();
     if (rc) return rc;
+    if (hv->narrow) {
+      form = 1;
+      continue;
+    }
     steps += hv->kdone;
     cycles++;
   }
@@ -2486,8 +2509,9 @@ int capture_members(int n, SislCore* const* cores, F&& record, SislStepGraph** o
 }
 
 // One solve of every member as grouped launches, captured on st: the
-// restart loop is one conditional WHILE node (body captured on side) that
-// runs while any member continues; each member's own loop state (cycles,
+// restart loop is the two conditional WHILE nodes of gmres_run (bodies
+// captured on side), each running while any member continues in its form, a
+// member whose block lost columns waiting for the second; each member's own loop state (cycles,
 // convergence) lives in its GState and `running` flag.  The sequence of
 // phases per member is gmres_run's (transpose: the A^T / M^T iteration of
 // the custom_linear_solve transpose), so each member's result is the same
@@ -2496,8 +2520,6 @@ int capture_members(int n, SislCore* const* cores, F&& record, SislStepGraph** o
 template <typename T>
 int gmres_group_run(const GroupLaunch<T>& gl, cudaStream_t st, cudaStream_t side, int slot, int transpose) {
   const int R = gl.R;
-  int cols[GM_MAXR];
-  const int nblocks = gm_block_plan(R, gl.S, gl.method, cols);
   grp_setup<T>(gl, transpose, st);
   if (gl.refine) grp_convert<T>(gl, 0, st);
   grp_dots<T>(gl, 0, GV_B, 1 /*BNORM*/, 0, st);
@@ -2531,7 +2553,9 @@ int gmres_group_run(const GroupLaunch<T>& gl, cudaStream_t st, cudaStream_t side
     }
     grp_dots<T>(gl, 0, GV_V0, 3 /*RNORM*/, 0, s);
   };
-  auto cycle = [&](cudaStream_t s) {
+  auto cycle = [&](cudaStream_t s, int S) {
+    int cols[GM_MAXR];
+    const int nblocks = gm_block_plan(R, S, gl.method, cols);
     grp_begin_cycle<T>(gl, s);
     for (int b = 0, j0 = 0; b < nblocks; j0 += cols[b++]) {
       for (int j = j0; j < j0 + cols[b]; ++j) {
@@ -2543,7 +2567,7 @@ int gmres_group_run(const GroupLaunch<T>& gl, cudaStream_t st, cudaStream_t side
           grp_precond<T>(gl, 0, j + 1, 1, s);
         }
       }
-      if (gl.S == 1) {
+      if (S == 1) {
         grp_dots<T>(gl, j0 + 1, GV_V0 + j0 + 1, 0 /*PROJ*/, 1, s);
         grp_update_arnoldi<T>(gl, j0 + 1, s);
       } else {
@@ -2555,39 +2579,16 @@ int gmres_group_run(const GroupLaunch<T>& gl, cudaStream_t st, cudaStream_t side
     grp_update_x<T>(gl, s);
   };
   residual(st);
-  cudaStreamCaptureStatus cs;
-  cudaGraph_t gr;
-  const cudaGraphNode_t* deps = nullptr;
-  size_t nd = 0;
-  if (cuda_failed(cudaStreamGetCaptureInfo(st, &cs, nullptr, &gr, &deps, &nd), "cudaStreamGetCaptureInfo") ||
-      cs != cudaStreamCaptureStatusActive)
-    return SISL_ERR_ARG;
-  cudaGraphConditionalHandle h;
-  if (cuda_failed(cudaGraphConditionalHandleCreate(&h, gr, 0, cudaGraphCondAssignDefault),
-                  "cudaGraphConditionalHandleCreate"))
-    return SISL_ERR_CUDA;
-  grp_gate<T>(gl, h, 0, st);
-  if (cuda_failed(cudaStreamGetCaptureInfo(st, &cs, nullptr, &gr, &deps, &nd), "cudaStreamGetCaptureInfo"))
-    return SISL_ERR_CUDA;
-  cudaGraphNodeParams np{};
-  np.type = cudaGraphNodeTypeConditional;
-  np.conditional.handle = h;
-  np.conditional.type = cudaGraphCondTypeWhile;
-  np.conditional.size = 1;
-  cudaGraphNode_t node;
-  if (cuda_failed(cudaGraphAddNode(&node, gr, deps, nd, &np), "cudaGraphAddNode(conditional)")) return SISL_ERR_CUDA;
-  cudaGraph_t body = np.conditional.phGraph_out[0];
-  if (cuda_failed(cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies),
-                  "cudaStreamUpdateCaptureDependencies"))
-    return SISL_ERR_CUDA;
-  if (cuda_failed(cudaStreamBeginCaptureToGraph(side, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed),
-                  "cudaStreamBeginCaptureToGraph"))
-    return SISL_ERR_CUDA;
-  cycle(side);
-  residual(side);
-  grp_gate<T>(gl, h, 1, side);
-  cudaGraph_t body_out = nullptr;
-  if (cuda_failed(cudaStreamEndCapture(side, &body_out), "cudaStreamEndCapture(body)")) return SISL_ERR_CUDA;
+  for (int form = gl.S > 1 ? 1 : 0; form >= 0; --form) {
+    const int rc = capture_while(
+        st, side,
+        [&](cudaGraphConditionalHandle h, int after, cudaStream_t s) { grp_gate<T>(gl, h, after, form, s); },
+        [&](cudaStream_t s) {
+          cycle(s, form ? gl.S : 1);
+          residual(s);
+        });
+    if (rc) return rc;
+  }
   grp_info<T>(gl, slot, st);
   if (gl.refine) grp_convert<T>(gl, 2, st);
   g_launches += 1;

@@ -185,7 +185,7 @@ void gm_setup(GState* gs, double eps, double tol, double atol_in, int restart, i
               cudaStream_t st);
 void gm_init_tol(GState* gs, cudaStream_t st);
 struct GDevInfo;
-void gm_gate(GState* gs, cudaGraphConditionalHandle h, int maxiter, int after_cycle, cudaStream_t st);
+void gm_gate(GState* gs, cudaGraphConditionalHandle h, int maxiter, int after_cycle, int block, cudaStream_t st);
 void gm_info(const GState* gs, GDevInfo* o, cudaStream_t st);
 void gm_begin_cycle(GState* gs, cudaStream_t st);
 void gm_small_solve(GState* gs, int restart, cudaStream_t st);

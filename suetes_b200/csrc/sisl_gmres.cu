@@ -19,9 +19,12 @@
 // Berkeley 2010).  block_dots forms all products of the basis with Z and of Z
 // with itself in one pass over memory, block_update the new vectors in a
 // second one, and the Hessenberg columns follow from the small matrices
-// (block_finish), so a cycle spans the same Krylov space and minimises over
-// it as the one-step form does.  256x256x80 float32, restart 30: vector passes
-// per cycle 1020 -> 220.
+// (block_finish).  A cycle whose blocks keep all their columns spans the same
+// Krylov space and minimises over it as the one-step form does; a cycle in
+// which a column is lost to rounding is narrow: it is dropped and done over
+// one column at a time, and so are the solve's later ones (gmres_run in
+// sisl_api.cu).  256x256x80 float32, restart 30: vector passes per cycle 1020
+// -> 220.
 //
 // One column per block is the classical form: the dots and update kernels with
 // their one-step bookkeeping.  It stays for the cores and calls whose rule
@@ -615,7 +618,10 @@ __device__ __forceinline__ void block_finish(GState* gs, const double (&gram)[GM
       gs->err = fabs(gs->beta[j + 1]);
       if (!(gs->err > gs->ptol)) active = 0;
     }
-    if (keep < s) active = 0;  // a shortened block ends its cycle
+    if (keep < s && active) {  // columns lost to rounding, and the cycle not over: see small_solve_state
+      gs->narrow = 1;
+      active = 0;
+    }
     gs->kdone = j0 + done;
     gs->active = active;
     done_s = done;
@@ -952,6 +958,7 @@ __device__ void setup_state(GState* gs, double eps, double tol, double atol_in, 
   gs->active = 1;
   gs->kdone = 0;
   gs->breakdown = 0;
+  gs->narrow = 0;
   gs->cycles = 0;
   gs->steps = 0;
   for (int q = 0; q < GM_MAXR + 2; ++q) gs->s[q] = 0.0;
@@ -962,16 +969,23 @@ __global__ void setup_kernel(GState* gs, double eps, double tol, double atol_in,
   setup_state(gs, eps, tol, atol_in, restart, method, columns);
 }
 
+// The restart loop runs in the block form (block = 1) until a cycle is narrow
+// or it ends, then one column at a time (block = 0).  A narrow cycle is not
+// counted.
+__device__ __forceinline__ void count_cycle(GState* gs) {
+  if (gs->narrow) return;
+  gs->cycles += 1;
+  gs->steps += gs->kdone;
+}
+__device__ __forceinline__ bool another_cycle(const GState* gs, int maxiter, int block) {
+  return gs->rnorm > gs->atol && gs->cycles < maxiter && (gs->columns > 1) == (block != 0);
+}
 // Graph mode: after a residual, count the finished cycle and set the WHILE
-// condition: another cycle while ||M r|| > atol and cycles < maxiter.
-__global__ void gate_kernel(GState* gs, cudaGraphConditionalHandle h, int maxiter, int after_cycle) {
+// condition: another cycle of this form while ||M r|| > atol and cycles < maxiter.
+__global__ void gate_kernel(GState* gs, cudaGraphConditionalHandle h, int maxiter, int after_cycle, int block) {
   grid_chain();
-  if (after_cycle) {
-    gs->cycles += 1;
-    gs->steps += gs->kdone;
-  }
-  const bool more = (gs->rnorm > gs->atol) && (gs->cycles < maxiter);
-  cudaGraphSetConditional(h, more ? 1u : 0u);
+  if (after_cycle) count_cycle(gs);
+  cudaGraphSetConditional(h, another_cycle(gs, maxiter, block) ? 1u : 0u);
 }
 
 __device__ void info_state(const GState* gs, GDevInfo* o) {
@@ -1007,6 +1021,7 @@ __device__ void begin_cycle_state(GState* gs) {
     gs->active = 1;
     gs->kdone = 0;
     gs->breakdown = 0;
+    gs->narrow = 0;
   }
 }
 __global__ void begin_cycle_kernel(GState* gs) {
@@ -1059,6 +1074,14 @@ __device__ void small_solve_state(GState* gs) {
   __shared__ double b2[GM_MAXR];
   __shared__ double y[GM_MAXR];
   __shared__ double rd[GM_MAXR];  // reciprocal diagonal of a triangular solve
+  if (gs->narrow) {  // nothing of the cycle is used: x stays, and it is done over one column at a time
+    __syncthreads();
+    if (tid == 0) {
+      gs->kdone = 0;
+      gs->columns = 1;
+    }
+    return;
+  }
   if (gs->method == 0) {
     // _lstsq(H.T, beta): normal equations (H H^T) y = H beta, Cholesky solve, over the cycle's kd steps.  A row past them
     // is an identity row (begin_cycle): as an unknown it would meet the last step's subdiagonal equation for nothing
@@ -1169,6 +1192,7 @@ __global__ void snapshot_kernel(const GState* gs, GHostView* v) {
   v->atol = gs->atol;
   v->bnorm = gs->bnorm;
   v->kdone = gs->kdone;
+  v->narrow = gs->narrow;
 }
 
 // ---------------------------------------------------------------------------
@@ -1317,19 +1341,16 @@ __global__ void __launch_bounds__(1024) group_small_solve_kernel(GroupMember<T>*
   if (g.running) small_solve_state(g.gs);
 }
 // one block: count the finished cycle of every running member, decide which
-// members continue, set the WHILE condition while any does
+// members continue in this form, set the WHILE condition while any does
 template <typename T>
-__global__ void group_gate_kernel(GroupMember<T>* mem, int M, cudaGraphConditionalHandle h, int after_cycle) {
+__global__ void group_gate_kernel(GroupMember<T>* mem, int M, cudaGraphConditionalHandle h, int after_cycle,
+                                  int block) {
   grid_chain();
   int any = 0;
   for (int m = threadIdx.x; m < M; m += blockDim.x) {
     GroupMember<T>& g = mem[m];
-    GState* gs = g.gs;
-    if (after_cycle && g.running) {
-      gs->cycles += 1;
-      gs->steps += gs->kdone;
-    }
-    const int more = g.running && (gs->rnorm > gs->atol) && (gs->cycles < g.maxiter);
+    if (after_cycle && g.running) count_cycle(g.gs);
+    const int more = (g.running || !after_cycle) && another_cycle(g.gs, g.maxiter, block);
     g.running = more;
     any |= more;
   }
@@ -1469,8 +1490,8 @@ void gm_setup(GState* gs, double eps, double tol, double atol_in, int restart, i
   launch_chained(setup_kernel, 1, 1, 0, st, gs, eps, tol, atol_in, restart, method, columns);
 }
 void gm_init_tol(GState* gs, cudaStream_t st) { launch_chained(init_tol_kernel, 1, 1, 0, st, gs); }
-void gm_gate(GState* gs, cudaGraphConditionalHandle h, int maxiter, int after_cycle, cudaStream_t st) {
-  launch_chained(gate_kernel, 1, 1, 0, st, gs, h, maxiter, after_cycle);
+void gm_gate(GState* gs, cudaGraphConditionalHandle h, int maxiter, int after_cycle, int block, cudaStream_t st) {
+  launch_chained(gate_kernel, 1, 1, 0, st, gs, h, maxiter, after_cycle, block);
 }
 void gm_info(const GState* gs, GDevInfo* o, cudaStream_t st) { launch_chained(info_kernel, 1, 1, 0, st, gs, o); }
 void gm_begin_cycle(GState* gs, cudaStream_t st) { launch_chained(begin_cycle_kernel, 1, 256, 0, st, gs); }
@@ -1563,8 +1584,8 @@ void grp_small_solve(const GroupLaunch<T>& g, cudaStream_t st) {
   launch_chained(group_small_solve_kernel<T>, g.M, small_solve_threads(g.R), small_solve_smem(g.R), st, g.mem);
 }
 template <typename T>
-void grp_gate(const GroupLaunch<T>& g, cudaGraphConditionalHandle h, int after_cycle, cudaStream_t st) {
-  launch_chained(group_gate_kernel<T>, 1, 256, 0, st, g.mem, g.M, h, after_cycle);
+void grp_gate(const GroupLaunch<T>& g, cudaGraphConditionalHandle h, int after_cycle, int block, cudaStream_t st) {
+  launch_chained(group_gate_kernel<T>, 1, 256, 0, st, g.mem, g.M, h, after_cycle, block);
 }
 template <typename T>
 void grp_info(const GroupLaunch<T>& g, int solve, cudaStream_t st) {
@@ -1587,7 +1608,7 @@ void grp_info(const GroupLaunch<T>& g, int solve, cudaStream_t st) {
   template void grp_init_tol<T>(const GroupLaunch<T>&, cudaStream_t);                                \
   template void grp_begin_cycle<T>(const GroupLaunch<T>&, cudaStream_t);                             \
   template void grp_small_solve<T>(const GroupLaunch<T>&, cudaStream_t);                             \
-  template void grp_gate<T>(const GroupLaunch<T>&, cudaGraphConditionalHandle, int, cudaStream_t);   \
+  template void grp_gate<T>(const GroupLaunch<T>&, cudaGraphConditionalHandle, int, int, cudaStream_t); \
   template void grp_info<T>(const GroupLaunch<T>&, int, cudaStream_t);
 SISL_GROUP_INST(float)
 SISL_GROUP_INST(double)

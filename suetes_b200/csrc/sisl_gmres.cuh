@@ -43,6 +43,7 @@ struct GState {
   int method;                       // 0 batched, 1 incremental
   int columns;                      // columns per block at most; 1: the classical form
   int breakdown;
+  int narrow;                       // a block of this cycle lost columns: the cycle is done over, one column at a time
   unsigned int counter;             // last-block-done ticket
   unsigned int group_counter[GM_BLOCKS / GM_GROUP + 1];
   int cycles, steps;                // restart cycles and Arnoldi steps taken (graph mode)
@@ -92,7 +93,7 @@ struct GDevInfo {
 struct GHostView {
   double rnorm, atol, bnorm;
   int kdone;
-  int pad;
+  int narrow;
 };
 
 }  // namespace sisl

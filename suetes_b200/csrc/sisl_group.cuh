@@ -126,7 +126,7 @@ void grp_small_solve(const GroupLaunch<T>& g, cudaStream_t st);
 // another cycle for member m while rnorm > atol and cycles < maxiter; the
 // WHILE condition is set while any member continues
 template <typename T>
-void grp_gate(const GroupLaunch<T>& g, cudaGraphConditionalHandle h, int after_cycle, cudaStream_t st);
+void grp_gate(const GroupLaunch<T>& g, cudaGraphConditionalHandle h, int after_cycle, int block, cudaStream_t st);
 template <typename T>
 void grp_info(const GroupLaunch<T>& g, int solve, cudaStream_t st);
 // matvec: mode 0 Arnoldi step j: V_j scaled by s_j -> V_{j+1} (u, v) | z;
