@@ -294,9 +294,9 @@ __global__ void __launch_bounds__(256) at_main_kernel(Dims d, Coef<T> c, CVec5<T
 // rounded products that the compiler may not fuse into a following add, so
 // that the column variants of M^T round identically
 
-template <typename T, int TPT, int TPC>
+template <typename T, int TPT, int TPC, bool SH>
 __global__ void __launch_bounds__(TPT) pt_column_kernel(Dims d, Coef<T> c, CVec5<T> y, Vec5<T> out,
-                                                        const int* active) {
+                                                        const int* active, Shift<T> sh) {
   grid_chain();
   if (active && *active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -317,6 +317,7 @@ __global__ void __launch_bounds__(TPT) pt_column_kernel(Dims d, Coef<T> c, CVec5
   T* __restrict__ ow = out.f[2];
   T* __restrict__ op = out.f[3];
   T* __restrict__ oW = out.f[4];
+  const ShiftBy<T, SH> by(sh);
   // G(K) = -adt cp thw (yw + yW) idzw / damp at interior w levels
   auto Gw = [&](int i, int K) -> T {
     const int kc = min(max(K, 1), nz - 1);
@@ -358,15 +359,18 @@ __global__ void __launch_bounds__(TPT) pt_column_kernel(Dims d, Coef<T> c, CVec5
     const int k = q / TPC, l = q % TPC, i = i0 + l;
     if (i >= nx) continue;
     const int p = i + nx * j + k * pm;
-    if (k < nz) op[p] = s_x[q] * ips;
+    const T xw = by.in(sh, 2, p), xW = by.in(sh, 4, p);
+    if (k < nz) op[p] = by.of(mul_rn(s_x[q], ips), by.in(sh, 3, p));
     if (k == 0 || k == nz) {
-      ow[p] = ld(yw, p);
-      oW[p] = ld(yW, p) * ld(c.dzw, p);
+      ow[p] = by.of(ld(yw, p), xw);
+      oW[p] = by.of(mul_rn(ld(yW, p), ld(c.dzw, p)), xW);
     } else {
       const T dvl = mul_rn(-ld(c.lpi, p - pm), s_x[q - TPC]), dv = mul_rn(-ld(c.lpi, p), s_x[q]);
       const T ep = ld(yW, p) + ld(c.rtw, p) * (dvl - dv);
-      oW[p] = ep * inva;
-      ow[p] = (ld(yw, p) + ep) * ld(c.idamp, p);
+      const T eta = mul_rn(ep, inva);
+      if (SH) sh.keep[p - pm] = eta;
+      oW[p] = by.of(eta, xW);
+      ow[p] = by.of(mul_rn(ld(yw, p) + ep, ld(c.idamp, p)), xw);
     }
   }
 }
@@ -375,8 +379,9 @@ __global__ void __launch_bounds__(TPT) pt_column_kernel(Dims d, Coef<T> c, CVec5
 // items' loads before it computes any of them (the forward tile's
 // batching).  Arithmetic is term for term that of pt_column_kernel, so the
 // results are bitwise those of every other column variant.
-template <typename T, int TPT, int TPC, int PU>
-__device__ __forceinline__ void pt_column_batched_block(const Dims& d, const Coef<T>& c, const CVec5<T>& y, const Vec5<T>& out, int bx, int by, int bz) {
+template <typename T, int TPT, int TPC, int PU, bool SH>
+__device__ __forceinline__ void pt_column_batched_block(const Dims& d, const Coef<T>& c, const CVec5<T>& y, const Vec5<T>& out,
+                                               const Shift<T>& sh, int bx, int by_, int bz) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
   const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -385,7 +390,7 @@ __device__ __forceinline__ void pt_column_batched_block(const Dims& d, const Coe
   T* s_lo = s_cp + nz * TPC;  // [nz][TPC]  lower
   T* s_iv = s_lo + nz * TPC;  // [nz][TPC]  1 / pivot
   const int i0 = bx * TPC;
-  const int j = by;
+  const int j = by_;
   const int tid = threadIdx.x;
   const int pm = nx * ny;
   const int nm = nz * TPC, nw = (nz + 1) * TPC;
@@ -396,6 +401,7 @@ __device__ __forceinline__ void pt_column_batched_block(const Dims& d, const Coe
   T* __restrict__ ow = out.f[2];
   T* __restrict__ op = out.f[3];
   T* __restrict__ oW = out.f[4];
+  const ShiftBy<T, SH> by(sh);
   (void)ny;
   // ---- A: pibar and the factorisation ----
   for (int q0 = tid; q0 < nm; q0 += PU * TPT) {
@@ -458,7 +464,7 @@ __device__ __forceinline__ void pt_column_batched_block(const Dims& d, const Coe
   __syncthreads();
   // ---- C: pi, w and eta_dot cotangents ----
   for (int q0 = tid; q0 < nw; q0 += PU * TPT) {
-    T c_w[PU], c_W[PU], c_a[PU], c_b[PU], c_r[PU], c_d[PU];
+    T c_w[PU], c_W[PU], c_a[PU], c_b[PU], c_r[PU], c_d[PU], xw[PU], xW[PU], xp[PU];
 #pragma unroll
     for (int u = 0; u < PU; ++u) {
       const int q = q0 + u * TPT;
@@ -467,6 +473,9 @@ __device__ __forceinline__ void pt_column_batched_block(const Dims& d, const Coe
         const int p = i + nx * j + k * pm;
         c_w[u] = ld(yw, p);
         c_W[u] = ld(yW, p);
+        xw[u] = by.in(sh, 2, p);
+        xW[u] = by.in(sh, 4, p);
+        xp[u] = by.in(sh, 3, min(p, nz * pm - 1));
         if (k == 0 || k == nz) {
           c_d[u] = ld(c.dzw, p);
         } else {
@@ -483,40 +492,45 @@ __device__ __forceinline__ void pt_column_batched_block(const Dims& d, const Coe
       const int k = q / TPC, i = i0 + q % TPC;
       if (q < nw && i < nx) {
         const int p = i + nx * j + k * pm;
-        if (k < nz) op[p] = s_x[q] * ips;
+        if (k < nz) op[p] = by.of(mul_rn(s_x[q], ips), xp[u]);
         if (k == 0 || k == nz) {
-          ow[p] = c_w[u];
-          oW[p] = c_W[u] * c_d[u];
+          ow[p] = by.of(c_w[u], xw[u]);
+          oW[p] = by.of(mul_rn(c_W[u], c_d[u]), xW[u]);
         } else {
           const T dvl = mul_rn(-c_a[u], s_x[q - TPC]), dv = mul_rn(-c_b[u], s_x[q]);
           const T ep = c_W[u] + c_r[u] * (dvl - dv);
-          oW[p] = ep * inva;
-          ow[p] = (c_w[u] + ep) * c_d[u];
+          const T eta = mul_rn(ep, inva);
+          if (SH) sh.keep[p - pm] = eta;
+          oW[p] = by.of(eta, xW[u]);
+          ow[p] = by.of(mul_rn(c_w[u] + ep, c_d[u]), xw[u]);
         }
       }
     }
   }
 }
-template <typename T, int TPT, int TPC, int PU>
+template <typename T, int TPT, int TPC, int PU, bool SH>
 __global__ void __launch_bounds__(TPT) pt_column_batched_kernel(Dims d, Coef<T> c, CVec5<T> y, Vec5<T> out,
-                                                                const int* active) {
+                                                                const int* active, Shift<T> sh) {
   grid_chain();
   if (active && *active == 0) return;
-  pt_column_batched_block<T, TPT, TPC, PU>(d, c, y, out, blockIdx.x, blockIdx.y, blockIdx.z);
+  pt_column_batched_block<T, TPT, TPC, PU, SH>(d, c, y, out, sh, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // ---------------------------------------------------------------------------
 // M^T, horizontal part: out_u = y_u + sum of the kinematic cotangent
 // kinbar = -alpha out_W over the interior w levels of the adjacent cells.
-template <typename T>
-__device__ __forceinline__ void pt_uv_block(const Dims& d, const Coef<T>& c, const CVec5<T>& y, const Vec5<T>& out, int bx, int by, int bz) {
+template <typename T, bool SH>
+__device__ __forceinline__ void pt_uv_block(const Dims& d, const Coef<T>& c, const CVec5<T>& y, const Vec5<T>& out,
+                                               const Shift<T>& sh, int bx, int by_, int bz) {
   const int i = bx * blockDim.x + threadIdx.x;
-  const int j = by * blockDim.y + threadIdx.y;
+  const int j = by_ * blockDim.y + threadIdx.y;
   const int k = bz * blockDim.z + threadIdx.z;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   if (i > nx || j > ny || k >= nz) return;
   const T qa = -(T)c.s.alpha * T(0.25);
-  const T* __restrict__ oW = out.f[4];
+  const ShiftBy<T, SH> by(sh);
+  const T* __restrict__ oW = SH ? sh.keep : out.f[4];  // interior level K at K - 1 when kept
+  const int down = SH ? nx * ny : 0;
   if (j < ny) {
     const int p = iu(d, i, j, k);
     T g = ld(y.f[0], p);
@@ -526,10 +540,10 @@ __device__ __forceinline__ void pt_uv_block(const Dims& d, const Coef<T>& c, con
       for (int K = k; K <= k + 1; ++K) {
         if (K <= 0 || K >= nz) continue;
         const int pw = iw(d, ii, j, K);
-        g += qa * m * ld(c.zxw, pw) * oW[pw];
+        g += qa * m * ld(c.zxw, pw) * oW[pw - down];
       }
     }
-    out.f[0][p] = g;
+    out.f[0][p] = by.of(g, by.in(sh, 0, p));
   }
   if (i < nx) {
     const int p = iv(d, i, j, k);
@@ -540,17 +554,18 @@ __device__ __forceinline__ void pt_uv_block(const Dims& d, const Coef<T>& c, con
       for (int K = k; K <= k + 1; ++K) {
         if (K <= 0 || K >= nz) continue;
         const int pw = iw(d, i, jj, K);
-        g += qa * m * ld(c.zew, pw) * oW[pw];
+        g += qa * m * ld(c.zew, pw) * oW[pw - down];
       }
     }
-    out.f[1][p] = g;
+    out.f[1][p] = by.of(g, by.in(sh, 1, p));
   }
 }
-template <typename T>
-__global__ void __launch_bounds__(256) pt_uv_kernel(Dims d, Coef<T> c, CVec5<T> y, Vec5<T> out, const int* active) {
+template <typename T, bool SH>
+__global__ void __launch_bounds__(256) pt_uv_kernel(Dims d, Coef<T> c, CVec5<T> y, Vec5<T> out, const int* active,
+                                                    Shift<T> sh) {
   grid_chain();
   if (active && *active == 0) return;
-  pt_uv_block<T>(d, c, y, out, blockIdx.x, blockIdx.y, blockIdx.z);
+  pt_uv_block<T, SH>(d, c, y, out, sh, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // ---------------------------------------------------------------------------
@@ -910,12 +925,13 @@ template void launch_tricubic_vjp<double>(int, int, int, int, int, int, const do
 // L^T z = w downward (z(k) = (w(k) - lower(k+1) z(k+1)) / pivot(k)), where
 // the w and eta_dot cotangents of the w level between z(k) and z(k+1) are
 // formed.  Shared memory per block: nz * NT values of T.
-template <typename T, int NT>
-__device__ __forceinline__ void pt_march_block(const Dims& d, const Coef<T>& c, const CVec5<T>& y, const Vec5<T>& out, int bx, int by, int bz) {
+template <typename T, int NT, bool SH>
+__device__ __forceinline__ void pt_march_block(const Dims& d, const Coef<T>& c, const CVec5<T>& y, const Vec5<T>& out,
+                                               const Shift<T>& sh, int bx, int by_, int bz) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* s_w = reinterpret_cast<T*>(smem_raw);  // [nz][NT]
   const int t = threadIdx.x;
-  const int i = bx * NT + t, j = by;
+  const int i = bx * NT + t, j = by_;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   if (i >= nx) return;
   const int pm = nx * ny, h = i + nx * j;
@@ -926,6 +942,7 @@ __device__ __forceinline__ void pt_march_block(const Dims& d, const Coef<T>& c, 
   T* __restrict__ ow = out.f[2];
   T* __restrict__ op = out.f[3];
   T* __restrict__ oW = out.f[4];
+  const ShiftBy<T, SH> by(sh);
   T G_lo = T(0), wprev = T(0), cprev = T(0);
 #pragma unroll 4
   for (int k = 0; k < nz; ++k) {
@@ -947,30 +964,32 @@ __device__ __forceinline__ void pt_march_block(const Dims& d, const Coef<T>& c, 
   for (int k = nz - 1; k >= 0; --k) {
     const int p = h + k * pm;
     const T z = (s_w[k * NT + t] - loh * zh) * ld(c.tinv, p);
-    op[p] = z * ips;
+    op[p] = by.of(mul_rn(z, ips), by.in(sh, 3, p));
     const T dv = mul_rn(-ld(c.lpi, p), z);
     if (k + 1 < nz) {
       const int pw = p + pm;
       const T ep = ld(yW, pw) + ld(c.rtw, pw) * (dv - dvh);
-      oW[pw] = ep * inva;
-      ow[pw] = (ld(yw, pw) + ep) * ld(c.idamp, pw);
+      const T eta = mul_rn(ep, inva);
+      if (SH) sh.keep[p] = eta;
+      oW[pw] = by.of(eta, by.in(sh, 4, pw));
+      ow[pw] = by.of(mul_rn(ld(yw, pw) + ep, ld(c.idamp, pw)), by.in(sh, 2, pw));
     }
     zh = z;
     loh = ld(c.tlo, p);
     dvh = dv;
   }
-  ow[h] = ld(yw, h);
-  oW[h] = ld(yW, h) * ld(c.dzw, h);
   const int ptop = h + nz * pm;
-  ow[ptop] = ld(yw, ptop);
-  oW[ptop] = ld(yW, ptop) * ld(c.dzw, ptop);
+  ow[h] = by.of(ld(yw, h), by.in(sh, 2, h));
+  oW[h] = by.of(mul_rn(ld(yW, h), ld(c.dzw, h)), by.in(sh, 4, h));
+  ow[ptop] = by.of(ld(yw, ptop), by.in(sh, 2, ptop));
+  oW[ptop] = by.of(mul_rn(ld(yW, ptop), ld(c.dzw, ptop)), by.in(sh, 4, ptop));
 }
-template <typename T, int NT>
+template <typename T, int NT, bool SH>
 __global__ void __launch_bounds__(NT) pt_march_kernel(Dims d, Coef<T> c, CVec5<T> y, Vec5<T> out,
-                                                      const int* active) {
+                                                      const int* active, Shift<T> sh) {
   grid_chain();
   if (active && *active == 0) return;
-  pt_march_block<T, NT>(d, c, y, out, blockIdx.x, blockIdx.y, blockIdx.z);
+  pt_march_block<T, NT, SH>(d, c, y, out, sh, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // ---------------------------------------------------------------------------
@@ -1036,7 +1055,7 @@ __global__ void __launch_bounds__(256) group_at_kernel(GroupMember<T>* mem, cons
 // stage 0: column tile (32 columns per block of 256, batched loads, the
 // autotuner's usual choice), stage 1: u and v faces.  mode 0: z -> V_tv
 // (gated when asked); mode 1: b -> V_1
-template <typename T>
+template <typename T, bool SH>
 __global__ void __launch_bounds__(256) group_pt_kernel(GroupMember<T>* mem, const int* __restrict__ first, int M,
                                                        int stage, int mode, int tv, int gated) {
   grid_chain();
@@ -1052,15 +1071,22 @@ __global__ void __launch_bounds__(256) group_pt_kernel(GroupMember<T>* mem, cons
     y.f[q] = src + g.off[q];
     out.f[q] = tgt + g.off[q];
   }
+  Shift<T> sh;
+  if (SH) {
+    const T* x = gvec_a(g, GV_V0 + tv - 1);
+    for (int q = 0; q < 5; ++q) sh.f[q] = x + g.off[q];
+    sh.s = &g.gs->s[tv - 1];
+    sh.keep = g.tmp;
+  }
   const int t = b - first[mi];
   if (stage == 0) {
     const int gx = (g.d.nx + 31) / 32;
     const int by = t / gx;
-    pt_column_batched_block<T, 256, 32, 4>(g.d, g.c, y, out, t - by * gx, by, 0);
+    pt_column_batched_block<T, 256, 32, 4, SH>(g.d, g.c, y, out, sh, t - by * gx, by, 0);
   } else {
     int bx, by, bz;
     group_box(t, g.d.nx + 1, g.d.ny + 1, bx, by, bz);
-    pt_uv_block<T>(g.d, g.c, y, out, bx, by, bz);
+    pt_uv_block<T, SH>(g.d, g.c, y, out, sh, bx, by, bz);
   }
 }
 
@@ -1091,76 +1117,89 @@ void grp_matvec_t(const GroupLaunch<T>& g, int mode, int j, cudaStream_t st) {
 }
 
 template <typename T>
-void grp_precond_t(const GroupLaunch<T>& g, int mode, int t, int gated, cudaStream_t st) {
+void grp_precond_t(const GroupLaunch<T>& g, int mode, int t, int gated, cudaStream_t st, int shift) {
   int nz_max = 1;
   for (int m = 0; m < g.M; ++m) nz_max = nz_max > g.nz_h[m] ? nz_max : g.nz_h[m];
   const size_t smem = (size_t)(4 * nz_max) * 32 * sizeof(T);
-  static SmemLimit attr_bytes;
-  ensure_smem_limit((const void*)group_pt_kernel<T>, attr_bytes, smem);
-  launch_chained(group_pt_kernel<T>, g.blocks(GT_PTM), 256, smem, st, g.mem, g.row(GT_PTM), g.M, 0, mode, t, gated);
-  launch_chained(group_pt_kernel<T>, g.blocks(GT_PTU), dim3(32, 4, 2), 0, st, g.mem, g.row(GT_PTU), g.M, 1, mode, t,
-                 gated);
+  auto run = [&](auto on) {
+    constexpr auto fn = group_pt_kernel<T, decltype(on)::value>;
+    static SmemLimit attr_bytes;
+    ensure_smem_limit((const void*)fn, attr_bytes, smem);
+    launch_chained(fn, g.blocks(GT_PTM), 256, smem, st, g.mem, g.row(GT_PTM), g.M, 0, mode, t, gated);
+    launch_chained(fn, g.blocks(GT_PTU), dim3(32, 4, 2), 0, st, g.mem, g.row(GT_PTU), g.M, 1, mode, t, gated);
+  };
+  if (shift) run(std::true_type{});
+  else run(std::false_type{});
 }
 
 template void grp_matvec_t<float>(const GroupLaunch<float>&, int, int, cudaStream_t);
 template void grp_matvec_t<double>(const GroupLaunch<double>&, int, int, cudaStream_t);
-template void grp_precond_t<float>(const GroupLaunch<float>&, int, int, int, cudaStream_t);
-template void grp_precond_t<double>(const GroupLaunch<double>&, int, int, int, cudaStream_t);
+template void grp_precond_t<float>(const GroupLaunch<float>&, int, int, int, cudaStream_t, int);
+template void grp_precond_t<double>(const GroupLaunch<double>&, int, int, int, cudaStream_t, int);
 
 template <typename T, int NT>
 void launch_pt_march(const Dims& d, const Coef<T>& c, CVec5<T> y, Vec5<T> out, const int* active,
-                     cudaStream_t st) {
+                     cudaStream_t st, const Shift<T>& sh) {
   const size_t smem = (size_t)d.nz * NT * sizeof(T);
-  static SmemLimit attr_bytes;  // per instantiation
-  ensure_smem_limit((const void*)pt_march_kernel<T, NT>, attr_bytes, smem);
-  launch_chained(pt_march_kernel<T, NT>, dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st, d, c, y, out, active);
+  with_shift(sh, [&](auto on) {
+    constexpr auto fn = pt_march_kernel<T, NT, decltype(on)::value>;
+    static SmemLimit attr_bytes;  // per instantiation
+    ensure_smem_limit((const void*)fn, attr_bytes, smem);
+    launch_chained(fn, dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st, d, c, y, out, active, sh);
+  });
 }
 
 template <typename T, int TPT, int TPC>
 void launch_pt_column(const Dims& d, const Coef<T>& c, CVec5<T> y, Vec5<T> out, const int* active,
-                      cudaStream_t st) {
+                      cudaStream_t st, const Shift<T>& sh) {
   const size_t smem = (size_t)(4 * d.nz) * TPC * sizeof(T);
-  static SmemLimit attr_bytes;  // per instantiation
-  ensure_smem_limit((const void*)pt_column_kernel<T, TPT, TPC>, attr_bytes, smem);
-  launch_chained(pt_column_kernel<T, TPT, TPC>, dim3((d.nx + TPC - 1) / TPC, d.ny), TPT, smem, st, d, c, y, out,
-                 active);
+  with_shift(sh, [&](auto on) {
+    constexpr auto fn = pt_column_kernel<T, TPT, TPC, decltype(on)::value>;
+    static SmemLimit attr_bytes;  // per instantiation
+    ensure_smem_limit((const void*)fn, attr_bytes, smem);
+    launch_chained(fn, dim3((d.nx + TPC - 1) / TPC, d.ny), TPT, smem, st, d, c, y, out, active, sh);
+  });
 }
 
 template <typename T, int TPT, int TPC, int PU>
 void launch_pt_column_batched(const Dims& d, const Coef<T>& c, CVec5<T> y, Vec5<T> out, const int* active,
-                              cudaStream_t st) {
+                              cudaStream_t st, const Shift<T>& sh) {
   const size_t smem = (size_t)(4 * d.nz) * TPC * sizeof(T);
-  static SmemLimit attr_bytes;  // per instantiation
-  ensure_smem_limit((const void*)pt_column_batched_kernel<T, TPT, TPC, PU>, attr_bytes, smem);
-  launch_chained(pt_column_batched_kernel<T, TPT, TPC, PU>, dim3((d.nx + TPC - 1) / TPC, d.ny), TPT, smem, st, d, c,
-                 y, out, active);
+  with_shift(sh, [&](auto on) {
+    constexpr auto fn = pt_column_batched_kernel<T, TPT, TPC, PU, decltype(on)::value>;
+    static SmemLimit attr_bytes;  // per instantiation
+    ensure_smem_limit((const void*)fn, attr_bytes, smem);
+    launch_chained(fn, dim3((d.nx + TPC - 1) / TPC, d.ny), TPT, smem, st, d, c, y, out, active, sh);
+  });
 }
 
 template <typename T>
 void launch_precond_t(const Dims& d, const Coef<T>& c, CVec5<T> y, Vec5<T> out, const int* active,
-                      cudaStream_t st) {
+                      cudaStream_t st, Shift<T> sh) {
   int v = d.tune_pct;
   if (v == 2 && (size_t)(4 * d.nz) * 64 * sizeof(T) > 200 * 1024) v = 0;  // 64-column tile too large
   switch (v) {
-    case 1: launch_pt_column<T, 128, 16>(d, c, y, out, active, st); break;
-    case 2: launch_pt_column<T, 256, 64>(d, c, y, out, active, st); break;
-    case 3: launch_pt_march<T, 128>(d, c, y, out, active, st); break;
+    case 1: launch_pt_column<T, 128, 16>(d, c, y, out, active, st, sh); break;
+    case 2: launch_pt_column<T, 256, 64>(d, c, y, out, active, st, sh); break;
+    case 3: launch_pt_march<T, 128>(d, c, y, out, active, st, sh); break;
     case 4:
       // at most one tile an SM: more threads a tile, as the forward preconditioner (61x47x40 float64 4.9 -> 4.2 us;
       // 128x128x64 float32 15.1 against 22.0)
-      if ((d.nx + 31) / 32 * d.ny <= 148) launch_pt_column_batched<T, 512, 32, 3>(d, c, y, out, active, st);
-      else launch_pt_column_batched<T, 256, 32, 4>(d, c, y, out, active, st);
+      if ((d.nx + 31) / 32 * d.ny <= 148) launch_pt_column_batched<T, 512, 32, 3>(d, c, y, out, active, st, sh);
+      else launch_pt_column_batched<T, 256, 32, 4>(d, c, y, out, active, st, sh);
       break;
-    default: launch_pt_column<T, 256, 32>(d, c, y, out, active, st); break;
+    default: launch_pt_column<T, 256, 32>(d, c, y, out, active, st, sh); break;
   }
   const dim3 blk = stencil_block(d.tune_mvt);
-  launch_chained(pt_uv_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz, blk), blk, 0, st, d, c, y, out, active);
+  with_shift(sh, [&](auto on) {
+    launch_chained(pt_uv_kernel<T, decltype(on)::value>, box_grid(d.nx + 1, d.ny + 1, d.nz, blk), blk, 0, st, d, c, y, out, active, sh);
+  });
 }
 
 template void launch_precond_t<float>(const Dims&, const Coef<float>&, CVec5<float>, Vec5<float>, const int*,
-                                      cudaStream_t);
+                                      cudaStream_t, Shift<float>);
 template void launch_precond_t<double>(const Dims&, const Coef<double>&, CVec5<double>, Vec5<double>, const int*,
-                                       cudaStream_t);
+                                       cudaStream_t, Shift<double>);
 
 // out = A^T (y * yscale), or out = b - A^T(...) when b is given; gzm_tmp is a
 // mass-point scratch field.

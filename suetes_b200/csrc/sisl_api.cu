@@ -547,6 +547,28 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
     else launch_precond<T>(d, cf, as_const(g.split(target, g.z())), g.view(target), act, s);
   };
   const int na = transpose ? 2 : 1, nm = transpose ? 2 : 1;
+  // V_{j+1} = (M A - I) (s_j V_j); the matvec's rows all go through z, whose u and v rows M reads unshifted
+  auto apply_shifted = [&](int j, cudaStream_t s) {
+    const int* act = &gs->active;
+    const CVec5<T> x = g.cview(g.V(j));
+    Vec5<T> out = g.view(g.V(j + 1));
+    Shift<T> sh;
+    for (int q = 0; q < 5; ++q) sh.f[q] = x.f[q];
+    sh.s = &gs->s[j];
+    sh.keep = g.tmp;
+    {
+      KScope k(c, SISL_K_MATVEC, s, na, transpose ? mvb : mvb + es * (field_size(d, LOC_U) + field_size(d, LOC_V)));
+      if (transpose) launch_matvec_t<T>(d, cf, x, sh.s, none, g.view(g.z()), g.tmp, act, s);
+      else launch_matvec<T>(d, cf, x, sh.s, none, g.view(g.z()), act, s, out.f[0], out.f[1]);
+    }
+    KScope k(c, SISL_K_PRECOND, s, nm, pcb + es * (field_size(d, LOC_M) + 2.0 * field_size(d, LOC_W)));
+    if (transpose) {
+      launch_precond_t<T>(d, cf, g.cview(g.z()), out, act, s, sh);
+    } else {
+      out.f[0] = out.f[1] = nullptr;  // the matvec wrote them
+      launch_precond<T>(d, cf, g.cview(g.z()), out, act, s, sh);
+    }
+  };
   if (method == SISL_GMRES_INCREMENTAL) {
     {
       KScope k(c, SISL_K_PRECOND, st, nm);
@@ -603,6 +625,10 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
     for (int b = 0, j0 = 0; b < nblocks; j0 += cols[b++]) {
       const int sc = cols[b];
       for (int j = j0; j < j0 + sc; ++j) {
+        if (S > 1) {
+          apply_shifted(j, s);
+          continue;
+        }
         {
           KScope k(c, SISL_K_MATVEC, s, na, mvb);
           apply_A(g.V(j), &gs->s[j], none, g.V(j + 1), &gs->active, s);
@@ -2561,10 +2587,10 @@ int gmres_group_run(const GroupLaunch<T>& gl, cudaStream_t st, cudaStream_t side
       for (int j = j0; j < j0 + cols[b]; ++j) {
         if (transpose) {
           grp_matvec_t<T>(gl, 0, j, s);
-          grp_precond_t<T>(gl, 0, j + 1, 1, s);
+          grp_precond_t<T>(gl, 0, j + 1, 1, s, S > 1);
         } else {
-          grp_matvec<T>(gl, 0, j, s);
-          grp_precond<T>(gl, 0, j + 1, 1, s);
+          grp_matvec<T>(gl, 0, j, s, S > 1);
+          grp_precond<T>(gl, 0, j + 1, 1, s, S > 1);
         }
       }
       if (S == 1) {

@@ -1,6 +1,8 @@
 // Coefficient sets and host-side launch wrappers shared by the SISL kernels.
 #pragma once
 
+#include <type_traits>
+
 #include "sisl_common.cuh"
 
 namespace sisl {
@@ -85,13 +87,45 @@ struct CVec5 {
   const T* f[5];
 };
 
-// out = A(x * xs) or out = b - A(x * xs) (residual mode, when b != nullptr)
+// What is subtracted from M A x to leave (M A - I) x, as the block Arnoldi
+// process wants it: the operator's own input x and its scale; f[0] null:
+// nothing.  The preconditioner kernels subtract it where they store their
+// result (shift_of).  M reads the u and v rows of A x and M^T the eta_dot
+// rows of its own result at neighbouring points, so those are kept unshifted
+// beside it: the forward matvec writes A x in full and the shifted u and v
+// rows as well (launch_matvec's su, sv), and M^T keeps the interior levels of
+// its eta_dot rows (keep, a mass-point field).  256x256x80 float32, a step of
+// two solves: 65.8 ms, and 71.5 with a pass of its own over the vectors; the
+// preconditioner 101 us with the shift's three more rows, 90 without.
+template <typename T>
+struct Shift {
+  const T* f[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+  const double* s = nullptr;
+  T* keep = nullptr;
+};
+template <typename T, bool SH>
+struct ShiftBy {
+  T c;
+  __device__ __forceinline__ explicit ShiftBy(const Shift<T>& sh) : c(SH ? -(T)(*sh.s) : T(0)) {}
+  // input value of field q at p, and the shifted result: one rounding, the same in every kernel
+  __device__ __forceinline__ T in(const Shift<T>& sh, int q, int p) const { return SH ? __ldg(sh.f[q] + p) : T(0); }
+  __device__ __forceinline__ T of(T v, T x) const { return SH ? fma(c, x, v) : v; }
+};
+// calls f with whether there is a shift as a compile-time constant: the kernels without one keep their registers
+template <typename T, typename F>
+inline void with_shift(const Shift<T>& sh, F&& f) {
+  if (sh.f[0]) f(std::true_type{});
+  else f(std::false_type{});
+}
+
+// out = A(x * xs) or out = b - A(x * xs) (residual mode, when b != nullptr);
+// su, sv: also the u and v rows less x * xs
 template <typename T>
 void launch_matvec(const Dims& d, const Coef<T>& c, CVec5<T> x, const double* xscale, CVec5<T> b,
-                   Vec5<T> out, const int* active, cudaStream_t st);
+                   Vec5<T> out, const int* active, cudaStream_t st, T* su = nullptr, T* sv = nullptr);
 template <typename T>
 void launch_precond(const Dims& d, const Coef<T>& c, CVec5<T> r, Vec5<T> out, const int* active,
-                    cudaStream_t st);
+                    cudaStream_t st, Shift<T> sh = Shift<T>());
 
 // transposes for the adjoint solve (sisl_adjoint.cu): out = A^T(y * ys), or
 // out = b - A^T(y * ys); gzm_tmp is a mass-point scratch field.  out = M^T y.
@@ -100,7 +134,7 @@ void launch_matvec_t(const Dims& d, const Coef<T>& c, CVec5<T> y, const double* 
                      T* gzm_tmp, const int* active, cudaStream_t st);
 template <typename T>
 void launch_precond_t(const Dims& d, const Coef<T>& c, CVec5<T> y, Vec5<T> out, const int* active,
-                      cudaStream_t st);
+                      cudaStream_t st, Shift<T> sh = Shift<T>());
 
 // grad += scale * (d tricubic / d field)^T cot  (coordinates carry no cotangent)
 template <typename T>

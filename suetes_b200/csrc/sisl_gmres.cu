@@ -13,18 +13,20 @@
 // The classical projection reads the whole basis twice per Arnoldi step (once
 // for the inner products, once for the update), which was two thirds of a
 // solve.  Here up to GM_S steps share those two reads: the operator is
-// applied to its own output s times, Z_1 = M A V_j, Z_i = M A Z_{i-1}, and
-// the s new vectors are orthogonalised together (s-step Arnoldi with a
-// monomial basis; Hoemmen, Communication-avoiding Krylov subspace methods,
-// Berkeley 2010).  block_dots forms all products of the basis with Z and of Z
-// with itself in one pass over memory, block_update the new vectors in a
-// second one, and the Hessenberg columns follow from the small matrices
-// (block_finish).  A cycle whose blocks keep all their columns spans the same
-// Krylov space and minimises over it as the one-step form does; a cycle in
-// which a column is lost to rounding is narrow: it is dropped and done over
-// one column at a time, and so are the solve's later ones (gmres_run in
-// sisl_api.cu).  256x256x80 float32, restart 30: vector passes per cycle 1020
-// -> 220.
+// applied to its own output s times, Z_1 = (M A - I) V_j, Z_i = (M A - I)
+// Z_{i-1}, and the s new vectors are orthogonalised together (s-step Arnoldi
+// with a shifted basis; Hoemmen, Communication-avoiding Krylov subspace
+// methods, Berkeley 2010).  The shift takes out the identity of M A = I + E:
+// E, the horizontal acoustic coupling, is small on smooth vectors, and
+// without it Z_i would be V_j over again there.  block_dots forms all products
+// of the basis with Z and of Z with itself in one pass over memory,
+// block_update the new vectors in a second one, and the Hessenberg columns
+// follow from the small matrices (block_finish).  A cycle whose blocks keep
+// all their columns spans the same Krylov space and minimises over it as the
+// one-step form does; a cycle in which a column is lost to rounding is
+// narrow: it is dropped and done over one column at a time, and so are the
+// solve's later ones (gmres_run in sisl_api.cu).  256x256x80 float32, restart
+// 30: vector passes per cycle 1020 -> 220.
 //
 // One column per block is the classical form: the dots and update kernels with
 // their one-step bookkeeping.  It stays for the cores and calls whose rule
@@ -289,7 +291,9 @@ __device__ __forceinline__ void block_coefs(GState* gs, const double* w, double*
   __syncthreads();
   if (tid == 0) {
     int keep = s;
-    const double lost = 32.0 * gs->eps;
+    // what is left of a healthy column, squared and against its length, is 5e-4 or more at six columns: acoustic
+    // radius 0.02 to 59, float32 and float64, cosine modes, noise and the states of the workloads
+    const double lost = fmax(32.0 * gs->eps, 1e-6);
     for (int i = 0; i < keep; ++i) {
       double piv = g[i][i];
       for (int q = 0; q < i; ++q) {
@@ -475,8 +479,8 @@ __global__ void __launch_bounds__(GT, 2) block_dots_kernel(const T* __restrict__
 // With rc^T rc = gram the new orthonormal vectors are Q_{m+i} = sum_q V_{m+q}
 // (rc^-1)[q][i], and in the basis Q the operator's inputs and outputs are
 // known columns C: C_0 the scaled V_j0, C_{i+1} = [r1_i; (rc r2)_i] the
-// vector Z_{i+1} = M A (input i).  H C_t = C_{t+1} gives the new columns of
-// H one after the other (a row per thread: a row of column t needs only the
+// vector Z_{i+1} = (M A - I) (input i).  H C_t = C_{t+1} + C_t gives the new
+// columns of H one after the other (a row per thread: a row of column t needs only the
 // same row of earlier columns).  For one column this is the classical
 // Arnoldi step.
 __device__ __forceinline__ void block_finish(GState* gs, const double (&gram)[GM_S][GM_S], int j0, int s) {
@@ -546,7 +550,7 @@ __device__ __forceinline__ void block_finish(GState* gs, const double (&gram)[GM
     for (int t = 0; t < GM_S; ++t) {
       h[t] = 0.0;
       if (t < keep) {
-        double v = C[t + 1][p] - a[t];
+        double v = C[t + 1][p] + C[t][p] - a[t];
 #pragma unroll
         for (int k = 0; k < GM_S; ++k)
           if (k < t) v -= h[k] * C[t][j0 + k];

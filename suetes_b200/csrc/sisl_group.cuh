@@ -133,17 +133,17 @@ void grp_info(const GroupLaunch<T>& g, int solve, cudaStream_t st);
 // mode 1 residual b - A x -> V_0 (u, v) | z; mode 2 float64 residual
 // b64 - A64 x64 -> r64 (refinement)
 template <typename T>
-void grp_matvec(const GroupLaunch<T>& g, int mode, int j, cudaStream_t st);
+void grp_matvec(const GroupLaunch<T>& g, int mode, int j, cudaStream_t st, int shift = 0);
 // preconditioner after the matvec: target V_t (u, v already there), w, pi,
 // eta from z; gated for the Arnoldi steps (t >= 1); mode 1: M b -> V_1
 template <typename T>
-void grp_precond(const GroupLaunch<T>& g, int mode, int t, int gated, cudaStream_t st);
+void grp_precond(const GroupLaunch<T>& g, int mode, int t, int gated, cudaStream_t st, int shift = 0);
 // transposed operators.  matvec^T: mode 0 Arnoldi step j (gated), V_j
 // scaled by s_j -> z; mode 1 b - A^T x -> z; mode 2 b64 - A64^T x64 -> r64.
 // preconditioner^T: mode 0 z -> V_t (gated when t >= 1); mode 1 b -> V_1
 template <typename T>
 void grp_matvec_t(const GroupLaunch<T>& g, int mode, int j, cudaStream_t st);
 template <typename T>
-void grp_precond_t(const GroupLaunch<T>& g, int mode, int t, int gated, cudaStream_t st);
+void grp_precond_t(const GroupLaunch<T>& g, int mode, int t, int gated, cudaStream_t st, int shift = 0);
 
 }  // namespace sisl

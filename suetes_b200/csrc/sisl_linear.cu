@@ -79,8 +79,8 @@ __device__ __forceinline__ void mv_rows(const Dims& d, const Coef<T>& c, const M
 // on a periodic axis the face-0 thread also writes the duplicate face n
 // (euler.py:412, 417).
 template <typename T>
-__device__ __forceinline__ void mv_store(const Dims& d, const CVec5<T>& b, const Vec5<T>& out, int i, int j, int k,
-                                         const T (&L)[5]) {
+__device__ __forceinline__ void mv_store(const Dims& d, const CVec5<T>& x, T xs, T xu_f, T xv_f, const CVec5<T>& b,
+                                         const Vec5<T>& out, T* su, T* sv, int i, int j, int k, const T (&L)[5]) {
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const bool do_u = (k < nz) && (j < ny) && !(d.px && i == nx);
   const bool do_v = (k < nz) && (i < nx) && !(d.py && j == ny);
@@ -88,17 +88,21 @@ __device__ __forceinline__ void mv_store(const Dims& d, const CVec5<T>& b, const
   if (do_u) {
     const int p = iu(d, i, j, k);
     out.f[0][p] = b.f[0] ? ld(b.f[0], p) - L[0] : L[0];
+    if (su) su[p] = fma(-xs, xu_f, L[0]);
     if (d.px && i == 0) {
       const int pn = iu(d, nx, j, k);
       out.f[0][pn] = b.f[0] ? ld(b.f[0], pn) - L[0] : L[0];
+      if (su) su[pn] = fma(-xs, ld(x.f[0], pn), L[0]);
     }
   }
   if (do_v) {
     const int p = iv(d, i, j, k);
     out.f[1][p] = b.f[1] ? ld(b.f[1], p) - L[1] : L[1];
+    if (sv) sv[p] = fma(-xs, xv_f, L[1]);
     if (d.py && j == 0) {
       const int pn = iv(d, i, ny, k);
       out.f[1][pn] = b.f[1] ? ld(b.f[1], pn) - L[1] : L[1];
+      if (sv) sv[pn] = fma(-xs, ld(x.f[1], pn), L[1]);
     }
   }
   if (own) {
@@ -115,7 +119,8 @@ __device__ __forceinline__ void mv_store(const Dims& d, const CVec5<T>& b, const
 // All rows of one point of the union box (the matvec_kernel body).
 template <typename T>
 __device__ __forceinline__ void matvec_point(const Dims& d, const Coef<T>& c, const CVec5<T>& x, const T xs,
-                                             const CVec5<T>& b, const Vec5<T>& out, int i, int j, int k) {
+                                             const CVec5<T>& b, const Vec5<T>& out, T* su, T* sv, int i, int j,
+                                             int k) {
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const T adt = (T)(c.s.alpha * c.s.dt), cp = (T)c.s.cp, a = (T)c.s.alpha, ps = (T)c.s.ps;
   const T sp = xs / ps;
@@ -200,17 +205,21 @@ __device__ __forceinline__ void matvec_point(const Dims& d, const Coef<T>& c, co
   if (do_u) {
     const int p = iu(d, i, j, k);
     out.f[0][p] = b.f[0] ? ld(b.f[0], p) - Lu : Lu;
+    if (su) su[p] = fma(-xs, xu_f, Lu);
     if (d.px && i == 0) {  // duplicate periodic face (euler.py:412)
       const int pn = iu(d, nx, j, k);
       out.f[0][pn] = b.f[0] ? ld(b.f[0], pn) - Lu : Lu;
+      if (su) su[pn] = fma(-xs, ld(xu, pn), Lu);
     }
   }
   if (do_v) {
     const int p = iv(d, i, j, k);
     out.f[1][p] = b.f[1] ? ld(b.f[1], p) - Lv : Lv;
+    if (sv) sv[p] = fma(-xs, xv_f, Lv);
     if (d.py && j == 0) {
       const int pn = iv(d, i, ny, k);
       out.f[1][pn] = b.f[1] ? ld(b.f[1], pn) - Lv : Lv;
+      if (sv) sv[pn] = fma(-xs, ld(xv, pn), Lv);
     }
   }
   if (own) {
@@ -230,7 +239,7 @@ __device__ __forceinline__ void matvec_point(const Dims& d, const Coef<T>& c, co
 template <typename T, int LV>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (LV == 1 ? 6 : 4) : (LV == 1 ? 4 : 3)) matvec_kernel(Dims d, Coef<T> c, CVec5<T> x,
                                                                             const double* xscale,
-                                                     CVec5<T> b, Vec5<T> out, const int* active) {
+                                                     CVec5<T> b, Vec5<T> out, const int* active, T* su, T* sv) {
   grid_chain();
   if (active && *active == 0) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -240,7 +249,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (LV == 1 ? 6 : 4) : (LV 
   const T xs = xscale ? (T)(*xscale) : T(1);
 #pragma unroll
   for (int l = 0; l < LV; ++l)
-    if (k0 + l <= d.nz) matvec_point(d, c, x, xs, b, out, i, j, k0 + l);
+    if (k0 + l <= d.nz) matvec_point(d, c, x, xs, b, out, su, sv, i, j, k0 + l);
 }
 
 // cp.async helpers (global -> shared, asynchronous, per thread)
@@ -287,7 +296,7 @@ struct MvB {  // the rest of level k (faces at mass level min(k, nz-1), w-level 
 template <typename T>
 __device__ __forceinline__ void matvec_march_block(const Dims& d, const Coef<T>& c, const CVec5<T>& x,
                                                    const double* xscale, const CVec5<T>& b, const Vec5<T>& out,
-                                                   int bx, int by, int bz, int gz) {
+                                                   T* su, T* sv, int bx, int by, int bz, int gz) {
   const int i = bx * blockDim.x + threadIdx.x;
   const int j = by * blockDim.y + threadIdx.y;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -448,7 +457,7 @@ __device__ __forceinline__ void matvec_march_block(const Dims& d, const Coef<T>&
     q.xp_k = a0.pO;
     T L[5];
     mv_rows(d, c, q, xs, u_lock, v_lock, k == 0 || k == nz, L);
-    mv_store(d, b, out, i, j, k, L);
+    mv_store(d, x, xs, q.xu_f, q.xv_f, b, out, su, sv, i, j, k, L);
     // one level up
     uw_a = b0.uO0, uw_b = b0.uO1, vw_a = b0.vO0, vw_b = b0.vO1;
     PmO = P0O, PmX = P0X, PmY = P0Y;
@@ -463,10 +472,11 @@ __device__ __forceinline__ void matvec_march_block(const Dims& d, const Coef<T>&
 template <typename T>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 2) matvec_march_kernel(Dims d, Coef<T> c, CVec5<T> x,
                                                                                   const double* xscale, CVec5<T> b,
-                                                                                  Vec5<T> out, const int* active) {
+                                                                                  Vec5<T> out, const int* active, T* su,
+                                                                                  T* sv) {
   grid_chain();
   if (active && *active == 0) return;
-  matvec_march_block<T>(d, c, x, xscale, b, out, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.z);
+  matvec_march_block<T>(d, c, x, xscale, b, out, su, sv, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.z);
 }
 
 // ---------------------------------------------------------------------------
@@ -516,9 +526,22 @@ __device__ __forceinline__ PrecondW<T> precond_wlevel(const Dims& d, const Coef<
   return o;
 }
 
-template <typename T, int PT, int PC>
+// ground and lid rows of a column (steppers.py:237-238, 244-245)
+template <typename T, bool SH>
+__device__ __forceinline__ void precond_ends(const Coef<T>& c, const Shift<T>& sh, const ShiftBy<T, SH>& by,
+                                             const T* __restrict__ rw, const T* __restrict__ rW, T* __restrict__ ow,
+                                             T* __restrict__ oW, int h, int top) {
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int p = h + (e ? top : 0);
+    ow[p] = by.of(ld(rw, p), by.in(sh, 2, p));
+    oW[p] = by.of(mul_rn(ld(rW, p), ld(c.dzw, p)), by.in(sh, 4, p));
+  }
+}
+
+template <typename T, int PT, int PC, bool SH>
 __global__ void __launch_bounds__(PT) precond_tile_kernel(Dims d, Coef<T> c, CVec5<T> r, Vec5<T> out,
-                                                          const int* active) {
+                                                          const int* active, Shift<T> sh) {
   grid_chain();
   if (active && *active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -540,20 +563,21 @@ __global__ void __launch_bounds__(PT) precond_tile_kernel(Dims d, Coef<T> c, CVe
   T* __restrict__ ow = out.f[2];
   T* __restrict__ op = out.f[3];
   T* __restrict__ oW = out.f[4];
+  const ShiftBy<T, SH> by(sh);
   const T inva = T(1) / (T)c.s.alpha;
   const T ips = (T)c.s.rps;
   const T ps = (T)c.s.ps;
   const int pm = nx * ny;
 
   // u and v pass straight through (steppers.py:247-249) unless aliased
-  if (out.f[0] != ru) {
+  if (out.f[0] && out.f[0] != ru) {
     const int ncol = min(PC + (i0 + PC >= nx ? 1 : 0), nx + 1 - i0);
     for (int q = tid; q < ncol * nz; q += PT) {
       const int k = q / ncol, ii = i0 + q % ncol;
       out.f[0][iu(d, ii, j, k)] = ld(ru, iu(d, ii, j, k));
     }
   }
-  if (out.f[1] != rv) {
+  if (out.f[1] && out.f[1] != rv) {
     const int ncol = min(PC, nx - i0);
     const int nj = (j == ny - 1) ? 2 : 1;  // the last block row also copies face ny
     for (int q = tid; q < ncol * nz * nj; q += PT) {
@@ -605,15 +629,16 @@ __global__ void __launch_bounds__(PT) precond_tile_kernel(Dims d, Coef<T> c, CVe
     const int k = q / PC, l = q % PC, i = i0 + l;
     if (i >= nx) continue;
     const int p = i + nx * j + k * pm;
+    const T xw = by.in(sh, 2, p), xW = by.in(sh, 4, p);
     if (k == 0 || k == nz) {  // boundary rows (steppers.py:237-238, 244-245)
-      ow[p] = ld(rw, p);
-      oW[p] = ld(rW, p) * ld(c.dzw, p);
+      ow[p] = by.of(ld(rw, p), xw);
+      oW[p] = by.of(mul_rn(ld(rW, p), ld(c.dzw, p)), xW);
     } else {
       const T wv = ld(rw, p) * ld(c.idamp, p) - ld(c.pbw, p) * (s_x[q] - s_x[q - PC]);
-      ow[p] = wv;
-      oW[p] = oW[p] + wv;
+      ow[p] = by.of(wv, xw);
+      oW[p] = by.of(oW[p] + wv, xW);
     }
-    if (k < nz) op[p] = s_x[q] * ps;
+    if (k < nz) op[p] = by.of(mul_rn(s_x[q], ps), by.in(sh, 3, p));
   }
 }
 
@@ -625,9 +650,9 @@ __global__ void __launch_bounds__(PT) precond_tile_kernel(Dims d, Coef<T> c, CVe
 // w-level phase reads six arrays instead of fifteen values.  Arithmetic is
 // term for term that of precond_wlevel and precond_tile_kernel: results
 // are bitwise those of every other column variant.
-template <typename T, int PT, int PC, int PU>
+template <typename T, int PT, int PC, int PU, bool SH>
 __global__ void __launch_bounds__(PT) precond_tile_batched_kernel(Dims d, Coef<T> c, CVec5<T> r, Vec5<T> out,
-                                                                  const int* active) {
+                                                                  const int* active, Shift<T> sh) {
   grid_chain();
   if (active && *active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -649,20 +674,21 @@ __global__ void __launch_bounds__(PT) precond_tile_batched_kernel(Dims d, Coef<T
   T* __restrict__ ow = out.f[2];
   T* __restrict__ op = out.f[3];
   T* __restrict__ oW = out.f[4];
+  const ShiftBy<T, SH> by(sh);
   const T inva = T(1) / (T)c.s.alpha;
   const T ips = (T)c.s.rps;
   const T ps = (T)c.s.ps;
   const int pm = nx * ny;
   const int nm = nz * PC, nw = (nz + 1) * PC;
 
-  if (out.f[0] != ru) {
+  if (out.f[0] && out.f[0] != ru) {
     const int ncol = min(PC + (i0 + PC >= nx ? 1 : 0), nx + 1 - i0);
     for (int q = tid; q < ncol * nz; q += PT) {
       const int k = q / ncol, ii = i0 + q % ncol;
       out.f[0][iu(d, ii, j, k)] = ld(ru, iu(d, ii, j, k));
     }
   }
-  if (out.f[1] != rv) {
+  if (out.f[1] && out.f[1] != rv) {
     const int ncol = min(PC, nx - i0);
     const int nj = (j == ny - 1) ? 2 : 1;
     for (int q = tid; q < ncol * nz * nj; q += PT) {
@@ -779,7 +805,7 @@ __global__ void __launch_bounds__(PT) precond_tile_batched_kernel(Dims d, Coef<T
   }
   __syncthreads();
   // ---- C: back substitution for w, eta_dot and the scaled pi ----
-  T ww[PU], id[PU], pb[PU];
+  T ww[PU], id[PU], pb[PU], xw[PU], xW[PU], xp[PU];
   auto c_load = [&](int q0) {
 #pragma unroll
     for (int u = 0; u < PU; ++u) {
@@ -791,6 +817,9 @@ __global__ void __launch_bounds__(PT) precond_tile_batched_kernel(Dims d, Coef<T
         const bool edge = (k == 0 || k == nz);
         id[u] = edge ? ld(rW, p) : ld(c.idamp, p);
         pb[u] = edge ? ld(c.dzw, p) : ld(c.pbw, p);
+        xw[u] = by.in(sh, 2, p);
+        xW[u] = by.in(sh, 4, p);
+        xp[u] = by.in(sh, 3, min(p, nz * pm - 1));
       }
     }
   };
@@ -802,14 +831,14 @@ __global__ void __launch_bounds__(PT) precond_tile_batched_kernel(Dims d, Coef<T
       if (q < nw && i < nx) {
         const int p = i + nx * j + k * pm;
         if (k == 0 || k == nz) {
-          ow[p] = ww[u];
-          oW[p] = id[u] * pb[u];
+          ow[p] = by.of(ww[u], xw[u]);
+          oW[p] = by.of(mul_rn(id[u], pb[u]), xW[u]);
         } else {
           const T wv = ww[u] * id[u] - pb[u] * (s_x[q] - s_x[q - PC]);
-          ow[p] = wv;
-          oW[p] = oW[p] + wv;
+          ow[p] = by.of(wv, xw[u]);
+          oW[p] = by.of(oW[p] + wv, xW[u]);
         }
-        if (k < nz) op[p] = s_x[q] * ps;
+        if (k < nz) op[p] = by.of(mul_rn(s_x[q], ps), xp[u]);
       }
     }
   };
@@ -823,24 +852,24 @@ __global__ void __launch_bounds__(PT) precond_tile_batched_kernel(Dims d, Coef<T
 
 template <typename T>
 void launch_matvec(const Dims& d, const Coef<T>& c, CVec5<T> x, const double* xscale, CVec5<T> b,
-                   Vec5<T> out, const int* active, cudaStream_t st) {
+                   Vec5<T> out, const int* active, cudaStream_t st, T* su, T* sv) {
   if (d.tune_mv >= 6 && d.nz >= 2) {  // column march in 1, 2 or 4 z chunks
     const dim3 blk(32, 4, 1);
     dim3 grd((d.nx + 1 + 31) / 32, (d.ny + 1 + 3) / 4, d.tune_mv == 7 ? 2 : (d.tune_mv == 8 ? 4 : 1));
-    launch_chained(matvec_march_kernel<T>, grd, blk, 0, st, d, c, x, xscale, b, out, active);
+    launch_chained(matvec_march_kernel<T>, grd, blk, 0, st, d, c, x, xscale, b, out, active, su, sv);
     return;
   }
   if (d.tune_mv == 4 || d.tune_mv == 5) {  // two or four levels per thread
     const dim3 blk(32, 8, 1);
     const int lv = d.tune_mv == 4 ? 2 : 4;
     dim3 grd((d.nx + 1 + 31) / 32, (d.ny + 1 + 7) / 8, (d.nz + lv) / lv);
-    if (lv == 2) launch_chained(matvec_kernel<T, 2>, grd, blk, 0, st, d, c, x, xscale, b, out, active);
-    else launch_chained(matvec_kernel<T, 4>, grd, blk, 0, st, d, c, x, xscale, b, out, active);
+    if (lv == 2) launch_chained(matvec_kernel<T, 2>, grd, blk, 0, st, d, c, x, xscale, b, out, active, su, sv);
+    else launch_chained(matvec_kernel<T, 4>, grd, blk, 0, st, d, c, x, xscale, b, out, active, su, sv);
     return;
   }
   const dim3 blk = stencil_block(d.tune_mv);
   dim3 grd((d.nx + 1 + blk.x - 1) / blk.x, (d.ny + 1 + blk.y - 1) / blk.y, (d.nz + 1 + blk.z - 1) / blk.z);
-  launch_chained(matvec_kernel<T, 1>, grd, blk, 0, st, d, c, x, xscale, b, out, active);
+  launch_chained(matvec_kernel<T, 1>, grd, blk, 0, st, d, c, x, xscale, b, out, active, su, sv);
 }
 
 // ---------------------------------------------------------------------------
@@ -854,9 +883,9 @@ void launch_matvec(const Dims& d, const Coef<T>& c, CVec5<T> x, const double* xs
 // writes pi, w and eta_dot at the w level between x(k) and x(k+1).
 // Shared memory per block: nz * NT values of T.
 // ---------------------------------------------------------------------------
-template <typename T, int NT>
+template <typename T, int NT, bool SH>
 __global__ void __launch_bounds__(NT) precond_march_kernel(Dims d, Coef<T> c, CVec5<T> r, Vec5<T> out,
-                                                           const int* active) {
+                                                           const int* active, Shift<T> sh) {
   grid_chain();
   if (active && *active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -876,6 +905,7 @@ __global__ void __launch_bounds__(NT) precond_march_kernel(Dims d, Coef<T> c, CV
   T* __restrict__ ow = out.f[2];
   T* __restrict__ op = out.f[3];
   T* __restrict__ oW = out.f[4];
+  const ShiftBy<T, SH> by(sh);
   const T mq = T(0.25) * ld(c.mm, h);
   const int ub = iu(d, i, j, 0), vb = iv(d, i, j, 0);
   // u over faces i, i+1 and v over faces j, j+1 at mass level k
@@ -903,37 +933,37 @@ __global__ void __launch_bounds__(NT) precond_march_kernel(Dims d, Coef<T> c, CV
     wt_lo = wt_hi;
   }
   T xh = dprev;
-  op[h + (nz - 1) * pm] = xh * ps;
+  const int pl = h + (nz - 1) * pm;
+  op[pl] = by.of(mul_rn(xh, ps), by.in(sh, 3, pl));
 #pragma unroll 4
   for (int k = nz - 2; k >= 0; --k) {  // steppers.py:227-245
     const int p = h + k * pm;
     const T x = s_d[k * NT + t] - ld(c.tcp, p) * xh;
-    op[p] = x * ps;
+    op[p] = by.of(mul_rn(x, ps), by.in(sh, 3, p));
     const int pw = p + pm;
     const T wv = ld(rw, pw) * ld(c.idamp, pw) - ld(c.pbw, pw) * (xh - x);
-    ow[pw] = wv;
-    oW[pw] = oW[pw] + wv;
+    ow[pw] = by.of(wv, by.in(sh, 2, pw));
+    oW[pw] = by.of(oW[pw] + wv, by.in(sh, 4, pw));
     xh = x;
   }
-  ow[h] = ld(rw, h);  // ground and lid rows (steppers.py:237-238, 244-245)
-  oW[h] = ld(rW, h) * ld(c.dzw, h);
-  const int ptop = h + nz * pm;
-  ow[ptop] = ld(rw, ptop);
-  oW[ptop] = ld(rW, ptop) * ld(c.dzw, ptop);
+  precond_ends<T, SH>(c, sh, by, rw, rW, ow, oW, h, nz * pm);
 }
 
 template <typename T, int NT>
 void launch_precond_march(const Dims& d, const Coef<T>& c, CVec5<T> r, Vec5<T> out, const int* active,
-                          cudaStream_t st) {
+                          cudaStream_t st, const Shift<T>& sh) {
   const size_t smem = (size_t)d.nz * NT * sizeof(T);
-  static SmemLimit attr_bytes;  // per instantiation
-  ensure_smem_limit((const void*)precond_march_kernel<T, NT>, attr_bytes, smem);
   // u and v pass straight through (steppers.py:247-249) unless aliased
-  if (out.f[0] != r.f[0])
+  if (out.f[0] && out.f[0] != r.f[0])
     cudaMemcpyAsync(out.f[0], r.f[0], sizeof(T) * field_size(d, LOC_U), cudaMemcpyDeviceToDevice, st);
-  if (out.f[1] != r.f[1])
+  if (out.f[1] && out.f[1] != r.f[1])
     cudaMemcpyAsync(out.f[1], r.f[1], sizeof(T) * field_size(d, LOC_V), cudaMemcpyDeviceToDevice, st);
-  launch_chained(precond_march_kernel<T, NT>, dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st, d, c, r, out, active);
+  with_shift(sh, [&](auto on) {
+    constexpr auto fn = precond_march_kernel<T, NT, decltype(on)::value>;
+    static SmemLimit attr_bytes;  // per instantiation
+    ensure_smem_limit((const void*)fn, attr_bytes, smem);
+    launch_chained(fn, dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st, d, c, r, out, active, sh);
+  });
 }
 
 // ---------------------------------------------------------------------------
@@ -988,17 +1018,17 @@ struct PcUp {  // inputs of upward step k: faces at mass level k + 1, w level k 
   T u0, u1, v0, v1, zx, ze, W, rt, w, id, p, l, lo, inv;
 };
 template <typename T>
-struct PcDown {  // inputs of downward step k: mass level k, w level k + 1
-  T cp, w, id, pb, ep;
+struct PcDown {  // inputs of downward step k: mass level k, w level k + 1 (xp, xw, xW: the shift's)
+  T cp, w, id, pb, ep, xp, xw, xW;
 };
 
-template <typename T, int NT, int HINT>
+template <typename T, int NT, int HINT, bool SH>
 __device__ __forceinline__ void precond_pipe_block(const Dims& d, const Coef<T>& c, const CVec5<T>& r,
-                                                   const Vec5<T>& out, int bx, int by) {
+                                                   const Vec5<T>& out, const Shift<T>& sh, int bx, int by_) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* s_d = reinterpret_cast<T*>(smem_raw);  // [nz][NT]
   const int t = threadIdx.x;
-  const int i = bx * NT + t, j = by;
+  const int i = bx * NT + t, j = by_;
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   if (i >= nx) return;
   const int pm = nx * ny, h = i + nx * j;
@@ -1012,6 +1042,7 @@ __device__ __forceinline__ void precond_pipe_block(const Dims& d, const Coef<T>&
   T* __restrict__ ow = out.f[2];
   T* __restrict__ op = out.f[3];
   T* __restrict__ oW = out.f[4];
+  const ShiftBy<T, SH> by(sh);
   const uint64_t keep = HINT ? l2_policy_evict_last() : 0, once = HINT ? l2_policy_evict_first() : 0;
   const T mq = T(0.25) * ld(c.mm, h);
   const int ub = iu(d, i, j, 0), vb = iv(d, i, j, 0);
@@ -1069,37 +1100,39 @@ __device__ __forceinline__ void precond_pipe_block(const Dims& d, const Coef<T>&
     e.id = ldp<T, HINT>(c.idamp, pw, keep);
     e.pb = ldp<T, HINT>(c.pbw, pw, once);
     e.ep = oW[pw];
+    if (SH) {
+      e.xp = ldp<T, HINT>(sh.f[3], p, once);
+      e.xw = ldp<T, HINT>(sh.f[2], pw, once);
+      e.xW = ldp<T, HINT>(sh.f[4], pw, once);
+    }
     return e;
   };
   T xh = dprev;
-  op[h + (nz - 1) * pm] = xh * ps;
+  const int pl = h + (nz - 1) * pm;
+  op[pl] = by.of(mul_rn(xh, ps), by.in(sh, 3, pl));
   if (nz >= 2) {
     PcDown<T> e = down(nz - 2), f = down(max(nz - 3, 0));
     for (int k = nz - 2; k >= 0; --k) {  // steppers.py:227-245
       const PcDown<T> gnext = down(max(k - 2, 0));
       const int p = h + k * pm, pw = p + pm;
       const T x = s_d[k * NT + t] - e.cp * xh;
-      op[p] = x * ps;
+      op[p] = by.of(mul_rn(x, ps), e.xp);
       const T wv = e.w * e.id - e.pb * (xh - x);
-      ow[pw] = wv;
-      oW[pw] = e.ep + wv;
+      ow[pw] = by.of(wv, e.xw);
+      oW[pw] = by.of(e.ep + wv, e.xW);
       xh = x;
       e = f;
       f = gnext;
     }
   }
-  ow[h] = ld(rw, h);  // ground and lid rows (steppers.py:237-238, 244-245)
-  oW[h] = ld(rW, h) * ld(c.dzw, h);
-  const int ptop = h + nz * pm;
-  ow[ptop] = ld(rw, ptop);
-  oW[ptop] = ld(rW, ptop) * ld(c.dzw, ptop);
+  precond_ends<T, SH>(c, sh, by, rw, rW, ow, oW, h, nz * pm);
 }
-template <typename T, int NT, int HINT>
+template <typename T, int NT, int HINT, bool SH>
 __global__ void __launch_bounds__(NT) precond_pipe_kernel(Dims d, Coef<T> c, CVec5<T> r, Vec5<T> out,
-                                                          const int* active) {
+                                                          const int* active, Shift<T> sh) {
   grid_chain();
   if (active && *active == 0) return;
-  precond_pipe_block<T, NT, HINT>(d, c, r, out, blockIdx.x, blockIdx.y);
+  precond_pipe_block<T, NT, HINT, SH>(d, c, r, out, sh, blockIdx.x, blockIdx.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -1110,9 +1143,9 @@ __global__ void __launch_bounds__(NT) precond_pipe_kernel(Dims d, Coef<T> c, CVe
 // thread reads back only what it copied itself (no block barrier).
 // Shared memory per block: (nz + 16 S) * NT values of T.
 // ---------------------------------------------------------------------------
-template <typename T, int NT, int S>
+template <typename T, int NT, int S, bool SH>
 __global__ void __launch_bounds__(NT) precond_async_kernel(Dims d, Coef<T> c, CVec5<T> r, Vec5<T> out,
-                                                           const int* active) {
+                                                           const int* active, Shift<T> sh) {
   grid_chain();
   if (active && *active == 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1134,6 +1167,7 @@ __global__ void __launch_bounds__(NT) precond_async_kernel(Dims d, Coef<T> c, CV
   T* __restrict__ ow = out.f[2];
   T* __restrict__ op = out.f[3];
   T* __restrict__ oW = out.f[4];
+  const ShiftBy<T, SH> by(sh);
   const T mq = T(0.25) * ld(c.mm, h);
   const int ub = iu(d, i, j, 0), vb = iv(d, i, j, 0);
   // the 14 inputs of upward step k into ring slot `slot` (clamped in bounds)
@@ -1197,7 +1231,8 @@ __global__ void __launch_bounds__(NT) precond_async_kernel(Dims d, Coef<T> c, CV
     cp_async_t(q + 4 * NT, oW + pw);  // this thread's own eta_dot/alpha - kin of the upward sweep
   };
   T xh = dprev;
-  op[h + (nz - 1) * pm] = xh * ps;
+  const int pl = h + (nz - 1) * pm;
+  op[pl] = by.of(mul_rn(xh, ps), by.in(sh, 3, pl));
   if (nz >= 2) {
 #pragma unroll
     for (int q = 0; q < S - 1; ++q) {
@@ -1211,90 +1246,96 @@ __global__ void __launch_bounds__(NT) precond_async_kernel(Dims d, Coef<T> c, CV
       const T* e = ring + (n % S) * 16 * NT + t;
       const int p = h + k * pm, pw = p + pm;
       const T x = s_d[k * NT + t] - e[0 * NT] * xh;
-      op[p] = x * ps;
+      op[p] = by.of(mul_rn(x, ps), by.in(sh, 3, p));
       const T wv = e[1 * NT] * e[2 * NT] - e[3 * NT] * (xh - x);
-      ow[pw] = wv;
-      oW[pw] = e[4 * NT] + wv;
+      ow[pw] = by.of(wv, by.in(sh, 2, pw));
+      oW[pw] = by.of(e[4 * NT] + wv, by.in(sh, 4, pw));
       xh = x;
     }
     cp_async_wait<0>();
   }
-  ow[h] = ld(rw, h);  // ground and lid rows (steppers.py:237-238, 244-245)
-  oW[h] = ld(rW, h) * ld(c.dzw, h);
-  const int ptop = h + nz * pm;
-  ow[ptop] = ld(rw, ptop);
-  oW[ptop] = ld(rW, ptop) * ld(c.dzw, ptop);
+  precond_ends<T, SH>(c, sh, by, rw, rW, ow, oW, h, nz * pm);
 }
 
 template <typename T, int NT, int S>
 void launch_precond_async(const Dims& d, const Coef<T>& c, CVec5<T> r, Vec5<T> out, const int* active,
-                          cudaStream_t st) {
+                          cudaStream_t st, const Shift<T>& sh) {
   const size_t smem = (size_t)(d.nz + 16 * S) * NT * sizeof(T);
-  static SmemLimit attr_bytes;  // per instantiation
-  ensure_smem_limit((const void*)precond_async_kernel<T, NT, S>, attr_bytes, smem);
-  if (out.f[0] != r.f[0])
+  if (out.f[0] && out.f[0] != r.f[0])
     cudaMemcpyAsync(out.f[0], r.f[0], sizeof(T) * field_size(d, LOC_U), cudaMemcpyDeviceToDevice, st);
-  if (out.f[1] != r.f[1])
+  if (out.f[1] && out.f[1] != r.f[1])
     cudaMemcpyAsync(out.f[1], r.f[1], sizeof(T) * field_size(d, LOC_V), cudaMemcpyDeviceToDevice, st);
-  launch_chained(precond_async_kernel<T, NT, S>, dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st, d, c, r, out,
-                 active);
+  with_shift(sh, [&](auto on) {
+    constexpr auto fn = precond_async_kernel<T, NT, S, decltype(on)::value>;
+    static SmemLimit attr_bytes;  // per instantiation
+    ensure_smem_limit((const void*)fn, attr_bytes, smem);
+    launch_chained(fn, dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st, d, c, r, out, active, sh);
+  });
 }
 
 template <typename T, int NT, int HINT>
 void launch_precond_pipe(const Dims& d, const Coef<T>& c, CVec5<T> r, Vec5<T> out, const int* active,
-                         cudaStream_t st) {
+                         cudaStream_t st, const Shift<T>& sh) {
   const size_t smem = (size_t)d.nz * NT * sizeof(T);
-  static SmemLimit attr_bytes;  // per instantiation
-  ensure_smem_limit((const void*)precond_pipe_kernel<T, NT, HINT>, attr_bytes, smem);
   // u and v pass straight through (steppers.py:247-249) unless aliased
-  if (out.f[0] != r.f[0])
+  if (out.f[0] && out.f[0] != r.f[0])
     cudaMemcpyAsync(out.f[0], r.f[0], sizeof(T) * field_size(d, LOC_U), cudaMemcpyDeviceToDevice, st);
-  if (out.f[1] != r.f[1])
+  if (out.f[1] && out.f[1] != r.f[1])
     cudaMemcpyAsync(out.f[1], r.f[1], sizeof(T) * field_size(d, LOC_V), cudaMemcpyDeviceToDevice, st);
-  launch_chained(precond_pipe_kernel<T, NT, HINT>, dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st, d, c, r, out,
-                 active);
+  with_shift(sh, [&](auto on) {
+    constexpr auto fn = precond_pipe_kernel<T, NT, HINT, decltype(on)::value>;
+    static SmemLimit attr_bytes;  // per instantiation
+    ensure_smem_limit((const void*)fn, attr_bytes, smem);
+    launch_chained(fn, dim3((d.nx + NT - 1) / NT, d.ny), NT, smem, st, d, c, r, out, active, sh);
+  });
 }
 
 template <typename T, int PT, int PC>
 void launch_precond_tile(const Dims& d, const Coef<T>& c, CVec5<T> r, Vec5<T> out, const int* active,
-                         cudaStream_t st) {
+                         cudaStream_t st, const Shift<T>& sh) {
   const size_t smem = (size_t)(5 * d.nz + 1) * PC * sizeof(T);
-  static SmemLimit attr_bytes;  // per instantiation
-  ensure_smem_limit((const void*)precond_tile_kernel<T, PT, PC>, attr_bytes, smem);
   dim3 grd((d.nx + PC - 1) / PC, d.ny);
-  launch_chained(precond_tile_kernel<T, PT, PC>, grd, PT, smem, st, d, c, r, out, active);
+  with_shift(sh, [&](auto on) {
+    constexpr auto fn = precond_tile_kernel<T, PT, PC, decltype(on)::value>;
+    static SmemLimit attr_bytes;  // per instantiation
+    ensure_smem_limit((const void*)fn, attr_bytes, smem);
+    launch_chained(fn, grd, PT, smem, st, d, c, r, out, active, sh);
+  });
 }
 
 template <typename T, int PT, int PC, int PU>
 void launch_precond_tile_batched(const Dims& d, const Coef<T>& c, CVec5<T> r, Vec5<T> out, const int* active,
-                                 cudaStream_t st) {
+                                 cudaStream_t st, const Shift<T>& sh) {
   const size_t smem = (size_t)(5 * d.nz + 1) * PC * sizeof(T);
-  static SmemLimit attr_bytes;  // per instantiation
-  ensure_smem_limit((const void*)precond_tile_batched_kernel<T, PT, PC, PU>, attr_bytes, smem);
   dim3 grd((d.nx + PC - 1) / PC, d.ny);
-  launch_chained(precond_tile_batched_kernel<T, PT, PC, PU>, grd, PT, smem, st, d, c, r, out, active);
+  with_shift(sh, [&](auto on) {
+    constexpr auto fn = precond_tile_batched_kernel<T, PT, PC, PU, decltype(on)::value>;
+    static SmemLimit attr_bytes;  // per instantiation
+    ensure_smem_limit((const void*)fn, attr_bytes, smem);
+    launch_chained(fn, grd, PT, smem, st, d, c, r, out, active, sh);
+  });
 }
 
 template <typename T>
 void launch_precond(const Dims& d, const Coef<T>& c, CVec5<T> r, Vec5<T> out, const int* active,
-                    cudaStream_t st) {
+                    cudaStream_t st, Shift<T> sh) {
   int v = d.tune_pc;
   if (v == 2 && (size_t)(5 * d.nz + 1) * 64 * sizeof(T) > 200 * 1024) v = 0;  // 64-column tile too large
   switch (v) {
-    case 1: launch_precond_tile<T, 128, 16>(d, c, r, out, active, st); break;
-    case 2: launch_precond_tile<T, 256, 64>(d, c, r, out, active, st); break;
-    case 3: launch_precond_march<T, 128>(d, c, r, out, active, st); break;
+    case 1: launch_precond_tile<T, 128, 16>(d, c, r, out, active, st, sh); break;
+    case 2: launch_precond_tile<T, 256, 64>(d, c, r, out, active, st, sh); break;
+    case 3: launch_precond_march<T, 128>(d, c, r, out, active, st, sh); break;
     case 4:
       // At most one tile an SM: a thread per level or two, so that every phase is one round of loads (float32
       // 48x41x33 7.2 -> 6.0 us, float64 64x64x48 12.1 -> 9.6, 61x47x40 11.4 -> 9.0); with more tiles than SMs
       // several smaller blocks hide more (128x128x64 float32 19.4 against 39.8).
-      if ((d.nx + 31) / 32 * d.ny <= 148) launch_precond_tile_batched<T, 1024, 32, 2>(d, c, r, out, active, st);
-      else launch_precond_tile_batched<T, 256, 32, 4>(d, c, r, out, active, st);
+      if ((d.nx + 31) / 32 * d.ny <= 148) launch_precond_tile_batched<T, 1024, 32, 2>(d, c, r, out, active, st, sh);
+      else launch_precond_tile_batched<T, 256, 32, 4>(d, c, r, out, active, st, sh);
       break;
-    case 5: launch_precond_pipe<T, 64, 0>(d, c, r, out, active, st); break;
-    case 6: launch_precond_pipe<T, 64, 1>(d, c, r, out, active, st); break;
-    case 7: launch_precond_async<T, 32, 6>(d, c, r, out, active, st); break;
-    default: launch_precond_tile<T, 256, 32>(d, c, r, out, active, st); break;
+    case 5: launch_precond_pipe<T, 64, 0>(d, c, r, out, active, st, sh); break;
+    case 6: launch_precond_pipe<T, 64, 1>(d, c, r, out, active, st, sh); break;
+    case 7: launch_precond_async<T, 32, 6>(d, c, r, out, active, st, sh); break;
+    default: launch_precond_tile<T, 256, 32>(d, c, r, out, active, st, sh); break;
   }
 }
 
@@ -1307,12 +1348,13 @@ __device__ __forceinline__ T* gvec_l(const GroupMember<T>& g, int v) {
   return g.vec + (size_t)v * g.npad;
 }
 
-// mode 0: Arnoldi step j (gated), V_j scaled by s_j -> V_{j+1} (u, v) | z;
+// mode 0: Arnoldi step j (gated), V_j scaled by s_j -> V_{j+1} (u, v) | z, with shift -> z and the shifted u, v rows
+// -> V_{j+1};
 // mode 1: b - A x -> V_0 (u, v) | z; mode 2 (U = double): b64 - A64 x64 -> r64
 template <typename T, typename U>
 __global__ void __launch_bounds__(128, sizeof(U) == 4 ? 3 : 2) group_matvec_kernel(GroupMember<T>* mem,
                                                                                   const int* __restrict__ first,
-                                                                                  int M, int mode, int j) {
+                                                                                  int M, int mode, int j, int shift) {
   grid_chain();
   const int b = blockIdx.x;
   const int mi = group_find(first, M, b);
@@ -1336,9 +1378,10 @@ __global__ void __launch_bounds__(128, sizeof(U) == 4 ? 3 : 2) group_matvec_kern
     for (int q = 0; q < 5; ++q) {
       x.f[q] = src + g.off[q];
       bb.f[q] = (mode == 1) ? bv + g.off[q] : nullptr;
-      out.f[q] = (q < 2 ? tgt : z) + g.off[q];
+      out.f[q] = (q < 2 && !shift ? tgt : z) + g.off[q];
     }
-    matvec_march_block<T>(g.d, g.c, x, xsp, bb, out, bx, by, bz, 1);
+    matvec_march_block<T>(g.d, g.c, x, xsp, bb, out, shift ? tgt + g.off[0] : nullptr, shift ? tgt + g.off[1] : nullptr,
+                          bx, by, bz, 1);
   } else {
     CVec5<double> x, bb;
     Vec5<double> out;
@@ -1347,13 +1390,13 @@ __global__ void __launch_bounds__(128, sizeof(U) == 4 ? 3 : 2) group_matvec_kern
       bb.f[q] = g.b64 + g.off[q];
       out.f[q] = g.r64 + g.off[q];
     }
-    matvec_march_block<double>(g.d, g.c64, x, xsp, bb, out, bx, by, bz, 1);
+    matvec_march_block<double>(g.d, g.c64, x, xsp, bb, out, nullptr, nullptr, bx, by, bz, 1);
   }
 }
 
 // mode 0: target V_t: u, v already there, w, pi, eta_dot from z (gated when
-// t >= 1); mode 1: M b -> V_1 (u, v copied by the caller)
-template <typename T, int NT>
+// t >= 1), with shift less s V_{t-1} and A's u, v rows from z; mode 1: M b -> V_1 (u, v copied by the caller)
+template <typename T, int NT, bool SH>
 __global__ void __launch_bounds__(NT) group_precond_kernel(GroupMember<T>* mem, const int* __restrict__ first, int M,
                                                            int mode, int tv, int gated) {
   grid_chain();
@@ -1369,10 +1412,16 @@ __global__ void __launch_bounds__(NT) group_precond_kernel(GroupMember<T>* mem, 
   CVec5<T> r;
   Vec5<T> out;
   for (int q = 0; q < 5; ++q) {
-    r.f[q] = (q < 2 && mode == 0 ? tgt : src) + g.off[q];
+    r.f[q] = (q < 2 && mode == 0 && !SH ? tgt : src) + g.off[q];
     out.f[q] = tgt + g.off[q];
   }
-  precond_pipe_block<T, NT, 1>(g.d, g.c, r, out, bx, by);
+  Shift<T> sh;
+  if (SH) {
+    const T* x = gvec_l(g, GV_V0 + tv - 1);
+    for (int q = 0; q < 5; ++q) sh.f[q] = x + g.off[q];
+    sh.s = &g.gs->s[tv - 1];
+  }
+  precond_pipe_block<T, NT, 1, SH>(g.d, g.c, r, out, sh, bx, by);
 }
 
 // ---------------------------------------------------------------------------
@@ -1383,40 +1432,43 @@ int group_matvec_blocks(const Dims& d) { return ((d.nx + 1 + 31) / 32) * ((d.ny 
 int group_precond_blocks(const Dims& d) { return ((d.nx + GROUP_PC_NT - 1) / GROUP_PC_NT) * d.ny; }
 
 template <typename T>
-void grp_matvec(const GroupLaunch<T>& g, int mode, int j, cudaStream_t st) {
+void grp_matvec(const GroupLaunch<T>& g, int mode, int j, cudaStream_t st, int shift) {
   const int nb = g.blocks(GT_MV);
   if (mode == 2) {
     if constexpr (sizeof(T) == 4) launch_chained(group_matvec_kernel<T, double>, nb, dim3(32, 4), 0, st, g.mem,
-                                                 g.row(GT_MV), g.M, 2, 0);
+                                                 g.row(GT_MV), g.M, 2, 0, 0);
     return;
   }
-  launch_chained(group_matvec_kernel<T, T>, nb, dim3(32, 4), 0, st, g.mem, g.row(GT_MV), g.M, mode, j);
+  launch_chained(group_matvec_kernel<T, T>, nb, dim3(32, 4), 0, st, g.mem, g.row(GT_MV), g.M, mode, j, shift);
 }
 
 template <typename T>
-void grp_precond(const GroupLaunch<T>& g, int mode, int t, int gated, cudaStream_t st) {
+void grp_precond(const GroupLaunch<T>& g, int mode, int t, int gated, cudaStream_t st, int shift) {
   int nz_max = 1;
   for (int m = 0; m < g.M; ++m) nz_max = nz_max > g.nz_h[m] ? nz_max : g.nz_h[m];
   const size_t smem = (size_t)nz_max * GROUP_PC_NT * sizeof(T);
-  static SmemLimit attr_bytes;
-  ensure_smem_limit((const void*)group_precond_kernel<T, GROUP_PC_NT>, attr_bytes, smem);
-  launch_chained(group_precond_kernel<T, GROUP_PC_NT>, g.blocks(GT_PC), GROUP_PC_NT, smem, st, g.mem, g.row(GT_PC),
-                 g.M, mode, t,
-                                                                                   gated);
+  auto run = [&](auto on) {
+    constexpr auto fn = group_precond_kernel<T, GROUP_PC_NT, decltype(on)::value>;
+    static SmemLimit attr_bytes;
+    ensure_smem_limit((const void*)fn, attr_bytes, smem);
+    launch_chained(fn, g.blocks(GT_PC), GROUP_PC_NT, smem, st, g.mem, g.row(GT_PC), g.M, mode, t, gated);
+  };
+  if (shift) run(std::true_type{});
+  else run(std::false_type{});
 }
 
-template void grp_matvec<float>(const GroupLaunch<float>&, int, int, cudaStream_t);
-template void grp_matvec<double>(const GroupLaunch<double>&, int, int, cudaStream_t);
-template void grp_precond<float>(const GroupLaunch<float>&, int, int, int, cudaStream_t);
-template void grp_precond<double>(const GroupLaunch<double>&, int, int, int, cudaStream_t);
+template void grp_matvec<float>(const GroupLaunch<float>&, int, int, cudaStream_t, int);
+template void grp_matvec<double>(const GroupLaunch<double>&, int, int, cudaStream_t, int);
+template void grp_precond<float>(const GroupLaunch<float>&, int, int, int, cudaStream_t, int);
+template void grp_precond<double>(const GroupLaunch<double>&, int, int, int, cudaStream_t, int);
 
 template void launch_matvec<float>(const Dims&, const Coef<float>&, CVec5<float>, const double*, CVec5<float>,
-                                   Vec5<float>, const int*, cudaStream_t);
+                                   Vec5<float>, const int*, cudaStream_t, float*, float*);
 template void launch_matvec<double>(const Dims&, const Coef<double>&, CVec5<double>, const double*,
-                                    CVec5<double>, Vec5<double>, const int*, cudaStream_t);
+                                    CVec5<double>, Vec5<double>, const int*, cudaStream_t, double*, double*);
 template void launch_precond<float>(const Dims&, const Coef<float>&, CVec5<float>, Vec5<float>, const int*,
-                                    cudaStream_t);
+                                    cudaStream_t, Shift<float>);
 template void launch_precond<double>(const Dims&, const Coef<double>&, CVec5<double>, Vec5<double>,
-                                     const int*, cudaStream_t);
+                                     const int*, cudaStream_t, Shift<double>);
 
 }  // namespace sisl
