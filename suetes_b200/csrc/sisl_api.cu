@@ -412,33 +412,6 @@ void default_shapes(Dims& d, size_t es) {
   d.tune_pct = d.nz >= 2 ? 4 : 0;
 }
 
-// Columns per orthogonalisation block of the Krylov cycles.  The monomial
-// basis M A V, (M A)^2 V, .. of a block is well conditioned when the operator
-// M A = I + E is dominated by E, the horizontal acoustic coupling, whose
-// spectrum is close to imaginary with radius alpha dt times the grid's largest
-// acoustic frequency.  From radius 3 a block of 6 loses nothing against
-// one-step orthogonalisation (flat mountain wave, float32 vectors, residual
-// after 3 cycles 3.7823e-10 against 3.7836e-10 at radius 3.8, and the same
-// digits at 7, 15 and 61); at 1.9, where one cycle already converges to
-// the vectors' rounding, the first cycle ends at 1.6e-6 against 5.8e-7, so
-// such small steps keep one column at a time.
-//
-// The forward solves of a float32 step recorded for its VJP keep one column
-// too: the objective of a gradient run is compared between runs (finite
-// differences, Taylor tests) as a float32 number, where the last bit of the
-// state shows in full, and one column per block forms the states to the bit
-// as the one-step Arnoldi process does.  128x128x64 float32, two steps and
-// their sweep: 243 ms with one column everywhere, 187 ms with blocks in the
-// transposed solves only (this rule), 152 ms with blocks in both.
-int block_columns(const SislCore* c, bool taped) {
-  if (taped && c->grid.dtype == SISL_F32) return 1;
-  const Scalars& s = c->s;
-  const double sound = std::sqrt(s.cp / s.cvd * s.Rd * 300.0);
-  const double radius =
-      2.0 * s.alpha * s.dt * sound * std::sqrt(1.0 / (c->d.dx * c->d.dx) + 1.0 / (c->d.dy * c->d.dy));
-  return radius >= 3.0 ? GM_S : 1;
-}
-
 // A conditional WHILE node at the tail of st's capture: gate(handle,
 // after_pass, stream) launches the kernel that sets its condition, before it
 // and after every pass; body(stream) records one pass, captured on side.
@@ -498,14 +471,13 @@ int capture_while(cudaStream_t st, cudaStream_t side, Gate&& gate, Body&& body) 
 // synchronisation: the whole solve replays inside one graph launch.
 template <typename T>
 int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, SislSolveInfo* info,
-              int transpose = 0, GDevInfo* dev_info = nullptr, bool taped = false) {
+              int transpose = 0, GDevInfo* dev_info = nullptr) {
   const Dims& d = c->d;
   const int R = g.R;
   const size_t n = g.npad;
   const int method = (transpose && c->adj_method >= 0) ? c->adj_method : c->prm.solve_method;
   const double eps = (sizeof(T) == 8) ? 2.220446049250313e-16 : 1.1920928955078125e-07;
   GState* gs = g.gs;
-  const int S = block_columns(c, taped);
   CVec5<T> none{};
   const double es = sizeof(T), vb = es * (double)n;
   const double mvb = matvec_bytes(d, sizeof(T)), pcb = precond_bytes(d, sizeof(T));
@@ -525,7 +497,7 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
   {
     KScope k(c, SISL_K_OTHER, st);
     const double tol = (transpose && c->adj_tol > 0.0) ? c->adj_tol : c->prm.solver_tol;
-    gm_setup(gs, eps, tol, c->prm.solver_atol, R, method, S, st);
+    gm_setup(gs, eps, tol, c->prm.solver_atol, R, method, GM_S, st);
   }
   {
     KScope k(c, SISL_K_DOTS, st);
@@ -677,7 +649,7 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
   if (dev_info) {  // ---- graph mode ----
     if (!c->cap_side) return SISL_ERR_ARG;
     residual(st);
-    for (int form = S > 1 ? 1 : 0; form >= 0; --form) {
+    for (int form = 1; form >= 0; --form) {
       const int rc = capture_while(
           st, c->cap_side,
           [&](cudaGraphConditionalHandle h, int after, cudaStream_t s) {
@@ -685,7 +657,7 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
             gm_gate(gs, h, maxiter, after, form, s);
           },
           [&](cudaStream_t s) {
-            cycle(s, form ? S : 1);
+            cycle(s, form ? GM_S : 1);
             residual(s);
           });
       if (rc) return rc;
@@ -713,14 +685,14 @@ int gmres_run(SislCore* c, const Coef<T>& cf, GWork<T>& g, cudaStream_t st, Sisl
   residual(st);
   int rc = read();
   if (rc) return rc;
-  int cycles = 0, steps = 0, form = S;
+  int cycles = 0, steps = 0, columns = GM_S;
   while (cycles < maxiter && hv->rnorm > hv->atol) {
-    cycle(st, form);
+    cycle(st, columns);
     residual(st);
     rc = read();
     if (rc) return rc;
     if (hv->narrow) {
-      form = 1;
+      columns = 1;
       continue;
     }
     steps += hv->kdone;
@@ -1103,7 +1075,7 @@ int step_impl(SislCore* c, const SislState* in, const SislState* out, const Sisl
   for (int it = 0; it < 2; ++it) {
     step_pre_solve<T>(r, it);
     SislSolveInfo si{};
-    rc = gmres_run<T>(c, r.cf, r.w.g, st, &si, 0, dev_info ? dev_info + it : nullptr, tape != nullptr);
+    rc = gmres_run<T>(c, r.cf, r.w.g, st, &si, 0, dev_info ? dev_info + it : nullptr);
     rc = step_post_solve<T>(r, it, rc, si);
     if (rc) return rc;
   }
@@ -2605,12 +2577,12 @@ int gmres_group_run(const GroupLaunch<T>& gl, cudaStream_t st, cudaStream_t side
     grp_update_x<T>(gl, s);
   };
   residual(st);
-  for (int form = gl.S > 1 ? 1 : 0; form >= 0; --form) {
+  for (int form = 1; form >= 0; --form) {
     const int rc = capture_while(
         st, side,
         [&](cudaGraphConditionalHandle h, int after, cudaStream_t s) { grp_gate<T>(gl, h, after, form, s); },
         [&](cudaStream_t s) {
-          cycle(s, form ? gl.S : 1);
+          cycle(s, form ? GM_S : 1);
           residual(s);
         });
     if (rc) return rc;
@@ -2627,7 +2599,7 @@ int gmres_group_run(const GroupLaunch<T>& gl, cudaStream_t st, cudaStream_t side
 // grouped GMRES over all members (gmres_group_run).  transpose: the solves
 // are the reverse sweep's transposed ones, the step's second solve first.
 template <typename T, typename Open, typename Work, typename Phase>
-int capture_grouped(int n, SislCore* const* cores, int transpose, bool taped, Open&& open, Work&& gwork, Phase&& phase,
+int capture_grouped(int n, SislCore* const* cores, int transpose, Open&& open, Work&& gwork, Phase&& phase,
                     SislStepGraph** out) {
   SislStepGraph* g = new (std::nothrow) SislStepGraph();
   if (!g) return SISL_ERR_ARG;
@@ -2698,8 +2670,6 @@ int capture_grouped(int n, SislCore* const* cores, int transpose, bool taped, Op
   gl.R = R;
   gl.method = method;
   gl.refine = refine;
-  gl.S = GM_S;
-  for (int m = 0; m < n; ++m) gl.S = std::min(gl.S, block_columns(cores[m], taped));
   gl.first_h.assign((size_t)NT * (n + 1), 0);
   gl.nz_h.resize(n);
   for (int m = 0; m < n; ++m) {
@@ -2798,7 +2768,7 @@ int capture_grouped_step(int n, SislCore* const* cores, const SislState* ins, co
   std::vector<StepRun<T>> runs(n);
   const SislSolveInfo none{};
   return capture_grouped<T>(
-      n, cores, 0, solves != nullptr,
+      n, cores, 0,
       [&](int m, cudaStream_t s) {
         return step_open<T>(runs[m], cores[m], &ins[m], &outs[m], relax ? relax[m] : nullptr, ws[m], ws_bytes[m],
                             s, nullptr, solves ? solves + 10 * m : nullptr, nullptr);
@@ -2832,7 +2802,7 @@ int capture_grouped_vjp(int n, SislCore* const* cores, const SislState* ins, voi
   std::vector<VjpRun<T>> runs(n);
   const SislSolveInfo none{};
   return capture_grouped<T>(
-      n, cores, 1, false,
+      n, cores, 1,
       [&](int m, cudaStream_t s) {
         return vjp_open<T>(runs[m], cores[m], &ins[m], solves + 10 * m, relax ? relax[m] : nullptr, &out_bars[m],
                            &in_bars[m], ws[m], ws_bytes[m], s, nullptr);

@@ -28,9 +28,8 @@
 // solve's later ones (gmres_run in sisl_api.cu).  256x256x80 float32, restart
 // 30: vector passes per cycle 1020 -> 220.
 //
-// One column per block is the classical form: the dots and update kernels with
-// their one-step bookkeeping.  It stays for the cores and calls whose rule
-// says so (block_columns in sisl_api.cu).
+// One column at a time is the classical form: the dots and update kernels with
+// their one-step bookkeeping, for what follows a narrow cycle.
 //
 // The block form's stored vectors V carry a small triangular factor per block (GState::B)
 // instead of being normalised in memory: the Gram matrix of the vectors as
@@ -1534,7 +1533,7 @@ int group_convert_blocks(size_t n) { return flat_grid(n, 256 * 8) < 296 ? flat_g
 
 template <typename T>
 void grp_setup(const GroupLaunch<T>& g, int transpose, cudaStream_t st) {
-  launch_chained(group_setup_kernel<T>, (g.M + 127) / 128, 128, 0, st, g.mem, g.M, g.R, g.method, transpose, g.S);
+  launch_chained(group_setup_kernel<T>, (g.M + 127) / 128, 128, 0, st, g.mem, g.M, g.R, g.method, transpose, GM_S);
 }
 template <typename T>
 void grp_dots(const GroupLaunch<T>& g, int m, int w, int mode, int gated, cudaStream_t st) {

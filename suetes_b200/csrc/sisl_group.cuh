@@ -61,7 +61,6 @@ struct GroupLaunch {
   std::vector<int> first_h;  // host copy
   std::vector<int> nz_h;     // members' level counts (preconditioner shared memory)
   int M = 0, R = 0, method = 0;
-  int S = 1;                 // columns per orthogonalisation block, the same for every member
   bool refine = false;
   const int* row(int t) const { return first + (size_t)t * (M + 1); }
   int blocks(int t) const { return first_h[(size_t)t * (M + 1) + M]; }

@@ -108,9 +108,11 @@ def test_cycle_takes_all_its_steps(waves, dt, restart, dtype, method):
     p = Problem(dt, method, restart)
     rhs = smooth_rhs(waves)
     _, info = p.solve(rhs, dtype)
-    # an incremental cycle may leave when its estimate meets the tolerance (float64 at the smallest step)
-    assert info["cycles"] == 1 and (info["arnoldi_steps"] == restart or info["converged"]), info
     first, least = p.reference(rhs, dtype, info["arnoldi_steps"])
+    # an incremental cycle leaves when its estimate meets the tolerance (float64 at the smallest step) or nothing above
+    # the rounding of its vectors is left to orthogonalise (float32 there: the residual is at 4 eps of the first)
+    spent = info["converged"] or info["residual_norm"] <= 4 * torch.finfo(dtype).eps * first
+    assert info["cycles"] == 1 and (info["arnoldi_steps"] == restart or spent), (info, first)
     assert info["residual_norm"] <= RATIO * least + FLOOR[dtype] * first, (info, least, first)
 
 
@@ -130,7 +132,7 @@ def test_transposed_cycle_takes_all_its_steps(dt, dtype):
 # launches and about 20 others of a solve.
 @pytest.mark.parametrize("method", ["batched", "incremental"])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
-@pytest.mark.parametrize("dt", [3.2, 8.0, 16.0])
+@pytest.mark.parametrize("dt", [0.2, 1.0, 3.2, 8.0, 16.0])
 @pytest.mark.parametrize("waves", [(0, 1, 1), (1, 1, 1), (2, 1, 0)])
 def test_smooth_blocks_keep_their_columns(waves, dt, dtype, method):
     from suetes_b200.core import kernel_launches
