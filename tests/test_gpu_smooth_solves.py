@@ -10,7 +10,7 @@ import math
 import pytest
 import torch
 
-from _cases import build, mountain, shapes5, to_cuda
+from _cases import build, mountain, random_fields, rel_l2, shapes5, to_cuda
 
 pytestmark = pytest.mark.gpu
 
@@ -41,10 +41,11 @@ def smooth_rhs(waves, shape=SHAPE):
 class Problem:
     """The package's solver from a zero guess, and the reference cycle on the same operator."""
 
-    def __init__(self, dt, method, restart=30, maxiter=1, tol=1e-14, h=None, shape=SHAPE, transpose=False):
+    def __init__(self, dt, method, restart=30, maxiter=1, tol=1e-14, h=None, shape=SHAPE, transpose=False,
+                 periodic=()):
         from suetes_b200 import SemiImplicitSolver3D
         from suetes_b200.steppers import VerticalPreconditioner
-        p = build("cuda", *shape, *SPACING, h=h, device="cuda", dt=dt)
+        p = build("cuda", *shape, *SPACING, h=h, periodic=periodic, device="cuda", dt=dt)
         self.bg = p[2].precompute_bg(p[2].bg_state_ref())
         self.shapes = shapes5(*shape)
         self.solver = SemiImplicitSolver3D(p[2], dt, solver_tol=tol, solver_maxiter=maxiter, solver_restart=restart,
@@ -142,6 +143,33 @@ def test_smooth_blocks_keep_their_columns(waves, dt, dtype, method):
     before = kernel_launches()
     p.solve(rhs, dtype)
     assert kernel_launches() - before < 60 + 14 + 40
+
+
+# Periodic axes, whose duplicate faces are unknowns of their own: a right-hand side that differs there too.  One
+# float64 cycle of 13 against the oracle's; the bound is that of the one-cycle tests of test_gpu_block_arnoldi.
+@pytest.mark.parametrize("periodic", [(0,), (1,), (0, 1)])
+def test_periodic_cycle_is_the_oracles(periodic):
+    from oracle.steppers import SemiImplicitSolver3D as Oracle
+    from suetes_b200 import SemiImplicitSolver3D
+    shape, dt = (11, 9, 7), 8.0
+    rhs = random_fields(shapes5(*shape), 7, {"u": 1.0, "v": 1.0, "w": 0.5, "pi": 1e-3, "eta_dot": 1e-3})
+    kw = dict(solver_tol=1e-14, solver_maxiter=1, solver_restart=13)
+    o = build("oracle", *shape, *SPACING, h=mountain, periodic=periodic, dt=dt)[2]
+    p = build("cuda", *shape, *SPACING, h=mountain, periodic=periodic, device="cuda", dt=dt)[2]
+    ref = Oracle(o, dt, **kw).solve(rhs, o.precompute_bg(o.bg_state_ref()))
+    out = SemiImplicitSolver3D(p, dt, **kw).solve(to_cuda(rhs), p.precompute_bg(p.bg_state_ref()))
+    for k in ref:
+        assert rel_l2(out[k], ref[k]) < 1e-9, (k, rel_l2(out[k], ref[k]))
+
+
+@pytest.mark.parametrize("periodic", [(0,), (1,), (0, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_periodic_transposed_cycle(periodic, dtype):
+    p = Problem(8.0, "batched", 13, h=mountain, transpose=True, periodic=periodic)
+    rhs = random_fields(p.shapes, 7, {"u": 1.0, "v": 1.0, "w": 0.5, "pi": 1e3, "eta_dot": 0.0})
+    _, info = p.solve(rhs, dtype)
+    first, least = p.reference(rhs, dtype, 13)
+    assert info["residual_norm"] <= RATIO * least + FLOOR[dtype] * first, (info, least, first)
 
 
 # A cycle that is cut short is still the least residual of the steps it took
