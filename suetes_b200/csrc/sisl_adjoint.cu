@@ -380,8 +380,8 @@ __global__ void __launch_bounds__(TPT) pt_column_kernel(Dims d, Coef<T> c, CVec5
 // batching).  Arithmetic is term for term that of pt_column_kernel, so the
 // results are bitwise those of every other column variant.
 template <typename T, int TPT, int TPC, int PU, bool SH>
-__device__ __forceinline__ void pt_column_batched_block(const Dims& d, const Coef<T>& c, const CVec5<T>& y, const Vec5<T>& out,
-                                               const Shift<T>& sh, int bx, int by_, int bz) {
+__device__ __forceinline__ void pt_column_batched_block(const Dims& d, const Coef<T>& c, const CVec5<T>& y,
+                                                        const Vec5<T>& out, const Shift<T>& sh, int bx, int by_, int bz) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* sm = reinterpret_cast<T*>(smem_raw);
   const int nx = d.nx, ny = d.ny, nz = d.nz;
@@ -520,8 +520,8 @@ __global__ void __launch_bounds__(TPT) pt_column_batched_kernel(Dims d, Coef<T> 
 // M^T, horizontal part: out_u = y_u + sum of the kinematic cotangent
 // kinbar = -alpha out_W over the interior w levels of the adjacent cells.
 template <typename T, bool SH>
-__device__ __forceinline__ void pt_uv_block(const Dims& d, const Coef<T>& c, const CVec5<T>& y, const Vec5<T>& out,
-                                               const Shift<T>& sh, int bx, int by_, int bz) {
+__device__ __forceinline__ void pt_uv_block(const Dims& d, const Coef<T>& c, const CVec5<T>& y,
+                                            const Vec5<T>& out, const Shift<T>& sh, int bx, int by_, int bz) {
   const int i = bx * blockDim.x + threadIdx.x;
   const int j = by_ * blockDim.y + threadIdx.y;
   const int k = bz * blockDim.z + threadIdx.z;
@@ -870,9 +870,7 @@ void launch_tricubic_vjp(int sx, int sy, int sz, int dx, int dy, int dz, const T
                          const T* cot, T* grad, int use_limiter, T scale, cudaStream_t st) {
   dim3 blk(32, 4, 2);
   launch_chained(tricubic_vjp_kernel<T>, box_grid(dx, dy, dz, blk), blk, 0, st, sx, sy, sz, dx, dy, dz, field,
-                 coords3[0],
-                                                                    coords3[1], coords3[2], cot, grad,
-                                                                    use_limiter, scale);
+                 coords3[0], coords3[1], coords3[2], cot, grad, use_limiter, scale);
 }
 size_t tricubic_vjp_det_scratch_bytes(int sx, int sy, int sz, int elem_bytes) {
   return 256 + (elem_bytes == 8 ? 2 : 1) * sizeof(unsigned long long) * (size_t)sx * sy * sz;
@@ -892,19 +890,17 @@ void launch_tricubic_vjp_det(int sx, int sy, int sz, int dx, int dy, int dz, con
   const dim3 grd = box_grid(dx, dy, dz, blk);
   if (relative)
     launch_chained(tricubic_vjp_count_kernel<T, 1>, grd, blk, 0, st, sx, sy, sz, dx, dy, dz, coords3[0], coords3[1],
-                                                         coords3[2], cot, scale, (int*)acc, hdr);
+                   coords3[2], cot, scale, (int*)acc, hdr);
   else
     launch_chained(tricubic_vjp_count_kernel<T, 0>, grd, blk, 0, st, sx, sy, sz, dx, dy, dz, coords3[0], coords3[1],
-                                                         coords3[2], cot, scale, (int*)acc, hdr);
+                   coords3[2], cot, scale, (int*)acc, hdr);
   cudaMemsetAsync(acc, 0, (sizeof(T) == 8 ? 2 : 1) * sizeof(unsigned long long) * n, st);
   if (relative)
     launch_chained(tricubic_vjp_fixed_kernel<T, 1>, grd, blk, 0, st, sx, sy, sz, dx, dy, dz, field, coords3[0],
-                   coords3[1],
-                                                         coords3[2], cot, acc, hdr, use_limiter, scale);
+                   coords3[1], coords3[2], cot, acc, hdr, use_limiter, scale);
   else
     launch_chained(tricubic_vjp_fixed_kernel<T, 0>, grd, blk, 0, st, sx, sy, sz, dx, dy, dz, field, coords3[0],
-                   coords3[1],
-                                                         coords3[2], cot, acc, hdr, use_limiter, scale);
+                   coords3[1], coords3[2], cot, acc, hdr, use_limiter, scale);
   const size_t nb = (n + 255) / 256;
   launch_chained(tricubic_vjp_finish_kernel<T>, (unsigned)(nb < 148 * 16 ? nb : 148 * 16), 256, 0, st, n, acc, hdr,
                  grad);
@@ -926,8 +922,8 @@ template void launch_tricubic_vjp<double>(int, int, int, int, int, int, const do
 // the w and eta_dot cotangents of the w level between z(k) and z(k+1) are
 // formed.  Shared memory per block: nz * NT values of T.
 template <typename T, int NT, bool SH>
-__device__ __forceinline__ void pt_march_block(const Dims& d, const Coef<T>& c, const CVec5<T>& y, const Vec5<T>& out,
-                                               const Shift<T>& sh, int bx, int by_, int bz) {
+__device__ __forceinline__ void pt_march_block(const Dims& d, const Coef<T>& c, const CVec5<T>& y,
+                                               const Vec5<T>& out, const Shift<T>& sh, int bx, int by_, int bz) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* s_w = reinterpret_cast<T*>(smem_raw);  // [nz][NT]
   const int t = threadIdx.x;
@@ -1209,9 +1205,8 @@ void launch_matvec_t(const Dims& d, const Coef<T>& c, CVec5<T> y, const double* 
   const dim3 blk = stencil_block(d.tune_mvt);
   launch_chained(at_gzm_kernel<T>, box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st, d, c, y.f[0], y.f[1], yscale,
                  gzm_tmp, active);
-  launch_chained(at_main_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, c, y, yscale,
-                 gzm_tmp, b, out,
-                                                                              active);
+  launch_chained(at_main_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, c, y, yscale, gzm_tmp,
+                 b, out, active);
 }
 
 template void launch_matvec_t<float>(const Dims&, const Coef<float>&, CVec5<float>, const double*, CVec5<float>,

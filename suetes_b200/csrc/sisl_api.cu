@@ -351,8 +351,7 @@ void scale5(SislCore* c, const Coef<T>& cf, CVec5<T> src, Vec5<T> dst, T pi_mul,
   KScope k(c, SISL_K_OTHER, st);
   dim3 blk(32, 4, 2);
   launch_chained(scale5_kernel<T>, box(c->d.nx + 1, c->d.ny + 1, c->d.nz + 1, blk), blk, 0, st, c->d, src, dst,
-                 pi_mul,
-                                                                                   eta_mode, cf.dzw, cf.idzw);
+                 pi_mul, eta_mode, cf.dzw, cf.idzw);
 }
 
 template <typename T>
@@ -379,18 +378,19 @@ double precond_bytes(const Dims& d, size_t es) {
 }
 
 // Launch shapes of a core that has not been tuned; every shape gives the same
-// bits, so only time decides.  Lines drawn from whole solves (us per Arnoldi
-// step, cold coefficients) at grids from 48x41x33 to 384x384x96.
+// bits, so only time decides.  Lines drawn from whole solves of one cycle of
+// 30 (us per Arnoldi step) at grids from 48x41x33 to 384x384x96.
 //
 // Matvec.  The column march (6) holds one thread per column: it needs
 // four blocks on every SM to hide memory, and then beats the
 // several-levels-per-thread shapes (4: two, 5: four), which hide latency with
-// threads instead (256x256x80 float32 449 against 473; 192x192x64, at 0.6 of a
-// wave, 255 against 237; 64x64x48 104 against 70).  Past one wave of blocks,
-// four z chunks (8) even out the second one (384x384x96 1202 against 1257).
-// In float64 the march has half the threads resident and never wins by more
-// than 1 %; shape 5 from about 20,000 columns (150x131x60 222.5 against 224.2,
-// 96x96x48 114 against 110).
+// threads instead (256x256x80 float32 451 against 493; 192x192x64, at 0.6 of a
+// wave, 231 against 229; 64x64x48 64 against 42).  Past one wave of blocks,
+// four z chunks (8) even out the second one (384x384x96 1226 against 1270).
+// In float64 the march has half the threads resident and does not win
+// (150x131x60 234 against 211); 4 and 5 are within 1.5 % of each other from
+// 20,000 columns (192x192x64 385 and 386), below it 4 wins (96x96x48 87
+// against 93).
 int default_matvec(const Dims& d, size_t es) {
   if (es == 8) return d.nx * d.ny < 20000 ? 4 : 5;
   const int blocks = ((d.nx + 1 + 31) / 32) * ((d.ny + 1 + 3) / 4), wave = 4 * 148;
@@ -399,11 +399,12 @@ int default_matvec(const Dims& d, size_t es) {
 // Preconditioner.  The 32-column tile with batched loads (4) works on a
 // column with eight threads outside the tridiagonal sweep, the pipelined
 // march (6) with one: the tile wins while the columns alone do not fill the
-// chip (64x64x48 float32 46 against 70, 192x192x64 227 against 237, float64
-// 150x131x60 216 against 224) and loses after (256x256x80 487 against 473.5,
-// float64 192x192x64 385 against 380).  Of the transposed ones the batched
-// tile is never slower (256x256x80 float32 613 against 643, float64 948
-// against 1118).
+// chip (64x64x48 float32 42 against 68, 128x128x64 116 against 143, float64
+// 150x131x60 211 against 233), past the lines the two are within a few per
+// cent (256x256x80 463 against 452, 384x384x96 1201 against 1225, float64
+// 192x192x64 377 against 387).  Of the transposed ones the batched tile is
+// never slower (256x256x80 float32 640 against 681, float64 192x192x64 449
+// against 478).
 void default_shapes(Dims& d, size_t es) {
   d.tune_mv = default_matvec(d, es);
   const bool fits = d.nz >= 2 && (size_t)(5 * d.nz + 1) * 32 * es <= 200 * 1024;
@@ -719,8 +720,7 @@ void solve_prep(SislCore* c, const Coef<T>& cf, GWork<T>& g, CVec5<T> rhs, const
   {
     KScope k(c, SISL_K_OTHER, st);
     launch_chained(zero_gaps_kernel<T>, g.R + 4, 256, 0, st, g.vec, g.npad, g.R + 4, g.off[0], g.off[1], g.off[2],
-                   g.off[3],
-                                                g.off[4], g.sz[0], g.sz[1], g.sz[2], g.sz[3], g.sz[4]);
+                   g.off[3], g.off[4], g.sz[0], g.sz[1], g.sz[2], g.sz[3], g.sz[4]);
   }
   const T ps = (T)c->s.ps;
   scale5<T>(c, cf, rhs, g.view(g.bg()), ps, 0, st);       // rhs_scaled: pi * pi_scale
@@ -750,8 +750,7 @@ int solve_t_prep(SislCore* c, const Coef<T>& cf, GWork<T>& g, CVec5<T> xbar, con
   {
     KScope k(c, SISL_K_OTHER, st);
     launch_chained(zero_gaps_kernel<T>, g.R + 4, 256, 0, st, g.vec, g.npad, g.R + 4, g.off[0], g.off[1], g.off[2],
-                   g.off[3],
-                                                g.off[4], g.sz[0], g.sz[1], g.sz[2], g.sz[3], g.sz[4]);
+                   g.off[3], g.off[4], g.sz[0], g.sz[1], g.sz[2], g.sz[3], g.sz[4]);
   }
   scale5<T>(c, cf, xbar, g.view(g.bg()), (T)(1.0 / c->s.ps), 2, st);  // pi / ps, eta / dz_w
   // initial guess: zero as in bwd_solve, or a caller's guess in the units of

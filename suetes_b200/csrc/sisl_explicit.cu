@@ -433,8 +433,7 @@ void launch_corrector_theta(const Dims& d, const Coef<T>& c, const T* th_adv, co
                             const T* w_next, T* th_next, cudaStream_t st) {
   dim3 blk(32, 4, 2);
   launch_chained(corrector_theta_kernel<T>, box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st, d, c, th_adv, tth, w_now,
-                 w_next,
-                                                                            th_next);
+                 w_next, th_next);
 }
 
 template <typename T>

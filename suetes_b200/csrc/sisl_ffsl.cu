@@ -255,8 +255,7 @@ bool launch_ffsl_tile(const Dims& d, const Coef<T>& c, const T* in, const T* vel
   ensure_smem_limit((const void*)ffsl_tile_kernel<T, AXIS>, attr_bytes, smem);
   const double scale = AXIS == 0 ? dt / d.dx : AXIS == 1 ? dt / d.dy : dt;  // of the interface Courant number
   launch_chained(ffsl_tile_kernel<T, AXIS>, (nlines + FL - 1) / FL, FL * FW, smem, st, d, c, in, vel, out, periodic,
-                 scale,
-                                                                         from_density, to_density);
+                 scale, from_density, to_density);
   return true;
 }
 template <typename T>
@@ -510,14 +509,11 @@ int launch_ffsl_vjp(const Dims& d, const Coef<T>& c, const T* field, const T* u,
   launch_ffsl_sweep<T>(d, c, 1, mx, v, my, M, d.py, dt, 0, st);
   // reverse z, y, x
   launch_chained(ffsl_sweep_vjp_kernel<T>, (d.nx * d.ny + tb - 1) / tb, tb, 0, st, d, c, 2, my, eta, out_bar, b1,
-                 eta_bar, M,
-                                                                     Mb, 0, dt, 1, 0);
+                 eta_bar, M, Mb, 0, dt, 1, 0);
   launch_chained(ffsl_sweep_vjp_kernel<T>, (d.nx * d.nz + tb - 1) / tb, tb, 0, st, d, c, 1, mx, v, b1, b2, v_bar, M,
-                 Mb, d.py,
-                                                                     dt, 0, 0);
+                 Mb, d.py, dt, 0, 0);
   launch_chained(ffsl_sweep_vjp_kernel<T>, (d.ny * d.nz + tb - 1) / tb, tb, 0, st, d, c, 0, mass, u, b2, field_bar,
-                 u_bar, M,
-                                                                     Mb, d.px, dt, 0, 1);
+                 u_bar, M, Mb, d.px, dt, 0, 1);
   return 6;  // kernels launched
 }
 
@@ -525,8 +521,7 @@ template <typename T>
 void launch_ffsl_lines_vjp(int N, int nlines, const T* scalar, const T* cfl, const T* out_bar, T* scalar_bar,
                            T* cfl_bar, double* M, double* Mb, int periodic, cudaStream_t st) {
   launch_chained(ffsl_line_vjp_kernel<T>, (nlines + 127) / 128, 128, 0, st, N, nlines, scalar, cfl, out_bar,
-                 scalar_bar, cfl_bar,
-                                                                M, Mb, periodic);
+                 scalar_bar, cfl_bar, M, Mb, periodic);
 }
 
 template <typename T>

@@ -1086,10 +1086,10 @@ __device__ void small_solve_state(GState* gs) {
     return;
   }
   if (gs->method == 0) {
-    // _lstsq(H.T, beta): normal equations (H H^T) y = H beta, Cholesky solve, over the cycle's kd steps.  A row past them
-    // is an identity row (begin_cycle): as an unknown it would meet the last step's subdiagonal equation for nothing
-    // and leave the square Hessenberg system in the least-squares problem's place.  Row p of H ends at column p + 1,
-    // and the lower triangle is enough.
+    // _lstsq(H.T, beta): normal equations (H H^T) y = H beta, Cholesky solve, over the cycle's kd steps.  A row past
+    // them is an identity row (begin_cycle): as an unknown it would meet the last step's subdiagonal equation for
+    // nothing and leave the square Hessenberg system in the least-squares problem's place.  Row p of H ends at column
+    // p + 1, and the lower triangle is enough.
     const int P = R | 1;
     double* ht = a2 + (size_t)R * R;  // [SS_C][P]: columns c0 .. of H, transposed
     for (int q = tid; q < kd * R; q += blockDim.x) a2[q] = 0.0;
@@ -1504,8 +1504,9 @@ void gm_small_solve(GState* gs, int restart, cudaStream_t st) {
   ensure_smem_limit((const void*)small_solve_kernel, attr_bytes, small_solve_smem(GM_MAXR));
   launch_chained(small_solve_kernel, 1, small_solve_threads(restart), smem, st, gs);
 }
-void gm_snapshot(const GState* gs, GHostView* v, cudaStream_t st) { launch_chained(snapshot_kernel, 1, 1, 0, st, gs,
-    v); }
+void gm_snapshot(const GState* gs, GHostView* v, cudaStream_t st) {
+  launch_chained(snapshot_kernel, 1, 1, 0, st, gs, v);
+}
 
 // ---------------------------------------------------------------------------
 // grouped host wrappers

@@ -424,8 +424,8 @@ template <typename T>
 void launch_departure(const Dims& d, int loc, double dt, const T* const* vel3, int iterations, T* const* coords3,
                       int relative, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  launch_chained(departure_kernel<T>, box_grid(ext_x(d, loc), ext_y(d, loc), ext_z(d, loc), blk), blk, 0, st,
-      d, loc, (T)dt, vel3[0], vel3[1], vel3[2], iterations, coords3[0], coords3[1], coords3[2], relative);
+  launch_chained(departure_kernel<T>, box_grid(ext_x(d, loc), ext_y(d, loc), ext_z(d, loc), blk), blk, 0, st, d, loc,
+                 (T)dt, vel3[0], vel3[1], vel3[2], iterations, coords3[0], coords3[1], coords3[2], relative);
 }
 
 template <typename T>
@@ -433,8 +433,7 @@ void launch_tricubic_ext(int sx, int sy, int sz, int dx, int dy, int dz, const T
                          T* out, int use_limiter, T scale, cudaStream_t st) {
   dim3 blk(32, 4, 2);
   launch_chained(tricubic_kernel<T>, box_grid(dx, dy, dz, blk), blk, 0, st, Ext{sx, sy, sz}, Ext{dx, dy, dz}, field,
-                                                               coords3[0], coords3[1], coords3[2], out,
-                                                               use_limiter, scale);
+                 coords3[0], coords3[1], coords3[2], out, use_limiter, scale);
 }
 
 template <typename T>
@@ -442,16 +441,16 @@ void launch_trilinear_ext(int sx, int sy, int sz, int dx, int dy, int dz, const 
                           T* out, cudaStream_t st) {
   dim3 blk(32, 4, 2);
   launch_chained(trilinear_kernel<T>, box_grid(dx, dy, dz, blk), blk, 0, st, Ext{sx, sy, sz}, Ext{dx, dy, dz}, field,
-                                                                coords3[0], coords3[1], coords3[2], out);
+                 coords3[0], coords3[1], coords3[2], out);
 }
 
 template <typename T>
 void launch_sl_advect(const Dims& d, int loc, double dt, const T* const* vel3, int iterations, int nf,
                       const T* const* fields, T* const* outs, const T* scales, int use_limiter, cudaStream_t st) {
   dim3 blk(32, 4, 2);
-  launch_chained(sl_advect_kernel<T>, box_grid(ext_x(d, loc), ext_y(d, loc), ext_z(d, loc), blk), blk, 0, st,
-      d, loc, (T)dt, vel3[0], vel3[1], vel3[2], iterations, nf, fields[0], nf > 1 ? fields[1] : nullptr,
-      outs[0], nf > 1 ? outs[1] : nullptr, scales[0], nf > 1 ? scales[1] : T(0), use_limiter);
+  launch_chained(sl_advect_kernel<T>, box_grid(ext_x(d, loc), ext_y(d, loc), ext_z(d, loc), blk), blk, 0, st, d, loc,
+                 (T)dt, vel3[0], vel3[1], vel3[2], iterations, nf, fields[0], nf > 1 ? fields[1] : nullptr, outs[0],
+                 nf > 1 ? outs[1] : nullptr, scales[0], nf > 1 ? scales[1] : T(0), use_limiter);
 }
 
 #define SISL_INST_SL(T)                                                                                     \

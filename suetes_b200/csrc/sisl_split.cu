@@ -716,8 +716,7 @@ void launch_split_adv(const Dims& d, const Coef<T>& c, const T* u, const T* v, c
   const int tiles = ((d.nx + AX - 1) / AX) * ((d.ny + AY - 1) / AY);
   const int chunk = tiles * ((d.nz + 15) / 16) >= 2 * 148 ? 16 : 8;
   launch_chained(split_adv_kernel<T>, dim3((d.nx + AX - 1) / AX, (d.ny + AY - 1) / AY, (d.nz + chunk - 1) / chunk),
-                 blk, 0, st,
-      d, c, u, v, w, eta, th, eps_l, o, chunk);
+                 blk, 0, st, d, c, u, v, w, eta, th, eps_l, o, chunk);
 }
 
 template <typename T>

@@ -116,8 +116,7 @@ void launch_stagger(const int in_shape[3], int axis, int to_face, int periodic, 
                    src, dst);
   else
     launch_chained(stagger_t_kernel<T>, sgrid(in, blk), blk, 0, st, in, out, axis, to_face, periodic, stop_grad, c0,
-                   c1, mult,
-                                                        src, dst);
+                   c1, mult, src, dst);
 }
 
 template void launch_stagger<float>(const int*, int, int, int, int, int, float, float, const float*, const float*,

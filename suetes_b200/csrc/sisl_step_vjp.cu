@@ -1679,8 +1679,7 @@ void launch_corrector_theta_vjp(const Dims& d, const Coef<T>& c, const T* thn_ba
                                 T* w_now_bar, T* w_next_bar, cudaStream_t st) {
   dim3 blk(32, 4, 2);
   launch_chained(corrector_theta_vjp_kernel<T>, box_grid(d.nx, d.ny, d.nz + 1, blk), blk, 0, st, d, c, thn_bar,
-                 tha_bar,
-                                                                                   tth_bar, w_now_bar, w_next_bar);
+                 tha_bar, tth_bar, w_now_bar, w_next_bar);
 }
 
 template <typename T>
@@ -1714,8 +1713,7 @@ void launch_hyper_vjp(const Dims& d, const Coef<T>& c, PtrTable<T> hyp_bar, PtrT
   launch_chained(lap_t_faces_kernel<T>, gf, blk, 0, st, d, c, tmp4, gx4, gy4, T(1));
   launch_chained(lap_t_mass_kernel<T>, gm, blk, 0, st, d, c, gx4, gy4, hyp_bar);
   launch_chained(hyper_src_t_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, hyp_bar, u_bar,
-                 v_bar,
-                                                                                     w_bar, th_bar);
+                 v_bar, w_bar, th_bar);
 }
 
 // ---------------------------------------------------------------------------
@@ -1766,8 +1764,7 @@ void launch_split_end_vjp(const Dims& d, const T* const* out6, T* const* c6, T* 
     cb.p[q] = c6[q];
   }
   launch_chained(split_end_vjp_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, o, cb, th0b,
-                 upp, vpp,
-                                                                                     wpp, ppp, sfth, dtns);
+                 upp, vpp, wpp, ppp, sfth, dtns);
 }
 
 template <typename T>
@@ -1780,8 +1777,7 @@ void launch_split_init_vjp(const Dims& d, const T* upp, const T* vpp, const T* w
     cb.p[q] = c6[q];
   }
   launch_chained(split_init_vjp_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, upp, vpp, wpp,
-                 ppp, s,
-                                                                                      cb);
+                 ppp, s, cb);
 }
 
 template <typename T>
@@ -1808,9 +1804,8 @@ void launch_split_adv_vjp(const Dims& d, const Coef<T>& c, const T* u, const T* 
   PtrTable<T> qb{};
   for (int q = 0; q < 4; ++q) qb.p[q] = tmp4[q];
   launch_chained(split_adv_vjp_mass_kernel<T>, box_grid(d.nx, d.ny, d.nz, blk), blk, 0, st, d, c, in, qb, thb);
-  launch_chained(split_adv_vjp_faces_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, c, in,
-                 qb, ub, vb, wb,
-                                                                                           eb);
+  launch_chained(split_adv_vjp_faces_kernel<T>, box_grid(d.nx + 1, d.ny + 1, d.nz + 1, blk), blk, 0, st, d, c, in, qb,
+                 ub, vb, wb, eb);
 }
 
 #define SISL_INST_SPLIT_VJP(T)                                                                                 \
