@@ -1179,8 +1179,8 @@ void launch_precond_t(const Dims& d, const Coef<T>& c, CVec5<T> y, Vec5<T> out, 
     case 2: launch_pt_column<T, 256, 64>(d, c, y, out, active, st, sh); break;
     case 3: launch_pt_march<T, 128>(d, c, y, out, active, st, sh); break;
     case 4:
-      // at most one tile an SM: more threads a tile, as the forward preconditioner (61x47x40 float64 4.9 -> 4.2 us;
-      // 128x128x64 float32 15.1 against 22.0)
+      // at most one tile an SM: more threads a tile, as the forward preconditioner (without a shift, 61x47x40
+      // float64 4.9 -> 4.2 us; 128x128x64 float32 15.1 against 22.0)
       if ((d.nx + 31) / 32 * d.ny <= 148) launch_pt_column_batched<T, 512, 32, 3>(d, c, y, out, active, st, sh);
       else launch_pt_column_batched<T, 256, 32, 4>(d, c, y, out, active, st, sh);
       break;

@@ -1326,9 +1326,9 @@ void launch_precond(const Dims& d, const Coef<T>& c, CVec5<T> r, Vec5<T> out, co
     case 2: launch_precond_tile<T, 256, 64>(d, c, r, out, active, st, sh); break;
     case 3: launch_precond_march<T, 128>(d, c, r, out, active, st, sh); break;
     case 4:
-      // At most one tile an SM: a thread per level or two, so that every phase is one round of loads (float32
-      // 48x41x33 7.2 -> 6.0 us, float64 64x64x48 12.1 -> 9.6, 61x47x40 11.4 -> 9.0); with more tiles than SMs
-      // several smaller blocks hide more (128x128x64 float32 19.4 against 39.8).
+      // At most one tile an SM: a thread per level or two, so that every phase is one round of loads (without a
+      // shift, float32 48x41x33 7.2 -> 6.0 us, float64 64x64x48 12.1 -> 9.6, 61x47x40 11.4 -> 9.0); with more
+      // tiles than SMs several smaller blocks hide more (128x128x64 float32 19.4 against 39.8).
       if ((d.nx + 31) / 32 * d.ny <= 148) launch_precond_tile_batched<T, 1024, 32, 2>(d, c, r, out, active, st, sh);
       else launch_precond_tile_batched<T, 256, 32, 4>(d, c, r, out, active, st, sh);
       break;
