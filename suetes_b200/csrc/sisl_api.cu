@@ -3003,15 +3003,25 @@ int sisl_autotune_query(const SislCore* c, SislTuning* out) {
 
 namespace {
 // Time every candidate launch shape of the four tunable Helmholtz kernels on
-// this core's grid (CUDA events, warm launches) and keep the fastest.
+// this core's grid (CUDA events, warm launches) and keep the fastest: the
+// shifted forms that a block of the Krylov cycle launches.  Vectors: V_0 in, z,
+// V_1 out; a restart of 1 has no more.
 template <typename T>
 int autotune_impl(SislCore* c, void* ws, cudaStream_t st, SislTuning* out) {
   Carver cv{(char*)ws};
   GWork<T> g = carve_gmres<T>(cv, c->d, c->prm.solver_restart, false);
   const Coef<T> cf = coef_of<T>(c);
-  for (int q = 0; q < 3; ++q)
-    if (cuda_failed(cudaMemsetAsync(g.V(q), 0, sizeof(T) * g.npad, st), "cudaMemsetAsync")) return SISL_ERR_CUDA;
-  if (cuda_failed(cudaMemsetAsync(g.z(), 0, sizeof(T) * g.npad, st), "cudaMemsetAsync")) return SISL_ERR_CUDA;
+  for (T* v : {g.V(0), g.V(1), g.z()})
+    if (cuda_failed(cudaMemsetAsync(v, 0, sizeof(T) * g.npad, st), "cudaMemsetAsync")) return SISL_ERR_CUDA;
+  if (cuda_failed(cudaMemsetAsync(g.scal, 0, sizeof(double), st), "cudaMemsetAsync")) return SISL_ERR_CUDA;
+  const CVec5<T> x = g.cview(g.V(0));
+  const Vec5<T> out_t = g.view(g.V(1));
+  Vec5<T> out_m = out_t;
+  out_m.f[0] = out_m.f[1] = nullptr;  // the matvec writes the shifted u and v rows
+  Shift<T> sh;
+  for (int q = 0; q < 5; ++q) sh.f[q] = x.f[q];
+  sh.s = g.scal;
+  sh.keep = g.tmp;
   cudaEvent_t e0, e1;
   if (cuda_failed(cudaEventCreate(&e0), "cudaEventCreate") || cuda_failed(cudaEventCreate(&e1), "cudaEventCreate"))
     return SISL_ERR_CUDA;
@@ -3045,16 +3055,14 @@ int autotune_impl(SislCore* c, void* ws, cudaStream_t st, SislTuning* out) {
     *us_out = tbest;
   };
   pick(&d.tune_mv, N_MATVEC_SHAPES,
-       [&] { launch_matvec<T>(d, cf, g.cview(g.V(0)), nullptr, none, g.split(g.V(1), g.z()), nullptr, st); },
+       [&] { launch_matvec<T>(d, cf, x, sh.s, none, g.view(g.z()), nullptr, st, out_t.f[0], out_t.f[1]); },
        &out->us[0]);
-  pick(&d.tune_pc, N_PRECOND_SHAPES,
-       [&] { launch_precond<T>(d, cf, as_const(g.split(g.V(1), g.z())), g.view(g.V(2)), nullptr, st); },
+  pick(&d.tune_pc, N_PRECOND_SHAPES, [&] { launch_precond<T>(d, cf, g.cview(g.z()), out_m, nullptr, st, sh); },
        &out->us[1]);
   pick(&d.tune_mvt, N_STENCIL_BLOCKS,
-       [&] { launch_matvec_t<T>(d, cf, g.cview(g.V(0)), nullptr, none, g.view(g.z()), g.tmp, nullptr, st); },
-       &out->us[2]);
-  pick(&d.tune_pct, N_PRECOND_T_SHAPES,
-       [&] { launch_precond_t<T>(d, cf, g.cview(g.z()), g.view(g.V(2)), nullptr, st); }, &out->us[3]);
+       [&] { launch_matvec_t<T>(d, cf, x, sh.s, none, g.view(g.z()), g.tmp, nullptr, st); }, &out->us[2]);
+  pick(&d.tune_pct, N_PRECOND_T_SHAPES, [&] { launch_precond_t<T>(d, cf, g.cview(g.z()), out_t, nullptr, st, sh); },
+       &out->us[3]);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   out->matvec_block = d.tune_mv;
