@@ -114,7 +114,7 @@ typedef struct SislCore SislCore;
 
 typedef struct SislSolveInfo {
   int32_t cycles;          /* restart cycles run */
-  int32_t arnoldi_steps;   /* matvec + preconditioner applications inside cycles */
+  int32_t arnoldi_steps;   /* Arnoldi steps of these cycles */
   int32_t converged;       /* 1 when ||M(b - A x)|| <= atol */
   int32_t pad;
   double residual_norm;    /* final preconditioned residual norm */
@@ -414,9 +414,10 @@ int sisl_step_vjp(SislCore* core, const SislState* in, void* const solves[10], c
  * into outs[m] on core m with workspace ws[m]), captured once for these
  * buffers and replayed by sisl_step_graph_launch with no host
  * synchronisation.  Members are parallel branches of the graph; each GMRES
- * restart loop is a conditional WHILE node whose condition a kernel sets on
- * the device (rnorm > atol and cycles < maxiter), so a replay runs exactly
- * the cycles the host loop of sisl_step would.  The replay of lax.scan's
+ * restart loop is a pair of conditional WHILE nodes (cycles in blocks, then
+ * cycles of single Arnoldi steps where a block lost columns) whose conditions a
+ * kernel sets on the device (rnorm > atol and cycles < maxiter), so a replay
+ * runs exactly the cycles the host loop of sisl_step would.  The replay of lax.scan's
  * jitted step (steppers.py:692-714) in one launch; the ensemble launch of
  * the many-member configuration.  Cores must be distinct and have no timing
  * class selected; relax may be NULL (or hold NULL entries). */
@@ -465,8 +466,8 @@ int sisl_step_graph_create_taped(int n, SislCore* const* cores, const SislState*
  * branches, but each of the step's two solves runs as ONE restarted GMRES
  * over all members, every Krylov phase (matvec, preconditioner,
  * projections, update, small solves) a single launch that walks a
- * member/block table, and one device-decided WHILE node per solve that
- * loops while any member continues (convergence per member).  A member's
+ * member/block table, and the solve's two device-decided WHILE nodes loop
+ * while any member continues in their form (convergence per member).  A member's
  * share of each grouped launch is its own launch's partition, so every
  * member's step is the same bits as with sisl_step_graph_create.  Members
  * share the dtype, GMRES restart and method and the refinement switch, and
